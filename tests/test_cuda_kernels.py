@@ -1,6 +1,7 @@
 """Numerics of the sm_100a kernels against plain PyTorch fp32 references of the same op."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -561,6 +562,49 @@ def test_sdpa_dense(ops, dtype, D, S):
     qf, kf, vf = [t.float().reshape(B, S, H, D).transpose(1, 2) for t in (q, k, v)]
     ref = torch.nn.functional.scaled_dot_product_attention(qf, kf, vf).transpose(1, 2).reshape(B * S, H * D)
     assert _rel_err(out, ref) < 1e-2
+
+
+def _expected_draw(row: np.ndarray, temp: float, top_k: int, top_p: float, seed: int, step: int, index: int):
+    """The kept set in 64 bits and, for the random number of (seed, step, row), the tokens around the target: a target within 1e-5
+    of the total mass of a boundary between two tokens (fp32 sums of up to 128k terms) may fall on either side."""
+    def mix(z):
+        z = (z + 0x9E3779B97F4A7C15) & M
+        z = ((z ^ (z >> 30)) * 0xBF58476D1CE4E5B9) & M
+        z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & M
+        return z ^ (z >> 31)
+    M = (1 << 64) - 1
+    u = ((mix(seed ^ mix((step << 20) ^ index)) >> 40) + 0.5) / 16777216.0
+    p = np.exp((row.astype(np.float64) - row.max()) / temp)
+    order = np.argsort(-row, kind="stable")
+    thr = []
+    if 0 < top_k < len(row):
+        thr.append(row[order[top_k - 1]])
+    if top_p < 1.0:
+        thr.append(row[order[np.searchsorted(np.cumsum(p[order]), top_p * p.sum())]])
+    kept = np.nonzero(row >= max(thr))[0] if thr else np.arange(len(row))
+    cum = np.cumsum(p[kept]) / p[kept].sum()
+    at = [min(np.searchsorted(cum, u + d), len(kept) - 1) for d in (-1e-5, 1e-5)]
+    return {int(t) for t in kept[at[0]:at[1] + 1]}
+
+
+@pytest.mark.parametrize("V,ld,dtype", [(128256, 128256, torch.bfloat16), (32007, 32011, torch.bfloat16), (1, 8, torch.bfloat16), (9, 9, torch.float32),
+                                        (8191, 8192, torch.float32), (70001, 70001, torch.bfloat16)])
+@pytest.mark.parametrize("top_k,top_p", [(50, 0.95), (0, 1.0), (0, 0.6), (9000, 1.0), (1, 1.0)])
+def test_sampling_kernel_draws(ops, V, ld, dtype, top_k, top_p):
+    """Rows of aligned, odd and tiny lengths; kept sets that fit the per-warp lists and sets that do not (top_k 9000; equal logits)."""
+    g = torch.Generator(device="cuda").manual_seed(V + top_k)
+    rows = (torch.randn(5, ld, device="cuda", generator=g) * 2).to(dtype)
+    rows[3, :V] = 0.25                                       # all equal
+    rows[4, :V] = torch.arange(V, device="cuda").flip(0).to(dtype) * -1e-4   # large entries side by side: one warp's piece holds them all
+    rows[4, V // 2] = 3.0
+    step = torch.tensor([17], dtype=torch.int32, device="cuda")
+    got = ops.sample(rows[:, :V], 0.8, top_k=top_k, top_p=top_p, seed=21, step=step).cpu()
+    again = ops.sample(rows[:, :V], 0.8, top_k=top_k, top_p=top_p, seed=21, step=step).cpu()
+    ops.check_status("sample")
+    assert torch.equal(got, again)
+    for i in range(5):
+        want = _expected_draw(rows[i, :V].float().cpu().numpy(), 0.8, top_k, top_p, 21, 17, i)
+        assert int(got[i]) in want, (i, int(got[i]), want)
 
 
 def test_sampling_kernel(ops):
