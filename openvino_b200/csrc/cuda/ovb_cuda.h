@@ -95,12 +95,16 @@ typedef struct {
     int group_ldx, group_ldo;
     int x_cols;             // columns of x that may be read (0: the row pitch)
     float act_limit, act_slope, act_shift;
+    void* scratch;          // memory for expanded weights (ovb_gemm_scratch_bytes), not shared with calls that may overlap; may be NULL
+    int64_t scratch_bytes;
 } ovb_gemm_args;
 
 int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream);
 // Bytes of split-K workspace / number of counters that ovb_gemm may need for the given problem.
 int64_t ovb_gemm_ws_bytes(int T, int N, int K, int act);
 int ovb_gemm_num_counters(void);
+// Bytes of scratch memory with which ovb_gemm runs this problem (quantised weights, many tokens) faster; 0: none.
+int64_t ovb_gemm_scratch_bytes(const ovb_gemm_args* a);
 /* Conditional compilation: bit (log2(token tile) - 4) of the result is set when the GEMM variant (tile, wmode, fp16) has been
    launched in this process; ovb_cc_is_selective tells whether the library is a selective build. */
 unsigned ovb_cc_used_gemm(int wmode, int is_f16);

@@ -41,6 +41,7 @@ class GemmArgs(C.Structure):
         ("group_offsets", C.c_void_p), ("num_groups", C.c_int), ("group_mode", C.c_int),
         ("group_ldx", C.c_int), ("group_ldo", C.c_int), ("x_cols", C.c_int),
         ("act_limit", C.c_float), ("act_slope", C.c_float), ("act_shift", C.c_float),
+        ("scratch", C.c_void_p), ("scratch_bytes", C.c_int64),
     ]
 
 
@@ -129,6 +130,8 @@ def lib():
         l.ovb_last_error.restype = C.c_char_p
         l.ovb_status_ptr.restype = C.c_void_p
         l.ovb_gemm_ws_bytes.restype = C.c_int64
+        l.ovb_gemm_scratch_bytes.restype = C.c_int64
+        l.ovb_gemm_scratch_bytes.argtypes = [C.POINTER(GemmArgs)]
         l.ovb_pa_scratch_bytes.restype = C.c_int64
         l.ovb_channel_delta_record_floats.restype = C.c_int64
         l.ovb_gemm.argtypes = [C.POINTER(GemmArgs), C.c_void_p]
@@ -334,6 +337,11 @@ def gemm(x: torch.Tensor, w: PackedWeight, out: Optional[torch.Tensor] = None, r
         a.act_limit, a.act_slope, a.act_shift = glu
     elif act == ACT_SOFTCAP:
         a.act_limit = cap
+    if w.mode in (W_U4, W_U8, W_F8) and T >= 1024:      # expanded weights; the caching allocator keeps the memory, per stream
+        a.scratch_bytes = lib().ovb_gemm_scratch_bytes(C.byref(a))
+        if a.scratch_bytes:
+            scratch = torch.empty(a.scratch_bytes, dtype=torch.uint8, device=x.device)
+            a.scratch = scratch.data_ptr()
     _check(lib().ovb_gemm(C.byref(a), C.c_void_p(_stream())), "ovb_gemm")
     return out
 

@@ -660,3 +660,71 @@ def test_bounded_wait_reports_a_timeout_and_the_context_survives(ops):
     x = torch.randn(4, 256, device="cuda", dtype=torch.bfloat16)
     y = ops.rmsnorm(x, torch.ones(256, device="cuda", dtype=torch.bfloat16), 1e-5)
     assert torch.isfinite(y.float()).all()
+
+
+# Two correct kernels round the same fp32 sums (taken in another order) to bf16: each is off by 2^-9 / sqrt(3) of a value on average,
+# 1.6e-3 between the two in the 2-norm.
+PAIR_REL = 4e-3
+
+
+def _pair_weight(ops, fmt, N, K, dtype=torch.bfloat16):
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    if fmt == "dense":
+        return ops.PackedWeight.from_dense((torch.randn(N, K, device="cuda", generator=g) * 0.05).to(dtype))
+    if fmt == "u4":
+        q = torch.randint(0, 256, (N * K // 2,), dtype=torch.uint8, device="cuda", generator=g)
+        z = torch.randint(0, 256, (N * (K // 64) // 2,), dtype=torch.uint8, device="cuda", generator=g)
+        return ops.PackedWeight.from_ir_u4(q, (torch.rand(N, K // 64, device="cuda", generator=g) * 0.01 + 0.005).half(), z, N, K, 64)
+    if fmt == "u8":
+        q = torch.randint(0, 256, (N, K), dtype=torch.uint8, device="cuda", generator=g)
+        z = torch.randint(100, 156, (N, K // 128), dtype=torch.uint8, device="cuda", generator=g)
+        return ops.PackedWeight.from_ir_u8(q, (torch.rand(N, K // 128, device="cuda", generator=g) * 0.001 + 0.0005).half(), z, N, K, 128)
+    q = torch.randn(N, K, device="cuda", generator=g).to(torch.float8_e4m3fn)
+    return ops.PackedWeight.from_f8_block(q, torch.rand((N + 127) // 128, K // 128, device="cuda", generator=g) * 0.05 + 0.02, N, K)
+
+
+@pytest.mark.parametrize("fmt,T,N,K", [("dense", 129, 3328, 64), ("dense", 999, 6144, 448), ("dense", 257, 4224, 1024), ("dense", 2049, 384, 128), ("dense", 8191, 256, 512),
+                                       ("u4", 1024, 1280, 256), ("u4", 1031, 640, 4096), ("u8", 1025, 896, 256), ("f8", 1100, 768, 384), ("u4", 1024, 36864, 2048)])
+def test_gemm_pair(ops, fmt, T, N, K):
+    """Edges of the token tile, an odd number of 128-row tiles, one k-block, weights expanded in one piece and in several: against the
+    single-CTA kernel (an explicit token tile selects it), in every epilogue."""
+    torch.manual_seed(1)
+    x = torch.randn(T, K + 64, device="cuda", dtype=torch.bfloat16)[:, :K]
+    w = _pair_weight(ops, fmt, N, K)
+    out, ref = (torch.full((T, N + 2), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    ops.gemm(x, w, out=out[:, :N])
+    ops.gemm(x, w, out=ref[:, :N], block_t=256)
+    ops.check_status("gemm_pair")
+    assert _rel_err(out, ref) < PAIR_REL and (out[:, N:] == 7.0).all()
+    w.bias = torch.randn(N, device="cuda").to(torch.bfloat16)
+    res = torch.randn(T, N, device="cuda").to(torch.bfloat16)
+    for kw in (dict(residual=res), dict(residual=res, act=ops.ACT_GELU_ERF), dict(act=ops.ACT_RELU2), dict(out_f32=True), dict(out_f32=True, act=ops.ACT_SILU)):
+        a, b = ops.gemm(x, w, **kw), ops.gemm(x, w, block_t=256, **kw)
+        assert _rel_err(a, b) < (1e-5 if kw.get("out_f32") else PAIR_REL), kw
+    w.bias = None
+    for kw in (dict(act=ops.ACT_SWIGLU), dict(act=ops.ACT_GLU_LIMITED, glu=(7.0, 1.702, 1.0))):
+        assert _rel_err(ops.gemm(x, w, **kw), ops.gemm(x, w, block_t=256, **kw)) < PAIR_REL, kw
+    h = res.clone()
+    ops.gemm(x, w, out=h, residual=h)                       # in place, as the residual stream
+    assert _rel_err(h, ops.gemm(x, w, residual=res, block_t=256)) < PAIR_REL
+    ops.check_status("gemm_pair")
+
+
+def test_gemm_pair_fp16_window_and_groups(ops):
+    torch.manual_seed(2)
+    x = torch.randn(700, 512, device="cuda", dtype=torch.float16)
+    w = _pair_weight(ops, "dense", 2560, 1024, torch.float16)
+    win = w.window(128, 2304, 256, 512)
+    assert _rel_err(ops.gemm(x, win), ops.gemm(x, win, block_t=256)) < PAIR_REL
+    for mode, N in ((1, 384), (2, 512)):
+        sizes = [0, 130, 1, 517, 0, 256]
+        off = torch.tensor(np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32), device="cuda")
+        cap, K = 1000, 256
+        w = _pair_weight(ops, "dense", N * (6 if mode == 1 else 1), K * (6 if mode == 2 else 1))
+        xg = torch.randn(cap, K, device="cuda", dtype=torch.bfloat16)
+        out, ref = (torch.full((cap, N), 3.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        ops.gemm_grouped(xg, w, off, 6, mode, out, block_t=256)
+        ops.gemm_grouped(xg, w, off, 6, mode, ref, block_t=64)
+        ops.check_status("gemm_pair")
+        assert _rel_err(out, ref) < PAIR_REL and (out[sum(sizes):] == 3.0).all()
+
