@@ -405,6 +405,309 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
 }
 
+// Two query tiles per CTA (256 stacked rows) for long prompts: paged bf16 cache, head size 128, G query heads per KV head.
+//
+// What bounds the kernel above: with one tile per SM the softmax of a tile (128 exponentials of a thread, one warp per scheduler)
+// and its two products follow one another, 3700 cycles per 128 x 128 tile where the tensor pipe needs 1024 and the exponentials
+// 1024. Here warps 0-3 and 4-7 hold a tile each and take turns: while one tile's scores are being exponentiated, the tensor pipe
+// works on the other's products, and both share the K and V tiles in shared memory (half the reads). Tensor memory is full with
+// S and O of the two tiles (4 x 128 columns), so P overwrites the first half of its S, and the next QK product of a tile is issued
+// after the PV product that reads P has retired. K and V stages are released on their own: K as soon as both QK products have
+// read it, so that the next tile but one is on its way a whole turn earlier.
+// 1 x 8191 tokens, 32 query and 8 KV heads, at the clock of a prefill step: 1084 us with one tile per CTA, 753 us here.
+constexpr int kDuoThreads = 320;
+
+template <int G>
+__global__ void __launch_bounds__(kDuoThreads, 1)
+pa_prefill_duo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, PaKParams p,
+                      int* status) {
+    constexpr int D = 128, TOK = tile_tokens(G);
+    constexpr int T_BYTES = kBM * D * 2;                        // a query, key or value tile
+    constexpr uint32_t TM_S = 0, TM_O = 256;                    // + 128 for the second tile
+    constexpr uint32_t IDESC_QK = umma_idesc_f16(kBM, kBK, true);
+    constexpr uint32_t IDESC_PV = umma_idesc_f16(kBM, D, true) | (1u << 16);
+
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* sQ = smem;                                         // two tiles
+    uint8_t* sK = sQ + 2 * T_BYTES;                             // two stages
+    uint8_t* sV = sK + 2 * T_BYTES;                             // two stages
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * T_BYTES);
+    uint64_t* q_full = bars;
+    uint64_t* k_full = bars + 1;               // [2 stages]
+    uint64_t* v_full = bars + 3;               // [2 stages]
+    uint64_t* k_empty = bars + 5;              // [2 stages] both QK products have read the stage
+    uint64_t* v_empty = bars + 7;              // [2 stages] both PV products have read the stage
+    uint64_t* s_full = bars + 9;               // [2 tiles] QK has retired (and with it the tile's PV product before it)
+    uint64_t* p_full = bars + 11;              // [2 tiles] P written, S read
+    uint64_t* pv_done = bars + 13;             // [2 tiles] PV has retired
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* s_work = const_cast<int*>(abort_flag) + 1;   // [2]
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = blockIdx.y;
+    pdl_enter_attn();
+    if (threadIdx.x == 0) {
+        const int bx = gridDim.x - 1 - blockIdx.x;
+        int acc = 0, found = -1, tile = 0;
+        for (int b = 0; b < p.B; ++b) {
+            const int nt = (p.subsequence_begins[b + 1] - p.subsequence_begins[b] + 2 * TOK - 1) / (2 * TOK);
+            if (bx < acc + nt) { found = b; tile = bx - acc; break; }
+            acc += nt;
+        }
+        s_work[0] = found;
+        s_work[1] = tile;
+        *abort_flag = 0;
+        mbar_init(q_full, 1);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&k_full[i], 1);
+            mbar_init(&v_full[i], 1);
+            mbar_init(&k_empty[i], 1);
+            mbar_init(&v_empty[i], 1);
+            mbar_init(&s_full[i], 1);
+            mbar_init(&p_full[i], kBM);
+            mbar_init(&pv_done[i], 1);
+        }
+        mbar_fence_init();
+    }
+    __syncthreads();
+    const int b = s_work[0];
+    if (b < 0) return;                          // (uniform) nothing allocated yet
+    if (warp == 9) {
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = *tmem_slot;
+
+    const int tok_begin = p.subsequence_begins[b];
+    const int q_len = p.subsequence_begins[b + 1] - tok_begin;
+    const int past = p.past_lens[b];
+    const int blk_begin = p.block_indices_begins[b];
+    const int tq0 = s_work[1] * 2 * TOK;
+    const int tq1 = min(q_len, tq0 + 2 * TOK);
+    const int kv_end = p.causal ? past + tq1 : past + q_len;
+    const int kv_start = first_visible_key(past + tq0, p.sliding_window, p.chunk) / kBK * kBK;
+    const int ntiles = (kv_end - kv_start + kBK - 1) / kBK;
+
+    if (warp == 8) {
+        // ------------------------------------------------------------------ TMA producer
+        if (lane == 0) {
+            mbar_arrive_expect_tx(q_full, 2 * G * TOK * D * 2);
+            for (int x = 0; x < 2; ++x)
+                for (int g = 0; g < G; ++g)
+                    for (int hf = 0; hf < 2; ++hf)
+                        tma_load_2d(sQ + x * T_BYTES + hf * (kBM * 128) + g * (TOK * 128), &tmQ, q_full, (h * G + g) * p.q_head + hf * 64, tok_begin + tq0 + x * TOK);
+        }
+        bool ok = true;
+        for (int j = 0; j < ntiles && ok; ++j) {
+            const int st = j & 1;
+            const int j0 = kv_start + j * kBK;
+            const int npages = (min(kv_end, j0 + kBK) - j0 + kPage - 1) / kPage;
+            for (int kv = 0; kv < 2 && ok; ++kv) {
+                uint64_t* full = kv ? &v_full[st] : &k_full[st];
+                if (j >= 2) ok = mbar_wait(kv ? &v_empty[st] : &k_empty[st], ((j >> 1) - 1) & 1, abort_flag, status);
+                if (!ok) break;
+                if (lane == 0) mbar_arrive_expect_tx(full, npages * kPage * D * 2);
+                __syncwarp();
+                if (lane < npages * 2) {                         // a lane per (half, page)
+                    const int part = lane / npages, pg = lane % npages;
+                    const int blk = OVB_DBG_BLOCK(p.block_indices[blk_begin + j0 / kPage + pg]);
+                    tma_load_2d((kv ? sV : sK) + st * T_BYTES + part * (kBK * 128) + pg * (kPage * 128), kv ? &tmV : &tmK, full, part * 64, (blk * p.Hkv + h) * kPage);
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 9) {
+        // ------------------------------------------------------------------ MMA issuer (warp-uniform flow, one elected lane issues)
+        bool ok = mbar_wait(q_full, 0, abort_flag, status);
+        const uint64_t dq0 = umma_desc_k_sw128(smem_u32(sQ), 1024);
+        auto qk = [&](int x, int st) {
+            const uint64_t dq = dq0 + (uint64_t)((x * T_BYTES) >> 4), dk = umma_desc_k_sw128(smem_u32(sK + st * T_BYTES), 1024);
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks) {
+                const uint64_t off = (uint64_t)(((ks >> 2) * (kBM * 128) + (ks & 3) * 32) >> 4);
+                umma_f16_ss_elect(tmem + TM_S + x * 128, dq + off, dk + off, IDESC_QK, ks > 0 ? 1u : 0u);
+            }
+            umma_commit_elect(&s_full[x]);
+        };
+        ok = ok && mbar_wait(&k_full[0], 0, abort_flag, status);
+        if (ok) {
+            tc_fence_after_sync();
+            qk(0, 0);
+            qk(1, 0);
+            umma_commit_elect(&k_empty[0]);
+        }
+        for (int j = 0; j < ntiles && ok; ++j) {
+            const int st = j & 1, nx = (j + 1) & 1;
+            const uint32_t par = j & 1;
+            const int ksteps = (min(kBK, kv_end - (kv_start + j * kBK)) + 15) / 16;
+            const uint64_t dv = umma_desc_mn_sw128(smem_u32(sV + st * T_BYTES), kBK * 128, 1024);
+            for (int x = 0; x < 2 && ok; ++x) {
+                if (x == 0) ok = mbar_wait(&v_full[st], (j >> 1) & 1, abort_flag, status);
+                ok = ok && mbar_wait(&p_full[x], par, abort_flag, status);
+                if (!ok) break;
+                tc_fence_after_sync();
+                for (int kk = 0; kk < ksteps; ++kk)
+                    umma_f16_ts_elect(tmem + TM_O + x * 128, tmem + TM_S + x * 128 + kk * 8, dv + (uint64_t)((kk * 16 * 128) >> 4), IDESC_PV, (j > 0 || kk > 0) ? 1u : 0u);
+                umma_commit_elect(&pv_done[x]);
+                if (x == 1) umma_commit_elect(&v_empty[st]);
+                if (j + 1 < ntiles) {
+                    if (x == 0) ok = mbar_wait(&k_full[nx], ((j + 1) >> 1) & 1, abort_flag, status);
+                    ok = ok && mbar_wait(&pv_done[x], par, abort_flag, status);     // P, which QK overwrites, has been read
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    qk(x, nx);
+                    if (x == 1) umma_commit_elect(&k_empty[nx]);
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------------ softmax: one thread per stacked query row
+        const int x = warp >> 2;                         // query tile of this thread
+        const int r = threadIdx.x & 127;                 // tensor-memory lane
+        const int g = r / TOK, tl = x * TOK + r % TOK;
+        const int qpos = past + tq0 + tl;
+        const bool row_valid = tq0 + tl < q_len;
+        const int lo_row = first_visible_key(qpos, p.sliding_window, p.chunk);
+        const int first_pos = past + tq0 + x * TOK, lo_last = first_visible_key(first_pos + TOK - 1, p.sliding_window, p.chunk);
+        const bool all_valid = tq0 + (x + 1) * TOK <= q_len;
+        const uint32_t lane_base = tmem + (uint32_t((warp & 3) * 32) << 16);
+        const uint32_t tm_s = lane_base + TM_S + x * 128, tm_o = lane_base + TM_O + x * 128;
+        float m_used = -CUDART_INF_F, l_sum = 0.f;
+        bool ok = true;
+        for (int j = 0; j < ntiles && ok; ++j) {
+            ok = mbar_wait(&s_full[x], j & 1, abort_flag, status);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const int j0 = kv_start + j * kBK;
+            // does any row of this query tile need a mask? (uniform over its four warps)
+            const bool need_mask = j0 + kBK > kv_end || (p.causal && j0 + kBK - 1 > first_pos) || j0 < lo_last || !all_valid;
+            int hi = kBK, lo = 0;                        // keys [lo, hi) of the tile are visible to this row
+            if (need_mask) {
+                hi = min(hi, kv_end - j0);
+                if (p.causal) hi = min(hi, qpos - j0 + 1);
+                lo = max(lo, lo_row - j0);
+                if (!row_valid) hi = 0;
+            }
+            uint32_t v[kBK];
+#pragma unroll
+            for (int c = 0; c < kBK; c += 16) tmem_ld_x16(tm_s + c, v + c);
+            tmem_ld_wait();
+            float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+            if (need_mask) {
+#pragma unroll
+                for (int i = 0; i < kBK; ++i) {
+                    const bool vis = i >= lo && i < hi;
+                    if (!vis) v[i] = __float_as_uint(-CUDART_INF_F);
+                    mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < kBK; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
+            }
+            const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
+            // raise the running maximum only when the tile exceeds it by a factor of 2^8; the rescale of O is warp-collective.
+            // (S of this tile is there, so the PV product of the tile before has retired and O may be touched.)
+            const bool raise = m_tile > m_used + 8.f;
+            if (__any_sync(0xffffffffu, raise)) {
+                const float factor = !raise ? 1.f : (m_used == -CUDART_INF_F ? 0.f : fast_exp2(m_used - m_tile));
+                if (j > 0) {
+#pragma unroll 1
+                    for (int c = 0; c < D; c += 16) {
+                        uint32_t o[16];
+                        tmem_ld_x16(tm_o + c, o);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+                        tmem_st_x16(tm_o + c, o);
+                    }
+                    tmem_st_wait();
+                }
+                if (raise) {
+                    l_sum *= factor;
+                    m_used = m_tile;
+                }
+            }
+            const float neg_m = (m_used == -CUDART_INF_F) ? 0.f : -m_used;
+            float ls[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int i = 0; i < kBK; i += 2) {
+                const float e0 = fast_exp2(fmaf(__uint_as_float(v[i]), p.scale_log2, neg_m));
+                const float e1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, neg_m));
+                ls[(i >> 1) & 3] += e0 + e1;
+                v[i >> 1] = pack16<false>(e0, e1);
+            }
+            l_sum += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+#pragma unroll
+            for (int c = 0; c < kBK / 2; c += 16) tmem_st_x16(tm_s + c, v + c);
+            tmem_st_wait();
+            tc_fence_before_sync();
+            mbar_arrive(&p_full[x]);
+        }
+        if (ok && ntiles > 0) ok = mbar_wait(&pv_done[x], (ntiles - 1) & 1, abort_flag, status);
+        if (ok) {
+            tc_fence_after_sync();
+            const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
+            uint8_t* dst = reinterpret_cast<uint8_t*>(p.out) + ((size_t)(tok_begin + tq0 + tl) * p.ldo + (size_t)(h * G + g) * p.o_head) * 2;
+#pragma unroll
+            for (int c = 0; c < D; c += 16) {
+                uint32_t o[16];
+                tmem_ld_x16(tm_o + c, o);
+                tmem_ld_wait();
+                if (row_valid) {
+                    uint32_t w[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) w[i] = pack16<false>(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
+                    *reinterpret_cast<uint4*>(dst + c * 2) = make_uint4(w[0], w[1], w[2], w[3]);
+                    *reinterpret_cast<uint4*>(dst + c * 2 + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+                }
+            }
+        }
+    }
+
+    // ---------------------------------------------------------------- tear-down
+    tc_fence_before_sync();
+    __syncthreads();
+    if (*abort_flag) {
+        for (int i = 0; i < 200; ++i) __nanosleep(1000);   // copies still in flight land before the shared memory is reused
+        __syncthreads();
+    }
+    if (warp == 9) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
+template <int G>
+int launch_duo(PaKParams p, int num_q_tiles, cudaStream_t stream) {
+    p.q_head = p.o_head = p.dv_store = p.k_row = p.v_row = 128;
+    p.ldo = p.Hq * 128;
+    const int smem = 6 * kBM * 256 + 256 + 1024;
+    auto kern = pa_prefill_duo_kernel<G>;
+    static std::atomic<uint64_t> configured{0};
+    int dev = 0;
+    OVB_CHECK_CUDA(cudaGetDevice(&dev));
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(configured.load(std::memory_order_acquire) & bit)) {
+        OVB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        configured.fetch_or(bit, std::memory_order_release);
+    }
+    const CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    const uint64_t rows = p.cache_rows > 0 ? (uint64_t)p.cache_rows : 1ull << 30;
+    CUtensorMap tmQ, tmK, tmV;
+    if (int rc = make_tmap_2d(&tmQ, p.q, dt, 2, (uint64_t)p.T, (uint64_t)p.ldq, (uint64_t)p.ldq * 2, tile_tokens(G), 64, true)) return rc;
+    if (int rc = make_tmap_2d(&tmK, p.k_cache, dt, 2, rows, 128, 256, kPage, 64, true)) return rc;
+    if (int rc = make_tmap_2d(&tmV, p.v_cache, dt, 2, rows, 128, 256, kPage, 64, true)) return rc;
+    // a sequence of n single tiles has (n + 1) / 2 of these
+    OVB_CHECK_CUDA(launch_pdl(kern, dim3((num_q_tiles + p.B + 1) / 2, p.Hkv), dim3(kDuoThreads), (size_t)smem, stream, tmQ, tmK, tmV, p, status_word()));
+    return 0;
+}
+
 template <int KH, int RH, int VH, int G, int SRC, bool F16>
 int launch_tc_parts(const PaKParams& p, int num_q_tiles, cudaStream_t stream) {
     const int TOK = tile_tokens(G > 0 ? G : p.group);
@@ -459,6 +762,15 @@ int launch_prefill_tc(const PaKParams& p, int D, int G, bool paged, bool f16, in
         (reinterpret_cast<uintptr_t>(p.out) & 15) || p.ldq % 8 != 0 || (!paged && p.ld_kv % 8 != 0))
         return ERR_UNSUPPORTED;
     if (paged && !f16) {
+        // two tiles to a CTA once single tiles would fill the machine twice; fewer are better spread over the SMs
+        if (D == 128 && p.gate == nullptr && p.sink == nullptr && num_q_tiles * p.Hkv >= 2 * 148) {
+            switch (G) {
+                case 1: return launch_duo<1>(p, num_q_tiles, stream);
+                case 2: return launch_duo<2>(p, num_q_tiles, stream);
+                case 4: return launch_duo<4>(p, num_q_tiles, stream);
+                case 8: return launch_duo<8>(p, num_q_tiles, stream);
+            }
+        }
         if (D == 128) {
             switch (G) {
                 case 1: return launch_tc<128, 1, true, false>(p, num_q_tiles, stream);

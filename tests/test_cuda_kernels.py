@@ -728,3 +728,26 @@ def test_gemm_pair_fp16_window_and_groups(ops):
         ops.check_status("gemm_pair")
         assert _rel_err(out, ref) < PAIR_REL and (out[sum(sizes):] == 3.0).all()
 
+
+
+@pytest.mark.parametrize("q_lens,past_lens,Hq,Hkv,window", [
+    ([1300, 1, 77, 640], [3, 500, 0, 129], 32, 8, 0),   # two query tiles of one CTA, the second of them empty, one row, whole
+    ([1, 2500, 2600], [700, 0, 17], 8, 8, 0),           # one query head per KV head
+    ([2049, 511], [0, 1000], 16, 8, 300),               # two query heads; tiles that the window hides from one of the two
+    ([700, 33], [100, 0], 64, 8, 0),                    # eight query heads
+])
+def test_paged_attention_long_prompts(ops, q_lens, past_lens, Hq, Hkv, window):
+    torch.manual_seed(5)
+    D, bs, dev, T = 128, 16, "cuda", sum(q_lens)
+    pl_t, sb_t, bi_t, bib_t, total_blocks = _make_paged_batch(q_lens, past_lens, bs, dev)
+    k_cache = torch.randn(total_blocks, Hkv, bs, D, device=dev).to(torch.bfloat16)
+    v_cache = torch.randn(total_blocks, Hkv, bs, D, device=dev).to(torch.bfloat16)
+    qkv = (torch.randn(T, (Hq + 2 * Hkv) * D, device=dev) * 1.5).to(torch.bfloat16)     # some scores stand out: the running maximum is raised
+    scale = 1.0 / math.sqrt(D)
+    out = ops.paged_attention(qkv, k_cache, v_cache, pl_t, sb_t, bi_t, bib_t, Hq, Hkv, D, scale=scale, sliding_window=window,
+                              max_context_len=max(p + q for p, q in zip(past_lens, q_lens)), max_q_len=max(q_lens))
+    ops.check_status("paged_attention")
+    rows = [[c[bi_t[bib_t[b]:bib_t[b + 1]].long()].permute(0, 2, 1, 3).reshape(-1, Hkv, D)[:p + q].float() for b, (q, p) in enumerate(zip(q_lens, past_lens))]
+            for c in (k_cache, v_cache)]
+    ref = _attn_ref(qkv[:, :Hq * D].float().reshape(T, Hq, D), rows[0], rows[1], q_lens, past_lens, Hq, Hkv, D, scale, window)
+    assert _rel_err(out.reshape(T, Hq, D), ref) < 1e-2
