@@ -33,11 +33,23 @@ __device__ __forceinline__ __half from_float<__half>(float v) {
 // cap * tanh(v / cap); the error is of the order of an ulp of cap.
 __device__ __forceinline__ float soft_cap(float v, float cap) { return cap - __fdividef(2.0f * cap, 1.0f + __expf(__fdividef(2.0f * v, cap))); }
 
+// v * Phi(v) with erfc by Abramowitz and Stegun 7.1.26 (absolute error below 1.5e-7; the largest error of the result over [-12, 12] is
+// 3.3e-7, with erff and 1 + erf it is 4.5e-7). Two special-function instructions and a dozen FMAs instead of erff's two branches:
+// at K = 1024 the epilogue, not the products, set the time.
+// 6144 x 4096 x 1024 in fp16 (gemm_pair.cu): 148 us with erff in sixteen copies of the switch, 141 us with this, and see apply_act_n.
+__device__ __forceinline__ float gelu_erf(float v) {
+    const float z = fminf(fabsf(v), 30.f) * 0.70710678118654752f;       // bounded: 0 * inf below would be NaN
+    const float t = __fdividef(1.f, fmaf(0.3275911f, z, 1.f));
+    const float poly = t * fmaf(t, fmaf(t, fmaf(t, fmaf(t, 1.061405429f, -1.453152027f), 1.421413741f), -0.284496736f), 0.254829592f);
+    const float h = z * 0.70710678118654752f * poly * __expf(-z * z);   // |v| / 2 * erfc(z)
+    return v < 0.f ? -h : v - h;
+}
+
 // Activations of the epilogue; P carries `act` and the limits of the GEMM's arguments.
 template <class P>
 __device__ __forceinline__ float apply_act(float v, const P& p) {
     switch (p.act) {
-        case OVB_ACT_GELU_ERF: return 0.5f * v * (1.0f + erff(v * 0.70710678118654752f));
+        case OVB_ACT_GELU_ERF: return gelu_erf(v);
         case OVB_ACT_RELU: return v > 0.f ? v : 0.f;
         case OVB_ACT_SILU: return v / (1.0f + __expf(-v));
         case OVB_ACT_GELU_TANH: {
@@ -50,6 +62,40 @@ __device__ __forceinline__ float apply_act(float v, const P& p) {
     }
 }
 
+// The same for N values. The choice is outside the loop: sixteen unrolled copies of the switch do not fit the instruction cache.
+template <int N, class P>
+__device__ __forceinline__ void apply_act_n(float (&v)[N], const P& p) {
+    switch (p.act) {
+        case OVB_ACT_NONE: break;
+        case OVB_ACT_GELU_ERF:
+#pragma unroll
+            for (int j = 0; j < N; ++j) v[j] = gelu_erf(v[j]);
+            break;
+        case OVB_ACT_SILU:
+#pragma unroll
+            for (int j = 0; j < N; ++j) v[j] = v[j] / (1.0f + __expf(-v[j]));
+            break;
+        case OVB_ACT_RELU:
+#pragma unroll
+            for (int j = 0; j < N; ++j) v[j] = v[j] > 0.f ? v[j] : 0.f;
+            break;
+        case OVB_ACT_RELU2:
+#pragma unroll
+            for (int j = 0; j < N; ++j) v[j] = v[j] > 0.f ? v[j] * v[j] : 0.f;
+            break;
+        default:                            // the rare ones: one copy of the code
+#pragma unroll 1
+            for (int j = 0; j < N; ++j) {
+                float one = 0.f;
+#pragma unroll
+                for (int i = 0; i < N; ++i) one = i == j ? v[i] : one;
+                one = apply_act(one, p);
+#pragma unroll
+                for (int i = 0; i < N; ++i) v[i] = i == j ? one : v[i];
+            }
+    }
+}
+
 // Clamped gate and up values with a sigmoid of adjustable slope (OVB_ACT_GLU_LIMITED).
 template <class P>
 __device__ __forceinline__ float glu_limited(const P& p, float g, float u) {
@@ -58,21 +104,35 @@ __device__ __forceinline__ float glu_limited(const P& p, float g, float u) {
     return g / (1.0f + __expf(-p.act_slope * g)) * (u + p.act_shift);
 }
 
+// Integers to bf16 without shifts: the bits 0..7 of a bf16 are linear in value down to zero (sub-normals and the first binade have
+// the same spacing), so an integer b < 256 in the low byte of a 16-bit lane reads as b * 2^-133, and a nibble in bits 4..7 as
+// 16 q * 2^-133. One fused multiply-add by 2^127 (2^123) makes that (b - z) / 64, exact; the product with 64 * scale is then rounded
+// once, like (b - z) * scale. u4: five integer instructions per eight weights instead of eight (shift and merge per pair), which
+// bound the kernel (ALU pipe 67 % busy on average); u8: one per pair instead of conversions (XU pipe 76 % busy). Zero points are whole.
+// 128256 x 4096 weights: u4 T = 1 109 -> 94 us, T = 64 125 -> 109 us; u8 T = 24 177 -> 119 us (cold caches).
+struct RowScale {
+    __nv_bfloat162 m, s;        // -z / 64 and 64 * scale, twice each
+};
+// `szp`: (scale, bias + zero point) of a row and group; bias 16 for u4, 0 for u8
+__device__ __forceinline__ RowScale row_scale(__nv_bfloat162 szp, float bias) {
+    const __nv_bfloat162 zz = __halves2bfloat162(__high2bfloat16(szp), __high2bfloat16(szp)), ss = __halves2bfloat162(__low2bfloat16(szp), __low2bfloat16(szp));
+    return {__hmul2(__hsub2(__float2bfloat162_rn(bias), zz), __float2bfloat162_rn(0.015625f)), __hmul2(ss, __float2bfloat162_rn(64.f))};
+}
+__device__ __forceinline__ uint32_t lane_fma(uint32_t bits, uint32_t mul, const RowScale& r) {
+    const __nv_bfloat162 v = __hmul2(__hfma2(*reinterpret_cast<__nv_bfloat162*>(&bits), *reinterpret_cast<__nv_bfloat162*>(&mul), r.m), r.s);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+constexpr uint32_t kTwo127 = 0x7F007F00u, kTwo123 = 0x7D007D00u;      // bf16 pairs
 // Expand one u32 (8 packed u4 in the plugin nibble order) to 8 bf16: (q - zp) * scale.
-// A nibble placed in mantissa bits 3..6 of bf16 16.0 (0x4180) reads as 16 + q exactly.
-__device__ __forceinline__ uint4 dequant_u4x8(uint32_t x, __nv_bfloat162 zz, __nv_bfloat162 ss) {
-    uint32_t t[4];
-    t[0] = ((x << 3) & 0x00780078u) | 0x41804180u;
-    t[1] = ((x >> 1) & 0x00780078u) | 0x41804180u;
-    t[2] = ((x >> 5) & 0x00780078u) | 0x41804180u;
-    t[3] = ((x >> 9) & 0x00780078u) | 0x41804180u;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&t[i]);
-        v = __hmul2(__hsub2(v, zz), ss);
-        t[i] = *reinterpret_cast<uint32_t*>(&v);
-    }
-    return make_uint4(t[0], t[1], t[2], t[3]);
+__device__ __forceinline__ uint4 dequant_u4x8(uint32_t x, const RowScale& r) {
+    const uint32_t y = x >> 8;
+    return make_uint4(lane_fma(x & 0x000F000Fu, kTwo127, r), lane_fma(x & 0x00F000F0u, kTwo123, r), lane_fma(y & 0x000F000Fu, kTwo127, r),
+                      lane_fma(y & 0x00F000F0u, kTwo123, r));
+}
+// Four bytes -> four bf16: (b - zp) * scale.
+__device__ __forceinline__ void dequant_u8x4(uint32_t w, const RowScale& r, uint32_t& lo, uint32_t& hi) {
+    lo = lane_fma(__byte_perm(w, 0u, 0x4140), kTwo127, r);
+    hi = lane_fma(__byte_perm(w, 0u, 0x4342), kTwo127, r);
 }
 
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
@@ -90,9 +150,9 @@ constexpr int wq_bytes(int wmode) { return wmode == OVB_W_U4 ? TILE_N * 32 : ((w
 // Four fp8 e4m3 bytes -> four bf16 (two words), each scaled: an e4m3 byte placed at bits 4..10 (sign at 15) of a bf16
 // reads as value * 2^-120 (sub-normals included), and the per-block scale in `ss` already carries the 2^120.
 __device__ __forceinline__ void dequant_f8x4(uint32_t w, __nv_bfloat162 ss, uint32_t& lo, uint32_t& hi) {
-    const uint32_t y0 = __byte_perm(w, 0u, 0x4140), y1 = __byte_perm(w, 0u, 0x4342);
-    uint32_t t0 = ((y0 << 8) & 0x80008000u) | ((y0 << 4) & 0x07F007F0u);
-    uint32_t t1 = ((y1 << 8) & 0x80008000u) | ((y1 << 4) & 0x07F007F0u);
+    const uint32_t y0 = __byte_perm(w, 0u, 0x1404), y1 = __byte_perm(w, 0u, 0x3424);      // bytes in the upper halves of their lanes
+    uint32_t t0 = (y0 & 0x80008000u) | ((y0 >> 4) & 0x07F007F0u);
+    uint32_t t1 = (y1 & 0x80008000u) | ((y1 >> 4) & 0x07F007F0u);
     __nv_bfloat162 v0 = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&t0), ss);
     __nv_bfloat162 v1 = __hmul2(*reinterpret_cast<__nv_bfloat162*>(&t1), ss);
     lo = *reinterpret_cast<uint32_t*>(&v0);

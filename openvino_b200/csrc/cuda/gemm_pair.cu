@@ -294,11 +294,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                     }
                 } else if (p.out_f32) {
                     float* o = reinterpret_cast<float*>(p.out) + (size_t)tok * p.ldo + oc;
+                    float v[16];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const float v = apply_act(__uint_as_float(r[j]) + bias_v, p);
-                        if (store && tok + j < t.t_end) o[(size_t)j * p.ldo] = v;
-                    }
+                    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + bias_v;
+                    apply_act_n(v, p);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (store && tok + j < t.t_end) o[(size_t)j * p.ldo] = v[j];
                 } else {
                     uint32_t rc[8];
 #pragma unroll
@@ -307,10 +309,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
                     float v[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + bias_v;
-                    if (p.act != OVB_ACT_NONE) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) v[j] = apply_act(v[j], p);
-                    }
+                    apply_act_n(v, p);
                     E* o = reinterpret_cast<E*>(p.out) + (size_t)(tok + odd) * p.ldo + (oc & ~1);
 #pragma unroll
                     for (int j = 0; j < 16; j += 2) {
@@ -369,8 +368,7 @@ __global__ void __launch_bounds__(256) expand_weights_kernel(const uint8_t* __re
         for (int i = 0; i < 4; ++i) {
             const int r = r0 + i * 32;
             const __nv_bfloat162 szp = *reinterpret_cast<const __nv_bfloat162*>(&s[i]);
-            dst[r * 8 + (u ^ (r & 7))] = dequant_u4x8(q[i], __halves2bfloat162(__high2bfloat16(szp), __high2bfloat16(szp)),
-                                                      __halves2bfloat162(__low2bfloat16(szp), __low2bfloat16(szp)));
+            dst[r * 8 + (u ^ (r & 7))] = dequant_u4x8(q[i], row_scale(szp, 16.f));
         }
     } else {
         const size_t K = (size_t)KB * TILE_K;
@@ -392,13 +390,9 @@ __global__ void __launch_bounds__(256) expand_weights_kernel(const uint8_t* __re
                 dequant_f8x4(q[i].x, ss2, o[0], o[1]);
                 dequant_f8x4(q[i].y, ss2, o[2], o[3]);
             } else {
-                const float sf = __bfloat162float(__low2bfloat16(szp)), zf = __bfloat162float(__high2bfloat16(szp));
-                const uint32_t b[2] = {q[i].x, q[i].y};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int sh = (e & 1) * 16;
-                    o[e] = pack_bf16x2((float((b[e >> 1] >> sh) & 0xFF) - zf) * sf, (float((b[e >> 1] >> (sh + 8)) & 0xFF) - zf) * sf);
-                }
+                const RowScale rs = row_scale(szp, 0.f);
+                dequant_u8x4(q[i].x, rs, o[0], o[1]);
+                dequant_u8x4(q[i].y, rs, o[2], o[3]);
             }
             dst[r * 8 + (u ^ (r & 7))] = make_uint4(o[0], o[1], o[2], o[3]);
         }

@@ -490,13 +490,12 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
                 const __nv_bfloat162 szp = *reinterpret_cast<const __nv_bfloat162*>(&cur);
                 uint32_t r[32];
                 if (WMODE == OVB_W_U4) {
-                    const __nv_bfloat162 ss2 = __halves2bfloat162(__low2bfloat16(szp), __low2bfloat16(szp));
-                    const __nv_bfloat162 zz2 = __halves2bfloat162(__high2bfloat16(szp), __high2bfloat16(szp));
+                    const RowScale rs = row_scale(szp, 16.f);
                     const uint4 pk0 = lds128(slot_a + row * 16), pk1 = lds128(slot_a + TILE_N * 16 + row * 16);
                     const uint32_t xs[8] = {pk0.x, pk0.y, pk0.z, pk0.w, pk1.x, pk1.y, pk1.z, pk1.w};
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const uint4 e = dequant_u4x8(xs[j], zz2, ss2);
+                        const uint4 e = dequant_u4x8(xs[j], rs);
                         r[4 * j] = e.x; r[4 * j + 1] = e.y; r[4 * j + 2] = e.z; r[4 * j + 3] = e.w;
                     }
                 } else if (WMODE == OVB_W_F8) {
@@ -510,18 +509,14 @@ gemm_ws_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
                         dequant_f8x4(pk.w, ss2, r[h * 8 + 6], r[h * 8 + 7]);
                     }
                 } else {
-                    const float sf = __bfloat162float(__low2bfloat16(szp));
-                    const float zf = __bfloat162float(__high2bfloat16(szp));
+                    const RowScale rs = row_scale(szp, 0.f);
 #pragma unroll
                     for (int h = 0; h < 4; ++h) {
                         const uint4 pk = lds128(slot_a + row * ROW_PKT + h * 16);
-                        const uint32_t b[4] = {pk.x, pk.y, pk.z, pk.w};
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            const uint32_t w32 = b[e >> 1];
-                            const int sh = (e & 1) * 16;
-                            r[h * 8 + e] = pack_bf16x2((float((w32 >> sh) & 0xFF) - zf) * sf, (float((w32 >> (sh + 8)) & 0xFF) - zf) * sf);
-                        }
+                        dequant_u8x4(pk.x, rs, r[h * 8 + 0], r[h * 8 + 1]);
+                        dequant_u8x4(pk.y, rs, r[h * 8 + 2], r[h * 8 + 3]);
+                        dequant_u8x4(pk.z, rs, r[h * 8 + 4], r[h * 8 + 5]);
+                        dequant_u8x4(pk.w, rs, r[h * 8 + 6], r[h * 8 + 7]);
                     }
                 }
                 tmem_st_x16(a_lane + uint32_t(st * A_COLS), r);

@@ -751,3 +751,45 @@ def test_paged_attention_long_prompts(ops, q_lens, past_lens, Hq, Hkv, window):
             for c in (k_cache, v_cache)]
     ref = _attn_ref(qkv[:, :Hq * D].float().reshape(T, Hq, D), rows[0], rows[1], q_lens, past_lens, Hq, Hkv, D, scale, window)
     assert _rel_err(out.reshape(T, Hq, D), ref) < 1e-2
+
+
+def test_gelu_epilogue_range(ops):
+    """The erf form of GELU over its range, infinities and NaN, against 64 bits: 3.3e-7 of the function itself (its two special
+    functions and fp32 sums), two units in the last place of the fp32 product before it."""
+    v = torch.cat([torch.linspace(-12, 12, 4093), torch.tensor([float("inf"), float("-inf"), float("nan")])]).cuda().to(torch.bfloat16)
+    for T, kw in ((300, {}), (300, {"block_t": 64}), (5, {})):
+        x = torch.zeros(T, 128, device="cuda", dtype=torch.bfloat16)
+        x[:, 0] = 1.0
+        w = torch.zeros(4096, 128, device="cuda", dtype=torch.bfloat16)
+        w[:, 0] = v
+        got = ops.gemm(x, ops.PackedWeight.from_dense(w), act=ops.ACT_GELU_ERF, out_f32=True, **kw)[3].double()
+        want = 0.5 * v.double() * torch.special.erfc(-v.double() * math.sqrt(0.5))
+        assert (got[:4093] - want[:4093]).abs().max() < 1e-6
+        assert got[4093] == float("inf") and got[4094] == 0 and got[4095].isnan()
+
+
+@pytest.mark.parametrize("fmt", ["u4", "u8"])
+def test_expanded_weights_exact(ops, fmt):
+    """Every byte and zero point, with scales from the smallest to the largest fp16: one weight at a time through the product is
+    (q - z) * scale rounded once to bf16, bit for bit."""
+    K, N = 256, 2048
+    k = torch.arange(K, device="cuda")
+    n = torch.arange(N, device="cuda")
+    scale = torch.tensor([6e-8, 6.1e-5, 0.0137, 1.0, 333.25, 65504.0], device="cuda")[n % 6].half()
+    s = scale.bfloat16()
+    if fmt == "u4":
+        q = ((k[None] + n[:, None]) % 16).to(torch.uint8)
+        z = (n // 6 % 16).to(torch.uint8)
+        w = ops.PackedWeight.from_ir_u4((q[:, 0::2] | (q[:, 1::2] << 4)).reshape(-1), scale[:, None].repeat(1, 2).contiguous(), z[:, None].repeat(1, 2).contiguous(), N, K, 128,
+                                        zp_is_u8=True)
+    else:
+        q = k[None].repeat(N, 1).to(torch.uint8)
+        z = (n // 6 % 256).to(torch.uint8)
+        w = ops.PackedWeight.from_ir_u8(q, scale[:, None].repeat(1, 2).contiguous(), z[:, None].repeat(1, 2).contiguous(), N, K, 128)
+    want = ((q.double() - z.double()[:, None]) * s.double()[:, None]).to(torch.bfloat16)
+    x = torch.eye(K, device="cuda", dtype=torch.bfloat16)
+    for kw in ({"block_t": 64}, {"block_t": 256}):
+        assert torch.equal(ops.gemm(x, w, out_f32=True, **kw).t().contiguous(), want.float()), kw
+    many = ops.gemm(x.repeat(4, 1), w, out_f32=True)         # expanded in a pass of its own
+    assert torch.equal(many[:K].t().contiguous(), want.float()) and torch.equal(many[3 * K:].t().contiguous(), want.float())
+    ops.check_status("gemm")
