@@ -793,3 +793,16 @@ def test_expanded_weights_exact(ops, fmt):
     many = ops.gemm(x.repeat(4, 1), w, out_f32=True)         # expanded in a pass of its own
     assert torch.equal(many[:K].t().contiguous(), want.float()) and torch.equal(many[3 * K:].t().contiguous(), want.float())
     ops.check_status("gemm")
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 1016), (5, 1024), (6, 1032), (9, 256)])
+def test_layernorm_row_widths(ops, rows, cols):
+    """Rows of a warp and of a block, whole and ragged, with and without a residual."""
+    torch.manual_seed(rows)
+    x, r = (torch.randn(rows, cols, device="cuda", dtype=torch.float16) * 3 + 1 for _ in range(2))
+    g, b = (torch.randn(cols, device="cuda", dtype=torch.float16) for _ in range(2))
+    for res in (None, r):
+        y = ops.layernorm(x, g, b, 1e-5, residual=res)
+        h = x.double() + (res.double() if res is not None else 0)
+        ref = torch.nn.functional.layer_norm(h, (cols,), g.double(), b.double(), 1e-5)
+        assert _rel_err(y, ref) < 1e-3          # one rounding to fp16: 2^-11 of a value at most
