@@ -864,6 +864,16 @@ __global__ void pack_w16_kernel(const uint4* __restrict__ w, uint4* __restrict__
         w_out[dst] = w[i];
     }
 }
+__device__ __forceinline__ uint32_t pack_f8_word(uint32_t w) {
+    const uint32_t x = (w & 0xFFu) | ((w & 0xFF00u) << 8), y = ((w >> 16) & 0xFFu) | ((w >> 8) & 0xFF0000u);      // values 0, 1 and 2, 3 in the lanes
+    return ((x & 0x00800080u) << 8) | ((x & 0x007F007Fu) << 4) | ((y & 0x00800080u) << 4) | ((y & 0x00700070u) << 8) | (y & 0x000F000Fu);
+}
+__global__ void pack_f8_kernel(const uint4* __restrict__ w, uint4* __restrict__ w_out, size_t n) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const uint4 v = w[i];
+        w_out[i] = make_uint4(pack_f8_word(v.x), pack_f8_word(v.y), pack_f8_word(v.z), pack_f8_word(v.w));
+    }
+}
 // scales_ir [N, G] fp16 + zero points -> [G, N] pairs (bf16 scale, bf16 bias + zp); zps_out (optional) [G, N]
 __global__ void pack_scale_zp_kernel(const __half* __restrict__ scales_ir, const uint8_t* __restrict__ zps_ir,
                                      int zp_is_u8, __nv_bfloat16* __restrict__ scales_out,
@@ -1155,6 +1165,14 @@ int ovb_pack_w16(const void* w, void* w_out, int N, int K, ovb_stream_t stream_)
     const size_t npieces = (size_t)N * K / 8;
     OVB_CHECK_CUDA(launch_serial(pack_w16_kernel, dim3(grid_for(npieces, 256)), dim3(256), 0, stream, (const uint4*)w, (uint4*)w_out, npieces, K));
     OVB_CHECK_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int ovb_pack_f8(const void* w, void* w_out, long long words, ovb_stream_t stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    OVB_REQUIRE(w && w_out && words > 0 && words % 4 == 0, "ovb_pack_f8: a multiple of four words expected");
+    OVB_REQUIRE(((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(w_out)) & 15) == 0, "ovb_pack_f8: 16-byte aligned memory expected");
+    OVB_CHECK_CUDA(launch_serial(pack_f8_kernel, dim3(grid_for((size_t)words / 4, 256)), dim3(256), 0, stream, (const uint4*)w, (uint4*)w_out, (size_t)words / 4));
     return 0;
 }
 

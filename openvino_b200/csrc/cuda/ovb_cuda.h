@@ -40,7 +40,7 @@ enum {
     OVB_W_U4 = 1,     // W is packed u4 in the plugin layout made by ovb_pack_u4 (4608-byte chunks, see below)
     OVB_W_U8 = 2,     // W is u8 [N, K]
     OVB_W_F16 = 3,    // W and X are fp16 (BERT path)
-    OVB_W_F8 = 4,     // W is fp8 e4m3 [N, K]; the (scale, -) pair table carries the block scale of every (k-group, row) times 2^120
+    OVB_W_F8 = 4,     // W is fp8 e4m3 [N, K], four values of a row to a word in the bit order of dequant_f8x4 (gemm_common.cuh); the (scale, -) pair table carries the block scale of every (k-group, row) times 2^120
 };
 enum {
     OVB_ACT_NONE = 0,
@@ -122,6 +122,8 @@ int ovb_pack_u4(const void* w_ir, const void* scales_ir, const void* zps_ir, int
 // 64-column k-block one 16 KB chunk whose 16-byte pieces are already placed in the 128-byte swizzle
 // ((tile * K/64 + kb) * 128 + row) * 8 + (piece ^ (row & 7)). w_out holds ceil(N/128)*128 * K elements.
 int ovb_pack_w16(const void* w, void* w_out, int N, int K, ovb_stream_t stream);
+// fp8 e4m3 bytes in row order -> the bit order of OVB_W_F8, word by word (16-byte aligned, a multiple of four words).
+int ovb_pack_f8(const void* w, void* w_out, long long words, ovb_stream_t stream);
 
 // ---------------------------------------------------------------------------------------------
 // Normalisation / elementwise

@@ -289,7 +289,19 @@ class PackedWeight:
         The kernel reads the scales as a (k-group, row) table of bf16 values that already carry the 2^120 exponent
         shift of its byte-to-bf16 conversion."""
         assert block == 128 and K % block == 0
-        w8 = w8.view(torch.uint8).reshape(N, K).contiguous()
+        w8 = w8.view(torch.uint8).reshape(N, K)
+        # four values of a row to a 32-bit word, in the bits from which the kernels take bf16 pairs (dequant_f8x4 in gemm_common.cuh):
+        # 16-bit lane i holds value i as [sign | 0000 | exponent, mantissa | 0000] and value 2 + i in the gaps
+        w8 = w8.contiguous()
+        out = torch.empty((N, K), dtype=torch.uint8, device=w8.device)
+        if w8.is_cuda:
+            _check(lib().ovb_pack_f8(C.c_void_p(w8.data_ptr()), C.c_void_p(out.data_ptr()), C.c_longlong(N * K // 4), C.c_void_p(_stream())), "ovb_pack_f8")
+        else:
+            v = w8.reshape(-1, 4).to(torch.int32)
+            x, y = v[:, :2], v[:, 2:]
+            lane = ((x & 0x80) << 8) | ((x & 0x7F) << 4) | ((y & 0x80) << 4) | ((y & 0x70) << 8) | (y & 0x0F)
+            out.copy_(torch.stack([lane & 0xFF, lane >> 8], dim=-1).to(torch.uint8).reshape(N, K))
+        w8 = out
         G = K // block
         s = block_scales.float().reshape(-1, G)                                     # [N/128, G]
         per_row = s.repeat_interleave(block, dim=0)[:N]                             # [N, G]

@@ -768,7 +768,7 @@ def test_gelu_epilogue_range(ops):
         assert got[4093] == float("inf") and got[4094] == 0 and got[4095].isnan()
 
 
-@pytest.mark.parametrize("fmt", ["u4", "u8"])
+@pytest.mark.parametrize("fmt", ["u4", "u8", "f8"])
 def test_expanded_weights_exact(ops, fmt):
     """Every byte and zero point, with scales from the smallest to the largest fp16: one weight at a time through the product is
     (q - z) * scale rounded once to bf16, bit for bit."""
@@ -782,11 +782,19 @@ def test_expanded_weights_exact(ops, fmt):
         z = (n // 6 % 16).to(torch.uint8)
         w = ops.PackedWeight.from_ir_u4((q[:, 0::2] | (q[:, 1::2] << 4)).reshape(-1), scale[:, None].repeat(1, 2).contiguous(), z[:, None].repeat(1, 2).contiguous(), N, K, 128,
                                         zp_is_u8=True)
+    elif fmt == "f8":
+        q = ((k[None] * 5 + n[:, None]) % 256).to(torch.uint8)
+        q = torch.where((q & 0x7F) == 0x7F, 0, q).to(torch.uint8)                  # no NaN
+        blocks = torch.tensor([3e-5, 0.0137, 1.0, 117.25], device="cuda")[torch.arange(N // 128 * 2, device="cuda") % 4].reshape(N // 128, 2)
+        w = ops.PackedWeight.from_f8_block(q, blocks, N, K)
     else:
         q = k[None].repeat(N, 1).to(torch.uint8)
         z = (n // 6 % 256).to(torch.uint8)
         w = ops.PackedWeight.from_ir_u8(q, scale[:, None].repeat(1, 2).contiguous(), z[:, None].repeat(1, 2).contiguous(), N, K, 128)
-    want = ((q.double() - z.double()[:, None]) * s.double()[:, None]).to(torch.bfloat16)
+    if fmt == "f8":
+        want = (q.view(torch.float8_e4m3fn).double() * blocks.bfloat16().double().repeat_interleave(128, 0).repeat_interleave(128, 1)).to(torch.bfloat16)
+    else:
+        want = ((q.double() - z.double()[:, None]) * s.double()[:, None]).to(torch.bfloat16)
     x = torch.eye(K, device="cuda", dtype=torch.bfloat16)
     for kw in ({"block_t": 64}, {"block_t": 256}):
         assert torch.equal(ops.gemm(x, w, out_f32=True, **kw).t().contiguous(), want.float()), kw
