@@ -1494,6 +1494,7 @@ int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream_) {
         OVB_REQUIRE((a->wmode == OVB_W_U4 || (a->w_tiled && !quant)) && a->comm == nullptr && a->N % TILE_N == 0 && a->K % TILE_K == 0,
                     "ovb_gemm: grouped GEMM needs tile-packed weights (u4 or 16-bit), N %% 128 == 0, K %% 64 == 0 and no communicator");
     }
+    if (gemm_stream_takes(a)) return gemm_stream(a, stream);
     if (gemm_pair_takes(a)) return gemm_pair(a, stream);
     const int bt = a->block_t ? a->block_t : pick_block_t(a->T);
     const int splits = (swiglu || grouped) ? 1 : a->splits;   // 0: chosen at launch, where the kernel variant and its cluster occupancy are known

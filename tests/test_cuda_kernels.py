@@ -814,3 +814,47 @@ def test_layernorm_row_widths(ops, rows, cols):
         h = x.double() + (res.double() if res is not None else 0)
         ref = torch.nn.functional.layer_norm(h, (cols,), g.double(), b.double(), 1e-5)
         assert _rel_err(y, ref) < 1e-3          # one rounding to fp16: 2^-11 of a value at most
+
+
+@pytest.mark.parametrize("fmt,N,K", [("dense", 96, 64), ("dense", 4096, 1088), ("u4", 128, 128), ("u4", 6240, 4096), ("u4", 1024, 14336), ("u8", 32, 256), ("u8", 2080, 4096),
+                                     ("f8", 160, 128), ("f8", 4096, 7168)])
+@pytest.mark.parametrize("T", [1, 3, 4, 8])
+def test_gemm_stream(ops, fmt, N, K, T):
+    """Edges of the token fragment, one unit of K, K shared by a cluster, tiles that are no multiple of 128 rows: against the
+    tensor-memory kernel (an explicit token tile selects it) and, where the weights are known, no further from a 64-bit product."""
+    torch.manual_seed(T)
+    x = torch.randn(T, K + 8, device="cuda", dtype=torch.bfloat16)[:, :K]
+    if fmt == "u4":
+        g = torch.Generator(device="cuda").manual_seed(N)
+        q = torch.randint(0, 256, (N * K // 2,), dtype=torch.uint8, device="cuda", generator=g)
+        z = torch.randint(0, 16, (N, K // 128), dtype=torch.uint8, device="cuda", generator=g)
+        sc = (torch.rand(N, K // 128, device="cuda", generator=g) * 0.01 + 0.005).half()
+        w = ops.PackedWeight.from_ir_u4(q, sc, z, N, K, 128, zp_is_u8=True)
+        wide = (torch.stack([q & 15, q >> 4], -1).reshape(N, K // 128, 128).double() - z.double()[..., None]) * sc.bfloat16().double()[..., None]
+        exact = x.double() @ wide.reshape(N, K).t()
+        out, old = ops.gemm(x, w), ops.gemm(x, w, block_t=16)
+        # the sums are exact to fp32, so the result is the rounded product up to a rare neighbour (more tokens take the other kernel)
+        assert T > 4 or _rel_err(out, exact) <= 1.02 * _rel_err(exact.to(torch.bfloat16), exact) and _rel_err(out, exact) <= _rel_err(old, exact)
+    else:
+        w = _pair_weight(ops, fmt, N, K)
+    # weights rounded to bf16 (2^-9 / sqrt(3) each) against unrounded ones, and the two roundings of the results
+    for kw in (dict(), dict(out_f32=True, act=ops.ACT_SILU)):
+        assert _rel_err(ops.gemm(x, w, **kw), ops.gemm(x, w, block_t=16, **kw)) < PAIR_REL, kw
+    w.bias = torch.randn(N, device="cuda").to(torch.bfloat16)
+    h = torch.randn(T + 1, N, device="cuda").to(torch.bfloat16)
+    keep = h[T].clone()
+    want = ops.gemm(x, w, residual=h[:T], block_t=16)
+    ops.gemm(x, w, out=h[:T], residual=h[:T])
+    assert _rel_err(h[:T], want) < PAIR_REL and torch.equal(h[T], keep)
+    w.bias = None
+    if N % 128 == 0:
+        for kw in (dict(act=ops.ACT_SWIGLU), dict(act=ops.ACT_GLU_LIMITED, glu=(7.0, 1.702, 1.0))):
+            assert _rel_err(ops.gemm(x, w, **kw), ops.gemm(x, w, block_t=16, **kw)) < 2 * PAIR_REL, kw      # a product of two such values
+    ops.check_status("gemm_stream")
+
+
+def test_gemm_stream_fp16_and_window(ops):
+    torch.manual_seed(3)
+    x = torch.randn(5, 256, device="cuda", dtype=torch.float16)
+    w = _pair_weight(ops, "dense", 512, 1024, torch.float16).window(128, 256, 320, 256)
+    assert _rel_err(ops.gemm(x, w), ops.gemm(x, w, block_t=16)) < PAIR_REL
