@@ -348,7 +348,7 @@ __device__ __forceinline__ void store_decoded(const PaKParams& p, int tok, int h
 // makes exact whole numbers only, two instructions a pair: a score is scale_j * (q . b_j - zero_j * sum(q)), and the probabilities
 // take the value rows' scales before they are rounded; what their zero points contribute is the same for all columns and is
 // summed per row from the rounded probabilities.
-// 24 sequences of 1200 tokens, 32 / 8 heads: 43 us with rounded products, 33 us now.
+// 24 sequences of 1200 tokens, 32 / 8 heads: 43 us with rounded products and two expanded pages per warp, 30 us now.
 // DK / DV: key and value sizes, multiples of 64; cache rows may be shorter (p.k_row, p.v_row: the rest is filled with zeros).
 // GT: query heads per KV head, or 0: any number (p.group), up to eight of them per CTA.
 template <int DK, int DV, int GT, int PAGE, bool KVU8, int NST>
@@ -382,9 +382,11 @@ __global__ void __launch_bounds__(128) pa_decode_kernel(PaKParams p) {
     // the splits share the keys from the first page that the window or the chunk touches
     const int win_lo = first_visible_key(ctx - 1, p.sliding_window, p.chunk);
     const int k_first = win_lo / PAGE * PAGE;
-    // Each sequence shares out its own keys, 256 at least to a CTA: p.keys_per_split belongs to the longest context that a captured
-    // step may meet (the next power of two), and by it the first splits of shorter sequences had all the work. MEASURED_SPLIT
-    const int share = ((ctx - k_first + p.nsplit - 1) / p.nsplit + 63) / 64 * 64, per_split = min(p.keys_per_split, max(256, share));
+    // p.keys_per_split belongs to the longest context that a captured step may meet (the next power of two), and by it the first splits
+    // of shorter sequences have all the work. The byte form, bound by its expansion, shares out each sequence's own keys instead, 256
+    // at least to a CTA. The 16-bit form is bound by HBM, and more and shorter CTAs cost it more than the balance gives (64 sequences
+    // of 1150 tokens: 53 us, evenly shared 56 us).
+    const int share = ((ctx - k_first + p.nsplit - 1) / p.nsplit + 63) / 64 * 64, per_split = KVU8 ? min(p.keys_per_split, max(256, share)) : p.keys_per_split;
     const int k_lo = k_first + split * per_split;
     const int k_hi = min(ctx, k_lo + per_split);
     const int page_lo = k_lo / PAGE;
