@@ -569,47 +569,49 @@ pa_prefill_duo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     } else {
         // ------------------------------------------------------------------ softmax: one thread per stacked query row
         const int x = warp >> 2;                         // query tile of this thread
-        const int r = threadIdx.x & 127;                 // tensor-memory lane
-        const int g = r / TOK, tl = x * TOK + r % TOK;
-        const int qpos = past + tq0 + tl;
-        const bool row_valid = tq0 + tl < q_len;
-        const int lo_row = first_visible_key(qpos, p.sliding_window, p.chunk);
-        const int first_pos = past + tq0 + x * TOK, lo_last = first_visible_key(first_pos + TOK - 1, p.sliding_window, p.chunk);
-        const bool all_valid = tq0 + (x + 1) * TOK <= q_len;
-        const uint32_t lane_base = tmem + (uint32_t((warp & 3) * 32) << 16);
-        const uint32_t tm_s = lane_base + TM_S + x * 128, tm_o = lane_base + TM_O + x * 128;
+        // keys [lo_row, hi_row) from kv_start on are visible to this row, every row of the query tile sees those of [lo_last, lim). (With
+        // three warps on a scheduler a thread has 168 registers: a whole row of 128 scores beside the rest of the loop's state spilled.)
+        int hi_row, lo_row, lim, lo_last;
+        {
+            const int tl = x * TOK + (threadIdx.x & 127) % TOK, first_pos = past + tq0 + x * TOK;
+            hi_row = tq0 + tl >= q_len ? 0 : p.causal ? min(kv_end, past + tq0 + tl + 1) : kv_end;
+            lo_row = first_visible_key(past + tq0 + tl, p.sliding_window, p.chunk);
+            lim = tq0 + (x + 1) * TOK > q_len ? 0 : p.causal ? min(kv_end, first_pos + 1) : kv_end;
+            lo_last = first_visible_key(first_pos + TOK - 1, p.sliding_window, p.chunk);
+            hi_row -= kv_start;
+            lo_row -= kv_start;
+            lim -= kv_start;
+            lo_last -= kv_start;
+        }
+        const uint32_t tm_s = tmem + (uint32_t((warp & 3) * 32) << 16) + TM_S + x * 128;
         float m_used = -CUDART_INF_F, l_sum = 0.f;
         bool ok = true;
         for (int j = 0; j < ntiles && ok; ++j) {
             ok = mbar_wait(&s_full[x], j & 1, abort_flag, status);
             if (!ok) break;
             tc_fence_after_sync();
-            const int j0 = kv_start + j * kBK;
-            // does any row of this query tile need a mask? (uniform over its four warps)
-            const bool need_mask = j0 + kBK > kv_end || (p.causal && j0 + kBK - 1 > first_pos) || j0 < lo_last || !all_valid;
-            int hi = kBK, lo = 0;                        // keys [lo, hi) of the tile are visible to this row
-            if (need_mask) {
-                hi = min(hi, kv_end - j0);
-                if (p.causal) hi = min(hi, qpos - j0 + 1);
-                lo = max(lo, lo_row - j0);
-                if (!row_valid) hi = 0;
-            }
-            uint32_t v[kBK];
-#pragma unroll
-            for (int c = 0; c < kBK; c += 16) tmem_ld_x16(tm_s + c, v + c);
-            tmem_ld_wait();
+            const int j0 = j * kBK;
+            const bool need_mask = j0 + kBK > lim || j0 < lo_last;       // (uniform over the four warps of the query tile)
+            const int hi = hi_row - j0, lo = lo_row - j0;
+            // the upper half of the row is read for its maximum and again for its exponentials: a whole row does not fit the registers
+            uint32_t v[kBK / 2];
             float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-            if (need_mask) {
+            auto half_row = [&](int c0) {
 #pragma unroll
-                for (int i = 0; i < kBK; ++i) {
-                    const bool vis = i >= lo && i < hi;
-                    if (!vis) v[i] = __float_as_uint(-CUDART_INF_F);
-                    mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
+                for (int c = 0; c < kBK / 2; c += 16) tmem_ld_x16(tm_s + c0 + c, v + c);
+                tmem_ld_wait();
+                if (need_mask) {
+#pragma unroll
+                    for (int i = 0; i < kBK / 2; ++i)
+                        if (!(c0 + i >= lo && c0 + i < hi)) v[i] = __float_as_uint(-CUDART_INF_F);
                 }
-            } else {
+            };
+            half_row(kBK / 2);
 #pragma unroll
-                for (int i = 0; i < kBK; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
-            }
+            for (int i = 0; i < kBK / 2; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
+            half_row(0);
+#pragma unroll
+            for (int i = 0; i < kBK / 2; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
             const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
             // raise the running maximum only when the tile exceeds it by a factor of 2^8; the rescale of O is warp-collective.
             // (S of this tile is there, so the PV product of the tile before has retired and O may be touched.)
@@ -618,13 +620,13 @@ pa_prefill_duo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 const float factor = !raise ? 1.f : (m_used == -CUDART_INF_F ? 0.f : fast_exp2(m_used - m_tile));
                 if (j > 0) {
 #pragma unroll 1
-                    for (int c = 0; c < D; c += 16) {
-                        uint32_t o[16];
-                        tmem_ld_x16(tm_o + c, o);
+                    for (int c = 0; c < D; c += 8) {             // (eight columns at a time: the row of S is in registers)
+                        uint32_t o[8];
+                        tmem_ld_x8(tm_s + (TM_O - TM_S) + c, o);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
-                        tmem_st_x16(tm_o + c, o);
+                        for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+                        tmem_st_x8(tm_s + (TM_O - TM_S) + c, o);
                     }
                     tmem_st_wait();
                 }
@@ -635,16 +637,24 @@ pa_prefill_duo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             }
             const float neg_m = (m_used == -CUDART_INF_F) ? 0.f : -m_used;
             float ls[4] = {0.f, 0.f, 0.f, 0.f};
+            auto half_p = [&](int c0) {                  // P takes half the columns of S: those of the lower half first
 #pragma unroll
-            for (int i = 0; i < kBK; i += 2) {
-                const float e0 = fast_exp2(fmaf(__uint_as_float(v[i]), p.scale_log2, neg_m));
-                const float e1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, neg_m));
-                ls[(i >> 1) & 3] += e0 + e1;
-                v[i >> 1] = pack16<false>(e0, e1);
-            }
+                for (int c = 0; c < kBK / 4; c += 16) {
+                    uint32_t pk[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const float e0 = fast_exp2(fmaf(__uint_as_float(v[2 * (c + i)]), p.scale_log2, neg_m));
+                        const float e1 = fast_exp2(fmaf(__uint_as_float(v[2 * (c + i) + 1]), p.scale_log2, neg_m));
+                        ls[i & 3] += e0 + e1;
+                        pk[i] = pack16<false>(e0, e1);
+                    }
+                    tmem_st_x16(tm_s + c0 + c, pk);
+                }
+            };
+            half_p(0);
+            half_row(kBK / 2);
+            half_p(kBK / 4);
             l_sum += (ls[0] + ls[1]) + (ls[2] + ls[3]);
-#pragma unroll
-            for (int c = 0; c < kBK / 2; c += 16) tmem_st_x16(tm_s + c, v + c);
             tmem_st_wait();
             tc_fence_before_sync();
             mbar_arrive(&p_full[x]);
@@ -653,11 +663,17 @@ pa_prefill_duo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (ok) {
             tc_fence_after_sync();
             const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
-            uint8_t* dst = reinterpret_cast<uint8_t*>(p.out) + ((size_t)(tok_begin + tq0 + tl) * p.ldo + (size_t)(h * G + g) * p.o_head) * 2;
+            uint32_t tid;                                // all of this is read again: nothing of it is kept through the loop
+            asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+            const int b2 = *reinterpret_cast<volatile int*>(s_work), tq = *reinterpret_cast<volatile int*>(s_work + 1) * 2 * TOK;
+            const int begin = __ldg(p.subsequence_begins + b2), len = __ldg(p.subsequence_begins + b2 + 1) - begin;
+            const int r = tid & 127, g = r / TOK, tl = (int)(tid >> 7) * TOK + r % TOK;
+            const bool row_valid = tq + tl < len;
+            uint8_t* dst = reinterpret_cast<uint8_t*>(p.out) + ((size_t)(begin + tq + tl) * p.ldo + (size_t)((int)blockIdx.y * G + g) * p.o_head) * 2;
 #pragma unroll
             for (int c = 0; c < D; c += 16) {
                 uint32_t o[16];
-                tmem_ld_x16(tm_o + c, o);
+                tmem_ld_x16(tm_s + (TM_O - TM_S) + c, o);
                 tmem_ld_wait();
                 if (row_valid) {
                     uint32_t w[8];
