@@ -37,8 +37,8 @@ namespace ovb {
 
 // Warp roles: warp 0 weight producer, warp 1 MMA issuer, warps 2 .. 2+NDQ-1 dequantisation and epilogue, the last warp
 // token-tile producer (quantised modes). The kernel is written for NDQ = 8 or 16; measurements on B200 favour 8 with two
-// CTAs per SM for decode-sized quantised problems: the MMA-issuing warp, not the expansion arithmetic, is what limits
-// a CTA there (its instructions issue several times slower while the dequant warps run), and two CTAs bring two issuers.
+// CTAs per SM for decode-sized quantised problems: what limits an SM there is the issue of the expansion's instructions (65 % of the
+// slots busy, no pipe above 50 %), and a second CTA works while the first one waits for its barriers.
 constexpr int num_dq_warps(int bt, int wmode) { (void)bt; (void)wmode; return 8; }
 constexpr int gemm_threads(int bt, int wmode) { return (3 + num_dq_warps(bt, wmode)) * 32; }
 #ifndef OVB_GEMM_DIRECT
