@@ -486,7 +486,7 @@ static bool pair_shape(const ovb_gemm_args* a) {
 
 bool gemm_pair_takes(const ovb_gemm_args* a) {
     if (!pair_shape(a)) return false;
-    return !is_quant(a->wmode) || (a->scratch != nullptr && a->scratch_bytes >= (int64_t)256 * a->K * 2);
+    return !is_quant(a->wmode) || (a->scratch != nullptr && (reinterpret_cast<uintptr_t>(a->scratch) & 15) == 0 && a->scratch_bytes >= (int64_t)256 * a->K * 2);
 }
 
 template <bool F16>

@@ -1464,6 +1464,12 @@ int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream_) {
     OVB_REQUIRE(a && a->x && a->w && a->out, "ovb_gemm: null operand");
     OVB_REQUIRE(a->T > 0 && a->N > 0 && a->K > 0, "ovb_gemm: empty problem T=%d N=%d K=%d", a->T, a->N, a->K);
     OVB_REQUIRE(a->K % 8 == 0 && a->ldx % 8 == 0, "ovb_gemm: K and ldx must be multiples of 8 (TMA 16-byte rule)");
+    // what every kernel relies on, those of few and of many tokens too: they read weights with 16-byte loads where this file's kernel
+    // makes a tensor map, whose encoding would refuse a misaligned base
+    OVB_REQUIRE(a->wmode == OVB_W_BF16 || a->wmode == OVB_W_F16 || is_quant(a->wmode), "ovb_gemm: unknown wmode %d", a->wmode);
+    OVB_REQUIRE(a->block_t == 0 || a->block_t == 16 || a->block_t == 32 || a->block_t == 64 || a->block_t == 128 || a->block_t == 256,
+                "unsupported block_t %d", a->block_t);
+    OVB_REQUIRE(((reinterpret_cast<uintptr_t>(a->x) | reinterpret_cast<uintptr_t>(a->w)) & 15) == 0, "ovb_gemm: x and weights must be 16-byte aligned");
     const bool f16 = a->wmode == OVB_W_F16;
     const bool quant = is_quant(a->wmode);
     if (quant) {

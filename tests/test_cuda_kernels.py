@@ -858,3 +858,33 @@ def test_gemm_stream_fp16_and_window(ops):
     x = torch.randn(5, 256, device="cuda", dtype=torch.float16)
     w = _pair_weight(ops, "dense", 512, 1024, torch.float16).window(128, 256, 320, 256)
     assert _rel_err(ops.gemm(x, w), ops.gemm(x, w, block_t=16)) < PAIR_REL
+
+
+@pytest.mark.parametrize("T", [1, 5, 300, 1024])
+def test_gemm_refuses_what_it_cannot_read(ops, T):
+    """Misaligned operands, unknown weight formats and unknown token tiles are errors of the call at every size, whichever kernel the
+    size belongs to; scratch memory that cannot be used is not."""
+    import ctypes as C
+    N, K = 1280, 256
+    x = torch.randn(T, K, device="cuda", dtype=torch.bfloat16)
+    w = _pair_weight(ops, "u8", N, K)
+    room = torch.empty(N * K + 16, dtype=torch.uint8, device="cuda")
+    room[1:N * K + 1] = w.w.reshape(-1)
+    off = ops.PackedWeight(ops.W_U8, room[1:N * K + 1].reshape(N, K), N, K, w.scales, None, 128)
+    dense = _pair_weight(ops, "dense", N, K)
+    xoff = torch.empty(T * K + 1, device="cuda", dtype=torch.bfloat16)[1:].reshape(T, K)
+    for bad in (lambda: ops.gemm(x, off), lambda: ops.gemm(xoff, w), lambda: ops.gemm(xoff, dense), lambda: ops.gemm(x, dense, block_t=200),
+                lambda: ops.gemm(x, ops.PackedWeight(7, dense.w, N, K, tiled=True))):
+        with pytest.raises(ops.KernelLibraryError):
+            bad()
+    with pytest.raises(ops.KernelLibraryError):
+        ops.gemm_grouped(x, dense, torch.tensor([0, T], dtype=torch.int32, device="cuda"), 1, 1, torch.empty(T, N, device="cuda", dtype=torch.bfloat16), block_t=200)
+    a = ops.GemmArgs()
+    out = torch.empty(T, N, device="cuda", dtype=torch.bfloat16)
+    scratch = torch.empty((16 << 20) + 16, dtype=torch.uint8, device="cuda")
+    a.x, a.w, a.out, a.scales = x.data_ptr(), w.w.data_ptr(), out.data_ptr(), w.scales.data_ptr()
+    a.T, a.N, a.K, a.ldx, a.ldo, a.group_size, a.wmode = T, N, K, K, N, 128, ops.W_U8
+    a.scratch, a.scratch_bytes = scratch.data_ptr() + 8, 16 << 20
+    assert ops.lib().ovb_gemm(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    assert _rel_err(out, ops.gemm(x, w, block_t=64)) < PAIR_REL
+    ops.check_status("gemm")
