@@ -213,15 +213,32 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const E* __restr
         if (lane >= o) upto += up;
     }
     const float total = __shfl_sync(0xffffffffu, upto, 31);
-    const float mine = __shfl_sync(0xffffffffu, upto, warp);
-    const float below = __shfl_sync(0xffffffffu, upto, max(warp - 1, 0));
-    const float before = warp ? below : 0.f;
     const uint64_t r64 = mix64(seed ^ mix64(((uint64_t)(step_ptr ? *step_ptr : 0) << 20) ^ (uint64_t)row));
-    const float u = (float)((r64 >> 40) + 0.5) * (1.0f / 16777216.0f);      // (0, 1)
+    const float u = (float)((r64 >> 40) + 0.5) * (1.0f / 16777216.0f);      // (0, 1], the last value rounds to 1
     const float target = u * total;
-    if (target > before && target <= mine && local > 0.f) {
+    // One warp draws, and every warp finds the same one: the first with kept mass whose prefix reaches the target. The prefixes are sums
+    // in different orders, so they may fall by a unit in the last place from a warp to the next, and the total may lie above the last
+    // kept warp's: a target in such a gap belongs to the last warp with kept mass.
+    const bool has = part_mass[turn][lane] > 0.f;
+    const uint32_t kept = __ballot_sync(0xffffffffu, has), reach = __ballot_sync(0xffffffffu, has && target <= upto);
+    const int owner = reach ? __ffs(reach) - 1 : 31 - __clz(kept);          // -1: no mass at all
+    const float below = __shfl_sync(0xffffffffu, upto, max(owner - 1, 0));
+    const float before = owner > 0 ? below : 0.f;
+    if (owner < 0) {                    // no distribution to draw from (NaN or infinite logits): the first of the largest entries
+        int best = V;
+        each([&](const float* x, int v) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (v + j < v1 && x[j] == mx) best = min(best, v + j);
+        });
+        best = __reduce_min_sync(0xffffffffu, best);
+        if (lane == 0) part_cnt[turn][warp] = best;
+        __syncthreads();
+        best = __reduce_min_sync(0xffffffffu, part_cnt[turn][lane]);
+        if (threadIdx.x == 0) out_ids[row] = best < V ? best : 0;
+    } else if (warp == owner) {
         float acc = before;
-        int pick = -1, last = -1;       // last: the last kept entry, for a target that the rounding of the sums puts past it
+        int pick = -1, last = -1;       // last: the last entry with mass, for a target that the rounding of the sums puts past it
         for (int base = v0; base < v1 && pick < 0; base += 256) {
             const int v = base + lane * 8;
             float x[8];
@@ -229,8 +246,10 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const E* __restr
             float own = 0.f;
             int own_last = -1;
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (v + j < v1 && x[j] >= thr) { own += __expf((x[j] - mx) * inv_temp); own_last = v + j; }
+            for (int j = 0; j < 8; ++j) {
+                const float e = v + j < v1 && x[j] >= thr ? __expf((x[j] - mx) * inv_temp) : 0.f;
+                if (e > 0.f) { own += e; own_last = v + j; }
+            }
             float incl = own;
             for (int o = 1; o < 32; o <<= 1) {
                 const float up = __shfl_up_sync(0xffffffffu, incl, o);
@@ -244,12 +263,14 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const E* __restr
                     float a = acc + (lane ? left : 0.f);
                     bool done = false;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (!done && v + j < v1 && x[j] >= thr) {
-                            a += __expf((x[j] - mx) * inv_temp);
+                    for (int j = 0; j < 8; ++j) {
+                        const float e = v + j < v1 && x[j] >= thr ? __expf((x[j] - mx) * inv_temp) : 0.f;
+                        if (!done && e > 0.f) {
+                            a += e;
                             pick = v + j;
                             done = a >= target;
                         }
+                    }
                 }
                 pick = __shfl_sync(0xffffffffu, pick, who);
             } else {

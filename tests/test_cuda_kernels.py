@@ -607,6 +607,55 @@ def test_sampling_kernel_draws(ops, V, ld, dtype, top_k, top_p):
         assert int(got[i]) in want, (i, int(got[i]), want)
 
 
+def _seed_for(u_bits: int, step: int, index: int = 0) -> int:
+    """The seed with which row ``index`` of a step draws u = (u_bits + 0.5) / 2^24 (the mixing function is a bijection)."""
+    M = (1 << 64) - 1
+    def mix(z):
+        z = (z + 0x9E3779B97F4A7C15) & M
+        z = ((z ^ (z >> 30)) * 0xBF58476D1CE4E5B9) & M
+        z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & M
+        return z ^ (z >> 31)
+    def unshift(z, s):
+        x = z
+        for _ in range(64 // s + 1):
+            x = z ^ (x >> s)
+        return x
+    z = unshift(u_bits << 40, 31)
+    z = unshift(z * pow(0x94D049BB133111EB, -1, 1 << 64) & M, 27)
+    z = unshift(z * pow(0xBF58476D1CE4E5B9, -1, 1 << 64) & M, 30)
+    seed = ((z - 0x9E3779B97F4A7C15) & M) ^ mix((step << 20) ^ index)
+    assert mix(seed ^ mix((step << 20) ^ index)) == u_bits << 40
+    return seed
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_sampling_kernel_always_draws(ops, dtype):
+    """The largest random number (1 after rounding) and others, with a handful of kept entries spread over the row: the fp32 prefixes of
+    the 32 pieces and their total are rounded in different orders, so the target may lie above the last kept piece's prefix. A kept token
+    comes out all the same, and a row without a distribution gives its largest entry."""
+    V, step = 32000, torch.tensor([3], dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(4)
+    for i in range(150):
+        kept = 3 + i % 17
+        row = torch.full((1, V), -50.0, device="cuda", dtype=dtype)
+        at = torch.randperm(V, device="cuda", generator=g)[:kept]
+        row[0, at] = torch.randn(kept, device="cuda", generator=g).to(dtype)
+        for bits in ((1 << 24) - 1, (1 << 24) - 3, 0):
+            out = torch.full((1,), -7, dtype=torch.int32, device="cuda")
+            ops.sample(row, 0.8, top_k=kept, top_p=1.0, seed=_seed_for(bits, 3), step=step, out=out)
+            got = int(out[0])
+            assert got in set(at.tolist()), (i, bits, got)
+            if bits != 0:       # within 2^-22 of the whole mass: the last kept entry, whatever the rounding
+                assert got == int(at.max()), (i, bits, got)
+    for bad, want in ((float("nan"), 4), (float("inf"), 9000)):
+        row = torch.zeros((1, V), device="cuda", dtype=dtype)
+        row[0, 4], row[0, 9000] = 5.0, bad
+        out = torch.full((1,), -7, dtype=torch.int32, device="cuda")
+        ops.sample(row, 0.8, top_k=50, top_p=0.9, seed=1, step=step, out=out)
+        assert 0 <= int(out[0]) < V and (bad != bad or int(out[0]) == want), int(out[0])
+    ops.check_status("sample")
+
+
 def test_sampling_kernel(ops):
     torch.manual_seed(11)
     V = 1000
