@@ -122,7 +122,9 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const E* __restr
     float thr = -INFINITY;
     if (restrict_k || restrict_p) {
         // bisection on the threshold: keep(lo) is never smaller than the wanted set, keep(hi) may be
-        float lo = mn, hi = mx, z = 0.f;
+        // An entry more than 104 temperatures below the largest has no mass (e^-104 < 2^-149), so the range ends there: masked entries
+        // (-inf, or the type's lowest value) would otherwise hold the bisection off the entries that count.
+        float lo = fmaxf(mn, mx - 104.f / inv_temp), hi = mx, z = 0.f;
         int it = 0, most = V;            // most: largest number of entries >= lo in a warp's piece
         for (; it < 26 && most > kListWarp; ++it) {
             const float mid = 0.5f * (lo + hi);

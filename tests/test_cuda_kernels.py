@@ -607,6 +607,24 @@ def test_sampling_kernel_draws(ops, V, ld, dtype, top_k, top_p):
         assert int(got[i]) in want, (i, int(got[i]), want)
 
 
+@pytest.mark.parametrize("V", [130, 50257])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_sampling_kernel_masked_logits(ops, V, dtype):
+    """Masked entries (-inf, the type's lowest value) and entries far below the rest leave top-k and top-p as they are."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    for fill in (float("-inf"), torch.finfo(dtype).min, -1e30, -3000.0):
+        row = (torch.randn(1, V, device="cuda", generator=g) * 2).to(dtype)
+        row[0, torch.randperm(V, device="cuda", generator=g)[:V // 2]] = fill
+        for top_k, top_p in ((5, 1.0), (0, 0.3), (5, 0.5)):
+            for step in range(24):
+                got = int(ops.sample(row, 0.8, top_k=top_k, top_p=top_p, seed=9, step=torch.tensor([step], dtype=torch.int32, device="cuda"))[0])
+                assert got in _expected_draw(np.nan_to_num(row[0].float().cpu().numpy(), neginf=-1e30), 0.8, top_k, top_p, 9, step, 0), (fill, top_k, top_p, step)
+    few = torch.full((1, V), float("-inf"), device="cuda", dtype=dtype)      # fewer entries than top-k
+    few[0, 3], few[0, V - 1] = 1.0, 0.5
+    assert {int(ops.sample(few, 1.0, top_k=40, top_p=1.0, seed=s)[0]) for s in range(64)} == {3, V - 1}
+    ops.check_status("sample")
+
+
 def _seed_for(u_bits: int, step: int, index: int = 0) -> int:
     """The seed with which row ``index`` of a step draws u = (u_bits + 0.5) / 2^24 (the mixing function is a bijection)."""
     M = (1 << 64) - 1
