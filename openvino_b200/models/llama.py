@@ -38,18 +38,20 @@ def random_float_state(cfg: LlmConfig, seed: int = 0, device="cpu", std: float =
     return st
 
 
-def effective_state(cfg: LlmConfig, state: Dict[str, torch.Tensor]) -> Dict[str, torch.Tensor]:
+def effective_state(cfg: LlmConfig, state: Dict[str, torch.Tensor], scale_dtype: torch.dtype = torch.float16) -> Dict[str, torch.Tensor]:
     """The weights the compressed model actually computes with: linear weights quantised and
-    dequantised per cfg.weight_format, norms/embeddings rounded to bf16."""
+    dequantised per cfg.weight_format, norms/embeddings rounded to bf16. ``scale_dtype``: how the group scales are kept, fp16 in the IR,
+    bf16 in the tables of the CUDA kernels."""
     from ..utils import quant
     out = {}
     for k, v in state.items():
         if v.dim() == 2 and not k.endswith("embed_tokens") and not k.endswith("router"):
             if cfg.weight_format == "int4":
                 q, s, z = quant.quantize_u4_asym(v, cfg.group_size)
-                out[k] = quant.dequantize_u4(q, s, z, cfg.group_size)
+                out[k] = quant.dequantize_u4(q, s.to(scale_dtype), z, cfg.group_size)
             elif cfg.weight_format == "int8":
                 q, s, z = quant.quantize_u8_asym(v, cfg.group_size)
+                s = s.to(scale_dtype)
                 N, Kd = v.shape
                 out[k] = ((q.float().reshape(N, -1, cfg.group_size) - z.float().unsqueeze(-1)) * s.float().unsqueeze(-1)).reshape(N, Kd)
             else:
