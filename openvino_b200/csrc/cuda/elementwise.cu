@@ -506,8 +506,9 @@ __global__ void rope_kv_write_vec_kernel(__nv_bfloat16* __restrict__ qkv, const 
                         const int hh = h + 4 * i;
                         __nv_bfloat16* dst = (hh >= Hq ? k_cache + (((size_t)blk * Hkv + (hh - Hq)) * block_size + off) * D : row + hh * D) + d;
                         const float2 a = __bfloat1622float2(a2[i]), b = __bfloat1622float2(b2[i]);
-                        *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(a.x * c0 - b.x * s0, a.y * c1 - b.y * s1);
-                        *reinterpret_cast<__nv_bfloat162*>(dst + half) = __floats2bfloat162_rn(b.x * c0 + a.x * s0, b.y * c1 + a.y * s1);
+                        // which product of a sum is fused is written out: left to the compiler it changes with the loop around it
+                        *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(fmaf(a.x, c0, -__fmul_rn(b.x, s0)), fmaf(a.y, c1, -__fmul_rn(b.y, s1)));
+                        *reinterpret_cast<__nv_bfloat162*>(dst + half) = __floats2bfloat162_rn(fmaf(a.x, s0, __fmul_rn(b.x, c0)), fmaf(b.y, c1, __fmul_rn(a.y, s1)));
                     }
             }
         }

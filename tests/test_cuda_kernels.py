@@ -955,3 +955,25 @@ def test_gemm_refuses_what_it_cannot_read(ops, T):
     assert ops.lib().ovb_gemm(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
     assert _rel_err(out, ops.gemm(x, w, block_t=64)) < PAIR_REL
     ops.check_status("gemm")
+
+
+@pytest.mark.parametrize("T", [1, 64, 200, 700])
+def test_rotation_rounds_the_same_at_every_size(ops, T):
+    """Bit for bit the rounding that the fused multiply-adds of the kernel name, however many heads a block takes."""
+    D, Hq, Hkv, theta, dev = 128, 32, 8, 500000.0, "cuda"
+    g = torch.Generator(device=dev).manual_seed(T)
+    qkv = torch.randn(T, (Hq + 2 * Hkv) * D, device=dev, generator=g).bfloat16()
+    pos = torch.arange(T, device=dev, dtype=torch.int32) + 500
+    kc, vc = (torch.zeros(64, Hkv, 16, D, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    x = qkv.reshape(T, -1, D)[:, :Hq + Hkv].clone()
+    ops.rope_kv_write(qkv, pos, torch.arange(T, device=dev, dtype=torch.int32), kc, vc, Hq, Hkv, D, theta, 16)
+    ops.check_status("rope")
+    d = torch.arange(D // 2, device=dev, dtype=torch.float32)
+    log2_theta = torch.tensor(theta, dtype=torch.float32).log2().to(dev)
+    ang = pos.float()[:, None] * torch.exp2(-log2_theta * (2.0 * d / D))
+    a, b, c, s = x[..., :D // 2].double(), x[..., D // 2:].double(), ang.cos().double()[:, None], ang.sin().double()[:, None]
+    r = lambda v: v.float().double()                         # a product rounded to fp32; a fused sum is exact in 64 bits up to a last rounding
+    lo = (a * c - r(b * s)).float().bfloat16()
+    hi = torch.where((d % 2 == 0)[None, None], a * s + r(b * c), b * c + r(a * s)).float().bfloat16()
+    got = torch.cat([qkv.reshape(T, -1, D)[:, :Hq], kc.permute(0, 2, 1, 3).reshape(-1, Hkv, D)[:T]], 1)
+    assert torch.equal(got, torch.cat([lo, hi], -1))
