@@ -33,16 +33,64 @@ __device__ __forceinline__ __half from_float<__half>(float v) {
 // cap * tanh(v / cap); the error is of the order of an ulp of cap.
 __device__ __forceinline__ float soft_cap(float v, float cap) { return cap - __fdividef(2.0f * cap, 1.0f + __expf(__fdividef(2.0f * v, cap))); }
 
-// v * Phi(v) with erfc by Abramowitz and Stegun 7.1.26 (absolute error below 1.5e-7; the largest error of the result over [-12, 12] is
-// 3.3e-7, with erff and 1 + erf it is 4.5e-7). Two special-function instructions and a dozen FMAs instead of erff's two branches:
-// at K = 1024 the epilogue, not the products, set the time.
-// 6144 x 4096 x 1024 in fp16 (gemm_pair.cu): 148 us with erff in sixteen copies of the switch, 141 us with this, and see apply_act_n.
+// Two fp32 values in a register pair: one instruction for both.
+__device__ __forceinline__ uint64_t pair_of(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t pair_of(float a) { return pair_of(a, a); }
+__device__ __forceinline__ void unpair(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// v * Phi(v) of two values. With x = |v| and h = Phi(-x) it is max(v, 0) - x h: no cancellation for positive v, and for negative v none
+// that h does not have. h = 1/2 - x P(x^2) up to 1.6, exp(-x^2 / 2) Q(x) above (from 5.5 on, where h < 2e-8, with Q(5.5)). P and Q are
+// minimax fits (Lawson's iteration on Chebyshev nodes): P - a0, of degree 6, within 3e-9 of (Phi(x) - 1/2) / x; Q, of degree 7, such that
+// h is within 3e-9. Error against 64 bits, rms (largest): v in (0.01, 3) 2.9e-8 (1.1e-7) of the value, 0.5 v (1 + erff(v / sqrt 2))
+// has 3.8e-8 (1.3e-7); (-1, -0.01) 4.2e-8 (1.5e-7), there 5.0e-8 (2.2e-7); (-2, -1) 1.4e-7 (6.9e-7), there 1.9e-7 (1.0e-6).
+// The epilogue's instructions set the time of short products: 6144 x 4096 x 1024 in fp16, cold caches, 102 us with erff, 76 us with this (58 us
+// without an activation; erfc by Abramowitz and Stegun 7.1.26, four times as far off as erff over (0.01, 3), 78 us).
+__device__ __forceinline__ void gelu_erf2(float& v0, float& v1) {
+    const uint64_t v = pair_of(v0, v1), s = mul2(v, v);
+    const uint64_t nx = pair_of(fmaxf(-fabsf(v0), -5.5f), fmaxf(-fabsf(v1), -5.5f));      // -x
+    uint64_t p = pair_of(3.88307512e-07f);
+    p = fma2(p, s, pair_of(-8.56560655e-06f));
+    p = fma2(p, s, pair_of(0.000113983522f));
+    p = fma2(p, s, pair_of(-0.00118607341f));
+    p = fma2(p, s, pair_of(0.00997303519f));
+    p = fma2(p, s, pair_of(-0.0664903f));
+    p = fma2(p, s, pair_of(-1.34248355e-08f));
+    uint64_t q = pair_of(1.29784776e-05f);
+    q = fma2(q, nx, pair_of(0.000298278086f));
+    q = fma2(q, nx, pair_of(0.00303096278f));
+    q = fma2(q, nx, pair_of(0.0180309042f));
+    q = fma2(q, nx, pair_of(0.0701728687f));
+    q = fma2(q, nx, pair_of(0.189219281f));
+    q = fma2(q, nx, pair_of(0.363507748f));
+    q = fma2(q, nx, pair_of(0.490691155f));
+    float h0, h1, a0, a1, e0, e1;
+    unpair(fma2(nx, p, fma2(nx, pair_of(0.398942292f), pair_of(0.5f))), a0, a1);
+    unpair(mul2(s, pair_of(-0.72134752f)), e0, e1);
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e0));
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(e1));
+    unpair(mul2(pair_of(e0, e1), q), h0, h1);
+    if (fabsf(v0) <= 1.6f) h0 = a0;                    // (NaN takes the other branch and stays)
+    if (fabsf(v1) <= 1.6f) h1 = a1;
+    unpair(fma2(nx, pair_of(h0, h1), pair_of(fmaxf(v0, 0.f), fmaxf(v1, 0.f))), v0, v1);
+}
 __device__ __forceinline__ float gelu_erf(float v) {
-    const float z = fminf(fabsf(v), 30.f) * 0.70710678118654752f;       // bounded: 0 * inf below would be NaN
-    const float t = __fdividef(1.f, fmaf(0.3275911f, z, 1.f));
-    const float poly = t * fmaf(t, fmaf(t, fmaf(t, fmaf(t, 1.061405429f, -1.453152027f), 1.421413741f), -0.284496736f), 0.254829592f);
-    const float h = z * 0.70710678118654752f * poly * __expf(-z * z);   // |v| / 2 * erfc(z)
-    return v < 0.f ? -h : v - h;
+    float other = 0.f;
+    gelu_erf2(v, other);
+    return v;
 }
 
 // Activations of the epilogue; P carries `act` and the limits of the GEMM's arguments.
@@ -65,11 +113,12 @@ __device__ __forceinline__ float apply_act(float v, const P& p) {
 // The same for N values. The choice is outside the loop: sixteen unrolled copies of the switch do not fit the instruction cache.
 template <int N, class P>
 __device__ __forceinline__ void apply_act_n(float (&v)[N], const P& p) {
+    static_assert(N % 2 == 0, "pairs");
     switch (p.act) {
         case OVB_ACT_NONE: break;
         case OVB_ACT_GELU_ERF:
 #pragma unroll
-            for (int j = 0; j < N; ++j) v[j] = gelu_erf(v[j]);
+            for (int j = 0; j < N; j += 2) gelu_erf2(v[j], v[j + 1]);
             break;
         case OVB_ACT_SILU:
 #pragma unroll

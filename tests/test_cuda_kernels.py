@@ -821,8 +821,8 @@ def test_paged_attention_long_prompts(ops, q_lens, past_lens, Hq, Hkv, window):
 
 
 def test_gelu_epilogue_range(ops):
-    """The erf form of GELU over its range, infinities and NaN, against 64 bits: 3.3e-7 of the function itself (its two special
-    functions and fp32 sums), two units in the last place of the fp32 product before it."""
+    """The erf form of GELU over its range, infinities and NaN, against 64 bits: absolutely, and relative to the result where that is
+    of the size of an activation: erff is good to two units in the last place, its argument and 1 + erf to half a unit each."""
     v = torch.cat([torch.linspace(-12, 12, 4093), torch.tensor([float("inf"), float("-inf"), float("nan")])]).cuda().to(torch.bfloat16)
     for T, kw in ((300, {}), (300, {"block_t": 64}), (5, {})):
         x = torch.zeros(T, 128, device="cuda", dtype=torch.bfloat16)
@@ -832,7 +832,32 @@ def test_gelu_epilogue_range(ops):
         got = ops.gemm(x, ops.PackedWeight.from_dense(w), act=ops.ACT_GELU_ERF, out_f32=True, **kw)[3].double()
         want = 0.5 * v.double() * torch.special.erfc(-v.double() * math.sqrt(0.5))
         assert (got[:4093] - want[:4093]).abs().max() < 1e-6
+        z = v[:4093].double() * math.sqrt(0.5)
+        erf = torch.special.erf(z)
+        bound = (2.0 ** -22 * erf.abs() + z.abs() * torch.exp(-z * z) * 2 / math.sqrt(math.pi) * 2.0 ** -23 + 2.0 ** -24) / (1 + erf) + 2.0 ** -23
+        off = ((got[:4093] - want[:4093]).abs() / want[:4093].abs().clamp_min(1e-30))[z > -2]
+        assert (off <= bound[z > -2]).all(), (off / bound[z > -2]).max()
         assert got[4093] == float("inf") and got[4094] == 0 and got[4095].isnan()
+
+
+@pytest.mark.parametrize("T,kw", [(300, {}), (300, {"block_t": 64}), (5, {})])
+def test_gelu_epilogue_is_no_further_off_than_the_library_function(ops, T, kw):
+    """Per range of arguments, largest and mean error relative to the result: at most that of 0.5 v (1 + erf(v / sqrt 2)) in fp32."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.zeros(T, 128, device="cuda", dtype=torch.bfloat16)
+    x[:, 0], x[:, 1] = 1.0, 2.0 ** -8
+    w = torch.zeros(65536, 128, device="cuda", dtype=torch.bfloat16)
+    w[:, 0] = (torch.randn(65536, device="cuda", generator=g) * 1.5).bfloat16()
+    w[:, 1] = torch.randn(65536, device="cuda", generator=g).bfloat16()
+    pw = ops.PackedWeight.from_dense(w)
+    v = ops.gemm(x, pw, out_f32=True, **kw)[3]                   # two exact products: the argument as the epilogue has it
+    got = ops.gemm(x, pw, act=ops.ACT_GELU_ERF, out_f32=True, **kw)[3]
+    plain = 0.5 * v * (1 + torch.erf(v * math.sqrt(0.5)))
+    want = 0.5 * v.double() * torch.special.erfc(-v.double() * math.sqrt(0.5))
+    for lo, hi in ((0.01, 1), (1, 3), (3, 9), (-1, -0.01), (-2, -1), (-3, -2), (-4, -3)):
+        at = (v > lo) & (v < hi)
+        here, lib = (((y.double() - want).abs() / want.abs())[at] for y in (got, plain))
+        assert at.sum() > 50 and here.max() <= lib.max() and here.square().mean() <= lib.square().mean(), (lo, hi, here.max(), lib.max(), here.mean(), lib.mean())
 
 
 @pytest.mark.parametrize("fmt", ["u4", "u8", "f8"])
