@@ -765,6 +765,8 @@ extern "C" int ovb_debug_set_limits_attention(const ovb::DebugLimits* l) {
 extern "C" {
 using namespace ovb;
 
+int ovb_pa_two_query_tiles(int T, int B, int Hq, int Hkv) { return T > 0 && B > 0 && Hkv > 0 && Hq >= Hkv && ovb::two_query_tiles(T, B, Hq / Hkv, Hkv); }
+
 int64_t ovb_pa_scratch_bytes(int B, int Hq, int D, int max_context_len) {
     (void)max_context_len;
     return (int64_t)B * Hq * 32 * (D + 2) * (int64_t)sizeof(float);

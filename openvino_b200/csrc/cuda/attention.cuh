@@ -67,6 +67,8 @@ __host__ __device__ inline int latent_first_key(int past, int window) {
 // tcgen05 / TMA prefill and dense attention (attention_sm100.cu). Returns a negative code when the shape is not one it
 // serves (the caller then uses the mma.sync kernel): head size 64 or 128, 16-key pages, 1, 2, 4 or 8 query heads per KV head.
 int launch_prefill_tc(const PaKParams& p, int D, int G, bool paged, bool f16, int num_q_tiles, cudaStream_t stream);
+// Does a step of T tokens in B sequences run two query tiles per CTA? (paged 16-bit cache, head size 128, G query heads per KV head)
+bool two_query_tiles(int T, int B, int G, int Hkv);
 // The same kernel with key and value sizes of their own (up to three and two 64-column parts) and any group size up to 16; bf16.
 // dk, dv: padded sizes (multiples of 16). dshared > 0: latent attention with expanded heads (PaKParams::kv_rows).
 int launch_window_tc(PaKParams p, int dk, int dshared, int dv, cudaStream_t stream);

@@ -413,8 +413,10 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // works on the other's products, and both share the K and V tiles in shared memory (half the reads). Tensor memory is full with
 // S and O of the two tiles (4 x 128 columns), so P overwrites the first half of its S, and the next QK product of a tile is issued
 // after the PV product that reads P has retired. K and V stages are released on their own: K as soon as both QK products have
-// read it, so that the next tile but one is on its way a whole turn earlier.
-// 1 x 8191 tokens, 32 query and 8 KV heads, at the clock of a prefill step: 1084 us with one tile per CTA, 753 us here.
+// read it, so that the next tile but one is on its way a whole turn earlier. A CTA whose second tile has no rows (a sequence's odd last
+// tile, a decoding sequence) works on the first alone, one product after the other.
+// One launch, cold caches, 32 query and 8 KV heads: 1 x 8191 tokens 873 us with one tile per CTA, 592 us here; 8 x 1024 198 and 139 us;
+// 40 decoding sequences beside 2048 prompt tokens 149 and 132 us.
 constexpr int kDuoThreads = 320;
 
 template <int G>
@@ -489,6 +491,7 @@ pa_prefill_duo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const int blk_begin = p.block_indices_begins[b];
     const int tq0 = s_work[1] * 2 * TOK;
     const int tq1 = min(q_len, tq0 + 2 * TOK);
+    const int nq = tq0 + TOK < q_len ? 2 : 1;                   // query tiles with rows: one at the end of a sequence, or in a decoding one
     const int kv_end = p.causal ? past + tq1 : past + q_len;
     const int kv_start = first_visible_key(past + tq0, p.sliding_window, p.chunk) / kBK * kBK;
     const int ntiles = (kv_end - kv_start + kBK - 1) / kBK;
@@ -496,8 +499,8 @@ pa_prefill_duo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (warp == 8) {
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
-            mbar_arrive_expect_tx(q_full, 2 * G * TOK * D * 2);
-            for (int x = 0; x < 2; ++x)
+            mbar_arrive_expect_tx(q_full, nq * G * TOK * D * 2);
+            for (int x = 0; x < nq; ++x)
                 for (int g = 0; g < G; ++g)
                     for (int hf = 0; hf < 2; ++hf)
                         tma_load_2d(sQ + x * T_BYTES + hf * (kBM * 128) + g * (TOK * 128), &tmQ, q_full, (h * G + g) * p.q_head + hf * 64, tok_begin + tq0 + x * TOK);
@@ -538,7 +541,7 @@ pa_prefill_duo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (ok) {
             tc_fence_after_sync();
             qk(0, 0);
-            qk(1, 0);
+            if (nq == 2) qk(1, 0);
             umma_commit_elect(&k_empty[0]);
         }
         for (int j = 0; j < ntiles && ok; ++j) {
@@ -547,6 +550,7 @@ pa_prefill_duo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             const int ksteps = (min(kBK, kv_end - (kv_start + j * kBK)) + 15) / 16;
             const uint64_t dv = umma_desc_mn_sw128(smem_u32(sV + st * T_BYTES), kBK * 128, 1024);
             for (int x = 0; x < 2 && ok; ++x) {
+                if (x >= nq) break;
                 if (x == 0) ok = mbar_wait(&v_full[st], (j >> 1) & 1, abort_flag, status);
                 ok = ok && mbar_wait(&p_full[x], par, abort_flag, status);
                 if (!ok) break;
@@ -554,19 +558,19 @@ pa_prefill_duo_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 for (int kk = 0; kk < ksteps; ++kk)
                     umma_f16_ts_elect(tmem + TM_O + x * 128, tmem + TM_S + x * 128 + kk * 8, dv + (uint64_t)((kk * 16 * 128) >> 4), IDESC_PV, (j > 0 || kk > 0) ? 1u : 0u);
                 umma_commit_elect(&pv_done[x]);
-                if (x == 1) umma_commit_elect(&v_empty[st]);
+                if (x == 1 || nq == 1) umma_commit_elect(&v_empty[st]);
                 if (j + 1 < ntiles) {
                     if (x == 0) ok = mbar_wait(&k_full[nx], ((j + 1) >> 1) & 1, abort_flag, status);
                     ok = ok && mbar_wait(&pv_done[x], par, abort_flag, status);     // P, which QK overwrites, has been read
                     if (!ok) break;
                     tc_fence_after_sync();
                     qk(x, nx);
-                    if (x == 1) umma_commit_elect(&k_empty[nx]);
+                    if (x == 1 || nq == 1) umma_commit_elect(&k_empty[nx]);
                 }
             }
         }
         __syncwarp();
-    } else {
+    } else if ((warp >> 2) < nq) {
         // ------------------------------------------------------------------ softmax: one thread per stacked query row
         const int x = warp >> 2;                         // query tile of this thread
         // keys [lo_row, hi_row) from kv_start on are visible to this row, every row of the query tile sees those of [lo_last, lim). (With
@@ -772,14 +776,23 @@ int launch_tc(PaKParams p, int num_q_tiles, cudaStream_t stream) {
 
 }  // namespace
 
+// Two tiles to a CTA once single tiles would fill the machine twice (fewer are better spread over the SMs), and where the tokens make up
+// as many full tiles as there are sequences. A sequence with one tile gains nothing from the second and takes about 15 % longer in that
+// kernel, a pair of tiles 30 % less. One tile / two (us, cold, 32 and 8 heads, decoding sequences behind 1000 to 1300 tokens): 48 decoding +
+// a portion of 16 tokens 89 / 103, 40 + 512 85 / 93, 40 + 1024 112 / 112, 47 + 2 x 1024 138 / 134, 40 + 2048 149 / 132; 64 x 20 108 / 120,
+// 40 x 33 44 / 36.
+bool two_query_tiles(int T, int B, int G, int Hkv) {
+    const int tok = tile_tokens(G);
+    return (int64_t)(T / tok + B) * Hkv >= 2 * 148 && T - B >= (int64_t)B * tok;
+}
+
 int launch_prefill_tc(const PaKParams& p, int D, int G, bool paged, bool f16, int num_q_tiles, cudaStream_t stream) {
     if (paged && p.block_size != kPage) return ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(p.q) & 15) || (reinterpret_cast<uintptr_t>(p.k_cache) & 15) || (reinterpret_cast<uintptr_t>(p.v_cache) & 15) ||
         (reinterpret_cast<uintptr_t>(p.out) & 15) || p.ldq % 8 != 0 || (!paged && p.ld_kv % 8 != 0))
         return ERR_UNSUPPORTED;
     if (paged && !f16) {
-        // two tiles to a CTA once single tiles would fill the machine twice; fewer are better spread over the SMs
-        if (D == 128 && p.gate == nullptr && p.sink == nullptr && num_q_tiles * p.Hkv >= 2 * 148) {
+        if (D == 128 && p.gate == nullptr && p.sink == nullptr && two_query_tiles(p.T, p.B, G, p.Hkv)) {
             switch (G) {
                 case 1: return launch_duo<1>(p, num_q_tiles, stream);
                 case 2: return launch_duo<2>(p, num_q_tiles, stream);

@@ -265,6 +265,8 @@ typedef struct {
 } ovb_pa_args;
 int ovb_paged_attention(const ovb_pa_args* a, ovb_stream_t stream);
 int64_t ovb_pa_scratch_bytes(int B, int Hq, int D, int max_context_len);
+// 1: a prefill or mixed step of T tokens in B sequences (16-bit cache, head size 128) runs two query tiles per CTA, 0: one.
+int ovb_pa_two_query_tiles(int T, int B, int Hq, int Hkv);
 
 // Dense (non-paged) bidirectional attention for encoder models: q,k,v [B, S, H, D] fp16/bf16.
 int ovb_sdpa_dense(const void* q, const void* k, const void* v, void* out, int B, int S, int H, int D, int ld,

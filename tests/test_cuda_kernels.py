@@ -802,6 +802,9 @@ def test_gemm_pair_fp16_window_and_groups(ops):
     ([1, 2500, 2600], [700, 0, 17], 8, 8, 0),           # one query head per KV head
     ([2049, 511], [0, 1000], 16, 8, 300),               # two query heads; tiles that the window hides from one of the two
     ([700, 33], [100, 0], 64, 8, 0),                    # eight query heads
+    ([1] * 12 + [32, 33, 1500, 64], [40 * i for i in range(12)] + [5, 0, 130, 64], 32, 8, 0),     # CTAs with one tile: decoding rows, a whole tile; one row more
+    ([1] * 5 + [129, 2000, 128], [300 * i for i in range(5)] + [77, 0, 1], 8, 8, 200),            # the same with one query head and a window
+    ([1] * 40 + [64], [17 * i for i in range(40)] + [300], 32, 8, 0),                             # mostly decoding rows: one tile per CTA
 ])
 def test_paged_attention_long_prompts(ops, q_lens, past_lens, Hq, Hkv, window):
     torch.manual_seed(5)

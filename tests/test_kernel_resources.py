@@ -49,3 +49,13 @@ def test_kernels_of_layered_decoders_do_not_spill(gemm, stem):
     words = 16 if stem in ("attention_heads", "delta_rule") else 0
     assert res and all(r["spill_stores"] <= 4 * words and r["stack"] <= 4 * words for r in res.values()), \
         {n: r for n, r in res.items() if r["spill_stores"] or r["stack"]}
+
+
+@pytest.mark.parametrize("T,B,Hq,Hkv,two", [
+    (48 + 16, 49, 32, 8, 0), (40 + 64, 41, 32, 8, 0), (40 + 512, 41, 32, 8, 0), (64 * 20, 64, 32, 8, 0), (30 + 300, 31, 64, 8, 0),     # mostly decoding, short
+    (40 + 2048, 41, 32, 8, 1), (8191, 1, 32, 8, 1), (8 * 1024, 8, 32, 8, 1), (40 * 33, 40, 32, 8, 1), (2048, 1, 64, 8, 1),             # full tiles
+    (1, 1, 32, 8, 0), (1000, 1, 32, 8, 0), (3 * 333, 3, 32, 8, 0),                                                                    # too few tiles
+])
+def test_two_query_tiles_go_to_steps_of_full_tiles(gemm, T, B, Hq, Hkv, two):
+    from openvino_b200.ops import cuda as ops
+    assert ops.lib().ovb_pa_two_query_tiles(T, B, Hq, Hkv) == two
