@@ -7,9 +7,8 @@
 //  * warp 0: TMA producer; both CTAs report their bytes on the barrier of the even CTA, whose warp 1 issues the MMAs of the pair
 //  * warps 4 .. 11: epilogue, straight from the accumulator to global memory (no staging of the tile)
 //  * the token tile is any multiple of 32 up to 256, chosen on the host so that the last wave of tiles is nearly full
-// Quantised weights are expanded into 16-bit tiles first, a piece of at most kScratchBytes at a time (it mostly stays in L2): with
-// more than a thousand tokens the expansion is a few percent of the product, while the fused expansion of gemm_sm100.cu is
-// repeated for every token tile.
+// Quantised weights are expanded into 16-bit tiles first, a piece of at most kScratchBytes at a time, where that takes less time than the
+// fused expansion of gemm_sm100.cu, which is repeated for every token tile (expansion_pays).
 // Measured on B200, one launch, T = 8191, 28672 x 4096 int8 weights with the fused gate: 2765 us in the single-CTA kernel, 1365 us here
 // (expansion included, 1.41 PFLOP/s); T = 999, the same in bf16: 271 -> 197 us; top-2 of 8 experts, 4096 rows, 28672 x 4096: 969 -> 799 us.
 // One expansion of 128 MB of tiles takes 32 us (u4), 46 us (u8).
@@ -456,9 +455,32 @@ static int pick_piece(int T, int N, int K, int bt, int pairs, int64_t scratch_by
     return best * 256;
 }
 
-// From how many tokens on: 16-bit weights above one 128-token tile of the single-CTA kernel; quantised weights where the expansion pays.
+// From how many tokens on: 16-bit weights above one 128-token tile of the single-CTA kernel; quantised weights from 1024 on, where
+// expansion_pays says so (for bytes the two are already equal at about 400 tokens: 28672 x 4096, 384 tokens, 201 / 166 us; the callers
+// provide scratch memory from 1024 on).
 constexpr int kPairMinTokens = 129;
 constexpr int kPairMinTokensQuant = 1024;
+
+// Is the expansion with a product of 16-bit tiles after it faster than the fused one? Both are estimated in microseconds, constants fitted
+// to 156 measured pairs (the products of an 8B and a 70B model in u4, u8 and fp8, 1024 to 8192 tokens, cold caches): the faster one is
+// chosen in all but four, which lose 2 to 5 %. Fused / expanded, us: u4 28672 x 4096 1024 tokens 264 / 226, 8192 tokens 2006 / 1252; 4096 x
+// 14336 1024 tokens 86 / 112; 57344 x 8192 1024 tokens 793 / 986; u8 4096 x 14336 1024 tokens 158 / 118. The expansion loses where it writes
+// many bytes for few tokens, and where K is so long that a piece of the scratch memory does not fill the machine: 8192 x 28672 1024 tokens,
+// u4 324 / 685, u8 575 / 691.
+static bool expansion_pays(const ovb_gemm_args* a) {
+    constexpr int kPairs = 74, kSMs = 148;
+    const bool u4 = a->wmode == OVB_W_U4, gated = a->act == OVB_ACT_SWIGLU || a->act == OVB_ACT_GLU_LIMITED;
+    // fused: waves of 128 x 256 tiles
+    const double k_us = a->K * 1e-3, fused_wave = (u4 ? 3.5 : 0.0) + (gated ? 10.0 : 0.0) + k_us * (u4 ? 6.2 : a->wmode == OVB_W_U8 ? 10.6 : 11.0);
+    const double fused = ceil_div(ceil_div(a->N, TILE_N) * ceil_div(a->T, 256), kSMs) * fused_wave;
+    // expanded: launches and bytes of the expansion, waves of 256 x bt tiles of every piece
+    const int bt = pick_pair_tile(a->T, a->N, 0, kPairs), piece = pick_piece(a->T, a->N, a->K, bt, kPairs, kScratchBytes);
+    if (piece <= 0) return false;
+    int pieces = 0, waves = 0;
+    for (int n = 0; n < a->N; n += piece, ++pieces) waves += ceil_div(ceil_div(a->N - n < piece ? a->N - n : piece, 256) * ceil_div(a->T, bt), kPairs);
+    const double expanded = 3.0 * pieces + (double)a->N * a->K * 2 / (1 << 20) * (u4 ? 0.30 : 0.36) + waves * k_us * 5.7 * (bt + 32) / 288;
+    return expanded < fused;
+}
 
 static bool pair_shape(const ovb_gemm_args* a) {
     const bool quant = is_quant(a->wmode);
@@ -474,7 +496,7 @@ static bool pair_shape(const ovb_gemm_args* a) {
     } else if (ceil_div(a->N, 256) * ceil_div(a->T, 64) < 37) {
         return false;           // less than half of the pairs would have a tile: the other kernel splits K over a cluster
     }
-    if (quant && (a->w_kb_stride != 0 || a->group_size <= 0)) return false;
+    if (quant && (a->w_kb_stride != 0 || a->group_size <= 0 || !expansion_pays(a))) return false;
     if (a->out_f32) {
         if (a->residual != nullptr || swiglu || (reinterpret_cast<uintptr_t>(a->out) & 3) != 0) return false;
     } else {

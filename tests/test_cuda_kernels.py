@@ -750,6 +750,14 @@ def _pair_weight(ops, fmt, N, K, dtype=torch.bfloat16):
     return ops.PackedWeight.from_f8_block(q, torch.rand((N + 127) // 128, K // 128, device="cuda", generator=g) * 0.05 + 0.02, N, K)
 
 
+def _is_expanded(ops, T, w):
+    """Does a plain product of T tokens expand these weights first?"""
+    import ctypes as C
+    a = ops.GemmArgs()
+    a.x, a.w, a.out, a.T, a.N, a.K, a.ldx, a.group_size, a.wmode = 16, 16, 16, T, w.N, w.K, w.K, w.group_size, w.mode
+    return ops.lib().ovb_gemm_scratch_bytes(C.byref(a)) > 0
+
+
 @pytest.mark.parametrize("fmt,T,N,K", [("dense", 129, 3328, 64), ("dense", 999, 6144, 448), ("dense", 257, 4224, 1024), ("dense", 2049, 384, 128), ("dense", 8191, 256, 512),
                                        ("u4", 1024, 1280, 256), ("u4", 1031, 640, 4096), ("u8", 1025, 896, 256), ("f8", 1100, 768, 384), ("u4", 1024, 36864, 2048)])
 def test_gemm_pair(ops, fmt, T, N, K):
@@ -774,6 +782,17 @@ def test_gemm_pair(ops, fmt, T, N, K):
     h = res.clone()
     ops.gemm(x, w, out=h, residual=h)                       # in place, as the residual stream
     assert _rel_err(h, ops.gemm(x, w, residual=res, block_t=256)) < PAIR_REL
+    ops.check_status("gemm_pair")
+
+
+@pytest.mark.parametrize("fmt,T,N,K", [("u8", 1024, 36864, 2048), ("u8", 1025, 4992, 2048), ("f8", 1100, 4224, 4096), ("u4", 2560, 28800, 4096), ("u4", 2049, 33024, 4096)])
+def test_gemm_expanded_weights(ops, fmt, T, N, K):
+    """Problems whose weights are expanded, in one piece and in several, odd numbers of 128-row tiles among them."""
+    x = torch.randn(T, K, device="cuda", dtype=torch.bfloat16, generator=torch.Generator(device="cuda").manual_seed(T))
+    w = _pair_weight(ops, fmt, N, K)
+    assert _is_expanded(ops, T, w)
+    assert _rel_err(ops.gemm(x, w), ops.gemm(x, w, block_t=256)) < PAIR_REL
+    assert _rel_err(ops.gemm(x, w, act=ops.ACT_SWIGLU), ops.gemm(x, w, block_t=256, act=ops.ACT_SWIGLU)) < PAIR_REL
     ops.check_status("gemm_pair")
 
 
@@ -893,8 +912,9 @@ def test_expanded_weights_exact(ops, fmt):
     x = torch.eye(K, device="cuda", dtype=torch.bfloat16)
     for kw in ({"block_t": 64}, {"block_t": 256}):
         assert torch.equal(ops.gemm(x, w, out_f32=True, **kw).t().contiguous(), want.float()), kw
-    many = ops.gemm(x.repeat(4, 1), w, out_f32=True)         # expanded in a pass of its own
-    assert torch.equal(many[:K].t().contiguous(), want.float()) and torch.equal(many[3 * K:].t().contiguous(), want.float())
+    many = ops.gemm(x.repeat(32, 1), w, out_f32=True)        # expanded in a pass of its own
+    assert _is_expanded(ops, 32 * K, w)
+    assert torch.equal(many[:K].t().contiguous(), want.float()) and torch.equal(many[31 * K:].t().contiguous(), want.float())
     ops.check_status("gemm")
 
 

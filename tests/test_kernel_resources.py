@@ -59,3 +59,19 @@ def test_kernels_of_layered_decoders_do_not_spill(gemm, stem):
 def test_two_query_tiles_go_to_steps_of_full_tiles(gemm, T, B, Hq, Hkv, two):
     from openvino_b200.ops import cuda as ops
     assert ops.lib().ovb_pa_two_query_tiles(T, B, Hq, Hkv) == two
+
+
+@pytest.mark.parametrize("fmt,N,K,T,expanded", [
+    ("u4", 4096, 14336, 1024, 0), ("u4", 57344, 8192, 1024, 0), ("u4", 8192, 28672, 1024, 0), ("u4", 8192, 28672, 8192, 0), ("u8", 8192, 28672, 1024, 0),
+    ("f8", 8192, 28672, 1024, 0), ("u4", 10240, 8192, 1280, 0),
+    ("u4", 28672, 4096, 1024, 1), ("u4", 28672, 4096, 8192, 1), ("u4", 57344, 8192, 4096, 1), ("u8", 4096, 14336, 1024, 1), ("f8", 8192, 28672, 2048, 1),
+    ("u8", 28672, 4096, 1024, 1), ("u8", 28672, 4096, 1023, 0)])
+def test_weights_are_expanded_where_that_is_faster(gemm, fmt, N, K, T, expanded):
+    """Both sides of the rule at sizes that were measured on both kernels."""
+    import ctypes as C
+    from openvino_b200.ops import cuda as ops
+    a = ops.GemmArgs()
+    a.T, a.N, a.K, a.ldx, a.group_size, a.wmode = T, N, K, K, 128, {"u4": ops.W_U4, "u8": ops.W_U8, "f8": ops.W_F8}[fmt]
+    a.act = ops.ACT_SWIGLU if N in (28672, 57344) else ops.ACT_NONE
+    a.x = a.w = a.out = 16
+    assert (ops.lib().ovb_gemm_scratch_bytes(C.byref(a)) > 0) == bool(expanded)
