@@ -350,12 +350,21 @@ def gemm(x: torch.Tensor, w: PackedWeight, out: Optional[torch.Tensor] = None, r
     elif act == ACT_SOFTCAP:
         a.act_limit = cap
     if w.mode in (W_U4, W_U8, W_F8) and T >= 1024:      # expanded weights; the caching allocator keeps the memory, per stream
-        a.scratch_bytes = lib().ovb_gemm_scratch_bytes(C.byref(a))
-        if a.scratch_bytes:
-            scratch = torch.empty(a.scratch_bytes, dtype=torch.uint8, device=x.device)
-            a.scratch = scratch.data_ptr()
+        scratch = _gemm_scratch(lib().ovb_gemm_scratch_bytes(C.byref(a)), x.device)
+        if scratch is not None:
+            a.scratch, a.scratch_bytes = scratch.data_ptr(), scratch.numel()
     _check(lib().ovb_gemm(C.byref(a), C.c_void_p(_stream())), "ovb_gemm")
     return out
+
+
+def _gemm_scratch(nbytes: int, device) -> Optional[torch.Tensor]:
+    """Memory for expanded weights, or None where the device has none left: the product then runs without expanding them."""
+    if nbytes <= 0:
+        return None
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None
 
 
 def _gemm_f32(x: torch.Tensor, w: "PackedWeight", out: Optional[torch.Tensor], act: int = ACT_NONE, limit: float = 0.0) -> torch.Tensor:

@@ -796,6 +796,23 @@ def test_gemm_expanded_weights(ops, fmt, T, N, K):
     ops.check_status("gemm_pair")
 
 
+def test_gemm_runs_without_scratch_memory(ops, monkeypatch):
+    """A device without room for expanded weights still runs the product."""
+    x = torch.randn(1025, 2048, device="cuda", dtype=torch.bfloat16)
+    w = _pair_weight(ops, "u8", 4992, 2048)
+    assert _is_expanded(ops, 1025, w)
+    want = ops.gemm(x, w)
+    out = torch.empty_like(want)
+
+    def full(*size, **kw):
+        raise torch.OutOfMemoryError("no room")
+    with monkeypatch.context() as m:
+        m.setattr(ops.torch, "empty", full)
+        ops.gemm(x, w, out=out)
+    assert _rel_err(out, want) < PAIR_REL
+    ops.check_status("gemm")
+
+
 def test_gemm_pair_fp16_window_and_groups(ops):
     torch.manual_seed(2)
     x = torch.randn(700, 512, device="cuda", dtype=torch.float16)
