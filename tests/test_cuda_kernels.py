@@ -529,6 +529,41 @@ def test_u8_kv_cache_write_and_attention(ops, q_lens, past_lens, Hq, Hkv):
     assert _rel_err(out.reshape(T, Hq, D), ref) < 1e-2
 
 
+@pytest.mark.parametrize("Hq,Hkv,window", [(32, 8, 0), (8, 8, 0), (16, 8, 0), (64, 8, 0), (32, 8, 300), (64, 8, 77)])
+def test_u8_kv_cache_decode_shares_keys_per_sequence(ops, Hq, Hkv, window):
+    """A captured length (2048) above the real ones: the keys of every sequence are shared out by its own length, some splits stay
+    empty. Zero points far from 128, and rows that are not visible (behind the last key, before the window) hold pairs of NaN and inf."""
+    g = torch.Generator(device="cuda").manual_seed(Hq + window)
+    D, bs, dev, top = 128, 16, "cuda", 2048
+    ctx = ([1, 2, 15, 255, 256, 257, 300, 900, 1023, 1500, 1999, 2048] * 2)
+    B = len(ctx)
+    past, sub, bi, bib, blocks = _make_paged_batch([1] * B, [c - 1 for c in ctx], bs, dev)
+    caches, metas, wide = [], [], []
+    seen = torch.zeros(blocks, bs, dtype=torch.bool, device=dev)
+    for b in range(B):
+        pos = torch.arange(max(0, ctx[b] - window) if window else 0, ctx[b], device=dev)
+        seen[bi[bib[b]:bib[b + 1]].long()[pos // bs], pos % bs] = True
+    for _ in range(2):
+        q = torch.randint(0, 256, (blocks, Hkv, bs, D), dtype=torch.uint8, device=dev, generator=g)
+        scale = torch.rand(blocks, Hkv, bs, device=dev, generator=g) * 0.02 + 0.004
+        zero = torch.tensor([128.0, 0.0, 255.0, -300.0, 700.0, 131.5], device=dev)[torch.randint(0, 6, (blocks, Hkv, bs), device=dev, generator=g)]
+        meta = torch.stack([scale, zero], -1).half()
+        wide.append((q.double() - meta[..., 1:].double()) * meta[..., :1].double())
+        meta = torch.where(seen[:, None, :, None], meta, torch.tensor([float("nan"), float("inf")], device=dev, dtype=torch.float16))
+        caches.append(q)
+        metas.append(meta.contiguous())
+    qkv = (torch.randn(B, (Hq + 2 * Hkv) * D, device=dev, generator=g) * 0.3).bfloat16()
+    out = ops.paged_attention(qkv, *caches, past, sub, bi, bib, Hq, Hkv, D, scale=1.0 / math.sqrt(D), sliding_window=window, max_context_len=top, max_q_len=1,
+                              k_meta=metas[0], v_meta=metas[1])
+    ops.check_status("paged_attention u8")
+    rows = [[c[bi[bib[b]:bib[b + 1]].long()].permute(0, 2, 1, 3).reshape(-1, Hkv, D)[:ctx[b]] for b in range(B)] for c in wide]
+    ref = _attn_ref(qkv[:, :Hq * D].double().reshape(B, Hq, D), *rows, [1] * B, [c - 1 for c in ctx], Hq, Hkv, D, 1 / math.sqrt(D), window)
+    # the bytes, scales and sums are exact to fp32 and the weights of the values to 2^-17: what is left is the rounding of the result to
+    # bf16, uniform up to 2^-8 of a value and less towards the upper end of a binade: 1.7e-3 in the 2-norm of many values
+    off = (out.reshape(B, Hq, D).double() - ref).norm(dim=(1, 2)) / ref.norm(dim=(1, 2))
+    assert off.max() < 2.2e-3, off
+
+
 def test_paged_attention_sliding_window(ops):
     torch.manual_seed(7)
     Hq, Hkv, D, bs = 8, 2, 128, 16
