@@ -983,36 +983,52 @@ def test_layernorm_row_widths(ops, rows, cols):
         assert _rel_err(y, ref) < 1e-3          # one rounding to fp16: 2^-11 of a value at most
 
 
+def _weight_and_values(ops, fmt, N, K):
+    """A packed weight and its values in 64 bits (scales as the kernels' tables hold them)."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    if fmt == "dense":
+        d = (torch.randn(N, K, device="cuda", generator=g) * 0.05).bfloat16()
+        return ops.PackedWeight.from_dense(d), d.double()
+    if fmt == "f8":
+        q = torch.randn(N, K, device="cuda", generator=g).to(torch.float8_e4m3fn)
+        s = torch.rand((N + 127) // 128, K // 128, device="cuda", generator=g) * 0.05 + 0.02
+        return ops.PackedWeight.from_f8_block(q, s, N, K), q.double() * s.bfloat16().double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)
+    top = 16 if fmt == "u4" else 256
+    q = torch.randint(0, top, (N, K), dtype=torch.uint8, device="cuda", generator=g)
+    z = torch.randint(0, top, (N, K // 128), dtype=torch.uint8, device="cuda", generator=g)
+    s = ((torch.rand(N, K // 128, device="cuda", generator=g) + 0.5) * (0.16 / top)).half()
+    wide = ((q.reshape(N, -1, 128).double() - z.double()[..., None]) * s.bfloat16().double()[..., None]).reshape(N, K)
+    if fmt == "u8":
+        return ops.PackedWeight.from_ir_u8(q, s, z, N, K, 128), wide
+    return ops.PackedWeight.from_ir_u4((q[:, 0::2] | (q[:, 1::2] << 4)).reshape(-1), s, z, N, K, 128, zp_is_u8=True), wide
+
+
 @pytest.mark.parametrize("fmt,N,K", [("dense", 96, 64), ("dense", 4096, 1088), ("u4", 128, 128), ("u4", 6240, 4096), ("u4", 1024, 14336), ("u8", 32, 256), ("u8", 2080, 4096),
                                      ("f8", 160, 128), ("f8", 4096, 7168)])
-@pytest.mark.parametrize("T", [1, 3, 4, 8])
+@pytest.mark.parametrize("T", [1, 3, 4, 5, 8, 9])
 def test_gemm_stream(ops, fmt, N, K, T):
-    """Edges of the token fragment, one unit of K, K shared by a cluster, tiles that are no multiple of 128 rows: against the
-    tensor-memory kernel (an explicit token tile selects it) and, where the weights are known, no further from a 64-bit product."""
+    """Edges of the token fragment, one unit of K, K shared by a cluster, tiles that are no multiple of 128 rows, token counts on both sides
+    of the kernel's limit (8 with 16-bit weights, 4 with quantised ones): element by element against the product in 64 bits."""
     torch.manual_seed(T)
     x = torch.randn(T, K + 8, device="cuda", dtype=torch.bfloat16)[:, :K]
-    if fmt == "u4":
-        g = torch.Generator(device="cuda").manual_seed(N)
-        q = torch.randint(0, 256, (N * K // 2,), dtype=torch.uint8, device="cuda", generator=g)
-        z = torch.randint(0, 16, (N, K // 128), dtype=torch.uint8, device="cuda", generator=g)
-        sc = (torch.rand(N, K // 128, device="cuda", generator=g) * 0.01 + 0.005).half()
-        w = ops.PackedWeight.from_ir_u4(q, sc, z, N, K, 128, zp_is_u8=True)
-        wide = (torch.stack([q & 15, q >> 4], -1).reshape(N, K // 128, 128).double() - z.double()[..., None]) * sc.bfloat16().double()[..., None]
-        exact = x.double() @ wide.reshape(N, K).t()
-        out, old = ops.gemm(x, w), ops.gemm(x, w, block_t=16)
-        # the sums are exact to fp32, so the result is the rounded product up to a rare neighbour (more tokens take the other kernel)
-        assert T > 4 or _rel_err(out, exact) <= 1.02 * _rel_err(exact.to(torch.bfloat16), exact) and _rel_err(out, exact) <= _rel_err(old, exact)
-    else:
-        w = _pair_weight(ops, fmt, N, K)
-    # weights rounded to bf16 (2^-9 / sqrt(3) each) against unrounded ones, and the two roundings of the results
-    for kw in (dict(), dict(out_f32=True, act=ops.ACT_SILU)):
-        assert _rel_err(ops.gemm(x, w, **kw), ops.gemm(x, w, block_t=16, **kw)) < PAIR_REL, kw
+    w, wide = _weight_and_values(ops, fmt, N, K)
+    exact, size = x.double() @ wide.t(), x.double().abs() @ wide.abs().t()
+    # fp32 sums of exact products: K roundings of at most 2^-24 of the sum of magnitudes, in practice their root; behind the limit the weights are
+    # rounded to bf16 first (half a unit in the last place of 8 bits: up to 2^-8 of the value each), and a bf16 result once more
+    streamed = T <= (8 if fmt == "dense" else 4)
+    sums = 2.0 ** -18 * size if streamed or fmt == "dense" else 2.0 ** -8 * size
+    for f32 in (True, False):
+        y = ops.gemm(x, w, out_f32=f32)
+        assert ((y.double() - exact).abs() <= sums + (0.0 if f32 else 2.0 ** -8) * exact.abs()).all(), (f32, ((y.double() - exact).abs() / size).max())
+    if streamed or fmt == "dense":
+        assert _rel_err(ops.gemm(x, w, out_f32=True), exact) <= 1.5 * _rel_err(ops.gemm(x, w, out_f32=True, block_t=16), exact) + 2.0 ** -22
+    act = ops.gemm(x, w, out_f32=True, act=ops.ACT_SILU)
+    assert ((act.double() - torch.nn.functional.silu(exact)).abs() <= 1.2 * sums + 2.0 ** -20 * exact.abs()).all()       # |silu'| < 1.1
     w.bias = torch.randn(N, device="cuda").to(torch.bfloat16)
     h = torch.randn(T + 1, N, device="cuda").to(torch.bfloat16)
-    keep = h[T].clone()
-    want = ops.gemm(x, w, residual=h[:T], block_t=16)
+    keep, want = h[T].clone(), exact + w.bias.double() + h[:T].double()
     ops.gemm(x, w, out=h[:T], residual=h[:T])
-    assert _rel_err(h[:T], want) < PAIR_REL and torch.equal(h[T], keep)
+    assert ((h[:T].double() - want).abs() <= sums + 2.0 ** -8 * want.abs() + 2.0 ** -20).all() and torch.equal(h[T], keep)
     w.bias = None
     if N % 128 == 0:
         for kw in (dict(act=ops.ACT_SWIGLU), dict(act=ops.ACT_GLU_LIMITED, glu=(7.0, 1.702, 1.0))):
