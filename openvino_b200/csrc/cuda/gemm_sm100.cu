@@ -1458,6 +1458,8 @@ static int comm_packets(int world, int mode) {
     return world <= 2;
 }
 
+int ovb_gemm_route(const ovb_gemm_args* a) { return ovb::gemm_stream_takes(a) ? 2 : ovb::gemm_pair_takes(a) ? 1 : 0; }
+
 int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream_) {
     using namespace ovb;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);

@@ -307,7 +307,9 @@ constexpr int kStreamSmem = 112 * 1024;         // two CTAs on an SM
 static int stream_smem(int wmode, int T, int units_per_split) { return 2 * kStreamWarps * 8 * 36 * 4 + units_per_split * stream_unit(wmode) * T * 2; }
 
 // CTAs that share K. Time of a candidate: tiles that a cluster works off one after another, each as long as its bytes take at this
-// CTA's part of 6 TB/s, or as long as its loads wait (0.8 us a round); a cluster barrier costs about 1 us.
+// CTA's part of 6 TB/s, or as long as its loads wait (0.8 us a round); a cluster barrier costs about 1 us. Clusters of four and eight take one
+// tile each: their CTAs wait for the slowest at every tile (8192 x 28672 u4, four tokens, whose rows only fit shared memory by such
+// clusters: 100 us, gemm_sm100.cu 59 us). 0: no split serves the problem well.
 static int pick_stream_split(int wmode, int T, int N, int units, int* smem_bytes) {
     const double unit_us = 32.0 * stream_unit(wmode) * (wmode == OVB_W_U4 ? 0.5625 : wmode == OVB_W_BF16 ? 2.0 : 1.03) * 296 / 6.0e6;
     int best = 0;
@@ -317,6 +319,7 @@ static int pick_stream_split(int wmode, int T, int N, int units, int* smem_bytes
         const int per = ceil_div(units, s), smem = stream_smem(wmode, T, per);
         if (smem > kStreamSmem) continue;
         const int jobs = ceil_div(N / 32, 296 / s);
+        if (s > 2 && jobs > 1) continue;
         const double bytes_us = per * unit_us, wait_us = 0.8 * ceil_div(per, kStreamWarps * 2);
         const double t = jobs * ((bytes_us > wait_us ? bytes_us : wait_us) + (s > 1 ? 1.0 : 0.3)) + per * T * 0.0006;
         if (t < best_t) { best_t = t; best = s; *smem_bytes = smem; }

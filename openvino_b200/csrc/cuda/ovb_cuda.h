@@ -100,6 +100,8 @@ typedef struct {
 } ovb_gemm_args;
 
 int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream);
+// The kernel that ovb_gemm runs this problem on: 0 single CTAs (gemm_sm100.cu), 1 pairs of CTAs (gemm_pair.cu), 2 few tokens (gemm_stream.cu).
+int ovb_gemm_route(const ovb_gemm_args* a);
 // Bytes of split-K workspace / number of counters that ovb_gemm may need for the given problem.
 int64_t ovb_gemm_ws_bytes(int T, int N, int K, int act);
 int ovb_gemm_num_counters(void);

@@ -75,3 +75,14 @@ def test_weights_are_expanded_where_that_is_faster(gemm, fmt, N, K, T, expanded)
     a.act = ops.ACT_SWIGLU if N in (28672, 57344) else ops.ACT_NONE
     a.x = a.w = a.out = 16
     assert (ops.lib().ovb_gemm_scratch_bytes(C.byref(a)) > 0) == bool(expanded)
+
+
+@pytest.mark.parametrize("N,K,T,route", [(8192, 28672, 4, 0), (57344, 28672, 4, 0), (8192, 28672, 3, 2), (1024, 28672, 4, 2), (4096, 14336, 4, 2), (128256, 4096, 1, 2),
+                                         (4096, 4096, 5, 0)])
+def test_few_tokens_leave_clusters_that_would_share_many_tiles(gemm, N, K, T, route):
+    import ctypes as C
+    from openvino_b200.ops import cuda as ops
+    a = ops.GemmArgs()
+    a.x = a.w = a.out = 16
+    a.T, a.N, a.K, a.ldx, a.group_size, a.wmode = T, N, K, K, 128, ops.W_U4
+    assert ops.lib().ovb_gemm_route(C.byref(a)) == route
