@@ -97,6 +97,28 @@ int make_tmap_2d(CUtensorMap* out, const void* base, CUtensorMapDataType dtype, 
     return 0;
 }
 
+int make_tmap_blocks(CUtensorMap* out, const void* base, CUtensorMapDataType dtype, int elem_bytes, uint64_t rows, uint64_t cols, uint64_t pitch_bytes,
+                     uint32_t box_rows, uint32_t block_cols, uint32_t box_blocks) {
+    if (int rc = load_encode()) return rc;
+    if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (pitch_bytes & 15) != 0 || block_cols * elem_bytes != 128 || cols % block_cols != 0) {
+        set_error("TMA operand in blocks: base %p, pitch %llu, %llu columns in blocks of %u x %d bytes", base, (unsigned long long)pitch_bytes,
+                  (unsigned long long)cols, block_cols, elem_bytes);
+        return ERR_BAD_ARG;
+    }
+    cuuint64_t dims[3] = {block_cols, rows, cols / block_cols};
+    cuuint64_t strides[2] = {pitch_bytes, 128};
+    cuuint32_t box[3] = {block_cols, box_rows, box_blocks};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = g_encode(out, dtype, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        set_error("cuTensorMapEncodeTiled failed with %d (rows %llu cols %llu pitch %llu box %u x %u x %u elem %d)", (int)r, (unsigned long long)rows,
+                  (unsigned long long)cols, (unsigned long long)pitch_bytes, box_rows, block_cols, box_blocks, elem_bytes);
+        return ERR_TMAP;
+    }
+    return 0;
+}
+
 }  // namespace ovb
 
 extern "C" {

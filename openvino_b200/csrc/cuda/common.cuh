@@ -45,6 +45,11 @@ int* status_word();   // device pointer of the current device's status word (NUL
 int make_tmap_2d(CUtensorMap* out, const void* base, CUtensorMapDataType dtype, int elem_bytes, uint64_t rows,
                  uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols, bool swizzle128);
 
+// The same matrix cut into blocks of `block_cols` columns (128 bytes, swizzled): a box of `box_rows` rows of `box_blocks` blocks lands block
+// after block, so that one copy brings several k-blocks of an operand. Coordinates: 0, row, block.
+int make_tmap_blocks(CUtensorMap* out, const void* base, CUtensorMapDataType dtype, int elem_bytes, uint64_t rows, uint64_t cols, uint64_t pitch_bytes,
+                     uint32_t box_rows, uint32_t block_cols, uint32_t box_blocks);
+
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Programmatic dependent launch: kernels of a stream that call pdl_wait() (sm100_ptx.cuh) are launched with the

@@ -214,6 +214,9 @@ __device__ __forceinline__ void dequant_f8x4(uint32_t w, __nv_bfloat162 ss, uint
 // gemm_pair.cu: products of many tokens on pairs of CTAs. gemm_pair_takes() says whether it runs the problem.
 bool gemm_pair_takes(const ovb_gemm_args* a);
 int gemm_pair(const ovb_gemm_args* a, cudaStream_t stream);
+// gemm_few.cu: products of up to 64 tokens with quantised weights.
+bool gemm_few_takes(const ovb_gemm_args* a);
+int gemm_few(const ovb_gemm_args* a, cudaStream_t stream);
 // gemm_stream.cu: products of few tokens.
 bool gemm_stream_takes(const ovb_gemm_args* a);
 int gemm_stream(const ovb_gemm_args* a, cudaStream_t stream);

@@ -114,10 +114,6 @@ __device__ __forceinline__ void pair_commit_elect(uint64_t* bar) {
         ::"r"(smem_u32(bar)), "h"((uint16_t)3)
         : "memory");
 }
-__device__ __forceinline__ void arrive_cluster(uint32_t addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
-}
-
 template <bool F16>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const PairParams p) {

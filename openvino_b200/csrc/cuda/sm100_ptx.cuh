@@ -186,6 +186,16 @@ __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t addr) {
     return v;
 }
 
+// Arrive on a barrier of any CTA of the cluster (a dsmem_addr).
+__device__ __forceinline__ void arrive_cluster(uint32_t addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// 16 bytes into the shared memory of a CTA of the cluster, counted as bytes on a barrier of that CTA.
+__device__ __forceinline__ void st_async_v4(uint32_t addr, const uint32_t* v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(bar) : "memory");
+}
+
 // ---------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -1093,3 +1093,31 @@ def test_rotation_rounds_the_same_at_every_size(ops, T):
     hi = torch.where((d % 2 == 0)[None, None], a * s + r(b * c), b * c + r(a * s)).float().bfloat16()
     got = torch.cat([qkv.reshape(T, -1, D)[:, :Hq], kc.permute(0, 2, 1, 3).reshape(-1, Hkv, D)[:T]], 1)
     assert torch.equal(got, torch.cat([lo, hi], -1))
+
+
+@pytest.mark.parametrize("fmt", ["u4", "u8", "f8"])
+@pytest.mark.parametrize("T", [5, 16, 17, 32, 33, 48, 49, 64])
+def test_gemm_few(ops, fmt, T):
+    """Up to 64 tokens with quantised weights: every token tile's edge, one stage of K, shares of K that are no equal parts, tiles that clusters work
+    off in several rounds, every number of splits, against the product in 64 bits and bit for bit against a second run."""
+    torch.manual_seed(T)
+    for N, K, splits in ((128, 256, (0, 1)), (256, 1280, (0, 2, 3, 5)), (512, 2048, (4, 6, 7, 8)), (128 * 150, 256, (1,)), (128 * 76, 512, (2,)), (128 * 19, 2048, (8,))):
+        x = torch.randn(T, K + 8, device="cuda", dtype=torch.bfloat16)[:, :K]
+        w, wide = _weight_and_values(ops, fmt, N, K)
+        exact, size = x.double() @ wide.t(), x.double().abs() @ wide.abs().t()
+        sums = 2.0 ** -8 * size                            # weights rounded to bf16 (fp32 sums are far closer)
+        res = torch.randn(T, N, device="cuda").to(torch.bfloat16)
+        bias = torch.randn(N, device="cuda").to(torch.bfloat16)
+        for s in splits:
+            y = ops.gemm(x, w, out_f32=True, splits=s)
+            assert ((y.double() - exact).abs() <= sums).all(), (N, K, s, ((y.double() - exact).abs() / size).max())
+            assert _rel_err(y, exact) < PAIR_REL and torch.equal(y, ops.gemm(x, w, out_f32=True, splits=s))
+            w.bias = bias
+            h = torch.randn(T + 1, N, device="cuda").to(torch.bfloat16)
+            keep, want = h[T].clone(), exact + bias.double() + res.double()
+            ops.gemm(x, w, out=h[:T], residual=res, splits=s)
+            assert ((h[:T].double() - want).abs() <= sums + 2.0 ** -8 * want.abs() + 2.0 ** -20).all() and torch.equal(h[T], keep)
+            w.bias = None
+            for kw in (dict(act=ops.ACT_SWIGLU), dict(act=ops.ACT_GLU_LIMITED, glu=(7.0, 1.702, 1.0)), dict(act=ops.ACT_SILU)):
+                assert _rel_err(ops.gemm(x, w, splits=s, **kw), ops.gemm(x, w, block_t=64, **kw)) < 2 * PAIR_REL, kw
+    ops.check_status("gemm_few")
