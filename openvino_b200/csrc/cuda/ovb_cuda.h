@@ -273,6 +273,62 @@ int64_t ovb_pa_scratch_bytes(int B, int Hq, int D, int max_context_len);
 // 1: a prefill or mixed step of T tokens in B sequences (16-bit cache, head size 128) runs two query tiles per CTA, 0: one.
 int ovb_pa_two_query_tiles(int T, int B, int Hq, int Hkv);
 
+// ---------------------------------------------------------------------------------------------
+// One step of a dense decoder-only model as one call (llm_step.cu): token ids and embedding, all layers, and the logits of every sequence's last
+// token. All buffers are contiguous; no address is kept.
+typedef struct {
+    const void* w;
+    const void* scales;
+    const void* bias;
+    int N, K, group_size, wmode, w_tiled, w_kb_stride;   // as in ovb_gemm_args
+    int act;                  // gate_up: OVB_ACT_SWIGLU (rows interleaved for the fused gate) or OVB_ACT_NONE
+    int reserved;
+} ovb_llm_weight;
+typedef struct {
+    ovb_llm_weight qkv, o, gate_up, down;
+    const void* norm1;
+    const void* norm2;
+    void* k_cache;
+    void* v_cache;
+    void* k_meta;             // u8 cache
+    void* v_meta;
+} ovb_llm_layer;
+typedef struct {
+    const ovb_llm_layer* layers;
+    ovb_llm_weight head;
+    const void* embed;
+    const void* final_norm;
+    int* ids;
+    const int* tok_src;
+    const int* last_token;
+    const int* positions;
+    const int* slot_map;
+    const int* past_lens;
+    const int* subsequence_begins;
+    const int* block_indices;
+    const int* block_indices_begins;
+    const int* logit_idx;
+    void* h;                  // [T, hidden]
+    void* x;                  // [T, hidden]
+    void* qkv;                // [T, (Hq + 2 Hkv) D]
+    void* attn;               // [T, Hq D]
+    void* gu;                 // [T, 2 ffn]
+    void* act;                // [T, ffn]
+    void* last_h;             // [B, hidden]
+    void* last_x;             // [B, hidden]
+    void* logits;             // [B, head_cols]
+    float* gemm_ws;
+    int* gemm_counters;
+    float* pa_scratch;
+    void* scratch;            // expanded weights (ovb_llm_scratch_bytes), may be NULL
+    int64_t gemm_ws_bytes, pa_scratch_bytes, scratch_bytes;
+    int num_layers, T, B, hidden, ffn, Hq, Hkv, D, vocab, head_cols, block_size, max_ctx, max_q_len, sliding_window, kv_u8;
+    float theta, eps;
+    int reserved;
+} ovb_llm_step;
+int64_t ovb_llm_scratch_bytes(const ovb_llm_step* s);
+int ovb_llm_step_run(const ovb_llm_step* s, ovb_stream_t stream);
+
 // Dense (non-paged) bidirectional attention for encoder models: q,k,v [B, S, H, D] fp16/bf16.
 int ovb_sdpa_dense(const void* q, const void* k, const void* v, void* out, int B, int S, int H, int D, int ld,
                    float scale, int is_f16, int causal, ovb_stream_t stream);

@@ -57,6 +57,36 @@ class PaArgs(C.Structure):
     ]
 
 
+class LlmStep(C.Structure):
+    """ovb_llm_step. ``layers`` and ``head`` hold weights as ``llm_weight_words`` packs them."""
+    POINTERS = ("embed", "final_norm", "ids", "tok_src", "last_token", "positions", "slot_map", "past_lens", "subsequence_begins", "block_indices",
+                "block_indices_begins", "logit_idx", "h", "x", "qkv", "attn", "gu", "act", "last_h", "last_x", "logits", "gemm_ws", "gemm_counters", "pa_scratch",
+                "scratch")
+    INTS = ("num_layers", "T", "B", "hidden", "ffn", "Hq", "Hkv", "D", "vocab", "head_cols", "block_size", "max_ctx", "max_q_len", "sliding_window", "kv_u8")
+    _fields_ = ([("layers", C.c_void_p), ("head", C.c_ubyte * 56)] + [(n, C.c_void_p) for n in POINTERS]
+                + [(n, C.c_int64) for n in ("gemm_ws_bytes", "pa_scratch_bytes", "scratch_bytes")] + [(n, C.c_int) for n in INTS]
+                + [("theta", C.c_float), ("eps", C.c_float), ("reserved", C.c_int)])
+
+
+LLM_WEIGHT = "QQQ8i"          # ovb_llm_weight
+LLM_LAYER = "<" + 4 * LLM_WEIGHT + "6Q"
+
+
+def llm_weight_words(w: "PackedWeight", act: int = ACT_NONE):
+    return (w.w.data_ptr(), 0 if w.scales is None else w.scales.data_ptr(), 0 if w.bias is None else w.bias.data_ptr(), w.N, w.K, w.group_size, w.mode,
+            1 if (w.tiled and w.mode in (W_BF16, W_F16)) else 0, int(w.kb_stride or 0), act, 0)
+
+
+def llm_step(step: "LlmStep", device) -> None:
+    """One step of a dense decoder (see ovb_llm_step). Memory for expanded weights comes from the caching allocator for the call."""
+    l = lib()
+    if step.T >= 1024:
+        scratch = _gemm_scratch(l.ovb_llm_scratch_bytes(C.byref(step)), device)
+        if scratch is not None:
+            step.scratch, step.scratch_bytes = scratch.data_ptr(), scratch.numel()
+    _check(l.ovb_llm_step_run(C.byref(step), C.c_void_p(_stream())), "ovb_llm_step")
+
+
 def _fields(pointers, ints, floats=()):
     return ([(n, C.c_void_p) for n in pointers] + [(n, C.c_int) for n in ints] + [(n, C.c_float) for n in floats])
 
@@ -132,6 +162,10 @@ def lib():
         l.ovb_gemm_ws_bytes.restype = C.c_int64
         l.ovb_gemm_scratch_bytes.restype = C.c_int64
         l.ovb_gemm_scratch_bytes.argtypes = [C.POINTER(GemmArgs)]
+        if hasattr(l, "ovb_llm_step_run"):          # not part of the library of layered decoders
+            l.ovb_llm_scratch_bytes.restype = C.c_int64
+            l.ovb_llm_scratch_bytes.argtypes = [C.POINTER(LlmStep)]
+            l.ovb_llm_step_run.argtypes = [C.POINTER(LlmStep), C.c_void_p]
         l.ovb_pa_scratch_bytes.restype = C.c_int64
         l.ovb_channel_delta_record_floats.restype = C.c_int64
         l.ovb_gemm.argtypes = [C.POINTER(GemmArgs), C.c_void_p]

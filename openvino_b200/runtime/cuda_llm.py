@@ -10,7 +10,9 @@ produced by SDPAToPagedAttention (src/core/src/pass/sdpa_to_paged_attention.cpp)
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
+import struct
 from dataclasses import dataclass, field
 from typing import List, Optional
 
@@ -427,6 +429,8 @@ class CudaLlmExecutor(LlmExecutor):
     # -- one forward pass over the buffers of `sb`
     def _forward(self, sb: StepBuffers, shp: StepShape) -> None:
         cfg, w, ws = self.cfg, self.w, self.ws
+        if self.tp_size == 1 and not cfg.num_experts and all(p.mode != K.W_F32 for lw in w.layers for p in (lw.qkv, lw.o, lw.gate_up, lw.down)):
+            return self._forward_native(sb, shp)
         T, B = shp.T, shp.B
         D = cfg.head_dim
         ids = sb.view("ids")[:T]
@@ -486,6 +490,34 @@ class CudaLlmExecutor(LlmExecutor):
         K.gemm(last_x, w.lm_head, out=logits, ws=ws)
         self._sample(sb, B)
         self.kernel_launches += n + 5
+
+    def _forward_native(self, sb: StepBuffers, shp: StepShape) -> None:
+        """The pass of a dense model on one GPU: one call into the kernel library, which launches what `_forward` launches one by one. The addresses
+        are collected anew for every pass."""
+        cfg, w, ws, T, B = self.cfg, self.w, self.ws, shp.T, shp.B
+        if T > sb.Tcap or B > sb.Bcap:
+            raise ValueError("a step of %d tokens in %d sequences does not fit buffers of %d and %d" % (T, B, sb.Tcap, sb.Bcap))
+        size, plain = struct.calcsize(K.LLM_LAYER), 0
+        layers = C.create_string_buffer(size * len(w.layers))
+        for l, lw in enumerate(w.layers):
+            gated = getattr(lw.gate_up, "swiglu", False)
+            plain += not gated
+            struct.pack_into(K.LLM_LAYER, layers, size * l, *K.llm_weight_words(lw.qkv), *K.llm_weight_words(lw.o),
+                             *K.llm_weight_words(lw.gate_up, K.ACT_SWIGLU if gated else K.ACT_NONE), *K.llm_weight_words(lw.down), lw.norm1.data_ptr(),
+                             lw.norm2.data_ptr(), self.k_cache[l].data_ptr(), self.v_cache[l].data_ptr(),
+                             self.k_meta[l].data_ptr() if self.kv_u8 else 0, self.v_meta[l].data_ptr() if self.kv_u8 else 0)
+        desc = sb.desc.data_ptr()
+        at = {name: desc + 4 * off for name, (off, _) in sb.offsets.items()}
+        step = K.LlmStep(C.addressof(layers), (C.c_ubyte * 56).from_buffer_copy(struct.pack("<" + K.LLM_WEIGHT, *K.llm_weight_words(w.lm_head))), w.embed.data_ptr(), w.final_norm.data_ptr(),
+                         at["ids"], at["tok_src"], self.last_token.data_ptr(), at["positions"], at["slot_map"], at["past_lens"], at["subsequence_begins"],
+                         at["block_indices"], at["block_indices_begins"], at["logit_idx"],
+                         *(t.data_ptr() for t in (sb.h, sb.x, sb.qkv, sb.attn, sb.gu, sb.act, sb.last_h, sb.last_x, sb.logits, ws.gemm_ws, ws.counters, ws.pa_scratch)),
+                         None, ws.gemm_ws.numel() * 4, ws.pa_scratch.numel() * 4, 0, len(w.layers), T, B, cfg.hidden_size, cfg.ffn_size, self.hq, self.hkv,
+                         cfg.head_dim, w.embed.shape[0], sb.logits.shape[1], self.block_size, shp.max_ctx, shp.max_q_len, cfg.sliding_window,
+                         1 if self.kv_u8 else 0, cfg.rope_theta, cfg.rms_eps, 0)
+        K.llm_step(step, self.device)
+        self._sample(sb, B)
+        self.kernel_launches += 3 + 8 * len(w.layers) + plain + 5
 
     def _moe_gathered(self, sb: StepBuffers, l: int, T: int, x: torch.Tensor, h: torch.Tensor) -> int:
         """Experts on their own tokens only (prefill-sized batches), without a host round trip: the position of every
