@@ -217,7 +217,12 @@ int gemm_pair(const ovb_gemm_args* a, cudaStream_t stream);
 // gemm_few.cu: products of up to 64 tokens with quantised weights.
 bool gemm_few_takes(const ovb_gemm_args* a);
 int gemm_few(const ovb_gemm_args* a, cudaStream_t stream);
-// gemm_stream.cu: products of few tokens.
+// Clusters of this many CTAs that the device holds, one CTA of gemm_few.cu's size per SM, asked of the driver once.
+int cluster_capacity(int size);
+// gemm_ring.cu: products of up to four tokens with u4 weights.
+bool gemm_ring_takes(const ovb_gemm_args* a);
+int gemm_ring(const ovb_gemm_args* a, cudaStream_t stream);
+// gemm_stream.cu: products of few tokens, small ones.
 bool gemm_stream_takes(const ovb_gemm_args* a);
 int gemm_stream(const ovb_gemm_args* a, cudaStream_t stream);
 

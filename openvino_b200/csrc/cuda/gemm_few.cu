@@ -449,8 +449,7 @@ static bool few_layout(int wmode, int nt, FewPlan* f) {
     return f->smem <= kFewSmem;
 }
 
-// Clusters of this many CTAs that the device holds, one CTA per SM, asked of the driver once.
-static int few_clusters(int splits) {
+int cluster_capacity(int splits) {
     static std::mutex mu;
     static int table[9] = {0, 148, 74, 45, 35, 27, 22, 18, 16};       // (without a device)
     std::lock_guard<std::mutex> lk(mu);
@@ -492,7 +491,7 @@ static bool few_plan(int wmode, int T, int N, int K, int forced, FewPlan* best) 
         FewPlan f;
         f.splits = s;
         if (!few_layout(wmode, nt, &f)) continue;
-        f.clusters = few_clusters(s);
+        f.clusters = cluster_capacity(s);
         const int per = ceil_div(ks, s), full = tiles / f.clusters, rest = tiles % f.clusters;
         auto round_us = [&](int clusters) {
             const double sm = per * stage_us, hbm = (double)clusters * s * per * bytes_us;

@@ -100,7 +100,7 @@ typedef struct {
 } ovb_gemm_args;
 
 int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream);
-// The kernel that ovb_gemm runs this problem on: 0 single CTAs (gemm_sm100.cu, gemm_few.cu), 1 pairs of CTAs (gemm_pair.cu), 2 few tokens (gemm_stream.cu).
+// The kernel that ovb_gemm runs this problem on: 0 single CTAs (gemm_sm100.cu, gemm_few.cu), 1 pairs of CTAs (gemm_pair.cu), 2 few tokens (gemm_ring.cu, gemm_stream.cu).
 int ovb_gemm_route(const ovb_gemm_args* a);
 // The plan of gemm_few.cu for a product: splits of K, clusters, ring stages, token stages, expanding groups, bytes of shared memory. `splits` 0: its
 // own choice. Returns 0 where no plan fits.
