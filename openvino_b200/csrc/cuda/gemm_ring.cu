@@ -1,7 +1,8 @@
 // Products of up to four tokens with u4 weights: out[T, N] = epilogue(X[T, K] * dequant(W[N, K])^T), a single user's decode step.
 //
 // What bounds it: the read of the weights. gemm_stream.cu, which ran all of these before and keeps the small ones, reads them into registers: a few
-// units per warp are on their way, and its warps meet after every 32 rows (128256 x 4096: 71 us, 4.0 TB/s). Here
+// units per warp are on their way, and its warps meet after every 32 rows (128256 x 4096 with the norm before it 75.5 us, here 59.8; the products of
+// a step of one token through four layers of an 8B model 258 -> 200). Here
 //  * one lane streams stages of 128 rows x 256 columns (18 KB, one bulk copy) into a ring of 6 to 10 of them, requested before the kernel that
 //    writes the tokens is done;
 //  * sixteen warps share a stage: warp w of a half takes 16 rows and 128 columns. ldmatrix hands a lane the 32-bit word (8 nibbles) that its place in
@@ -112,7 +113,8 @@ __global__ void __launch_bounds__(kRingThreads, 1) gemm_ring_kernel(const RingPa
         const bool gated = p.act == OVB_ACT_SWIGLU || p.act == OVB_ACT_GLU_LIMITED;
         const uint32_t lane_off = smem_u32(ring) + half * 9216 + (lane >> 4) * 2048 + (row0 + (lane & 15)) * 16;
         const uint32_t sz_off = smem_u32(ring) + half * 9216 + 4096 + (row0 + g) * 4;
-        const uint8_t* xlane = xs + (size_t)half * 4 * T * 64 + g * 64 + t * 16;
+        // (columns behind the last token repeat it: nothing reads their sums)
+        const uint32_t xlane = smem_u32(xs) + half * 4 * T * 64 + min(g, T - 1) * 64 + t * 16, xpiece = T * 64;
         int slot = 0, turn = 0;
         uint32_t par = 0;
         bool ok = true;
@@ -126,33 +128,35 @@ __global__ void __launch_bounds__(kRingThreads, 1) gemm_ring_kernel(const RingPa
                 for (int c = 0; c < 2; ++c) ldsm_x4(lane_off + slot * kRingStage + c * 4608, q[c][0], q[c][1], q[c][2], q[c][3]);
                 asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sz[0]) : "r"(sz_off + slot * kRingStage));
                 asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sz[1]) : "r"(sz_off + slot * kRingStage + 32));
-                uint32_t minus[2];                                // -z / 64, twice each
+                uint32_t minus[2];                                // -z / 64 (the table holds 16 + z), twice each
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    const RowScale rs = row_scale(*reinterpret_cast<const __nv_bfloat162*>(&sz[i]), 16.f);
-                    minus[i] = *reinterpret_cast<const uint32_t*>(&rs.m);
+                    const __nv_bfloat162 zz = __high2bfloat162(*reinterpret_cast<const __nv_bfloat162*>(&sz[i]));
+                    const __nv_bfloat162 m = __hfma2(zz, __float2bfloat162_rn(-0.015625f), __float2bfloat162_rn(0.25f));
+                    minus[i] = *reinterpret_cast<const uint32_t*>(&m);
                 }
                 auto whole = [&](uint32_t bits, uint32_t mul, uint32_t m) {
                     const __nv_bfloat162 v = __hfma2(*reinterpret_cast<__nv_bfloat162*>(&bits), *reinterpret_cast<__nv_bfloat162*>(&mul), *reinterpret_cast<__nv_bfloat162*>(&m));
                     return *reinterpret_cast<const uint32_t*>(&v);
                 };
-                float part[2][4] = {};
+                float part[4] = {};
+                uint32_t xa = xlane + j * 8 * xpiece;
 #pragma unroll
                 for (int s = 0; s < 4; ++s) {                     // pieces of 32 columns
-                    uint4 xb = make_uint4(0, 0, 0, 0);
-                    if (g < T) xb = *reinterpret_cast<const uint4*>(xlane + ((size_t)j * 8 + s) * T * 64);
+                    const uint4 xb = lds128(xa);
+                    xa += xpiece;
                     const uint32_t lo = q[s >> 1][(s & 1) * 2], hi = q[s >> 1][(s & 1) * 2 + 1], ly = lo >> 8, hy = hi >> 8;
                     const uint32_t a0[4] = {whole(lo & 0x000F000Fu, kTwo127, minus[0]), whole(hi & 0x000F000Fu, kTwo127, minus[1]),
                                             whole(lo & 0x00F000F0u, kTwo123, minus[0]), whole(hi & 0x00F000F0u, kTwo123, minus[1])};
                     const uint32_t a1[4] = {whole(ly & 0x000F000Fu, kTwo127, minus[0]), whole(hy & 0x000F000Fu, kTwo127, minus[1]),
                                             whole(ly & 0x00F000F0u, kTwo123, minus[0]), whole(hy & 0x00F000F0u, kTwo123, minus[1])};
-                    mma16816<false>(part[s & 1], a0, xb.x, xb.y);
-                    mma16816<false>(part[s & 1], a1, xb.z, xb.w);
+                    mma16816<false>(part, a0, xb.x, xb.y);
+                    mma16816<false>(part, a1, xb.z, xb.w);
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[slot]);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[e] += __uint_as_float(sz[e >> 1] << 16) * 64.f * (part[0][e] + part[1][e]);
+                for (int e = 0; e < 4; ++e) acc[e] += __uint_as_float(sz[e >> 1] << 16) * part[e];
                 if (++slot == P) { slot = 0; par ^= 1; }
             }
             // the halves of K meet; another tile's sums go to the other buffer meanwhile
@@ -160,7 +164,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) gemm_ring_kernel(const RingPa
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int tok = 2 * t + (e & 1);
-                if (tok < T) mine[tok * 128 + row0 + (e >> 1) * 8 + g] = acc[e];
+                if (tok < T) mine[tok * 128 + row0 + (e >> 1) * 8 + g] = 64.f * acc[e];
             }
             ring_barrier();
             const float* a = red + turn * 2 * kRingTokens * 128;
@@ -236,7 +240,8 @@ static bool ring_plan(int T, int N, int K, RingPlan* f) {
     return true;
 }
 
-constexpr int64_t kRingMinWeights = 4ll << 20;
+// Below, a launch costs as much either way (2048 x 2048 5.7 us, gemm_stream.cu 5.2; 1024 x 4096 5.7 / 5.8; 4096 x 4096 6.9 / 7.6).
+constexpr int64_t kRingMinWeights = 8ll << 20;
 
 bool gemm_ring_takes(const ovb_gemm_args* a) {
     if (a->wmode != OVB_W_U4 || a->T > kRingTokens || a->comm != nullptr || a->group_offsets != nullptr || a->group_mode == 3 || a->block_t != 0 || a->splits > 1) return false;
