@@ -21,6 +21,7 @@
 #include "attention.cuh"
 #include "common.cuh"
 #include "debug_bounds.cuh"
+#include "gemm_common.cuh"
 #include "mma_sync.cuh"
 #include "sm100_ptx.cuh"
 
@@ -352,12 +353,29 @@ __device__ __forceinline__ void store_decoded(const PaKParams& p, int tok, int h
 // 24 sequences of 1200 tokens, 32 / 8 heads: 43 us with rounded products and two expanded pages per warp, 30 us now.
 // DK / DV: key and value sizes, multiples of 64; cache rows may be shorter (p.k_row, p.v_row: the rest is filled with zeros).
 // GT: query heads per KV head, or 0: any number (p.group), up to eight of them per CTA.
-template <int DK, int DV, int GT, int PAGE, bool KVU8, int NST>
+// ROPE: q and the new key are rotated here (rope_kv_write_vec_kernel's arithmetic), while the first pages are on their way; the CTA whose keys end with
+// the new one writes it and its value to the cache and puts both into their page's copy in shared memory.
+// p.cluster: the splits of a (sequence, KV head) are a cluster, and push their sums to its first CTA (st.async), which writes the outputs.
+template <int DK, int DV, int GT, int PAGE, bool KVU8, int NST, bool ROPE>
 __global__ void __launch_bounds__(128) pa_decode_kernel(PaKParams p) {
+    __shared__ uint64_t recv_full;
+    __shared__ volatile int abort_flag;
+    const bool cluster = GT > 0 && p.cluster != 0;
+    if (cluster) {
+        if (threadIdx.x == 0) {
+            mbar_init(&recv_full, 1);
+            mbar_fence_init();
+            abort_flag = 0;
+            if (blockIdx.z == 0) mbar_arrive_expect_tx(&recv_full, (uint32_t)((p.nsplit - 1) * GT * (DV + 4) * 4));
+        }
+        __syncthreads();
+        cluster_arrive();
+    }
     pdl_enter_attn();
     constexpr int CHK = DK / 8, CHV = DV / 8;
     constexpr int GMAX = GT > 0 ? GT : 8;
     static_assert(!KVU8 || (DK == DV && GT > 0), "byte cache: one head size");
+    static_assert(!ROPE || (DK == 128 && DV == 128 && GT > 0 && !KVU8), "rotation: packed heads of 128");
     constexpr int D = DK;                                              // (byte cache)
     constexpr int U8_PAGE = PAGE * D + PAGE * 4;                       // bytes of one staged u8 page (rows, then the pairs)
     constexpr int STAGE = KVU8 ? 2 * U8_PAGE : PAGE * (DK + DV) * 2;   // K and V of one stage (NST page stages per warp)
@@ -393,14 +411,22 @@ __global__ void __launch_bounds__(128) pa_decode_kernel(PaKParams p) {
     const int page_lo = k_lo / PAGE;
     const int page_hi = (k_hi + PAGE - 1) / PAGE;         // exclusive
 
+    // the new key: its page, and whether this CTA's keys end with it
+    const int new_page = (ctx - 1) / PAGE, new_row = (ctx - 1) % PAGE;
+    uint8_t* sNew = smem + 16 * DK * 2 + 4 * WARP_BYTES;               // ROPE: rotated key, value, cosines and sines
+    float2* sAngle = reinterpret_cast<float2*>(sNew + 2 * DK * 2);
+    const int slot = ROPE ? OVB_DBG_SLOT(p.slot_map[tok], PAGE) : -1;
+    const bool keep_new = ROPE && slot >= 0 && k_lo < ctx && k_hi == ctx;
+
     // Q: G real rows, the rest zero
+    if (!ROPE)
     for (int i = threadIdx.x; i < 16 * CHK; i += 128) {
         const int r = i / CHK, c = i % CHK;
         const bool valid = r < G && (GT > 0 || c * 8 < p.k_row);
         const uint8_t* src = reinterpret_cast<const uint8_t*>(p.q) + ((size_t)tok * p.ldq + (size_t)(hq0 + (valid ? r : 0)) * p.q_head) * 2 + (valid ? c : 0) * 16;
         cp_async16(sQ + tile_off<DK>(r, c), src, valid);
     }
-    cp_async_commit();
+    if (!ROPE) cp_async_commit();
 
     auto load_page = [&](int page, int st) {
         const bool pv = page < page_hi;
@@ -454,7 +480,57 @@ __global__ void __launch_bounds__(128) pa_decode_kernel(PaKParams p) {
         load_page(page + s * 4, s);
         cp_async_commit();
     }
-    cp_async_wait<NST - 1>();   // Q landed (oldest group)
+    if (ROPE) {
+        constexpr int HALF = DK / 2;
+        if (threadIdx.x < HALF) {
+            float sn, cs;
+            sincosf(float(p.positions[tok]) * exp2f(-p.log2_theta * (2.0f * float(threadIdx.x) / float(DK))), &sn, &cs);
+            sAngle[threadIdx.x] = make_float2(cs, sn);
+        }
+        const __nv_bfloat16* base = reinterpret_cast<const __nv_bfloat16*>(p.q) + (size_t)tok * p.ldq;
+        // two columns of a head's lower half and the same of its upper half; heads: G of q, then the key
+        constexpr int ITEMS = (GT + 1) * (HALF / 2), MINE = (ITEMS + 127) / 128;
+        __nv_bfloat162 lo[MINE], hi[MINE];
+#pragma unroll
+        for (int n = 0; n < MINE; ++n) {
+            const int i = threadIdx.x + n * 128, r = i / (HALF / 2), d = i % (HALF / 2) * 2;
+            if (i < ITEMS) {
+                const __nv_bfloat16* src = base + (size_t)(r < GT ? hq0 + r : p.Hq + h) * DK + d;
+                lo[n] = *reinterpret_cast<const __nv_bfloat162*>(src);
+                hi[n] = *reinterpret_cast<const __nv_bfloat162*>(src + HALF);
+            }
+        }
+        uint2 val = make_uint2(0, 0);
+        if (threadIdx.x < DV / 4) val = *reinterpret_cast<const uint2*>(base + (size_t)(p.Hq + p.Hkv + h) * DV + threadIdx.x * 4);
+        for (int i = threadIdx.x; i < (16 - GT) * CHK; i += 128) sts128(smem_u32(sQ + tile_off<DK>(GT + i / CHK, i % CHK)), make_uint4(0, 0, 0, 0));
+        __syncthreads();
+        const size_t at = keep_new ? (((size_t)(slot / PAGE) * p.Hkv + h) * PAGE + slot % PAGE) * DK : 0;
+#pragma unroll
+        for (int n = 0; n < MINE; ++n) {
+            const int i = threadIdx.x + n * 128, r = i / (HALF / 2), d = i % (HALF / 2) * 2;
+            if (i < ITEMS) {
+                const float2 a = __bfloat1622float2(lo[n]), b = __bfloat1622float2(hi[n]), w0 = sAngle[d], w1 = sAngle[d + 1];
+                const __nv_bfloat162 l2 = __floats2bfloat162_rn(fmaf(a.x, w0.x, -__fmul_rn(b.x, w0.y)), fmaf(a.y, w1.x, -__fmul_rn(b.y, w1.y)));
+                const __nv_bfloat162 h2 = __floats2bfloat162_rn(fmaf(a.x, w0.y, __fmul_rn(b.x, w0.x)), fmaf(b.y, w1.x, __fmul_rn(a.y, w1.y)));
+                if (r < GT) {
+                    *reinterpret_cast<__nv_bfloat162*>(sQ + tile_off<DK>(r, d / 8) + (d % 8) * 2) = l2;
+                    *reinterpret_cast<__nv_bfloat162*>(sQ + tile_off<DK>(r, (d + HALF) / 8) + (d % 8) * 2) = h2;
+                } else if (keep_new) {
+                    *reinterpret_cast<__nv_bfloat162*>(sNew + d * 2) = l2;
+                    *reinterpret_cast<__nv_bfloat162*>(sNew + (d + HALF) * 2) = h2;
+                    __nv_bfloat16* kc = reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(p.k_cache)) + at + d;
+                    *reinterpret_cast<__nv_bfloat162*>(kc) = l2;
+                    *reinterpret_cast<__nv_bfloat162*>(kc + HALF) = h2;
+                }
+            }
+        }
+        if (keep_new && threadIdx.x < DV / 4) {
+            *reinterpret_cast<uint2*>(sNew + DK * 2 + threadIdx.x * 8) = val;
+            *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(const_cast<void*>(p.v_cache)) + at + threadIdx.x * 4) = val;
+        }
+    } else {
+        cp_async_wait<NST - 1>();   // Q landed (oldest group)
+    }
     __syncthreads();
     uint32_t qf[DK / 16][4];
 #pragma unroll
@@ -489,6 +565,11 @@ __global__ void __launch_bounds__(128) pa_decode_kernel(PaKParams p) {
         __syncwarp();
         const uint8_t* kS = sKV + st * STAGE;
         const uint8_t* vS = kS + PAGE * DK * 2;
+        if (ROPE && keep_new && page == new_page) {                    // (the copy may have read the row before it was written)
+            const bool value = lane >= CHK;
+            sts128(smem_u32((value ? vS : kS) + tile_off<DK>(new_row, lane % CHK)), lds128(smem_u32(sNew + (value ? DK * 2 : 0) + (lane % CHK) * 16)));
+            __syncwarp();
+        }
         if (KVU8) {
             const uint8_t* uk = sKV + st * STAGE;
             expand_u8_whole<D>(uk, sExp, PAGE, lane);
@@ -608,6 +689,56 @@ __global__ void __launch_bounds__(128) pa_decode_kernel(PaKParams p) {
         if ((lane & 3) == 0) { dst[DV] = m_run; dst[DV + 1] = l_run; }
     }
     __syncthreads();
+    if (cluster) {
+        // [split][row] of DV sums, then maximum and denominator
+        float* recv = reinterpret_cast<float*>(smem + 16 * DK * 2 + 4 * WARP_BYTES + (ROPE ? 2 * DK * 2 + DK / 2 * 8 : 0));
+        cluster_wait();
+        const uint32_t full0 = dsmem_addr(smem_u32(&recv_full), 0);
+        for (int i = threadIdx.x; i < G * DV / 4; i += 128) {
+            const int rr = i / (DV / 4), d = i % (DV / 4) * 4;
+            float m = -CUDART_INF_F, l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int w = 0; w < 4; ++w) m = fmaxf(m, merge_row(w, rr)[DV]);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const float* src = merge_row(w, rr);
+                const float sc = (src[DV] == -CUDART_INF_F) ? 0.f : exp2f(src[DV] - m);
+                l += src[DV + 1] * sc;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[e] += src[d + e] * sc;
+            }
+            const uint32_t at = smem_u32(recv + (split * GMAX + rr) * (DV + 4));
+            const uint32_t v[4] = {__float_as_uint(o[0]), __float_as_uint(o[1]), __float_as_uint(o[2]), __float_as_uint(o[3])};
+            const uint32_t ml[4] = {__float_as_uint(m), __float_as_uint(l), 0u, 0u};
+            if (split == 0) {
+                sts128(at + d * 4, make_uint4(v[0], v[1], v[2], v[3]));
+                if (d == 0) sts128(at + DV * 4, make_uint4(ml[0], ml[1], 0u, 0u));
+            } else {
+                st_async_v4(dsmem_addr(at + d * 4, 0), v, full0);
+                if (d == 0) st_async_v4(dsmem_addr(at + DV * 4, 0), ml, full0);
+            }
+        }
+        if (split == 0) {
+            __syncthreads();
+            const bool ok = mbar_wait(&recv_full, 0, &abort_flag, p.status);
+            for (int i = threadIdx.x; ok && i < G * DV; i += 128) {
+                const int rr = i / DV, d = i % DV;
+                float mx = -CUDART_INF_F, l = 0.f, o = 0.f;
+                for (int z = 0; z < p.nsplit; ++z) mx = fmaxf(mx, recv[(z * GMAX + rr) * (DV + 4) + DV]);
+                for (int z = 0; z < p.nsplit; ++z) {
+                    const float* src = recv + (z * GMAX + rr) * (DV + 4);
+                    const float sc = src[DV] == -CUDART_INF_F ? 0.f : exp2f(src[DV] - mx);
+                    l += src[DV + 1] * sc;
+                    o += src[d] * sc;
+                }
+                if (p.sink != nullptr) l += exp2f(p.sink[hq0 + rr] * 1.4426950408889634f - mx);
+                store_decoded(p, tok, hq0 + rr, d, l > 0.f ? o / l : 0.f);
+            }
+        }
+        cluster_arrive();       // no CTA leaves while a peer may still store to it
+        cluster_wait();
+        return;
+    }
     for (int i = threadIdx.x; i < G * DV; i += 128) {
         const int rr = i / DV, d = i % DV;
         float m = -CUDART_INF_F;
@@ -693,15 +824,35 @@ int launch_decode_combine(const PaKParams& p, int dv, cudaStream_t stream) {
     return 0;
 }
 
-template <int DK, int DV, int G, bool KVU8, int NST>
+template <int DK, int DV, int G, bool KVU8, int NST, bool ROPE = false>
 static int launch_decode_sizes(const PaKParams& p, cudaStream_t stream) {
     constexpr int PAGE = 16;
     const int warp_bytes = KVU8 ? NST * 2 * (PAGE * DK + PAGE * 4) + PAGE * DK * 2 : NST * PAGE * (DK + DV) * 2;
-    const int smem = 16 * DK * 2 + 4 * warp_bytes + 128;
-    auto kern = pa_decode_kernel<DK, DV, G, PAGE, KVU8, NST>;
+    const int smem = 16 * DK * 2 + 4 * warp_bytes + 128 + (ROPE ? 2 * DK * 2 + DK / 2 * 8 : 0) + (G > 0 && p.cluster ? p.nsplit * G * (DV + 4) * 4 : 0);
+    constexpr int most = 16 * DK * 2 + 4 * (KVU8 ? NST * 2 * (PAGE * DK + PAGE * 4) + PAGE * DK * 2 : NST * PAGE * (DK + DV) * 2) + 128 + 2 * DK * 2 + DK / 2 * 8 + 8 * (G > 0 ? G : 1) * (DV + 4) * 4;
+    auto kern = pa_decode_kernel<DK, DV, G, PAGE, KVU8, NST, ROPE>;
     static std::atomic<uint64_t> configured{0};
-    if (int rc = set_smem_once(configured, reinterpret_cast<const void*>(kern), smem)) return rc;
+    if (int rc = set_smem_once(configured, reinterpret_cast<const void*>(kern), most)) return rc;
     dim3 grid(p.B, p.Hkv * (G > 0 ? 1 : (p.group + 7) / 8), p.nsplit);
+    if (G > 0 && p.cluster) {
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(128);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = p.nsplit;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = pdl_enabled() ? 2 : 1;
+        OVB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<PaKParams>(p)));
+        return 0;
+    }
     OVB_CHECK_CUDA(launch_pdl(kern, dim3(grid), dim3(128), smem, stream, p));
     OVB_CHECK_CUDA(cudaGetLastError());
     return p.nsplit > 1 ? launch_decode_combine(p, DV, stream) : 0;
@@ -712,6 +863,7 @@ template <int D, int G, bool KVU8 = false>
 static int launch_decode(PaKParams p, cudaStream_t stream) {
     p.q_head = p.o_head = p.dv_store = p.k_row = p.v_row = D;
     p.ldo = p.Hq * D;
+    if (!KVU8 && p.positions != nullptr) return launch_decode_sizes<D, D, G, false, 3, !KVU8>(p, stream);
     return launch_decode_sizes<D, D, G, KVU8, 3>(p, stream);
 }
 
@@ -781,7 +933,31 @@ int64_t ovb_pa_scratch_bytes(int B, int Hq, int D, int max_context_len) {
     return (int64_t)B * Hq * 32 * (D + 2) * (int64_t)sizeof(float);
 }
 
-int ovb_paged_attention(const ovb_pa_args* a, ovb_stream_t stream_) {
+// A step whose CTAs are all resident at once: launches count, and what they would do costs little inside the attention (one sequence of 650
+// keys, 32 / 8 heads: rotation 2.3, attention 6.0 and sum 3.4 us as three launches). With more CTAs every wave of them pays for it (64 sequences of
+// 1150: 60 us as three launches, 71 as one).
+static bool decode_is_small(const ovb_pa_args* a) { return a->B * a->Hkv * decode_nsplit(a->B, a->Hkv, a->max_context_len) <= 444; }
+
+int ovb_decode_attention_rotates(const ovb_pa_args* a) { return ovb_decode_attention_takes(a) && !a->kv_u8 && decode_is_small(a); }
+
+int ovb_decode_attention_takes(const ovb_pa_args* a) {
+    const int G = a->Hkv > 0 ? a->Hq / a->Hkv : 0;
+    return a->max_q_len == 1 && a->T == a->B && a->D == 128 && a->block_size == 16 && (G == 1 || G == 2 || G == 4 || G == 8);
+}
+
+static int paged_attention(const ovb_pa_args* a, const int* positions, const int* slot_map, float theta, bool alone, ovb_stream_t stream_);
+
+int ovb_paged_attention(const ovb_pa_args* a, ovb_stream_t stream) { return paged_attention(a, nullptr, nullptr, 0.f, false, stream); }
+
+int ovb_decode_attention(const ovb_pa_args* a, const int* positions, const int* slot_map, float theta, ovb_stream_t stream) {
+    OVB_REQUIRE(a && ovb_decode_attention_takes(a) && (positions == nullptr || (slot_map && !a->kv_u8 && a->ldq >= (a->Hq + 2 * a->Hkv) * a->D)),
+                "ovb_decode_attention: one token per sequence, heads of 128, blocks of 16, 1, 2, 4 or 8 query heads per KV head; the rotation needs a 16-bit cache");
+    OVB_REQUIRE(((reinterpret_cast<uintptr_t>(a->q) | reinterpret_cast<uintptr_t>(a->k_cache) | reinterpret_cast<uintptr_t>(a->v_cache)) & 15) == 0,
+                "ovb_decode_attention: 16-byte aligned tensors expected");
+    return paged_attention(a, positions, slot_map, theta, true, stream);
+}
+
+static int paged_attention(const ovb_pa_args* a, const int* positions, const int* slot_map, float theta, bool alone, ovb_stream_t stream_) {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     OVB_REQUIRE(a && a->q && a->out && a->k_cache && a->v_cache, "ovb_paged_attention: null operand");
     OVB_REQUIRE(a->past_lens && a->subsequence_begins && a->block_indices && a->block_indices_begins,
@@ -800,6 +976,10 @@ int ovb_paged_attention(const ovb_pa_args* a, ovb_stream_t stream_) {
     p.scale_log2 = a->scale * 1.4426950408889634f;
     p.causal = 1;
     p.nsplit = 1;
+    p.positions = positions;
+    p.slot_map = slot_map;
+    p.log2_theta = positions != nullptr ? log2f(theta) : 0.f;
+    p.status = status_word();
     p.kv_u8 = a->kv_u8;
     p.k_meta = a->k_meta;
     p.v_meta = a->v_meta;
@@ -816,6 +996,7 @@ int ovb_paged_attention(const ovb_pa_args* a, ovb_stream_t stream_) {
         p.nsplit = ns;
         int kps = (a->max_context_len + ns - 1) / ns;
         p.keys_per_split = ((kps + 63) / 64) * 64;   // whole pages, and page index % 4 == warp stays aligned
+        p.cluster = alone && ns >= 2 && ns <= 8 && decode_is_small(a);
         if (a->kv_u8) {
             switch (G) {
                 case 1: return launch_decode<128, 1, true>(p, stream);

@@ -46,6 +46,13 @@ struct PaKParams {
     // read from the paged cache `shared` (rows of shared_row elements) at column shared_col, and meets the query's columns from q_shared on.
     const int* kv_rows;
     const void* shared;
+    // Decode with the rotation of the step's own rows (attention.cu): q is the row of all heads before the rotation, keys behind the query heads,
+    // values behind the keys. NULL: the rows have been rotated and written.
+    const int* positions;
+    const int* slot_map;
+    float log2_theta;
+    int cluster;              // decode: 1: the splits are a cluster and its first CTA sums them; 0: pa_decode_combine_kernel does
+    int* status;
     int cache_rows;           // rows of the paged caches (0: not known); copies are bounded by it
     int kv_total, kv_ld, k_head, v_head, shared_row, shared_col, q_shared;
 };

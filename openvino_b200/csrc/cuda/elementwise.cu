@@ -52,12 +52,28 @@ template <int THREADS, int MAXV>
 __global__ void __launch_bounds__(THREADS)
 rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                const __nv_bfloat16* __restrict__ gamma, __nv_bfloat16* __restrict__ y,
-               __nv_bfloat16* __restrict__ residual_out, int cols, float eps) {
+               __nv_bfloat16* __restrict__ residual_out, int cols, float eps, const int* __restrict__ row_idx, int x_rows) {
     pdl_enter();
     __shared__ float red[32];
     const size_t row = blockIdx.x;
     const int nvec = cols >> 3;
-    const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
+    size_t from = row;
+    if (row_idx != nullptr) {
+        int id = row_idx[row];
+        if (id < 0 || id >= x_rows) {            // as an embedding does
+            (void)OVB_DBG_ROW(-1, 1);
+            id = 0;
+        }
+        from = (size_t)id;
+    }
+    const uint4* xr = reinterpret_cast<const uint4*>(x + from * cols);
+    // the weights come with the row, not behind the sum: a step of few tokens waits for these loads
+    uint4 gv[MAXV];
+#pragma unroll
+    for (int i = 0; i < MAXV; ++i) {
+        const int v = threadIdx.x + i * THREADS;
+        if (v < nvec) gv[i] = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+    }
     const uint4* rr = residual ? reinterpret_cast<const uint4*>(residual + row * cols) : nullptr;
     float vals[MAXV][8];
     float ss = 0.f;
@@ -87,14 +103,18 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
             for (int j = 0; j < 8; ++j) ss += vals[i][j] * vals[i][j];
         }
     }
-    const float tot = block_sum<THREADS>(ss, red);
+    // every warp sums all warps' parts: one barrier
+    ss = warp_sum(ss);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    const float tot = warp_sum((threadIdx.x & 31) < THREADS / 32 ? red[threadIdx.x & 31] : 0.f);
     const float inv = rsqrtf(tot / float(cols) + eps);
 #pragma unroll
     for (int i = 0; i < MAXV; ++i) {
         const int v = threadIdx.x + i * THREADS;
         if (v < nvec) {
             Pack8 g, o;
-            g.u = reinterpret_cast<const uint4*>(gamma)[v];
+            g.u = gv[i];
 #pragma unroll
             for (int j = 0; j < 8; ++j) o.b[j] = __float2bfloat16_rn(vals[i][j] * inv * __bfloat162float(g.b[j]));
             reinterpret_cast<uint4*>(y + row * cols)[v] = o.u;
@@ -358,11 +378,120 @@ __global__ void scatter_tokens_kernel(const int* __restrict__ tokens, const int*
     }
 }
 
+// resolve_ids_kernel and embedding_kernel<int> in one: a position with a source never reads its own id, so that writing it is no race.
+__global__ void embed_tokens_kernel(int* __restrict__ ids, const int* __restrict__ tok_src, const int* __restrict__ last_token, const uint4* __restrict__ table,
+                                    uint4* __restrict__ out, int rows, int vec_per_row, int vocab) {
+    pdl_enter();
+    const size_t total = (size_t)rows * vec_per_row;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t r = i / vec_per_row;
+        const int c = int(i - r * vec_per_row), s = tok_src[r];
+        int id = s >= 0 ? last_token[s] : ids[r];
+        if (s >= 0 && c == 0) ids[r] = id;
+        if (id < 0 || id >= vocab) {
+            (void)OVB_DBG_ROW(-1, 1);
+            id = 0;
+        }
+        out[i] = table[(size_t)id * vec_per_row + c];
+    }
+}
+
 // ------------------------------------------------------------------------------------ argmax
+// A row of a vocabulary read by one SM takes 6 us (128256 entries); with few rows eight CTAs (a cluster) share one: each keeps the best of its
+// piece, the others push theirs to the first (st.async), which also hands the token on (tok_dst, last_token; see scatter_tokens_kernel).
+// One row, 128256 entries, with the hand-over: 7.6 -> 3.9 us.
+constexpr int kArgmaxThreads = 512, kArgmaxPieces = 8;
+__global__ void __launch_bounds__(kArgmaxThreads) argmax_pieces_kernel(const __nv_bfloat16* __restrict__ logits, int ld, int vocab, void* __restrict__ out_ids, int ids_i32,
+                                                                       float* __restrict__ out_max, const int* __restrict__ tok_dst, int* __restrict__ last_token,
+                                                                       int* __restrict__ status) {
+    __shared__ __align__(16) uint32_t got[kArgmaxPieces][4];
+    __shared__ uint64_t got_full;
+    __shared__ float sv[kArgmaxThreads / 32];
+    __shared__ int si[kArgmaxThreads / 32];
+    __shared__ volatile int abort_flag;
+    const uint32_t rank = cluster_ctarank();
+    if (threadIdx.x == 0) {
+        mbar_init(&got_full, 1);
+        mbar_fence_init();
+        abort_flag = 0;
+        if (rank == 0) mbar_arrive_expect_tx(&got_full, (kArgmaxPieces - 1) * 16);
+    }
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();
+    pdl_enter();
+    const int row = blockIdx.x / kArgmaxPieces, nvec = vocab >> 3, per = (nvec + kArgmaxPieces - 1) / kArgmaxPieces;
+    const __nv_bfloat16* lr = logits + (size_t)row * ld;
+    const int v1 = min(nvec, ((int)rank + 1) * per);
+    float best = -CUDART_INF_F;
+    int bi = 0x7fffffff;
+    for (int v0 = (int)rank * per + threadIdx.x; v0 < v1; v0 += 4 * kArgmaxThreads) {
+        Pack8 a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (v0 + i * kArgmaxThreads < v1) a[i].u = reinterpret_cast<const uint4*>(lr)[v0 + i * kArgmaxThreads];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (v0 + i * kArgmaxThreads < v1) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float f = __bfloat162float(a[i].b[j]);
+                    if (f > best) { best = f; bi = (v0 + i * kArgmaxThreads) * 8 + j; }
+                }
+            }
+    }
+    if (rank == kArgmaxPieces - 1)
+        for (int i = nvec * 8 + threadIdx.x; i < vocab; i += kArgmaxThreads) {
+            const float f = __bfloat162float(lr[i]);
+            if (f > best) { best = f; bi = i; }
+        }
+    auto across = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+            if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+        }
+    };
+    across();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) { sv[warp] = best; si[warp] = bi; }
+    __syncthreads();
+    if (warp == 0) {
+        best = lane < kArgmaxThreads / 32 ? sv[lane] : -CUDART_INF_F;
+        bi = lane < kArgmaxThreads / 32 ? si[lane] : 0x7fffffff;
+        across();
+        if (rank != 0) {
+            const uint32_t v[4] = {__float_as_uint(best), (uint32_t)bi, 0u, 0u};
+            if (lane == 0) st_async_v4(dsmem_addr(smem_u32(got[rank]), 0), v, dsmem_addr(smem_u32(&got_full), 0));
+        } else {
+            const bool ok = mbar_wait(&got_full, 0, &abort_flag, status);
+            if (ok && lane > 0 && lane < kArgmaxPieces) {
+                best = __uint_as_float(got[lane][0]);
+                bi = (int)got[lane][1];
+            } else if (lane > 0) {
+                best = -CUDART_INF_F;
+                bi = 0x7fffffff;
+            }
+            across();
+            if (lane == 0) {
+                const int res = bi == 0x7fffffff ? 0 : bi;
+                if (ids_i32) reinterpret_cast<int*>(out_ids)[row] = res;
+                else reinterpret_cast<int64_t*>(out_ids)[row] = res;
+                if (out_max) out_max[row] = best;
+                if (tok_dst != nullptr && tok_dst[row] >= 0) last_token[tok_dst[row]] = res;
+            }
+        }
+    }
+    // no CTA leaves while a peer may still store to it
+    cluster_arrive();
+    cluster_wait();
+}
+
 template <int THREADS, class E>
 __global__ void __launch_bounds__(THREADS)
 argmax_kernel(const E* __restrict__ logits, int ld, int vocab, void* __restrict__ out_ids, int ids_i32,
-              float* __restrict__ out_max) {
+              float* __restrict__ out_max, const int* __restrict__ tok_dst, int* __restrict__ last_token) {
     pdl_enter();
     __shared__ float sv[THREADS / 32];
     __shared__ int si[THREADS / 32];
@@ -415,6 +544,7 @@ argmax_kernel(const E* __restrict__ logits, int ld, int vocab, void* __restrict_
             if (ids_i32) reinterpret_cast<int*>(out_ids)[row] = res;
             else reinterpret_cast<int64_t*>(out_ids)[row] = res;
             if (out_max) out_max[row] = best;
+            if (tok_dst != nullptr && tok_dst[row] >= 0) last_token[tok_dst[row]] = res;
         }
     }
 }
@@ -914,8 +1044,8 @@ extern "C" int ovb_debug_set_limits_elementwise(const ovb::DebugLimits* l) {
 extern "C" {
 using namespace ovb;
 
-int ovb_rmsnorm(const void* x, const void* residual, const void* gamma, void* y, void* residual_out, int rows,
-                int cols, float eps, ovb_stream_t stream_) {
+static int rmsnorm(const void* x, const void* residual, const void* gamma, void* y, void* residual_out, int rows, int cols, float eps, const int* row_idx,
+                   int x_rows, ovb_stream_t stream_) {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     OVB_REQUIRE(x && gamma && y && rows > 0, "ovb_rmsnorm: null operand");
     OVB_REQUIRE(cols % 8 == 0 && cols <= 256 * 8 * 8, "ovb_rmsnorm: cols=%d must be a multiple of 8 and <= 16384", cols);
@@ -925,12 +1055,20 @@ int ovb_rmsnorm(const void* x, const void* residual, const void* gamma, void* y,
     auto Y = (__nv_bfloat16*)y;
     auto RO = (__nv_bfloat16*)residual_out;
     const int nvec = cols / 8;
-    if (nvec <= 256) OVB_CHECK_CUDA(launch_pdl(rmsnorm_kernel<256, 1>, dim3(rows), dim3(256), 0, stream, X, R, G, Y, RO, cols, eps));
-    else if (nvec <= 512) OVB_CHECK_CUDA(launch_pdl(rmsnorm_kernel<256, 2>, dim3(rows), dim3(256), 0, stream, X, R, G, Y, RO, cols, eps));
-    else if (nvec <= 1024) OVB_CHECK_CUDA(launch_pdl(rmsnorm_kernel<256, 4>, dim3(rows), dim3(256), 0, stream, X, R, G, Y, RO, cols, eps));
-    else OVB_CHECK_CUDA(launch_pdl(rmsnorm_kernel<256, 8>, dim3(rows), dim3(256), 0, stream, X, R, G, Y, RO, cols, eps));
+    auto kern = nvec <= 256 ? rmsnorm_kernel<256, 1> : nvec <= 512 ? rmsnorm_kernel<256, 2> : nvec <= 1024 ? rmsnorm_kernel<256, 4> : rmsnorm_kernel<256, 8>;
+    OVB_CHECK_CUDA(launch_pdl(kern, dim3(rows), dim3(256), 0, stream, X, R, G, Y, RO, cols, eps, row_idx, x_rows));
     OVB_CHECK_CUDA(cudaGetLastError());
     return 0;
+}
+
+int ovb_rmsnorm(const void* x, const void* residual, const void* gamma, void* y, void* residual_out, int rows,
+                int cols, float eps, ovb_stream_t stream) {
+    return rmsnorm(x, residual, gamma, y, residual_out, rows, cols, eps, nullptr, 0, stream);
+}
+
+int ovb_rmsnorm_rows(const void* x, const int* row_idx, const void* gamma, void* y, int rows, int cols, float eps, int x_rows, ovb_stream_t stream) {
+    OVB_REQUIRE(row_idx && x_rows > 0, "ovb_rmsnorm_rows: no rows");
+    return rmsnorm(x, nullptr, gamma, y, nullptr, rows, cols, eps, row_idx, x_rows, stream);
 }
 
 int ovb_layernorm(const void* x, const void* residual, const void* gamma, const void* beta, void* y, int rows,
@@ -1076,18 +1214,61 @@ int ovb_scatter_tokens(const int* tokens, const int* tok_dst, int* last_token, i
     return 0;
 }
 
+int ovb_embed_tokens(int* ids, const int* tok_src, const int* last_token, const void* table, void* out, int rows, int cols, int vocab, ovb_stream_t stream) {
+    OVB_REQUIRE(ids && tok_src && last_token && table && out && rows > 0 && cols % 8 == 0, "ovb_embed_tokens: bad arguments");
+    OVB_CHECK_CUDA(launch_pdl(embed_tokens_kernel, dim3(grid_for((size_t)rows * (cols / 8), 256)), dim3(256), 0, static_cast<cudaStream_t>(stream), ids, tok_src,
+                              last_token, (const uint4*)table, (uint4*)out, rows, cols / 8, vocab));
+    return 0;
+}
+
+// Rows that several CTAs share: few of them, long, and readable in 16-byte pieces. (64 rows of 128256: 8.4 us, shared 5.9; from 148 rows on every SM
+// has a row of its own.)
+static bool argmax_in_pieces(const void* logits, int ld, int rows, int vocab) {
+    return rows < 148 && vocab >= 16384 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+}
+
+static int launch_argmax_pieces(const void* logits, int ld, int rows, int vocab, void* out_ids, int ids_i32, float* out_max, const int* tok_dst, int* last_token,
+                                cudaStream_t stream) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(rows * kArgmaxPieces);
+    cfg.blockDim = dim3(kArgmaxThreads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kArgmaxPieces;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    OVB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, argmax_pieces_kernel, (const __nv_bfloat16*)logits, ld, vocab, out_ids, ids_i32, out_max, tok_dst, last_token, status_word()));
+    return 0;
+}
+
 int ovb_argmax(const void* logits, int ld, int rows, int vocab, void* out_ids, int ids_i32, float* out_max,
                ovb_stream_t stream_) {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     OVB_REQUIRE(logits && out_ids && rows > 0 && vocab > 0, "ovb_argmax: bad arguments");
-    OVB_CHECK_CUDA(launch_pdl(argmax_kernel<1024, __nv_bfloat16>, dim3(rows), dim3(1024), 0, stream, (const __nv_bfloat16*)logits, ld, vocab, out_ids, ids_i32, out_max));
+    if (argmax_in_pieces(logits, ld, rows, vocab)) return launch_argmax_pieces(logits, ld, rows, vocab, out_ids, ids_i32, out_max, nullptr, nullptr, stream);
+    OVB_CHECK_CUDA(launch_pdl(argmax_kernel<1024, __nv_bfloat16>, dim3(rows), dim3(1024), 0, stream, (const __nv_bfloat16*)logits, ld, vocab, out_ids, ids_i32, out_max, (const int*)nullptr, (int*)nullptr));
     OVB_CHECK_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int ovb_argmax_scatter(const void* logits, int ld, int rows, int vocab, int* out_ids, const int* tok_dst, int* last_token, ovb_stream_t stream) {
+    OVB_REQUIRE(logits && out_ids && tok_dst && last_token && rows > 0 && vocab > 0, "ovb_argmax_scatter: bad arguments");
+    if (argmax_in_pieces(logits, ld, rows, vocab))
+        return launch_argmax_pieces(logits, ld, rows, vocab, out_ids, 1, nullptr, tok_dst, last_token, static_cast<cudaStream_t>(stream));
+    OVB_CHECK_CUDA(launch_pdl(argmax_kernel<1024, __nv_bfloat16>, dim3(rows), dim3(1024), 0, static_cast<cudaStream_t>(stream), (const __nv_bfloat16*)logits, ld, vocab,
+                              out_ids, 1, (float*)nullptr, tok_dst, last_token));
     return 0;
 }
 
 int ovb_argmax_f32(const float* logits, int ld, int rows, int vocab, void* out_ids, int ids_i32, float* out_max, ovb_stream_t stream) {
     OVB_REQUIRE(logits && out_ids && rows > 0 && vocab > 0, "ovb_argmax_f32: bad arguments");
-    OVB_CHECK_CUDA(launch_pdl(argmax_kernel<1024, float>, dim3(rows), dim3(1024), 0, static_cast<cudaStream_t>(stream), logits, ld, vocab, out_ids, ids_i32, out_max));
+    OVB_CHECK_CUDA(launch_pdl(argmax_kernel<1024, float>, dim3(rows), dim3(1024), 0, static_cast<cudaStream_t>(stream), logits, ld, vocab, out_ids, ids_i32, out_max, (const int*)nullptr, (int*)nullptr));
     return 0;
 }
 

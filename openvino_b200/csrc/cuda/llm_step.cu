@@ -88,17 +88,11 @@ int ovb_llm_step_run(const ovb_llm_step* s, ovb_stream_t stream) {
         const int rc_ = (call);    \
         if (rc_ != 0) return rc_;  \
     } while (0)
-    OVB_STEP(ovb_resolve_ids(s->ids, s->tok_src, s->last_token, T, stream));
-    OVB_STEP(ovb_embedding(s->ids, 1, s->embed, s->h, T, H, s->vocab, stream));
+    OVB_STEP(ovb_embed_tokens(s->ids, s->tok_src, s->last_token, s->embed, s->h, T, H, s->vocab, stream));
     for (int i = 0; i < s->num_layers; ++i) {
         const ovb_llm_layer* l = &s->layers[i];
         OVB_STEP(ovb_rmsnorm(s->h, nullptr, l->norm1, s->x, nullptr, T, H, s->eps, stream));
         OVB_STEP(run_gemm(s, &l->qkv, s->x, s->qkv, nullptr, T, rows, stream));
-        if (s->kv_u8)
-            OVB_STEP(ovb_rope_kv_write_u8(s->qkv, s->positions, s->slot_map, l->k_cache, l->v_cache, l->k_meta, l->v_meta, T, s->Hq, s->Hkv, s->D, s->theta,
-                                          s->block_size, stream));
-        else
-            OVB_STEP(ovb_rope_kv_write(s->qkv, s->positions, s->slot_map, l->k_cache, l->v_cache, T, s->Hq, s->Hkv, s->D, s->theta, s->block_size, stream));
         ovb_pa_args pa;
         memset(&pa, 0, sizeof(pa));
         pa.q = s->qkv;
@@ -126,7 +120,16 @@ int ovb_llm_step_run(const ovb_llm_step* s, ovb_stream_t stream) {
             pa.k_meta = l->k_meta;
             pa.v_meta = l->v_meta;
         }
-        OVB_STEP(ovb_paged_attention(&pa, stream));
+        const bool decode = ovb_decode_attention_takes(&pa), rotates = decode && ovb_decode_attention_rotates(&pa);
+        if (s->kv_u8)
+            OVB_STEP(ovb_rope_kv_write_u8(s->qkv, s->positions, s->slot_map, l->k_cache, l->v_cache, l->k_meta, l->v_meta, T, s->Hq, s->Hkv, s->D, s->theta,
+                                          s->block_size, stream));
+        else if (!rotates)
+            OVB_STEP(ovb_rope_kv_write(s->qkv, s->positions, s->slot_map, l->k_cache, l->v_cache, T, s->Hq, s->Hkv, s->D, s->theta, s->block_size, stream));
+        if (decode)
+            OVB_STEP(ovb_decode_attention(&pa, rotates ? s->positions : nullptr, s->slot_map, s->theta, stream));
+        else
+            OVB_STEP(ovb_paged_attention(&pa, stream));
         OVB_STEP(run_gemm(s, &l->o, s->attn, s->h, s->h, T, H, stream));
         OVB_STEP(ovb_rmsnorm(s->h, nullptr, l->norm2, s->x, nullptr, T, H, s->eps, stream));
         if (l->gate_up.act == OVB_ACT_SWIGLU) {
@@ -138,8 +141,7 @@ int ovb_llm_step_run(const ovb_llm_step* s, ovb_stream_t stream) {
         OVB_STEP(run_gemm(s, &l->down, s->act, s->h, s->h, T, H, stream));
     }
     // logits only for the last token of every sequence
-    OVB_STEP(ovb_embedding(s->logit_idx, 1, s->h, s->last_h, B, H, T, stream));
-    OVB_STEP(ovb_rmsnorm(s->last_h, nullptr, s->final_norm, s->last_x, nullptr, B, H, s->eps, stream));
+    OVB_STEP(ovb_rmsnorm_rows(s->h, s->logit_idx, s->final_norm, s->last_x, B, H, s->eps, T, stream));
     OVB_STEP(run_gemm(s, &s->head, s->last_x, s->logits, nullptr, B, s->head_cols, stream));
 #undef OVB_STEP
     return 0;

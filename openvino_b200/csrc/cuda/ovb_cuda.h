@@ -135,6 +135,8 @@ int ovb_pack_f8(const void* w, void* w_out, long long words, ovb_stream_t stream
 // y = rmsnorm(x (+ residual)) * gamma ;  if residual_out != NULL it receives x + residual.
 int ovb_rmsnorm(const void* x, const void* residual, const void* gamma, void* y, void* residual_out, int rows,
                 int cols, float eps, ovb_stream_t stream);
+// The norm of rows row_idx[0 .. rows) of x (an index outside [0, x_rows) reads row 0).
+int ovb_rmsnorm_rows(const void* x, const int* row_idx, const void* gamma, void* y, int rows, int cols, float eps, int x_rows, ovb_stream_t stream);
 int ovb_layernorm(const void* x, const void* residual, const void* gamma, const void* beta, void* y, int rows,
                   int cols, float eps, int is_f16, ovb_stream_t stream);
 // Linear recurrences (fp32, contiguous). `state` is read, advanced over the L tokens of every sequence and written back.
@@ -224,6 +226,10 @@ int ovb_moe_route_topk(const float* logits, float* weights, int T, int E, int k,
 // SwiGLU of the `nloc` local experts [e0, e0 + nloc) stacked along the feature axis, scaled by the routing weight:
 // gu [rows, nloc * 2F] (gate block then up block per expert) -> out [rows, nloc * F]; rows not routed to an expert get zeros.
 int ovb_moe_silu_mul_scale(const void* gu, const float* weights, void* out, int rows, int F, int nloc, int E, int e0, ovb_stream_t stream);
+// ovb_argmax (int32 ids) and ovb_scatter_tokens in one.
+int ovb_argmax_scatter(const void* logits, int ld, int rows, int vocab, int* out_ids, const int* tok_dst, int* last_token, ovb_stream_t stream);
+// ovb_resolve_ids and ovb_embedding (int32 ids) in one.
+int ovb_embed_tokens(int* ids, const int* tok_src, const int* last_token, const void* table, void* out, int rows, int cols, int vocab, ovb_stream_t stream);
 // Device-side token feedback between chained steps (see elementwise.cu).
 int ovb_resolve_ids(int* ids, const int* tok_src, const int* last_token, int T, ovb_stream_t stream);
 int ovb_scatter_tokens(const int* tokens, const int* tok_dst, int* last_token, int B, ovb_stream_t stream);
@@ -269,6 +275,12 @@ typedef struct {
     const void* v_meta;
 } ovb_pa_args;
 int ovb_paged_attention(const ovb_pa_args* a, ovb_stream_t stream);
+// A decode step's attention with what surrounds it. `positions` (and slot_map, theta as in ovb_rope_kv_write; NULL: not): q points at the fused qkv
+// rows before the rotation; queries and the new key are rotated and the new rows written to the cache. The splits of a small step are summed
+// in the same launch.
+int ovb_decode_attention(const ovb_pa_args* a, const int* positions, const int* slot_map, float theta, ovb_stream_t stream);
+int ovb_decode_attention_takes(const ovb_pa_args* a);
+int ovb_decode_attention_rotates(const ovb_pa_args* a);      // 1: the rotation inside the attention is the faster way
 int64_t ovb_pa_scratch_bytes(int B, int Hq, int D, int max_context_len);
 // 1: a prefill or mixed step of T tokens in B sequences (16-bit cache, head size 128) runs two query tiles per CTA, 0: one.
 int ovb_pa_two_query_tiles(int T, int B, int Hq, int Hkv);

@@ -593,6 +593,21 @@ def layernorm(x, gamma, beta, eps, residual=None, out=None):
     return out
 
 
+def rmsnorm_rows(x, row_idx, gamma, eps, out):
+    """The norm of the rows ``row_idx`` (int32) of ``x``."""
+    _check(lib().ovb_rmsnorm_rows(C.c_void_p(x.data_ptr()), C.c_void_p(row_idx.data_ptr()), C.c_void_p(gamma.data_ptr()), C.c_void_p(out.data_ptr()),
+                                  C.c_int(out.shape[0]), C.c_int(x.shape[1]), C.c_float(eps), C.c_int(x.shape[0]), C.c_void_p(_stream())), "ovb_rmsnorm_rows")
+    return out
+
+
+def embed_tokens(ids, tok_src, last_token, table, out):
+    """``resolve_ids`` and ``embedding`` (int32 ids), one launch."""
+    vocab, cols = table.shape
+    _check(lib().ovb_embed_tokens(C.c_void_p(ids.data_ptr()), C.c_void_p(tok_src.data_ptr()), C.c_void_p(last_token.data_ptr()), C.c_void_p(table.data_ptr()),
+                                  C.c_void_p(out.data_ptr()), C.c_int(ids.numel()), C.c_int(cols), C.c_int(vocab), C.c_void_p(_stream())), "ovb_embed_tokens")
+    return out
+
+
 def silu_mul(gu, out=None, nrows: Optional[torch.Tensor] = None):
     """silu(gate) * up over [rows, 2F] -> [rows, F]; ``nrows`` (int32 device tensor) limits the rows without a host read."""
     rows, F2 = gu.shape
@@ -834,6 +849,14 @@ def argmax(logits, out=None, out_max=None):
     return out
 
 
+def argmax_scatter(logits, out, tok_dst, last_token):
+    """``argmax`` into int32 ``out`` and ``scatter_tokens`` of the result, one launch (16-bit logits)."""
+    rows, vocab = logits.shape
+    assert out.dtype == torch.int32 and logits.dtype == torch.bfloat16
+    _check(lib().ovb_argmax_scatter(C.c_void_p(logits.data_ptr()), C.c_int(logits.stride(0)), C.c_int(rows), C.c_int(vocab), C.c_void_p(out.data_ptr()),
+                                    C.c_void_p(tok_dst.data_ptr()), C.c_void_p(last_token.data_ptr()), C.c_void_p(_stream())), "ovb_argmax_scatter")
+
+
 def resolve_ids(ids, tok_src, last_token):
     _check(lib().ovb_resolve_ids(C.c_void_p(ids.data_ptr()), C.c_void_p(tok_src.data_ptr()),
                                  C.c_void_p(last_token.data_ptr()), C.c_int(ids.numel()), C.c_void_p(_stream())),
@@ -869,6 +892,25 @@ def paged_attention(q, k_cache, v_cache, past_lens, subsequence_begins, block_in
                     scale=None, max_context_len=0, max_q_len=0, sliding_window=0, block_size=16, out=None, ws=None, k_meta=None, v_meta=None):
     """q: [T, >=Hq*D] (row pitch = q.stride(0)); caches [num_blocks, Hkv, block_size, D] (16-bit, or uint8 with the
     (scale, zero point) tables ``k_meta`` / ``v_meta``)."""
+    a, out = _pa_args(q, k_cache, v_cache, past_lens, subsequence_begins, block_indices, block_indices_begins, Hq, Hkv, D, scale, max_context_len, max_q_len,
+                      sliding_window, block_size, out, ws, k_meta, v_meta)
+    _check(lib().ovb_paged_attention(C.byref(a), C.c_void_p(_stream())), "ovb_paged_attention")
+    return out
+
+
+def decode_attention(qkv, k_cache, v_cache, past_lens, subsequence_begins, block_indices, block_indices_begins, Hq, Hkv, D, positions=None, slot_map=None, theta=0.0,
+                     scale=None, max_context_len=0, sliding_window=0, block_size=16, out=None, ws=None, k_meta=None, v_meta=None):
+    """Attention of a decode step (one token per sequence). With ``positions`` and ``slot_map`` the rows of ``qkv`` are those before the rotation: queries
+    and the new key are rotated and the new rows written to the 16-bit cache. A small step needs no launch of its own for the sum of the splits."""
+    a, out = _pa_args(qkv, k_cache, v_cache, past_lens, subsequence_begins, block_indices, block_indices_begins, Hq, Hkv, D, scale, max_context_len, 1,
+                      sliding_window, block_size, out, ws, k_meta, v_meta)
+    _check(lib().ovb_decode_attention(C.byref(a), C.c_void_p(_ptr(positions)), C.c_void_p(_ptr(slot_map)), C.c_float(theta), C.c_void_p(_stream())),
+           "ovb_decode_attention")
+    return out
+
+
+def _pa_args(q, k_cache, v_cache, past_lens, subsequence_begins, block_indices, block_indices_begins, Hq, Hkv, D, scale, max_context_len, max_q_len, sliding_window,
+             block_size, out, ws, k_meta, v_meta):
     T = q.shape[0]
     B = past_lens.numel()
     if out is None:
@@ -889,8 +931,7 @@ def paged_attention(q, k_cache, v_cache, past_lens, subsequence_begins, block_in
     if k_cache.dtype == torch.uint8:
         assert k_meta is not None and v_meta is not None
         a.kv_u8, a.k_meta, a.v_meta = 1, k_meta.data_ptr(), v_meta.data_ptr()
-    _check(lib().ovb_paged_attention(C.byref(a), C.c_void_p(_stream())), "ovb_paged_attention")
-    return out
+    return a, out
 
 
 def sdpa_dense(q, k, v, B, S, H, D, ld, scale=None, causal=False, out=None):

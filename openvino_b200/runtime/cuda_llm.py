@@ -324,6 +324,9 @@ class LlmExecutor:
             else:
                 K.sample(sb.logits[:B], temp, top_k, top_p, seed, self.sample_step, out=sb.tokens[:B])
             self.kernel_launches += 1
+        elif self.tp_size == 1 and sb.logits.dtype == torch.bfloat16:
+            K.argmax_scatter(sb.logits[:B], sb.tokens[:B], sb.view("tok_dst")[:B], self.last_token)
+            return
         elif self.tp_size == 1:
             K.argmax(sb.logits[:B], out=sb.tokens[:B])
         else:
@@ -517,7 +520,8 @@ class CudaLlmExecutor(LlmExecutor):
                          1 if self.kv_u8 else 0, cfg.rope_theta, cfg.rms_eps, 0)
         K.llm_step(step, self.device)
         self._sample(sb, B)
-        self.kernel_launches += 3 + 8 * len(w.layers) + plain + 5
+        decode = shp.max_q_len == 1 and cfg.head_dim == 128                       # rotation and sum of the splits inside the attention
+        self.kernel_launches += 3 + (7 if decode and not self.kv_u8 else 8) * len(w.layers) + plain + (1 if self.sampling is None else 2)
 
     def _moe_gathered(self, sb: StepBuffers, l: int, T: int, x: torch.Tensor, h: torch.Tensor) -> int:
         """Experts on their own tokens only (prefill-sized batches), without a host round trip: the position of every

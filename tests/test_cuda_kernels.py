@@ -1121,3 +1121,75 @@ def test_gemm_few(ops, fmt, T):
             for kw in (dict(act=ops.ACT_SWIGLU), dict(act=ops.ACT_GLU_LIMITED, glu=(7.0, 1.702, 1.0)), dict(act=ops.ACT_SILU)):
                 assert _rel_err(ops.gemm(x, w, splits=s, **kw), ops.gemm(x, w, block_t=64, **kw)) < 2 * PAIR_REL, kw
     ops.check_status("gemm_few")
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(4, 4), (4, 2), (32, 8), (16, 2)])
+@pytest.mark.parametrize("ctxs,bucket,window", [((1,), 256, 0), ((16, 17, 64, 65), 256, 0), ((256, 257, 512, 1000, 3, 700), 1024, 0), ((2049, 4000, 1), 4096, 0),
+                                                ((300, 900), 1024, 100)])
+def test_decode_attention_with_its_rotation(ops, Hq, Hkv, ctxs, bucket, window):
+    """One launch against rotation, attention and sum of the splits as launches of their own: the last key on every place of a page and of a split,
+    splits without keys, a sequence without a slot."""
+    B, D, dev, theta = len(ctxs), 128, "cuda", 500000.0
+    g = torch.Generator(device=dev).manual_seed(B + Hq)
+    nb = [(c + 15) // 16 for c in ctxs]
+    tables = torch.randperm(sum(nb) + 3, device=dev, generator=g)[:sum(nb)].int()
+    begins = torch.tensor([sum(nb[:i]) for i in range(B + 1)], dtype=torch.int32, device=dev)
+    caches = [torch.randn(sum(nb) + 3, Hkv, 16, D, device=dev, generator=g).bfloat16() for _ in range(2)]
+    past = torch.tensor([c - 1 for c in ctxs], dtype=torch.int32, device=dev)
+    slots = torch.tensor([int(tables[int(begins[i]) + (c - 1) // 16]) * 16 + (c - 1) % 16 for i, c in enumerate(ctxs)], dtype=torch.int32, device=dev)
+    if B > 2:
+        slots[1] = -1
+    sub = torch.arange(B + 1, dtype=torch.int32, device=dev)
+    qkv = torch.randn(B, (Hq + 2 * Hkv) * D, device=dev, generator=g).bfloat16()
+    want_kv, qkv2 = [c.clone() for c in caches], qkv.clone()
+    ops.rope_kv_write(qkv2, past, slots, *want_kv, Hq, Hkv, D, theta, 16)
+    want = ops.paged_attention(qkv2, *want_kv, past, sub, tables, begins, Hq, Hkv, D, max_context_len=bucket, max_q_len=1, sliding_window=window)
+    for at in (past, None):
+        kv = [t.clone() for t in (caches if at is not None else want_kv)]
+        got = ops.decode_attention(qkv if at is not None else qkv2, *kv, past, sub, tables, begins, Hq, Hkv, D, at, slots, theta, max_context_len=bucket, sliding_window=window)
+        # the same rows in the cache to the bit; the same products, the splits' sums in another order
+        assert torch.equal(kv[0], want_kv[0]) and torch.equal(kv[1], want_kv[1])
+        assert _rel_err(got, want.double()) < 1e-3
+    ops.check_status("decode attention")
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 16384), (3, 32000), (64, 128256), (147, 16392), (148, 16384), (2, 16387)])
+def test_argmax_in_pieces(ops, rows, vocab):
+    """Ties across the pieces, rows of -inf and NaN, odd tails, both sides of the limits; the token is handed on where it has a place."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    l = torch.randn(rows, vocab, device="cuda", generator=g).bfloat16()
+    l[0, 5000 % vocab] = l[0, vocab - 1] = 50.0
+    if rows > 2:
+        l[1], l[2] = float("-inf"), float("nan")
+        l[2, vocab // 2] = 1.0
+    want = torch.where(l.isnan(), torch.full_like(l, float("-inf")), l).float().argmax(-1)
+    out, top = torch.empty(rows, dtype=torch.int32, device="cuda"), torch.empty(rows, dtype=torch.float32, device="cuda")
+    ops.argmax(l, out=out, out_max=top)
+    assert torch.equal(out.long(), want) and (rows <= 2 or float(top[2]) == 1.0)
+    dst = torch.arange(rows, dtype=torch.int32, device="cuda") * 2 - 2
+    last = torch.full((2 * rows + 1,), -7, dtype=torch.int32, device="cuda")
+    tok = torch.empty(rows, dtype=torch.int32, device="cuda")
+    ops.argmax_scatter(l, tok, dst, last)
+    assert torch.equal(tok, out)
+    keep = torch.full_like(last, -7)
+    keep[dst[1:].long()] = out[1:]
+    assert torch.equal(last, keep)
+    ops.check_status("argmax")
+
+
+def test_step_edges_in_one_launch(ops):
+    """Embedding of resolved ids, and the norm of gathered rows, as the launches that they replace."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    for T, H in ((1, 256), (5, 4096), (700, 8192)):
+        table, gamma = torch.randn(90, H, device="cuda", generator=g).bfloat16(), torch.randn(H, device="cuda", generator=g).bfloat16()
+        ids = torch.randint(-2, 95, (T,), dtype=torch.int32, device="cuda", generator=g)
+        src = torch.randint(-1, 8, (T,), dtype=torch.int32, device="cuda", generator=g)
+        last = torch.randint(0, 90, (8,), dtype=torch.int32, device="cuda", generator=g)
+        ids2 = ids.clone()
+        ops.resolve_ids(ids2, src, last)
+        want = ops.embedding(ids2, table)
+        h = torch.empty(T, H, dtype=torch.bfloat16, device="cuda")
+        ops.embed_tokens(ids, src, last, table, h)
+        assert torch.equal(h, want) and torch.equal(ids, ids2)
+        rows = torch.randint(-1, T + 1, (6,), dtype=torch.int32, device="cuda", generator=g)
+        assert torch.equal(ops.rmsnorm_rows(h, rows, gamma, 1e-5, torch.empty(6, H, dtype=torch.bfloat16, device="cuda")), ops.rmsnorm(ops.embedding(rows, h), gamma, 1e-5))
