@@ -219,11 +219,78 @@ bool gemm_few_takes(const ovb_gemm_args* a);
 int gemm_few(const ovb_gemm_args* a, cudaStream_t stream);
 // Clusters of this many CTAs that the device holds, one CTA of gemm_few.cu's size per SM, asked of the driver once.
 int cluster_capacity(int size);
+// The RMS norm of a product's few rows, by the whole CTA: every thread holds HOLD pieces of eight columns of each of T rows of x (it reads the rows in
+// whole, whatever part of K its CTA has) and calls put(token, piece of eight columns, normalised values). `part`: [warps][TMAX] floats of shared
+// memory. The caller's barrier must follow. Loads come from L2: the rows were written by the kernel before.
+template <int THREADS, int TMAX, int HOLD, class P, class F>
+__device__ __forceinline__ void norm_rows(const P& p, float (*part)[TMAX], F&& put) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pieces = p.K >> 3;
+    uint4 x[TMAX][HOLD], g[HOLD];
+#pragma unroll
+    for (int h = 0; h < HOLD; ++h) {
+        const int k8 = threadIdx.x + h * THREADS;
+        if (k8 < pieces) g[h] = __ldg(reinterpret_cast<const uint4*>(p.x_norm) + k8);
+    }
+#pragma unroll
+    for (int t = 0; t < TMAX; ++t) {
+        if (t >= p.T) break;
+        int row = t;
+        if (p.x_rows != nullptr) {
+            row = p.x_rows[t];
+            if (row < 0 || row >= p.x_count) row = 0;
+        }
+        const uint4* src = reinterpret_cast<const uint4*>(p.x + (size_t)row * p.ldx * 2);
+#pragma unroll
+        for (int h = 0; h < HOLD; ++h) {
+            const int k8 = threadIdx.x + h * THREADS;
+            if (k8 < pieces) x[t][h] = __ldcg(src + k8);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < TMAX; ++t) {
+        if (t >= p.T) break;
+        float ss = 0.f;
+#pragma unroll
+        for (int h = 0; h < HOLD; ++h)
+            if (threadIdx.x + h * THREADS < pieces) {
+                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&x[t][h]);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) ss += __bfloat162float(e[j]) * __bfloat162float(e[j]);
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane == 0) part[warp][t] = ss;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+#pragma unroll
+    for (int t = 0; t < TMAX; ++t) {
+        if (t >= p.T) break;
+        float tot = lane < THREADS / 32 ? part[lane][t] : 0.f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        const float inv = rsqrtf(tot / float(p.K) + p.x_eps);
+#pragma unroll
+        for (int h = 0; h < HOLD; ++h) {
+            const int k8 = threadIdx.x + h * THREADS;
+            if (k8 >= pieces) continue;
+            const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&x[t][h]);
+            const __nv_bfloat16* ge = reinterpret_cast<const __nv_bfloat16*>(&g[h]);
+            uint4 o;
+            __nv_bfloat16* oe = reinterpret_cast<__nv_bfloat16*>(&o);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) oe[j] = __float2bfloat16_rn(__bfloat162float(e[j]) * inv * __bfloat162float(ge[j]));
+            put(t, k8, o);
+        }
+    }
+}
+
 // gemm_ring.cu: products of up to four tokens with u4 weights.
 bool gemm_ring_takes(const ovb_gemm_args* a);
+bool gemm_ring_norms(const ovb_gemm_args* a);
 int gemm_ring(const ovb_gemm_args* a, cudaStream_t stream);
 // gemm_stream.cu: products of few tokens, small ones.
 bool gemm_stream_takes(const ovb_gemm_args* a);
+bool gemm_stream_norms(const ovb_gemm_args* a);
 int gemm_stream(const ovb_gemm_args* a, cudaStream_t stream);
 
 }  // namespace ovb

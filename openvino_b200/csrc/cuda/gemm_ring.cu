@@ -24,6 +24,7 @@ constexpr int kRingTokens = 4;
 constexpr int kRingMaxSlots = 10;
 constexpr int kRingSmem = 216 * 1024;                             // the blocks of a norm fit beside a CTA
 constexpr int kRingMaxX = 64 * 1024;
+constexpr int kRingHold = 2;                                      // pieces of a token that a thread holds for a norm: up to 8192 columns
 
 struct RingParams {
     const uint8_t* w;
@@ -37,6 +38,10 @@ struct RingParams {
     int ring;
     int act, out_f32;
     float act_limit, act_slope, act_shift;
+    const void* x_norm;
+    const int* x_rows;
+    float x_eps;
+    int x_count;
 };
 
 __device__ __forceinline__ void ring_barrier() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
@@ -98,8 +103,15 @@ __global__ void __launch_bounds__(kRingThreads, 1) gemm_ring_kernel(const RingPa
     } else {
         const int half = warp >> 3, g = lane >> 2, t = lane & 3, row0 = (warp & 7) * 16;
         pdl_wait();
-        {
-            // the tokens of this CTA's part of K, in 16-byte pieces
+        // the tokens of this CTA's part of K, in 16-byte pieces
+        if (p.x_norm != nullptr) {
+            __shared__ float squares[16][kRingTokens];
+            norm_rows<512, kRingTokens, kRingHold>(p, squares, [&](int tok, int k8, uint4 v) {
+                const int k = k8 - s0 * 32;
+                if (k >= 0 && k < nks * 32) *reinterpret_cast<uint4*>(xs + ((size_t)(k >> 2) * T + tok) * 64 + (k & 3) * 16) = v;
+            });
+            ring_barrier();
+        } else {
             const int per = nks * 32;                             // pieces of a token
             for (int i = threadIdx.x; i < per * T; i += 512) {
                 const int tok = i / per, k8 = i - tok * per;
@@ -250,6 +262,8 @@ bool gemm_ring_takes(const ovb_gemm_args* a) {
     return ring_plan(a->T, a->N, a->K, &f);
 }
 
+bool gemm_ring_norms(const ovb_gemm_args* a) { return a->K <= kRingHold * 512 * 8; }
+
 int gemm_ring(const ovb_gemm_args* a, cudaStream_t stream) {
     const bool gated = a->act == OVB_ACT_SWIGLU || a->act == OVB_ACT_GLU_LIMITED;
     RingPlan f;
@@ -274,6 +288,10 @@ int gemm_ring(const ovb_gemm_args* a, cudaStream_t stream) {
     p.act_limit = a->act_limit;
     p.act_slope = a->act_slope;
     p.act_shift = a->act_shift;
+    p.x_norm = a->x_norm;
+    p.x_rows = a->x_rows;
+    p.x_eps = a->x_eps;
+    p.x_count = a->x_count;
     {
         static std::mutex mu;
         static uint64_t configured = 0;         // one bit per device

@@ -1460,6 +1460,11 @@ static int comm_packets(int world, int mode) {
 
 int ovb_gemm_route(const ovb_gemm_args* a) { return ovb::gemm_ring_takes(a) || ovb::gemm_stream_takes(a) ? 2 : ovb::gemm_pair_takes(a) ? 1 : 0; }
 
+int ovb_gemm_norms(const ovb_gemm_args* a) {
+    using namespace ovb;
+    return gemm_ring_takes(a) ? gemm_ring_norms(a) : gemm_stream_takes(a) && gemm_stream_norms(a);
+}
+
 int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream_) {
     using namespace ovb;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
@@ -1472,6 +1477,9 @@ int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream_) {
     OVB_REQUIRE(a->block_t == 0 || a->block_t == 16 || a->block_t == 32 || a->block_t == 64 || a->block_t == 128 || a->block_t == 256,
                 "unsupported block_t %d", a->block_t);
     OVB_REQUIRE(((reinterpret_cast<uintptr_t>(a->x) | reinterpret_cast<uintptr_t>(a->w)) & 15) == 0, "ovb_gemm: x and weights must be 16-byte aligned");
+    OVB_REQUIRE(a->x_norm == nullptr || ((reinterpret_cast<uintptr_t>(a->x_norm) & 15) == 0 && ovb_gemm_norms(a)),
+                "ovb_gemm: this product does not take a norm in (ovb_gemm_norms), or its weights are misaligned");
+    OVB_REQUIRE(a->x_rows == nullptr || (a->x_norm != nullptr && a->x_count > 0), "ovb_gemm: row indices belong to a norm");
     const bool f16 = a->wmode == OVB_W_F16;
     const bool quant = is_quant(a->wmode);
     if (quant) {

@@ -26,6 +26,7 @@ namespace ovb {
 
 constexpr int kStreamThreads = 256;
 constexpr int kStreamWarps = 8;
+constexpr int kStreamNormTokens = 4;     // rows that a norm inside the product takes, of up to 2048 columns
 
 struct StreamParams {
     const uint8_t* w;
@@ -41,6 +42,10 @@ struct StreamParams {
     int units, units_per_split;
     int act, out_f32;
     float act_limit, act_slope, act_shift;
+    const void* x_norm;
+    const int* x_rows;
+    float x_eps;
+    int x_count;
 };
 
 constexpr int stream_unit(int wmode) { return wmode == OVB_W_BF16 ? 64 : 128; }      // columns of K in a unit
@@ -160,6 +165,14 @@ __global__ void __launch_bounds__(kStreamThreads, 2) gemm_stream_kernel(const St
     pdl_wait();
     // the tokens of this warp's units: consecutive lanes copy consecutive 16-byte pieces of a token row
     constexpr int PPU = KU / 8;                                  // pieces of a unit
+    if (!F16 && p.x_norm != nullptr) {
+        __shared__ float squares[kStreamWarps][kStreamNormTokens];
+        norm_rows<kStreamThreads, kStreamNormTokens, 1>(p, squares, [&](int n, int k8, uint4 v) {
+            const int lu = k8 / PPU - u0, r = k8 % PPU;
+            if (lu >= 0 && lu < nu_all) *reinterpret_cast<uint4*>(xs + ((size_t)((lu * SP + r % SP) * p.T + n) * 4 + r / SP) * 16) = v;
+        });
+        __syncthreads();
+    } else
     for (int i = 0; i < nu; ++i) {
         const int lu = warp + i * kStreamWarps;
         for (int j = lane; j < p.T * PPU; j += 32) {
@@ -349,6 +362,8 @@ bool gemm_stream_takes(const ovb_gemm_args* a) {
     return pick_stream_split(wm, a->T, a->N, a->K / stream_unit(wm), &smem) > 0;
 }
 
+bool gemm_stream_norms(const ovb_gemm_args* a) { return a->wmode != OVB_W_F16 && a->T <= kStreamNormTokens && a->K <= kStreamThreads * 8; }
+
 template <int WMODE, bool F16>
 static int run_stream(const ovb_gemm_args* a, cudaStream_t stream) {
     const bool swiglu = a->act == OVB_ACT_SWIGLU || a->act == OVB_ACT_GLU_LIMITED;
@@ -374,6 +389,10 @@ static int run_stream(const ovb_gemm_args* a, cudaStream_t stream) {
     p.act_limit = a->act_limit;
     p.act_slope = a->act_slope;
     p.act_shift = a->act_shift;
+    p.x_norm = a->x_norm;
+    p.x_rows = a->x_rows;
+    p.x_eps = a->x_eps;
+    p.x_count = a->x_count;
     int smem = 0;
     const int splits = pick_stream_split(WMODE, a->T, a->N, p.units, &smem);
     p.units_per_split = ceil_div(p.units, splits);

@@ -45,6 +45,25 @@ static int run_gemm(const ovb_llm_step* s, const ovb_llm_weight* w, const void* 
     return ovb_gemm(&a, stream);
 }
 
+// A product of normalised rows (row_idx: of those rows of h): in one launch where the kernel takes the norm in.
+static int run_norm_gemm(ovb_llm_step* s, const ovb_llm_weight* w, const void* gamma, const int* row_idx, int h_rows, void* x, void* out, int T, int out_cols,
+                         ovb_stream_t stream) {
+    ovb_gemm_args a;
+    fill_gemm(&a, s, w, s->h, out, nullptr, T, out_cols);
+    if ((reinterpret_cast<uintptr_t>(gamma) & 15) == 0 && ovb_gemm_norms(&a)) {
+        a.x_norm = gamma;
+        a.x_eps = s->eps;
+        a.x_rows = row_idx;
+        a.x_count = h_rows;
+        return ovb_gemm(&a, stream);
+    }
+    const int rc = row_idx != nullptr ? ovb_rmsnorm_rows(s->h, row_idx, gamma, x, T, w->K, s->eps, h_rows, stream)
+                                      : ovb_rmsnorm(s->h, nullptr, gamma, x, nullptr, T, w->K, s->eps, stream);
+    if (rc != 0) return rc;
+    ++s->launches;
+    return run_gemm(s, w, x, out, nullptr, T, out_cols, stream);
+}
+
 // The shapes that the buffers of the step were made for.
 static int check_layer(const ovb_llm_step* s, const ovb_llm_layer* l, int i) {
     const int q = s->Hq * s->D, rows = (s->Hq + 2 * s->Hkv) * s->D;
@@ -76,10 +95,11 @@ int64_t ovb_llm_scratch_bytes(const ovb_llm_step* s) {
     return most;
 }
 
-int ovb_llm_step_run(const ovb_llm_step* s, ovb_stream_t stream) {
+int ovb_llm_step_run(ovb_llm_step* s, ovb_stream_t stream) {
     using namespace ovb;
     OVB_REQUIRE(s && s->layers && s->T > 0 && s->B > 0, "ovb_llm_step: empty step");
-    const int T = s->T, B = s->B, H = s->hidden, q = s->Hq * s->D, rows = (s->Hq + 2 * s->Hkv) * s->D;
+    s->launches = 0;
+    const int T = s->T, B = s->B, H = s->hidden, rows = (s->Hq + 2 * s->Hkv) * s->D;
     for (int i = 0; i < s->num_layers; ++i)
         if (int rc = check_layer(s, &s->layers[i], i)) return rc;
     OVB_REQUIRE(s->head.K == H && s->head.N <= s->head_cols, "ovb_llm_step: the vocabulary projection is %d x %d", s->head.N, s->head.K);
@@ -87,12 +107,12 @@ int ovb_llm_step_run(const ovb_llm_step* s, ovb_stream_t stream) {
     do {                           \
         const int rc_ = (call);    \
         if (rc_ != 0) return rc_;  \
+        ++s->launches;             \
     } while (0)
     OVB_STEP(ovb_embed_tokens(s->ids, s->tok_src, s->last_token, s->embed, s->h, T, H, s->vocab, stream));
     for (int i = 0; i < s->num_layers; ++i) {
         const ovb_llm_layer* l = &s->layers[i];
-        OVB_STEP(ovb_rmsnorm(s->h, nullptr, l->norm1, s->x, nullptr, T, H, s->eps, stream));
-        OVB_STEP(run_gemm(s, &l->qkv, s->x, s->qkv, nullptr, T, rows, stream));
+        OVB_STEP(run_norm_gemm(s, &l->qkv, l->norm1, nullptr, T, s->x, s->qkv, T, rows, stream));
         ovb_pa_args pa;
         memset(&pa, 0, sizeof(pa));
         pa.q = s->qkv;
@@ -131,18 +151,16 @@ int ovb_llm_step_run(const ovb_llm_step* s, ovb_stream_t stream) {
         else
             OVB_STEP(ovb_paged_attention(&pa, stream));
         OVB_STEP(run_gemm(s, &l->o, s->attn, s->h, s->h, T, H, stream));
-        OVB_STEP(ovb_rmsnorm(s->h, nullptr, l->norm2, s->x, nullptr, T, H, s->eps, stream));
         if (l->gate_up.act == OVB_ACT_SWIGLU) {
-            OVB_STEP(run_gemm(s, &l->gate_up, s->x, s->act, nullptr, T, s->ffn, stream));
+            OVB_STEP(run_norm_gemm(s, &l->gate_up, l->norm2, nullptr, T, s->x, s->act, T, s->ffn, stream));
         } else {
-            OVB_STEP(run_gemm(s, &l->gate_up, s->x, s->gu, nullptr, T, 2 * s->ffn, stream));
+            OVB_STEP(run_norm_gemm(s, &l->gate_up, l->norm2, nullptr, T, s->x, s->gu, T, 2 * s->ffn, stream));
             OVB_STEP(ovb_silu_mul_counted(s->gu, s->act, T, s->ffn, nullptr, stream));
         }
         OVB_STEP(run_gemm(s, &l->down, s->act, s->h, s->h, T, H, stream));
     }
     // logits only for the last token of every sequence
-    OVB_STEP(ovb_rmsnorm_rows(s->h, s->logit_idx, s->final_norm, s->last_x, B, H, s->eps, T, stream));
-    OVB_STEP(run_gemm(s, &s->head, s->last_x, s->logits, nullptr, B, s->head_cols, stream));
+    OVB_STEP(run_norm_gemm(s, &s->head, s->final_norm, s->logit_idx, T, s->last_x, s->logits, B, s->head_cols, stream));
 #undef OVB_STEP
     return 0;
 }

@@ -97,11 +97,19 @@ typedef struct {
     float act_limit, act_slope, act_shift;
     void* scratch;          // memory for expanded weights (ovb_gemm_scratch_bytes), not shared with calls that may overlap; may be NULL
     int64_t scratch_bytes;
+    // RMS norm of the rows of x before the product, where ovb_gemm_norms says that the kernel takes it in: x[t] becomes
+    // bf16(x[t] / sqrt(mean(x[t]^2) + x_eps) * x_norm), with the row x_rows[t] in the place of t when x_rows is given (an index outside [0, x_count) reads row 0).
+    const void* x_norm;     // [K] bf16, or NULL
+    const int* x_rows;
+    float x_eps;
+    int x_count;
 } ovb_gemm_args;
 
 int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream);
 // The kernel that ovb_gemm runs this problem on: 0 single CTAs (gemm_sm100.cu, gemm_few.cu), 1 pairs of CTAs (gemm_pair.cu), 2 few tokens (gemm_ring.cu, gemm_stream.cu).
 int ovb_gemm_route(const ovb_gemm_args* a);
+// 1: ovb_gemm takes x_norm in (products of up to four tokens); the fields x_norm and x_rows themselves are not looked at.
+int ovb_gemm_norms(const ovb_gemm_args* a);
 // The plan of gemm_few.cu for a product: splits of K, clusters, ring stages, token stages, expanding groups, bytes of shared memory. `splits` 0: its
 // own choice. Returns 0 where no plan fits.
 int ovb_gemm_few_plan(int wmode, int T, int N, int K, int splits, int* out);
@@ -336,10 +344,10 @@ typedef struct {
     int64_t gemm_ws_bytes, pa_scratch_bytes, scratch_bytes;
     int num_layers, T, B, hidden, ffn, Hq, Hkv, D, vocab, head_cols, block_size, max_ctx, max_q_len, sliding_window, kv_u8;
     float theta, eps;
-    int reserved;
+    int launches;             // out: operations launched by ovb_llm_step_run
 } ovb_llm_step;
 int64_t ovb_llm_scratch_bytes(const ovb_llm_step* s);
-int ovb_llm_step_run(const ovb_llm_step* s, ovb_stream_t stream);
+int ovb_llm_step_run(ovb_llm_step* s, ovb_stream_t stream);
 
 // Dense (non-paged) bidirectional attention for encoder models: q,k,v [B, S, H, D] fp16/bf16.
 int ovb_sdpa_dense(const void* q, const void* k, const void* v, void* out, int B, int S, int H, int D, int ld,

@@ -42,6 +42,7 @@ class GemmArgs(C.Structure):
         ("group_ldx", C.c_int), ("group_ldo", C.c_int), ("x_cols", C.c_int),
         ("act_limit", C.c_float), ("act_slope", C.c_float), ("act_shift", C.c_float),
         ("scratch", C.c_void_p), ("scratch_bytes", C.c_int64),
+        ("x_norm", C.c_void_p), ("x_rows", C.c_void_p), ("x_eps", C.c_float), ("x_count", C.c_int),
     ]
 
 
@@ -65,7 +66,7 @@ class LlmStep(C.Structure):
     INTS = ("num_layers", "T", "B", "hidden", "ffn", "Hq", "Hkv", "D", "vocab", "head_cols", "block_size", "max_ctx", "max_q_len", "sliding_window", "kv_u8")
     _fields_ = ([("layers", C.c_void_p), ("head", C.c_ubyte * 56)] + [(n, C.c_void_p) for n in POINTERS]
                 + [(n, C.c_int64) for n in ("gemm_ws_bytes", "pa_scratch_bytes", "scratch_bytes")] + [(n, C.c_int) for n in INTS]
-                + [("theta", C.c_float), ("eps", C.c_float), ("reserved", C.c_int)])
+                + [("theta", C.c_float), ("eps", C.c_float), ("launches", C.c_int)])
 
 
 LLM_WEIGHT = "QQQ8i"          # ovb_llm_weight
@@ -348,16 +349,22 @@ class PackedWeight:
 # ------------------------------------------------------------------------------------------ ops
 def gemm(x: torch.Tensor, w: PackedWeight, out: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
          act: int = ACT_NONE, out_f32: bool = False, ws: Optional[Workspace] = None, splits: int = 0,
-         block_t: int = 0, comm=None, glu=None, cap: float = 0.0) -> torch.Tensor:
+         block_t: int = 0, comm=None, glu=None, cap: float = 0.0, norm=None) -> torch.Tensor:
     """out[T, N] = act(x[T, K] @ dequant(W)^T + bias) + residual  on the tcgen05 GEMM.
 
     ``comm`` (a ``parallel.comm.CommStruct``): sum the product over the tensor-parallel ranks inside the epilogue.
+    ``norm`` (weights, eps[, row indices]): RMS norm of the rows (of the indexed rows) of ``x`` before the product, in the product's launch where its kernel takes
+    it in and in one of its own otherwise.
     ``glu`` (limit, slope, shift): parameters of ``ACT_GLU_LIMITED``; ``cap``: bound of ``ACT_SOFTCAP``. fp32 weights (``W_F32``) take the product without
     tensor cores; ``x`` and ``out`` are then fp32."""
     assert x.dim() == 2 and x.stride(1) == 1
-    T, K = x.shape
+    if norm is not None and len(norm) > 2:
+        T, K = norm[2].numel(), x.shape[1]
+    else:
+        T, K = x.shape
     assert K == w.K, (K, w.K)
     if w.mode == W_F32:
+        assert norm is None
         assert residual is None and comm is None
         return _gemm_f32(x, w, out, act, cap)
     if out is None:
@@ -387,6 +394,13 @@ def gemm(x: torch.Tensor, w: PackedWeight, out: Optional[torch.Tensor] = None, r
         scratch = _gemm_scratch(lib().ovb_gemm_scratch_bytes(C.byref(a)), x.device)
         if scratch is not None:
             a.scratch, a.scratch_bytes = scratch.data_ptr(), scratch.numel()
+    if norm is not None:
+        if x.is_contiguous() and lib().ovb_gemm_norms(C.byref(a)):
+            a.x_norm, a.x_eps, a.x_count = norm[0].data_ptr(), norm[1], x.shape[0]
+            a.x_rows = norm[2].data_ptr() if len(norm) > 2 else None
+        else:
+            y = rmsnorm(x.contiguous(), norm[0], norm[1]) if len(norm) < 3 else rmsnorm_rows(x.contiguous(), norm[2], norm[0], norm[1], torch.empty((T, K), dtype=x.dtype, device=x.device))
+            a.x, a.ldx = y.data_ptr(), K
     _check(lib().ovb_gemm(C.byref(a), C.c_void_p(_stream())), "ovb_gemm")
     return out
 

@@ -500,11 +500,10 @@ class CudaLlmExecutor(LlmExecutor):
         cfg, w, ws, T, B = self.cfg, self.w, self.ws, shp.T, shp.B
         if T > sb.Tcap or B > sb.Bcap:
             raise ValueError("a step of %d tokens in %d sequences does not fit buffers of %d and %d" % (T, B, sb.Tcap, sb.Bcap))
-        size, plain = struct.calcsize(K.LLM_LAYER), 0
+        size = struct.calcsize(K.LLM_LAYER)
         layers = C.create_string_buffer(size * len(w.layers))
         for l, lw in enumerate(w.layers):
             gated = getattr(lw.gate_up, "swiglu", False)
-            plain += not gated
             struct.pack_into(K.LLM_LAYER, layers, size * l, *K.llm_weight_words(lw.qkv), *K.llm_weight_words(lw.o),
                              *K.llm_weight_words(lw.gate_up, K.ACT_SWIGLU if gated else K.ACT_NONE), *K.llm_weight_words(lw.down), lw.norm1.data_ptr(),
                              lw.norm2.data_ptr(), self.k_cache[l].data_ptr(), self.v_cache[l].data_ptr(),
@@ -520,8 +519,7 @@ class CudaLlmExecutor(LlmExecutor):
                          1 if self.kv_u8 else 0, cfg.rope_theta, cfg.rms_eps, 0)
         K.llm_step(step, self.device)
         self._sample(sb, B)
-        decode = shp.max_q_len == 1 and cfg.head_dim == 128                       # rotation and sum of the splits inside the attention
-        self.kernel_launches += 3 + (7 if decode and not self.kv_u8 else 8) * len(w.layers) + plain + (1 if self.sampling is None else 2)
+        self.kernel_launches += step.launches + (1 if self.sampling is None else 2)
 
     def _moe_gathered(self, sb: StepBuffers, l: int, T: int, x: torch.Tensor, h: torch.Tensor) -> int:
         """Experts on their own tokens only (prefill-sized batches), without a host round trip: the position of every

@@ -1193,3 +1193,28 @@ def test_step_edges_in_one_launch(ops):
         assert torch.equal(h, want) and torch.equal(ids, ids2)
         rows = torch.randint(-1, T + 1, (6,), dtype=torch.int32, device="cuda", generator=g)
         assert torch.equal(ops.rmsnorm_rows(h, rows, gamma, 1e-5, torch.empty(6, H, dtype=torch.bfloat16, device="cuda")), ops.rmsnorm(ops.embedding(rows, h), gamma, 1e-5))
+
+
+@pytest.mark.parametrize("fmt,N,K", [("u4", 128, 128), ("u4", 1024, 2048), ("u4", 6144, 4096), ("u4", 1280, 8192), ("u4", 4096, 14336), ("u8", 512, 2048), ("f8", 512, 1024),
+                                     ("dense", 512, 2048)])
+@pytest.mark.parametrize("T", [1, 3, 4, 5])
+def test_norm_inside_the_product(ops, fmt, N, K, T):
+    """Products that normalise their rows themselves, at the limits of what a thread holds and with K shared by clusters, against norm and product as
+    two launches: the sums of squares differ in order only, so a normalised value is at most a neighbour away."""
+    import ctypes as C
+    g = torch.Generator(device="cuda").manual_seed(T)
+    w, _ = _weight_and_values(ops, fmt, N, K)
+    h, gamma = torch.randn(T + 3, K, device="cuda", generator=g).bfloat16() * 3, torch.randn(K, device="cuda", generator=g).bfloat16()
+    rows = torch.randint(-1, T + 4, (T,), dtype=torch.int32, device="cuda", generator=g)
+    for norm, x in (((gamma, 1e-5), h[:T]), ((gamma, 1e-5, rows), h)):
+        y = ops.rmsnorm(h[:T], gamma, 1e-5) if len(norm) < 3 else ops.rmsnorm_rows(h, rows, gamma, 1e-5, torch.empty(T, K, dtype=torch.bfloat16, device="cuda"))
+        assert _rel_err(ops.gemm(x, w, out_f32=True, norm=norm), ops.gemm(y, w, out_f32=True).double()) < 2.0 ** -9
+    a = ops.GemmArgs()
+    a.x, a.w, a.out, a.scales = h.data_ptr(), w.w.data_ptr(), h.data_ptr(), w.w.data_ptr()
+    a.T, a.N, a.K, a.ldx, a.group_size, a.wmode, a.w_tiled = T, N, K, K, 128, w.mode, 1 if fmt == "dense" else 0
+    takes = T <= 4 and K <= (8192 if fmt == "u4" and N * K >= 8 << 20 else 2048)
+    assert bool(ops.lib().ovb_gemm_norms(C.byref(a))) == takes
+    if not takes:
+        a.x_norm = gamma.data_ptr()
+        assert ops.lib().ovb_gemm(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)) != 0
+    ops.check_status("norm in a product")
