@@ -1218,3 +1218,30 @@ def test_norm_inside_the_product(ops, fmt, N, K, T):
         a.x_norm = gamma.data_ptr()
         assert ops.lib().ovb_gemm(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)) != 0
     ops.check_status("norm in a product")
+
+
+@pytest.mark.parametrize("V", [16384, 32000, 65537, 128256, 131072])
+@pytest.mark.parametrize("kind", ["spread", "peaked", "masked", "equal", "nan", "inf"])
+def test_sampling_by_a_cluster(ops, V, kind):
+    """A row shared by eight CTAs draws the token that one CTA draws (enough rows go to that kernel): kept sets in one CTA's piece and in all, ties,
+    masked entries, rows without a distribution, a vocabulary that fills the registers and one that is no multiple of eight."""
+    many, few = 131072 // 2700 + 1, 2
+    g = torch.Generator(device="cuda").manual_seed(V)
+    l = torch.randn(1, (V + 7) // 8 * 8, device="cuda", generator=g).bfloat16()[:, :V] * (0.01 if kind == "equal" else 3)
+    if kind == "peaked":
+        l[0, V - 1], l[0, 3] = 60.0, 59.5
+    elif kind == "masked":
+        l[0, 40:] = float("-inf")
+        l[0, V // 2] = torch.finfo(torch.bfloat16).min
+    elif kind == "equal":
+        l[0] = 1.0
+    elif kind == "nan":
+        l[0, 5] = float("nan")
+    elif kind == "inf":
+        l[0, V // 3] = float("inf")
+    rows = torch.empty(many, (V + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :V].copy_(l.expand(many, V))
+    for top_k, top_p, t in ((50, 0.95, 0.8), (1, 1.0, 1.0), (3000, 1.0, 2.0), (5, 0.5, 1.0)):
+        for seed in range(8):
+            one, shared = ops.sample(rows, t, top_k=top_k, top_p=top_p, seed=seed), ops.sample(rows[:few], t, top_k=top_k, top_p=top_p, seed=seed)
+            assert torch.equal(one[:few], shared), (top_k, top_p, seed, one[:few], shared)
+    ops.check_status("sample")
