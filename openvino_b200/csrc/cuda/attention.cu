@@ -1045,6 +1045,23 @@ static int paged_attention(const ovb_pa_args* a, const int* positions, const int
     return ERR_UNSUPPORTED;
 }
 
+int ovb_sdpa_masked(const void* q, const void* k, const void* v, const void* key_bias, int bias_stride, void* out, int B, int S, int H, int D, int ld, float scale,
+                    int is_f16, ovb_stream_t stream) {
+    OVB_REQUIRE(q && k && v && key_bias && out && B > 0 && S > 0 && H > 0, "ovb_sdpa_masked: bad arguments");
+    PaKParams p;
+    memset(&p, 0, sizeof(p));
+    p.q = q; p.out = out; p.k_cache = k; p.v_cache = v;
+    p.B = B; p.T = B * S; p.Hq = H; p.Hkv = H;
+    p.ldq = ld; p.ld_kv = ld; p.dense_S = S;
+    p.key_bias = key_bias;
+    p.bias_stride = bias_stride;
+    p.scale_log2 = scale * 1.4426950408889634f;
+    p.nsplit = 1;
+    const int rc = launch_prefill_tc(p, D, 1, /*paged=*/false, is_f16 != 0, B * ((S + 127) / 128), static_cast<cudaStream_t>(stream));
+    if (rc == ERR_UNSUPPORTED) set_error("ovb_sdpa_masked: head sizes 64 and 128, up to 8192 keys, 16-byte aligned rows");
+    return rc;
+}
+
 int ovb_sdpa_dense(const void* q, const void* k, const void* v, void* out, int B, int S, int H, int D, int ld,
                    float scale, int is_f16, int causal, ovb_stream_t stream_) {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);

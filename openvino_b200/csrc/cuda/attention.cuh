@@ -26,6 +26,9 @@ struct PaKParams {
     int dense_S;
     int ld_kv;
     int causal;
+    // dense mode: added to the scaled scores of key j of sequence b, key_bias[b * bias_stride + j] in the type of q; NULL: nothing
+    const void* key_bias;
+    int bias_stride;
     // u8 KV cache (kv_u8 != 0): k_cache / v_cache hold bytes [block, kv head, slot, D]; k_meta / v_meta hold one fp16 pair
     // (scale, zero point) per (block, kv head, slot): value = (byte - zero point) * scale
     int kv_u8;

@@ -25,6 +25,7 @@
 #include <math_constants.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "attention.cuh"
 #include "common.cuh"
@@ -107,6 +108,7 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* s_work = const_cast<int*>(abort_flag) + 1;   // [2]
+    float* sBias = reinterpret_cast<float*>(bars + 32);   // SRC_DENSE with a bias: of all keys, times log2(e)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = blockIdx.y;
@@ -249,6 +251,14 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const uint32_t lane_base = tmem + (uint32_t(warp * 32) << 16);
         float m_used = -CUDART_INF_F, l_sum = 0.f;
         bool ok = true;
+        const bool biased = SRC == SRC_DENSE && p.key_bias != nullptr;
+        const float scale = biased ? 1.f : p.scale_log2;      // (biased scores are scaled when the bias is added)
+        if (biased) {
+            using E = typename std::conditional<F16, __half, __nv_bfloat16>::type;
+            const E* kb = reinterpret_cast<const E*>(p.key_bias) + (size_t)b * p.bias_stride;
+            for (int i = r; i < ntiles * kBK; i += kBM) sBias[i] = i < kv_total ? float(kb[i]) * 1.4426950408889634f : 0.f;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
         for (int j = 0; j < ntiles && ok; ++j) {
             const int st = j & 1;
             ok = mbar_wait(&s_full[st], (j >> 1) & 1, abort_flag, status);
@@ -273,6 +283,16 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             tmem_ld_wait();
             tc_fence_before_sync();
             mbar_arrive(&s_free[st]);
+            if (biased) {
+#pragma unroll
+                for (int i = 0; i < kBK; i += 4) {
+                    const float4 kb = *reinterpret_cast<const float4*>(sBias + j0 + i);
+                    v[i] = __float_as_uint(fmaf(__uint_as_float(v[i]), p.scale_log2, kb.x));
+                    v[i + 1] = __float_as_uint(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, kb.y));
+                    v[i + 2] = __float_as_uint(fmaf(__uint_as_float(v[i + 2]), p.scale_log2, kb.z));
+                    v[i + 3] = __float_as_uint(fmaf(__uint_as_float(v[i + 3]), p.scale_log2, kb.w));
+                }
+            }
             // maximum of the visible part of the row (four independent chains)
             float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
             if (need_mask) {
@@ -286,7 +306,7 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
                 for (int i = 0; i < kBK; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
             }
-            float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;   // scale > 0: max commutes with scaling
+            float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale;   // scale > 0: max commutes with scaling
             // raise the running maximum only when the tile exceeds it by a factor of 2^8; the rescale of O is warp-collective
             const bool raise = m_tile > m_used + 8.f;
             if (__any_sync(0xffffffffu, raise)) {
@@ -318,8 +338,8 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             float ls[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int i = 0; i < kBK; i += 2) {
-                const float e0 = fast_exp2(fmaf(__uint_as_float(v[i]), p.scale_log2, neg_m));
-                const float e1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, neg_m));
+                const float e0 = fast_exp2(fmaf(__uint_as_float(v[i]), scale, neg_m));
+                const float e1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), scale, neg_m));
                 ls[(i >> 1) & 3] += e0 + e1;
                 v[i >> 1] = pack16<F16>(e0, e1);
             }
@@ -728,17 +748,20 @@ int launch_duo(PaKParams p, int num_q_tiles, cudaStream_t stream) {
     return 0;
 }
 
+constexpr int kMaxBiasedKeys = 8192;
+
 template <int KH, int RH, int VH, int G, int SRC, bool F16>
 int launch_tc_parts(const PaKParams& p, int num_q_tiles, cudaStream_t stream) {
     const int TOK = tile_tokens(G > 0 ? G : p.group);
-    const int smem = kBM * (KH + RH) * 128 + 2 * kBK * (KH + RH + VH) * 128 + 256 + 1024;
+    constexpr int plain = kBM * (KH + RH) * 128 + 2 * kBK * (KH + RH + VH) * 128 + 256 + 1024;
+    const int smem = plain + (SRC == SRC_DENSE && p.key_bias != nullptr ? ceil_div(p.dense_S, kBK) * kBK * 4 : 0);
     auto kern = pa_prefill_tc_kernel<KH, RH, VH, G, SRC, F16>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     OVB_CHECK_CUDA(cudaGetDevice(&dev));
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
-        OVB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        OVB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, plain + (SRC == SRC_DENSE ? kMaxBiasedKeys * 4 : 0)));
         configured.fetch_or(bit, std::memory_order_release);
     }
     const CUtensorMapDataType dt = F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -788,6 +811,7 @@ bool two_query_tiles(int T, int B, int G, int Hkv) {
 
 int launch_prefill_tc(const PaKParams& p, int D, int G, bool paged, bool f16, int num_q_tiles, cudaStream_t stream) {
     if (paged && p.block_size != kPage) return ERR_UNSUPPORTED;
+    if (p.key_bias != nullptr && (paged || p.dense_S > kMaxBiasedKeys)) return ERR_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(p.q) & 15) || (reinterpret_cast<uintptr_t>(p.k_cache) & 15) || (reinterpret_cast<uintptr_t>(p.v_cache) & 15) ||
         (reinterpret_cast<uintptr_t>(p.out) & 15) || p.ldq % 8 != 0 || (!paged && p.ld_kv % 8 != 0))
         return ERR_UNSUPPORTED;

@@ -349,6 +349,10 @@ typedef struct {
 int64_t ovb_llm_scratch_bytes(const ovb_llm_step* s);
 int ovb_llm_step_run(ovb_llm_step* s, ovb_stream_t stream);
 
+// The same with a value per key that is added to its scaled scores (a padding mask): key_bias[b * bias_stride + j], in the type of q; bias_stride 0:
+// one row for all sequences. Up to 8192 keys, not causal.
+int ovb_sdpa_masked(const void* q, const void* k, const void* v, const void* key_bias, int bias_stride, void* out, int B, int S, int H, int D, int ld, float scale,
+                    int is_f16, ovb_stream_t stream);
 // Dense (non-paged) bidirectional attention for encoder models: q,k,v [B, S, H, D] fp16/bf16.
 int ovb_sdpa_dense(const void* q, const void* k, const void* v, void* out, int B, int S, int H, int D, int ld,
                    float scale, int is_f16, int causal, ovb_stream_t stream);

@@ -958,3 +958,15 @@ def sdpa_dense(q, k, v, B, S, H, D, ld, scale=None, causal=False, out=None):
                                 C.c_float(sc), C.c_int(1 if q.dtype == torch.float16 else 0), C.c_int(1 if causal else 0),
                                 C.c_void_p(_stream())), "ovb_sdpa_dense")
     return out
+
+
+def sdpa_masked(q, k, v, key_bias, B, S, H, D, ld, scale=None, out=None):
+    """``sdpa_dense`` with ``key_bias`` ([1 or B, S], the type of q) added to the scaled scores of the keys."""
+    if out is None:
+        out = torch.empty((B * S, H * D), dtype=q.dtype, device=q.device)
+    assert key_bias.is_contiguous() and key_bias.dtype == q.dtype and key_bias.shape in ((B, S), (1, S))
+    _check(lib().ovb_sdpa_masked(C.c_void_p(q.data_ptr()), C.c_void_p(k.data_ptr()), C.c_void_p(v.data_ptr()), C.c_void_p(key_bias.data_ptr()),
+                                 C.c_int(S if key_bias.shape[0] == B else 0), C.c_void_p(out.data_ptr()), C.c_int(B), C.c_int(S), C.c_int(H), C.c_int(D), C.c_int(ld),
+                                 C.c_float(scale if scale is not None else 1.0 / math.sqrt(D)), C.c_int(1 if q.dtype == torch.float16 else 0), C.c_void_p(_stream())),
+           "ovb_sdpa_masked")
+    return out

@@ -862,6 +862,16 @@ def _sdpa(n, ins, ctx):
         pack = lambda t: _dense(t.transpose(1, 2)).reshape(B * S, H * D)
         out = K.sdpa_dense(pack(q), pack(k), pack(v), B, S, H, D, H * D, scale=scale, causal=bool(causal))
         return [out.reshape(B, S, H, D).transpose(1, 2)]
+    if (K is not None and not causal and mask is not None and mask.dim() == 4 and mask.dtype == q.dtype and q.dim() == 4 and q.dtype in (torch.float16, torch.bfloat16)
+            and q.shape[-1] in (64, 128) and q.shape == k.shape == v.shape and k.dtype == v.dtype == q.dtype and len(ins) <= 5
+            and mask.shape[1] == mask.shape[2] == 1 and mask.shape[3] == q.shape[2] <= 8192 and mask.shape[0] in (1, q.shape[0])):
+        # a value per key (a padding mask), added to the scores inside the kernel
+        B, H, S, D = q.shape
+        q, k, v = (_dense(t.transpose(1, 2)).reshape(B * S, H * D) for t in (q, k, v))
+        if all(t.data_ptr() % 16 == 0 for t in (q, k, v)):
+            out = K.sdpa_masked(q, k, v, mask.reshape(mask.shape[0], S).contiguous(), B, S, H, D, H * D, scale=scale)
+            return [out.reshape(B, S, H, D).transpose(1, 2)]
+        q, k, v = (t.reshape(B, S, H, D).transpose(1, 2) for t in (q, k, v))
     return [F.scaled_dot_product_attention(q, k.to(q.dtype), v.to(q.dtype), attn_mask=None if causal else mask, is_causal=bool(causal) and mask is None, scale=scale)]
 
 

@@ -1245,3 +1245,35 @@ def test_sampling_by_a_cluster(ops, V, kind):
             one, shared = ops.sample(rows, t, top_k=top_k, top_p=top_p, seed=seed), ops.sample(rows[:few], t, top_k=top_k, top_p=top_p, seed=seed)
             assert torch.equal(one[:few], shared), (top_k, top_p, seed, one[:few], shared)
     ops.check_status("sample")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,S", [(64, 1), (64, 100), (64, 128), (64, 129), (64, 384), (128, 257), (64, 1500)])
+def test_sdpa_with_a_value_per_key(ops, dtype, D, S):
+    """Padding masks of every kind (-10000, the type's lowest value, -inf, small biases; one row for all sequences), against softmax in 64 bits. A
+    sequence without any visible key gives zeros."""
+    B, H = 3, 2
+    g = torch.Generator(device="cuda").manual_seed(S)
+    qkv = torch.randn(B * S, 3 * H * D, device="cuda", generator=g).to(dtype)
+    q, k, v = (qkv[:, i * H * D:] for i in range(3))
+    lens = torch.tensor([max(1, S // 3), S, max(1, S - 1)], device="cuda")
+    far = torch.arange(S, device="cuda")[None] >= lens[:, None]
+    for kind in ("-10000", "lowest", "-inf", "soft", "shared", "none visible"):
+        bias = torch.zeros(B, S, device="cuda", dtype=dtype)
+        if kind == "soft":
+            bias = torch.randn(B, S, device="cuda", generator=g).to(dtype) * 3
+        elif kind == "shared":
+            bias = torch.randn(1, S, device="cuda", generator=g).to(dtype) * 3
+        else:
+            bias[far] = {"-10000": -10000.0, "lowest": torch.finfo(dtype).min}.get(kind, float("-inf"))
+        if kind == "none visible":
+            bias[1] = float("-inf")
+        out = ops.sdpa_masked(q, k, v, bias, B, S, H, D, 3 * H * D)
+        qd, kd, vd = (t[:, :H * D].reshape(B, S, H, D).transpose(1, 2).double() for t in (q, k, v))
+        want = torch.softmax(qd @ kd.transpose(-1, -2) / D ** 0.5 + bias.double()[:, None, None], -1).nan_to_num(0.0) @ vd
+        # probabilities rounded to 16 bits, and the result once more
+        assert _rel_err(out, want.transpose(1, 2).reshape(B * S, H * D)) < (2.0 ** -9 if dtype == torch.float16 else 2.0 ** -7), kind
+    with pytest.raises(ops.KernelLibraryError):
+        ops.sdpa_masked(torch.zeros(9000, 64, device="cuda", dtype=dtype), *(torch.zeros(9000, 64, device="cuda", dtype=dtype),) * 2,
+                        torch.zeros(1, 9000, device="cuda", dtype=dtype), 1, 9000, 1, 64, 64)
+    ops.check_status("sdpa_masked")
