@@ -78,8 +78,12 @@ __host__ __device__ constexpr int tile_tokens(int g) { return kBM / g / 8 * 8; }
 // KH / RH / VH: 64-column (128-byte) parts of a key row, of its shared second part, and of a value row. A part that reaches past
 // the end of a cache row is filled with zeros by the copy, so any size that is a multiple of 8 is served; what the query tile
 // holds behind a head's columns meets those zeros. GT: query heads per KV head, 0 = at run time (p.group).
+// Dense heads of 64 keep S and P once (256 columns of tensor memory), so that two CTAs share an SM and one's exponentials run beside the other's
+// products; the scores are read twice, 32 at a time, instead of being held. 16 x 384 tokens, 16 heads, with a mask: 49 us with one CTA per SM, 36 here.
+constexpr bool two_dense_ctas(int kh, int rh, int vh, int src) { return src == SRC_DENSE && kh == 1 && rh == 0 && vh == 1; }
+
 template <int KH, int RH, int VH, int GT, int SRC, bool F16>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(192, two_dense_ctas(KH, RH, VH, SRC) ? 2 : 1)
 pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                      const __grid_constant__ CUtensorMap tmR, PaKParams p, int* status) {
     constexpr bool PAGED = SRC != SRC_DENSE;                   // ragged batch with a descriptor
@@ -87,7 +91,8 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int G = GT > 0 ? GT : p.group;
     const int TOK = tile_tokens(G);            // tokens per tile
     constexpr int Q_BYTES = kBM * DK * 2, K_BYTES = kBK * DK * 2, V_BYTES = kBK * DV * 2;
-    constexpr uint32_t TM_S = 0, TM_O = 256, TM_P = 256 + DV;   // tensor-memory columns
+    constexpr int SB = two_dense_ctas(KH, RH, VH, SRC) ? 1 : 2;   // copies of S and P
+    constexpr uint32_t TM_S = 0, TM_O = SB * 128, TM_P = SB * 128 + DV, TM_COLS = SB == 1 ? 256 : 512;   // tensor-memory columns
     constexpr uint32_t IDESC_QK = umma_idesc_f16(kBM, kBK, !F16);
     constexpr uint32_t IDESC_PV = umma_idesc_f16(kBM, DV, !F16) | (1u << 16);   // B operand MN-major
 
@@ -146,7 +151,7 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int b = s_work[0];
     if (b < 0) return;                          // (uniform) nothing allocated yet
     if (warp == 5) {
-        tmem_alloc(tmem_slot, 512);
+        tmem_alloc(tmem_slot, TM_COLS);
         tmem_relinquish();
     }
     tc_fence_before_sync();
@@ -211,33 +216,33 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const uint64_t dq = umma_desc_k_sw128(smem_u32(sQ), 1024);
         for (int j = 0; j <= ntiles && ok; ++j) {
             if (j < ntiles) {
-                const int st = j & 1;
+                const int st = j & 1, sb = j % SB;
                 ok = ok && mbar_wait(&k_full[st], (j >> 1) & 1, abort_flag, status);
-                if (j >= 2) ok = ok && mbar_wait(&s_free[st], ((j >> 1) - 1) & 1, abort_flag, status);
+                if (j >= SB) ok = ok && mbar_wait(&s_free[sb], (j / SB - 1) & 1, abort_flag, status);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint64_t dk = umma_desc_k_sw128(smem_u32(sK + st * K_BYTES), 1024);
 #pragma unroll
                 for (int ks = 0; ks < DK / 16; ++ks) {
                     const uint64_t off = (uint64_t)(((ks >> 2) * (kBM * 128) + (ks & 3) * 32) >> 4);
-                    umma_f16_ss_elect(tmem + TM_S + st * kBK, dq + off, dk + off, IDESC_QK, ks > 0 ? 1u : 0u);
+                    umma_f16_ss_elect(tmem + TM_S + sb * kBK, dq + off, dk + off, IDESC_QK, ks > 0 ? 1u : 0u);
                 }
-                umma_commit_elect(&s_full[st]);
+                umma_commit_elect(&s_full[sb]);
             }
             if (j >= 1) {
-                const int i = j - 1, st = i & 1;
+                const int i = j - 1, st = i & 1, sb = i % SB;
                 ok = ok && mbar_wait(&v_full[st], (i >> 1) & 1, abort_flag, status);
-                ok = ok && mbar_wait(&p_full[st], (i >> 1) & 1, abort_flag, status);
+                ok = ok && mbar_wait(&p_full[sb], (i / SB) & 1, abort_flag, status);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const int keys = min(kBK, kv_end - (kv_start + i * kBK));
                 const int ksteps = (keys + 15) / 16;
                 const uint64_t dv = umma_desc_mn_sw128(smem_u32(sV + st * V_BYTES), kBK * 128, 1024);
                 for (int kk = 0; kk < ksteps; ++kk)
-                    umma_f16_ts_elect(tmem + TM_O, tmem + TM_P + st * 64 + kk * 8, dv + (uint64_t)((kk * 16 * 128) >> 4), IDESC_PV,
+                    umma_f16_ts_elect(tmem + TM_O, tmem + TM_P + sb * 64 + kk * 8, dv + (uint64_t)((kk * 16 * 128) >> 4), IDESC_PV,
                                       (i > 0 || kk > 0) ? 1u : 0u);
                 umma_commit_elect(&kv_empty[st]);
-                umma_commit_elect(&pv_done[st]);
+                umma_commit_elect(&pv_done[sb]);
             }
         }
         __syncwarp();
@@ -260,8 +265,8 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
         for (int j = 0; j < ntiles && ok; ++j) {
-            const int st = j & 1;
-            ok = mbar_wait(&s_full[st], (j >> 1) & 1, abort_flag, status);
+            const int st = j % SB;
+            ok = mbar_wait(&s_full[st], (j / SB) & 1, abort_flag, status);
             if (!ok) break;
             tc_fence_after_sync();
             const int j0 = kv_start + j * kBK;
@@ -275,36 +280,66 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 lo = max(lo, lo_row - j0);
                 if (!row_valid) hi = 0;
             }
-            // The whole row of S goes to registers in one round trip to tensor memory (eight loads in flight, one wait);
-            // S is then free for the QK product of tile j + 2 while this thread still works on the values.
-            uint32_t v[kBK];
+            // 32 scores of the row, biased and masked (SB == 1)
+            auto scores = [&](int c, uint32_t* w) {
+                tmem_ld_x16(lane_base + TM_S + c, w);
+                tmem_ld_x16(lane_base + TM_S + c + 16, w + 16);
+                tmem_ld_wait();
+                if (biased) {
 #pragma unroll
-            for (int c = 0; c < kBK; c += 16) tmem_ld_x16(lane_base + TM_S + st * kBK + c, v + c);
-            tmem_ld_wait();
-            tc_fence_before_sync();
-            mbar_arrive(&s_free[st]);
-            if (biased) {
-#pragma unroll
-                for (int i = 0; i < kBK; i += 4) {
-                    const float4 kb = *reinterpret_cast<const float4*>(sBias + j0 + i);
-                    v[i] = __float_as_uint(fmaf(__uint_as_float(v[i]), p.scale_log2, kb.x));
-                    v[i + 1] = __float_as_uint(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, kb.y));
-                    v[i + 2] = __float_as_uint(fmaf(__uint_as_float(v[i + 2]), p.scale_log2, kb.z));
-                    v[i + 3] = __float_as_uint(fmaf(__uint_as_float(v[i + 3]), p.scale_log2, kb.w));
+                    for (int i = 0; i < 32; i += 4) {
+                        const float4 kb = *reinterpret_cast<const float4*>(sBias + j0 + c + i);
+                        w[i] = __float_as_uint(fmaf(__uint_as_float(w[i]), p.scale_log2, kb.x));
+                        w[i + 1] = __float_as_uint(fmaf(__uint_as_float(w[i + 1]), p.scale_log2, kb.y));
+                        w[i + 2] = __float_as_uint(fmaf(__uint_as_float(w[i + 2]), p.scale_log2, kb.z));
+                        w[i + 3] = __float_as_uint(fmaf(__uint_as_float(w[i + 3]), p.scale_log2, kb.w));
+                    }
                 }
-            }
-            // maximum of the visible part of the row (four independent chains)
-            float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-            if (need_mask) {
+                if (need_mask) {
 #pragma unroll
-                for (int i = 0; i < kBK; ++i) {
-                    const bool vis = i >= lo && i < hi;
-                    if (!vis) v[i] = __float_as_uint(-CUDART_INF_F);
-                    mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
+                    for (int i = 0; i < 32; ++i)
+                        if (c + i < lo || c + i >= hi) w[i] = __float_as_uint(-CUDART_INF_F);
+                }
+            };
+            uint32_t v[SB == 1 ? 32 : kBK];
+            float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+            if constexpr (SB == 1) {
+#pragma unroll 1
+                for (int c = 0; c < kBK; c += 32) {
+                    scores(c, v);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
                 }
             } else {
+                // The whole row of S goes to registers in one round trip to tensor memory (eight loads in flight, one wait);
+                // S is then free for the QK product of tile j + 2 while this thread still works on the values.
 #pragma unroll
-                for (int i = 0; i < kBK; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
+                for (int c = 0; c < kBK; c += 16) tmem_ld_x16(lane_base + TM_S + st * kBK + c, v + c);
+                tmem_ld_wait();
+                tc_fence_before_sync();
+                mbar_arrive(&s_free[st]);
+                if (biased) {
+#pragma unroll
+                    for (int i = 0; i < kBK; i += 4) {
+                        const float4 kb = *reinterpret_cast<const float4*>(sBias + j0 + i);
+                        v[i] = __float_as_uint(fmaf(__uint_as_float(v[i]), p.scale_log2, kb.x));
+                        v[i + 1] = __float_as_uint(fmaf(__uint_as_float(v[i + 1]), p.scale_log2, kb.y));
+                        v[i + 2] = __float_as_uint(fmaf(__uint_as_float(v[i + 2]), p.scale_log2, kb.z));
+                        v[i + 3] = __float_as_uint(fmaf(__uint_as_float(v[i + 3]), p.scale_log2, kb.w));
+                    }
+                }
+                // maximum of the visible part of the row (four independent chains)
+                if (need_mask) {
+#pragma unroll
+                    for (int i = 0; i < kBK; ++i) {
+                        const bool vis = i >= lo && i < hi;
+                        if (!vis) v[i] = __float_as_uint(-CUDART_INF_F);
+                        mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < kBK; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(v[i]));
+                }
             }
             float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale;   // scale > 0: max commutes with scaling
             // raise the running maximum only when the tile exceeds it by a factor of 2^8; the rescale of O is warp-collective
@@ -312,7 +347,7 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             if (__any_sync(0xffffffffu, raise)) {
                 const float factor = !raise ? 1.f : (m_used == -CUDART_INF_F ? 0.f : fast_exp2(m_used - m_tile));
                 if (j > 0) {
-                    ok = mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag, status);
+                    ok = mbar_wait(&pv_done[(j - 1) % SB], ((j - 1) / SB) & 1, abort_flag, status);
                     if (!ok) break;
                     tc_fence_after_sync();
 #pragma unroll 1
@@ -333,24 +368,47 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                     m_used = m_tile;
                 }
             }
-            // exponentials (masked entries are -inf: exp2 gives 0), row sum, P as 16-bit pairs (packed in place)
             const float neg_m = (m_used == -CUDART_INF_F) ? 0.f : -m_used;
             float ls[4] = {0.f, 0.f, 0.f, 0.f};
+            if constexpr (SB == 1) {
+                // P of the tile before must have been consumed
+                if (j >= 1) {
+                    ok = mbar_wait(&pv_done[0], (j - 1) & 1, abort_flag, status);
+                    if (!ok) break;
+                }
+#pragma unroll 1
+                for (int c = 0; c < kBK; c += 32) {
+                    scores(c, v);
 #pragma unroll
-            for (int i = 0; i < kBK; i += 2) {
-                const float e0 = fast_exp2(fmaf(__uint_as_float(v[i]), scale, neg_m));
-                const float e1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), scale, neg_m));
-                ls[(i >> 1) & 3] += e0 + e1;
-                v[i >> 1] = pack16<F16>(e0, e1);
-            }
-            l_sum += (ls[0] + ls[1]) + (ls[2] + ls[3]);
-            // P of tile j - 2 (same buffer) must have been consumed
-            if (j >= 2) {
-                ok = mbar_wait(&pv_done[st], ((j >> 1) - 1) & 1, abort_flag, status);
-                if (!ok) break;
-            }
+                    for (int i = 0; i < 32; i += 2) {
+                        const float e0 = fast_exp2(fmaf(__uint_as_float(v[i]), scale, neg_m));
+                        const float e1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), scale, neg_m));
+                        ls[(i >> 1) & 3] += e0 + e1;
+                        v[i >> 1] = pack16<F16>(e0, e1);
+                    }
+                    tmem_st_x16(lane_base + TM_P + c / 2, v);
+                }
+                l_sum += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+                tc_fence_before_sync();
+                mbar_arrive(&s_free[0]);
+            } else {
+                // exponentials (masked entries are -inf: exp2 gives 0), row sum, P as 16-bit pairs (packed in place)
 #pragma unroll
-            for (int c = 0; c < kBK / 2; c += 16) tmem_st_x16(lane_base + TM_P + st * 64 + c, v + c);
+                for (int i = 0; i < kBK; i += 2) {
+                    const float e0 = fast_exp2(fmaf(__uint_as_float(v[i]), scale, neg_m));
+                    const float e1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), scale, neg_m));
+                    ls[(i >> 1) & 3] += e0 + e1;
+                    v[i >> 1] = pack16<F16>(e0, e1);
+                }
+                l_sum += (ls[0] + ls[1]) + (ls[2] + ls[3]);
+                // P of tile j - 2 (same buffer) must have been consumed
+                if (j >= 2) {
+                    ok = mbar_wait(&pv_done[st], ((j >> 1) - 1) & 1, abort_flag, status);
+                    if (!ok) break;
+                }
+#pragma unroll
+                for (int c = 0; c < kBK / 2; c += 16) tmem_st_x16(lane_base + TM_P + st * 64 + c, v + c);
+            }
             tmem_st_wait();
             tc_fence_before_sync();
             mbar_arrive(&p_full[st]);
@@ -373,7 +431,7 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             for (int c = 0; c < DV / 8; ++c)
                 if (c * 8 < p.dv_store) gw[c] = gate[c];
         }
-        if (ok && ntiles > 0) ok = mbar_wait(&pv_done[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1, abort_flag, status);
+        if (ok && ntiles > 0) ok = mbar_wait(&pv_done[(ntiles - 1) % SB], ((ntiles - 1) / SB) & 1, abort_flag, status);
         if (ok) {
             tc_fence_after_sync();
             if (sink != -CUDART_INF_F && m_used != -CUDART_INF_F) l_sum += exp2f(sink - m_used);
@@ -421,7 +479,7 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     if (warp == 5) {
         tc_fence_after_sync();
-        tmem_dealloc(tmem, 512);
+        tmem_dealloc(tmem, TM_COLS);
     }
 }
 
