@@ -6,11 +6,12 @@
 // tensor memory (2 x 256 columns): the epilogue of a tile runs under the main loop of the next.
 //  * warp 0: TMA producer; both CTAs report their bytes on the barrier of the even CTA, whose warp 1 issues the MMAs of the pair
 //  * warps 4 .. 11: epilogue, straight from the accumulator to global memory (no staging of the tile)
-//  * the token tile is any multiple of 32 up to 256, chosen on the host so that the last wave of tiles is nearly full
+//  * the token tile is any multiple of 32 up to 256, chosen on the host so that the last wave of tiles is nearly full; the tiles of one that
+//    is not are cut (pick_pair_tile)
 // Quantised weights are expanded into 16-bit tiles first, a piece of at most kScratchBytes at a time, where that takes less time than the
 // fused expansion of gemm_sm100.cu, which is repeated for every token tile (expansion_pays).
 // Measured on B200, one launch, T = 8192, 28672 x 4096 int8 weights with the fused gate: 2452 us in the single-CTA kernel, 1274 us here
-// (expansion included, 1.51 PFLOP/s); T = 999, the same in bf16: 271 -> 197 us; top-2 of 8 experts, 4096 rows, 28672 x 4096: 969 -> 799 us.
+// (expansion included, 1.51 PFLOP/s); T = 999, the same in bf16: 271 -> 159 us; top-2 of 8 experts, 4096 rows, 28672 x 4096: 969 -> 799 us.
 // Counters (2048 tokens, bf16, 1.54 PFLOP/s): tensor pipe 85 % of the cycles, weights and tokens read once.
 #include <mutex>
 
@@ -35,6 +36,7 @@ struct PairParams {
     int T, N, K;
     int ldo, ldr;
     int bt;
+    int full_tiles, cut;                            // (not grouped) tiles from full_tiles on are cut into `cut` parts along the tokens
     int kb_stride;                                  // chunks between consecutive weight tiles
     int num_groups, group_mode;
     int act, out_f32;
@@ -45,6 +47,7 @@ struct PairTile {
     int n0;            // first weight row of the pair
     int t0, t_end;     // first token row, one past the last valid one
     int w_tile, w_kb;  // first weight tile of the pair and first k-block in the stack
+    int bt;            // tokens of the tile
     bool valid;
 };
 
@@ -56,16 +59,24 @@ __device__ __forceinline__ void pair_coords(int idx, int tiles_n, int tiles_t, i
     n = band * kPairBand + (r - t * in_band);
 }
 
+template <bool CUT>
 __device__ __forceinline__ PairTile pair_tile(const PairParams& p, int idx) {
     const int tiles_n = (p.N + 255) / 256;
     PairTile r;
     int n, t;
     r.w_kb = 0;
+    r.bt = p.bt;
     if (p.group_off == nullptr) {
         const int tiles_t = (p.T + p.bt - 1) / p.bt;
+        int part = 0;
+        if (CUT && idx >= p.full_tiles) {
+            part = (idx - p.full_tiles) % p.cut;
+            idx = p.full_tiles + (idx - p.full_tiles) / p.cut;
+            r.bt = p.bt / p.cut;
+        }
         r.valid = idx < tiles_n * tiles_t;
         pair_coords(r.valid ? idx : 0, tiles_n, tiles_t, n, t);
-        r.t0 = t * p.bt;
+        r.t0 = t * p.bt + part * r.bt;
         r.t_end = p.T;
         r.w_tile = n * 2;
     } else {
@@ -114,9 +125,9 @@ __device__ __forceinline__ void pair_commit_elect(uint64_t* bar) {
         ::"r"(smem_u32(bar)), "h"((uint16_t)3)
         : "memory");
 }
-template <bool F16>
+template <bool F16, bool CUT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const PairParams p) {
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const PairParams p, const __grid_constant__ CUtensorMap tmCut) {
     using E = typename Elem<F16>::type;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -163,25 +174,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
     if (warp == 0) {
         if (lane == 0) {
-            const uint32_t tx = 2u * (TILE_N * 128 + (p.bt / 2) * 128);
             const int tiles_n128 = p.N / TILE_N;
             int s = 0;
             uint32_t phase = 1;
             bool ok = true;
             for (int idx = first; ok; idx += pairs) {
-                const PairTile t = pair_tile(p, idx);
+                const PairTile t = pair_tile<CUT>(p, idx);
                 if (!t.valid) break;
                 // an odd last tile: the second CTA loads the first one's rows again and stores nothing
                 const int own = (t.n0 / TILE_N + (int)rank) < tiles_n128 ? (int)rank : 0;
                 int w_row = ((t.w_tile + own) * p.kb_stride + t.w_kb) * TILE_N;
-                const int x_row = t.t0 + (int)rank * (p.bt / 2);
+                const int x_row = t.t0 + (int)rank * (t.bt / 2);
+                const uint32_t tx = 2u * (TILE_N * 128 + (t.bt / 2) * 128);
+                const CUtensorMap* tm = !CUT || t.bt == p.bt ? &tmX : &tmCut;
                 for (int kb = 0; kb < num_kb; ++kb) {
                     ok = mbar_wait(&empty[s], phase, abort_flag, p.status);
                     if (!ok) break;
                     const uint32_t st = smem_u32(smem) + s * kPairStageBytes, bar = smem_u32(&full[s]);
                     if (rank == 0) mbar_arrive_expect_tx(&full[s], tx);
                     pair_load_2d(st, &tmW, bar, 0, w_row);
-                    pair_load_2d(st + TILE_N * 128, &tmX, bar, kb * TILE_K, x_row);
+                    pair_load_2d(st + TILE_N * 128, tm, bar, kb * TILE_K, x_row);
                     w_row += TILE_N;
                     if (++s == kPairStages) { s = 0; phase ^= 1; }
                 }
@@ -191,13 +203,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         __syncwarp();
     } else if (warp == 1) {
         if (rank == 0) {
-            const uint32_t idesc = umma_idesc_f16(256, p.bt, !F16);
             const uint64_t desc0 = umma_desc_k_sw128(smem_u32(smem), 1024);
             int s = 0, buf = 0;
             uint32_t phase = 0, acc_phase = 1;
             bool ok = true;
             for (int idx = first; ok; idx += pairs) {
-                if (!pair_tile(p, idx).valid) break;
+                const PairTile t = pair_tile<CUT>(p, idx);
+                if (!t.valid) break;
+                const uint32_t idesc = umma_idesc_f16(256, t.bt, !F16);
                 ok = mbar_wait(&acc_empty[buf], acc_phase, abort_flag, p.status);
                 if (!ok) break;
                 tc_fence_after_sync();
@@ -220,15 +233,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         __syncwarp();
     } else if (warp >= 4) {
         const int q = warp & 3, half = (warp - 4) >> 2;
-        const int cols = p.bt / 2, cbeg = half * cols;           // this warp's token columns
         const int odd = lane & 1;
         const bool gated = p.act == OVB_ACT_SWIGLU || p.act == OVB_ACT_GLU_LIMITED;
         const uint32_t drained0 = dsmem_addr(smem_u32(&acc_empty[0]), 0);
         int buf = 0;
         uint32_t acc_phase = 0;
         for (int idx = first;; idx += pairs) {
-            const PairTile t = pair_tile(p, idx);
+            const PairTile t = pair_tile<CUT>(p, idx);
             if (!t.valid) break;
+            const int cols = t.bt / 2, cbeg = half * cols;       // this warp's token columns
             const int n0 = t.n0 + (int)rank * TILE_N;
             const bool store = n0 < p.N;
             const int oc = n0 + q * 32 + lane;
@@ -404,7 +417,8 @@ static int resident_pairs(int* pairs) {
     OVB_CHECK_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(mu);
     if (known[dev & 63] == 0) {
-        auto kern = gemm_pair_kernel<F16>;
+        auto kern = gemm_pair_kernel<F16, false>;
+        OVB_CHECK_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<F16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
         OVB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
         cudaLaunchConfig_t cfg;
         memset(&cfg, 0, sizeof(cfg));
@@ -419,19 +433,41 @@ static int resident_pairs(int* pairs) {
     return 0;
 }
 
+// The last wave, when it would leave most pairs idle: its tiles are cut along the tokens, into parts of a multiple of 32 and so few that each pair
+// has at most one.
+static int pick_cut(int bt, int rest, int pairs) {
+    int best = 1;
+    for (int f = 2; f <= 8; ++f)
+        if (rest > 0 && rest * f <= pairs && bt % (32 * f) == 0) best = f;
+    return best;
+}
+
 // Token tile: the smallest estimate of waves x (tile + 32); the constant stands for what a wave costs beside its MMAs (the pair that
 // finishes last, the epilogue of the last tile). With 999 tokens a 256-token tile of the 4096 x 4096 product fills 64 of 74 pairs
 // once, 6144 rows fill them 1.3 times and take 192-token tiles (two full waves) instead.
-static int pick_pair_tile(int T, int N, int groups, int pairs) {
+// A cut last wave has to be cheaper by 4 %: its parts read the weights once each. us without / with it, gate and up of 28672 x 4096:
+// 512 tokens 101 / 87, 999: 168 / 159, 2048: 315 / 309; 4096 x 14336, 4096 tokens: 346 / 324. Where nearly every pair has a tile it costs as
+// much as it gives (4096 x 4096, 1024 tokens, one cut wave of 64 tiles: 31 / 34 us), and so it does where the sum is short (4096 x 1024,
+// 4096 tokens: 36.3 / 37.0).
+constexpr int kCutMinK = 2048;
+static int pick_pair_tile(int T, int N, int K, int groups, int pairs, int* cut) {
     const int tiles_n = ceil_div(N, 256);
-    int best = 256;
+    int best = 256, best_cut = 1;
     double best_t = 1e30;
     for (int bt = 256; bt >= 64; bt -= 32) {
-        double tiles = groups > 0 ? (double)groups * tiles_n * ((double)T / groups / bt + 0.5) : (double)tiles_n * ceil_div(T, bt);
+        const double tiles = groups > 0 ? (double)groups * tiles_n * ((double)T / groups / bt + 0.5) : (double)tiles_n * ceil_div(T, bt);
         const double waves = groups > 0 ? tiles / pairs + 0.5 : (double)ceil_div((int)tiles, pairs);
         const double t = waves * (bt + 32);
         if (t < best_t * 0.999) { best_t = t; best = bt; }
     }
+    if (cut == nullptr || K < kCutMinK || (int64_t)tiles_n * ceil_div(T, 64) > (1 << 24)) return best;
+    best_t *= 0.96;
+    for (int bt = 256; bt >= 64; bt -= 32) {
+        const int tiles = tiles_n * ceil_div(T, bt), parts = tiles < pairs ? 1 : pick_cut(bt, tiles % pairs, pairs);
+        const double t = (double)(tiles / pairs) * (bt + 32) + bt / parts + 64;
+        if (parts > 1 && t < best_t) { best_t = t; best = bt; best_cut = parts; }
+    }
+    *cut = best_cut;
     return best;
 }
 
@@ -470,7 +506,7 @@ static bool expansion_pays(const ovb_gemm_args* a) {
     const double k_us = a->K * 1e-3, fused_wave = (u4 ? 3.5 : 0.0) + (gated ? 10.0 : 0.0) + k_us * (u4 ? 6.2 : a->wmode == OVB_W_U8 ? 10.6 : 11.0);
     const double fused = ceil_div(ceil_div(a->N, TILE_N) * ceil_div(a->T, 256), kSMs) * fused_wave;
     // expanded: launches and bytes of the expansion, waves of 256 x bt tiles of every piece
-    const int bt = pick_pair_tile(a->T, a->N, 0, kPairs), piece = pick_piece(a->T, a->N, a->K, bt, kPairs, kScratchBytes);
+    const int bt = pick_pair_tile(a->T, a->N, a->K, 0, kPairs, nullptr), piece = pick_piece(a->T, a->N, a->K, bt, kPairs, kScratchBytes);
     if (piece <= 0) return false;
     int pieces = 0, waves = 0;
     for (int n = 0; n < a->N; n += piece, ++pieces) waves += ceil_div(ceil_div(a->N - n < piece ? a->N - n : piece, 256) * ceil_div(a->T, bt), kPairs);
@@ -522,7 +558,8 @@ static int run_pair(const ovb_gemm_args* a, cudaStream_t stream) {
     p.K = a->K;
     p.ldo = a->ldo ? a->ldo : (swiglu ? a->N / 2 : a->N);
     p.ldr = a->ldr ? a->ldr : a->N;
-    p.bt = pick_pair_tile(a->T, a->N, grouped ? a->num_groups : 0, pairs);
+    p.cut = 1;
+    p.bt = pick_pair_tile(a->T, a->N, a->K, grouped ? a->num_groups : 0, pairs, grouped || quant ? nullptr : &p.cut);
     p.num_groups = a->num_groups;
     p.group_mode = a->group_mode;
     p.act = a->act;
@@ -532,7 +569,7 @@ static int run_pair(const ovb_gemm_args* a, cudaStream_t stream) {
     p.act_shift = a->act_shift;
     const int KB = a->K / TILE_K;
     const CUtensorMapDataType dt16 = F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    CUtensorMap tmW, tmX;
+    CUtensorMap tmW, tmX, tmCut;
     const int ldx = a->ldx ? a->ldx : a->K;
     if (int rc = make_tmap_2d(&tmX, a->x, dt16, 2, a->T, a->K, (uint64_t)ldx * 2, p.bt / 2, TILE_K, true)) return rc;
     const int piece = quant ? pick_piece(a->T, a->N, a->K, p.bt, pairs, a->scratch_bytes) : a->N;
@@ -569,9 +606,14 @@ static int run_pair(const ovb_gemm_args* a, cudaStream_t stream) {
         p.bias = a->bias ? static_cast<const uint8_t*>(a->bias) + (size_t)n * 2 : nullptr;
         p.residual = a->residual ? static_cast<const uint8_t*>(a->residual) + (size_t)n * 2 : nullptr;
         // every group may end with a partial row tile
-        const int64_t tiles = (int64_t)ceil_div(rows, 256) * (ceil_div(a->T, p.bt) + (grouped ? a->num_groups : 0));
+        int64_t tiles = (int64_t)ceil_div(rows, 256) * (ceil_div(a->T, p.bt) + (grouped ? a->num_groups : 0));
+        p.full_tiles = p.cut > 1 ? (int)(tiles / pairs * pairs) : 0;
+        tmCut = tmX;
+        if (p.cut > 1) tiles = p.full_tiles + (tiles - p.full_tiles) * p.cut;
+        if (p.cut > 1)
+            if (int rc = make_tmap_2d(&tmCut, a->x, dt16, 2, a->T, a->K, (uint64_t)ldx * 2, p.bt / p.cut / 2, TILE_K, true)) return rc;
         const int grid = 2 * (int)(tiles < pairs ? tiles : pairs);
-        OVB_CHECK_CUDA(launch_pdl(gemm_pair_kernel<F16>, dim3(grid), dim3(kPairThreads), kPairSmem, stream, tmW, tmX, p));
+        OVB_CHECK_CUDA(launch_pdl(p.cut > 1 ? gemm_pair_kernel<F16, true> : gemm_pair_kernel<F16, false>, dim3(grid), dim3(kPairThreads), kPairSmem, stream, tmW, tmX, p, tmCut));
         OVB_CHECK_CUDA(cudaGetLastError());
     }
     return 0;

@@ -848,6 +848,20 @@ def test_gemm_runs_without_scratch_memory(ops, monkeypatch):
     ops.check_status("gemm")
 
 
+@pytest.mark.parametrize("T,N,dtype", [(256, 19200, torch.bfloat16), (225, 19200, torch.float16), (999, 28672, torch.bfloat16), (512, 28544, torch.bfloat16), (4033, 4096, torch.float16)])
+def test_gemm_pair_cut_wave(ops, T, N, dtype):
+    """Products whose last wave is cut along the tokens (one tile in eight parts, parts behind the last token, an odd number of 128-row tiles):
+    the same sums in the same order as in whole tiles, up to the order of the single-CTA kernel."""
+    K = 2048
+    x = torch.randn(T, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(T)).to(dtype)
+    w = _pair_weight(ops, "dense", N, K, dtype)
+    res = torch.randn(T, N, device="cuda").to(dtype)
+    for kw in (dict(), dict(residual=res), dict(act=ops.ACT_SWIGLU), dict(out_f32=True)):
+        a, b = ops.gemm(x, w, **kw), ops.gemm(x, w, block_t=256, **kw)
+        assert a.shape == b.shape and _rel_err(a, b) < (1e-5 if kw.get("out_f32") else PAIR_REL), kw
+    ops.check_status("gemm_pair")
+
+
 def test_gemm_pair_fp16_window_and_groups(ops):
     torch.manual_seed(2)
     x = torch.randn(700, 512, device="cuda", dtype=torch.float16)
