@@ -11,7 +11,7 @@
 // Quantised weights are expanded into 16-bit tiles first, a piece of at most kScratchBytes at a time, where that takes less time than the
 // fused expansion of gemm_sm100.cu, which is repeated for every token tile (expansion_pays).
 // Measured on B200, one launch, T = 8192, 28672 x 4096 int8 weights with the fused gate: 2452 us in the single-CTA kernel, 1274 us here
-// (expansion included, 1.51 PFLOP/s); T = 999, the same in bf16: 271 -> 159 us; top-2 of 8 experts, 4096 rows, 28672 x 4096: 969 -> 799 us.
+// (expansion included, 1.51 PFLOP/s); T = 999, the same in bf16: 271 -> 159 us; top-2 of 8 experts, 4096 rows, 28672 x 4096: 969 -> 728 us.
 // Counters (2048 tokens, bf16, 1.54 PFLOP/s): tensor pipe 85 % of the cycles, weights and tokens read once.
 #include <mutex>
 
@@ -43,6 +43,14 @@ struct PairParams {
     float act_limit, act_slope, act_shift;
 };
 
+// Forms of the kernel: whole tiles; tiles of the last wave cut along the tokens; groups, whose rows are shared out evenly among as many tiles as
+// they need, each as wide as that. (Groups of about 512 rows need two tiles of 256 or three of 192; tiles of 256 and a rest cost three of 256.) The
+// token box that is loaded stays p.bt / 2 rows: boxes of 16 rows, as many as the tile has, took 1390 us where one wide box takes 817 (8 experts,
+// 4096 rows, 28672 x 4096). us with equal tiles -> even
+// ones: that product 780 -> 728, 4096 x 14336 443 -> 390 (341 with 512 rows in each group); 64 experts, 8192 rows, 3072 x 2048: 275 -> 185; 128
+// experts, 32768 rows, 1536 x 2048: 454 -> 318; 8 experts, 16384 rows, 4096 x 14336: the same. 256 is the best limit: with 192 the first took 813.
+constexpr int kPairWhole = 0, kPairCut = 1, kPairEven = 2;
+
 struct PairTile {
     int n0;            // first weight row of the pair
     int t0, t_end;     // first token row, one past the last valid one
@@ -59,7 +67,7 @@ __device__ __forceinline__ void pair_coords(int idx, int tiles_n, int tiles_t, i
     n = band * kPairBand + (r - t * in_band);
 }
 
-template <bool CUT>
+template <int FORM>
 __device__ __forceinline__ PairTile pair_tile(const PairParams& p, int idx) {
     const int tiles_n = (p.N + 255) / 256;
     PairTile r;
@@ -69,7 +77,7 @@ __device__ __forceinline__ PairTile pair_tile(const PairParams& p, int idx) {
     if (p.group_off == nullptr) {
         const int tiles_t = (p.T + p.bt - 1) / p.bt;
         int part = 0;
-        if (CUT && idx >= p.full_tiles) {
+        if (FORM == kPairCut && idx >= p.full_tiles) {
             part = (idx - p.full_tiles) % p.cut;
             idx = p.full_tiles + (idx - p.full_tiles) / p.cut;
             r.bt = p.bt / p.cut;
@@ -91,7 +99,11 @@ __device__ __forceinline__ PairTile pair_tile(const PairParams& p, int idx) {
         r.valid = g < p.num_groups;
         if (!r.valid) return r;
         pair_coords(idx - acc, tiles_n, (end - begin + p.bt - 1) / p.bt, n, t);
-        r.t0 = begin + t * p.bt;
+        if (FORM == kPairEven) {
+            const int rows = end - begin, n_t = (rows + p.bt - 1) / p.bt;
+            r.bt = ((rows + n_t - 1) / n_t + 31) & ~31;         // at most p.bt; n_t tiles of this width hold all rows, n_t - 1 do not
+        }
+        r.t0 = begin + t * r.bt;
         r.t_end = end;
         r.w_tile = n * 2 + (p.group_mode == 1 ? g * (p.N / TILE_N) : 0);
         r.w_kb = p.group_mode == 2 ? g * (p.K / TILE_K) : 0;
@@ -125,7 +137,7 @@ __device__ __forceinline__ void pair_commit_elect(uint64_t* bar) {
         ::"r"(smem_u32(bar)), "h"((uint16_t)3)
         : "memory");
 }
-template <bool F16, bool CUT>
+template <bool F16, int FORM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const PairParams p, const __grid_constant__ CUtensorMap tmCut) {
     using E = typename Elem<F16>::type;
@@ -179,14 +191,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             uint32_t phase = 1;
             bool ok = true;
             for (int idx = first; ok; idx += pairs) {
-                const PairTile t = pair_tile<CUT>(p, idx);
+                const PairTile t = pair_tile<FORM>(p, idx);
                 if (!t.valid) break;
                 // an odd last tile: the second CTA loads the first one's rows again and stores nothing
                 const int own = (t.n0 / TILE_N + (int)rank) < tiles_n128 ? (int)rank : 0;
                 int w_row = ((t.w_tile + own) * p.kb_stride + t.w_kb) * TILE_N;
                 const int x_row = t.t0 + (int)rank * (t.bt / 2);
-                const uint32_t tx = 2u * (TILE_N * 128 + (t.bt / 2) * 128);
-                const CUtensorMap* tm = !CUT || t.bt == p.bt ? &tmX : &tmCut;
+                const uint32_t tx = 2u * (TILE_N * 128 + ((FORM == kPairEven ? p.bt : t.bt) / 2) * 128);
+                const CUtensorMap* tm = FORM != kPairCut || t.bt == p.bt ? &tmX : &tmCut;
                 for (int kb = 0; kb < num_kb; ++kb) {
                     ok = mbar_wait(&empty[s], phase, abort_flag, p.status);
                     if (!ok) break;
@@ -208,7 +220,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
             uint32_t phase = 0, acc_phase = 1;
             bool ok = true;
             for (int idx = first; ok; idx += pairs) {
-                const PairTile t = pair_tile<CUT>(p, idx);
+                const PairTile t = pair_tile<FORM>(p, idx);
                 if (!t.valid) break;
                 const uint32_t idesc = umma_idesc_f16(256, t.bt, !F16);
                 ok = mbar_wait(&acc_empty[buf], acc_phase, abort_flag, p.status);
@@ -239,7 +251,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         int buf = 0;
         uint32_t acc_phase = 0;
         for (int idx = first;; idx += pairs) {
-            const PairTile t = pair_tile<CUT>(p, idx);
+            const PairTile t = pair_tile<FORM>(p, idx);
             if (!t.valid) break;
             const int cols = t.bt / 2, cbeg = half * cols;       // this warp's token columns
             const int n0 = t.n0 + (int)rank * TILE_N;
@@ -417,8 +429,9 @@ static int resident_pairs(int* pairs) {
     OVB_CHECK_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(mu);
     if (known[dev & 63] == 0) {
-        auto kern = gemm_pair_kernel<F16, false>;
-        OVB_CHECK_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<F16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
+        auto kern = gemm_pair_kernel<F16, kPairWhole>;
+        OVB_CHECK_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<F16, kPairCut>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
+        OVB_CHECK_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<F16, kPairEven>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
         OVB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem));
         cudaLaunchConfig_t cfg;
         memset(&cfg, 0, sizeof(cfg));
@@ -450,14 +463,12 @@ static int pick_cut(int bt, int rest, int pairs) {
 // much as it gives (4096 x 4096, 1024 tokens, one cut wave of 64 tiles: 31 / 34 us), and so it does where the sum is short (4096 x 1024,
 // 4096 tokens: 36.3 / 37.0).
 constexpr int kCutMinK = 2048;
-static int pick_pair_tile(int T, int N, int K, int groups, int pairs, int* cut) {
+static int pick_pair_tile(int T, int N, int K, int pairs, int* cut) {
     const int tiles_n = ceil_div(N, 256);
     int best = 256, best_cut = 1;
     double best_t = 1e30;
     for (int bt = 256; bt >= 64; bt -= 32) {
-        const double tiles = groups > 0 ? (double)groups * tiles_n * ((double)T / groups / bt + 0.5) : (double)tiles_n * ceil_div(T, bt);
-        const double waves = groups > 0 ? tiles / pairs + 0.5 : (double)ceil_div((int)tiles, pairs);
-        const double t = waves * (bt + 32);
+        const double t = (double)ceil_div(tiles_n * ceil_div(T, bt), pairs) * (bt + 32);
         if (t < best_t * 0.999) { best_t = t; best = bt; }
     }
     if (cut == nullptr || K < kCutMinK || (int64_t)tiles_n * ceil_div(T, 64) > (1 << 24)) return best;
@@ -506,7 +517,7 @@ static bool expansion_pays(const ovb_gemm_args* a) {
     const double k_us = a->K * 1e-3, fused_wave = (u4 ? 3.5 : 0.0) + (gated ? 10.0 : 0.0) + k_us * (u4 ? 6.2 : a->wmode == OVB_W_U8 ? 10.6 : 11.0);
     const double fused = ceil_div(ceil_div(a->N, TILE_N) * ceil_div(a->T, 256), kSMs) * fused_wave;
     // expanded: launches and bytes of the expansion, waves of 256 x bt tiles of every piece
-    const int bt = pick_pair_tile(a->T, a->N, a->K, 0, kPairs, nullptr), piece = pick_piece(a->T, a->N, a->K, bt, kPairs, kScratchBytes);
+    const int bt = pick_pair_tile(a->T, a->N, a->K, kPairs, nullptr), piece = pick_piece(a->T, a->N, a->K, bt, kPairs, kScratchBytes);
     if (piece <= 0) return false;
     int pieces = 0, waves = 0;
     for (int n = 0; n < a->N; n += piece, ++pieces) waves += ceil_div(ceil_div(a->N - n < piece ? a->N - n : piece, 256) * ceil_div(a->T, bt), kPairs);
@@ -559,7 +570,7 @@ static int run_pair(const ovb_gemm_args* a, cudaStream_t stream) {
     p.ldo = a->ldo ? a->ldo : (swiglu ? a->N / 2 : a->N);
     p.ldr = a->ldr ? a->ldr : a->N;
     p.cut = 1;
-    p.bt = pick_pair_tile(a->T, a->N, a->K, grouped ? a->num_groups : 0, pairs, grouped || quant ? nullptr : &p.cut);
+    p.bt = grouped ? 256 : pick_pair_tile(a->T, a->N, a->K, pairs, quant ? nullptr : &p.cut);
     p.num_groups = a->num_groups;
     p.group_mode = a->group_mode;
     p.act = a->act;
@@ -613,7 +624,7 @@ static int run_pair(const ovb_gemm_args* a, cudaStream_t stream) {
         if (p.cut > 1)
             if (int rc = make_tmap_2d(&tmCut, a->x, dt16, 2, a->T, a->K, (uint64_t)ldx * 2, p.bt / p.cut / 2, TILE_K, true)) return rc;
         const int grid = 2 * (int)(tiles < pairs ? tiles : pairs);
-        OVB_CHECK_CUDA(launch_pdl(p.cut > 1 ? gemm_pair_kernel<F16, true> : gemm_pair_kernel<F16, false>, dim3(grid), dim3(kPairThreads), kPairSmem, stream, tmW, tmX, p, tmCut));
+        OVB_CHECK_CUDA(launch_pdl(grouped ? gemm_pair_kernel<F16, kPairEven> : p.cut > 1 ? gemm_pair_kernel<F16, kPairCut> : gemm_pair_kernel<F16, kPairWhole>, dim3(grid), dim3(kPairThreads), kPairSmem, stream, tmW, tmX, p, tmCut));
         OVB_CHECK_CUDA(cudaGetLastError());
     }
     return 0;

@@ -862,6 +862,22 @@ def test_gemm_pair_cut_wave(ops, T, N, dtype):
     ops.check_status("gemm_pair")
 
 
+@pytest.mark.parametrize("sizes", [[31, 0, 257, 33, 512, 1], [513, 224, 225, 65], [770, 0, 0, 0], [96] * 9])
+@pytest.mark.parametrize("mode", [1, 2])
+def test_gemm_groups_of_even_tiles(ops, sizes, mode):
+    """Rows of a group shared out evenly among its tiles: one row, one more than a tile holds, empty groups, rows behind the last group."""
+    G, N, K, total = len(sizes), 640, 320, sum(sizes)
+    off = torch.tensor(np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32), device="cuda")
+    w = _pair_weight(ops, "dense", N * (G if mode == 1 else 1), K * (G if mode == 2 else 1))
+    x = torch.randn(total + 70, K, device="cuda", dtype=torch.bfloat16, generator=torch.Generator(device="cuda").manual_seed(G))
+    for act, n in ((ops.ACT_NONE, N), (ops.ACT_SWIGLU, N // 2)):
+        out, ref = (torch.full((total + 70, n), 3.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        ops.gemm_grouped(x, w, off, G, mode, out, act=act, block_t=256)
+        ops.gemm_grouped(x, w, off, G, mode, ref, act=act, block_t=64)
+        assert _rel_err(out, ref) < PAIR_REL and (out[total:] == 3.0).all()
+    ops.check_status("gemm_groups")
+
+
 def test_gemm_pair_fp16_window_and_groups(ops):
     torch.manual_seed(2)
     x = torch.randn(700, 512, device="cuda", dtype=torch.float16)
