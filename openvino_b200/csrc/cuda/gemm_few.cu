@@ -601,12 +601,3 @@ int gemm_few(const ovb_gemm_args* a, cudaStream_t stream) {
 }
 
 }  // namespace ovb
-
-
-extern "C" int ovb_gemm_few_plan(int wmode, int T, int N, int K, int splits, int* out) {
-    ovb::FewPlan f;
-    if (!ovb::few_plan(wmode, T, N, K, splits, &f)) return 0;
-    const int v[6] = {f.splits, f.clusters, f.ring, f.xslots, f.groups, f.smem};
-    for (int i = 0; i < 6; ++i) out[i] = v[i];
-    return 1;
-}

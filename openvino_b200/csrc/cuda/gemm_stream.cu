@@ -15,8 +15,9 @@
 //  * The loop over (tile, unit) is flat: weight loads run ahead, also across tiles and before the wait for the kernel that writes
 //    the tokens.
 //  * Few tiles: a cluster of 2, 4 or 8 CTAs shares K, partial sums are read through distributed shared memory in rank order.
-// What bounds it at 128256 x 4096 u4 (74 us, 4 TB/s): the latency of its loads, with 16 warps on an SM and issue slots half used. A step of
-// one token through a two-layer model of 256 channels: 82 -> 46 us; of four layers of an 8B model in u4: 421 -> 360 us.
+// What bounds it: the latency of its loads, with 16 warps on an SM and issue slots half used (128256 x 4096 u4 74 us, 4 TB/s). u4 weights of at
+// least 8 M values go to gemm_ring.cu, which streams them through shared memory (60 us), and here stay the small ones, where the launch counts: a
+// step of one token through a two-layer model of 256 channels takes 82 us without this kernel, 46 with it, 37 with the norms inside its products.
 #include <mutex>
 
 #include "gemm_common.cuh"
@@ -340,6 +341,7 @@ static int pick_stream_split(int wmode, int T, int N, int units, int* smem_bytes
     return best;
 }
 
+// (u4 weights that gemm_ring.cu takes are asked for there first.)
 // Where it is the faster one, cold weights, against gemm_sm100.cu (us): u4 128256 x 4096 T = 1 74 / 84, T = 8 82 / 84; 4096 x 14336 T = 1
 // 14 / 20, T = 4 20 / 20, T = 8 22 / 20: up to four tokens. Bytes cost a lane twice the loads for the same weights: u8 128256 x 4096 T = 1
 // 119 / 103, fp8 4096 x 14336 22 / 21, but 4096 x 4096 9 / 17, where the launch counts: up to 32 MB. 16-bit: likewise, up to 16 MB

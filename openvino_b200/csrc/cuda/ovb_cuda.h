@@ -110,9 +110,6 @@ int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream);
 int ovb_gemm_route(const ovb_gemm_args* a);
 // 1: ovb_gemm takes x_norm in (products of up to four tokens); the fields x_norm and x_rows themselves are not looked at.
 int ovb_gemm_norms(const ovb_gemm_args* a);
-// The plan of gemm_few.cu for a product: splits of K, clusters, ring stages, token stages, expanding groups, bytes of shared memory. `splits` 0: its
-// own choice. Returns 0 where no plan fits.
-int ovb_gemm_few_plan(int wmode, int T, int N, int K, int splits, int* out);
 // Bytes of split-K workspace / number of counters that ovb_gemm may need for the given problem.
 int64_t ovb_gemm_ws_bytes(int T, int N, int K, int act);
 int ovb_gemm_num_counters(void);
@@ -334,7 +331,6 @@ typedef struct {
     void* attn;               // [T, Hq D]
     void* gu;                 // [T, 2 ffn]
     void* act;                // [T, ffn]
-    void* last_h;             // [B, hidden]
     void* last_x;             // [B, hidden]
     void* logits;             // [B, head_cols]
     float* gemm_ws;

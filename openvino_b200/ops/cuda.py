@@ -61,7 +61,7 @@ class PaArgs(C.Structure):
 class LlmStep(C.Structure):
     """ovb_llm_step. ``layers`` and ``head`` hold weights as ``llm_weight_words`` packs them."""
     POINTERS = ("embed", "final_norm", "ids", "tok_src", "last_token", "positions", "slot_map", "past_lens", "subsequence_begins", "block_indices",
-                "block_indices_begins", "logit_idx", "h", "x", "qkv", "attn", "gu", "act", "last_h", "last_x", "logits", "gemm_ws", "gemm_counters", "pa_scratch",
+                "block_indices_begins", "logit_idx", "h", "x", "qkv", "attn", "gu", "act", "last_x", "logits", "gemm_ws", "gemm_counters", "pa_scratch",
                 "scratch")
     INTS = ("num_layers", "T", "B", "hidden", "ffn", "Hq", "Hkv", "D", "vocab", "head_cols", "block_size", "max_ctx", "max_q_len", "sliding_window", "kv_u8")
     _fields_ = ([("layers", C.c_void_p), ("head", C.c_ubyte * 56)] + [(n, C.c_void_p) for n in POINTERS]

@@ -513,7 +513,7 @@ class CudaLlmExecutor(LlmExecutor):
         step = K.LlmStep(C.addressof(layers), (C.c_ubyte * 56).from_buffer_copy(struct.pack("<" + K.LLM_WEIGHT, *K.llm_weight_words(w.lm_head))), w.embed.data_ptr(), w.final_norm.data_ptr(),
                          at["ids"], at["tok_src"], self.last_token.data_ptr(), at["positions"], at["slot_map"], at["past_lens"], at["subsequence_begins"],
                          at["block_indices"], at["block_indices_begins"], at["logit_idx"],
-                         *(t.data_ptr() for t in (sb.h, sb.x, sb.qkv, sb.attn, sb.gu, sb.act, sb.last_h, sb.last_x, sb.logits, ws.gemm_ws, ws.counters, ws.pa_scratch)),
+                         *(t.data_ptr() for t in (sb.h, sb.x, sb.qkv, sb.attn, sb.gu, sb.act, sb.last_x, sb.logits, ws.gemm_ws, ws.counters, ws.pa_scratch)),
                          None, ws.gemm_ws.numel() * 4, ws.pa_scratch.numel() * 4, 0, len(w.layers), T, B, cfg.hidden_size, cfg.ffn_size, self.hq, self.hkv,
                          cfg.head_dim, w.embed.shape[0], sb.logits.shape[1], self.block_size, shp.max_ctx, shp.max_q_len, cfg.sliding_window,
                          1 if self.kv_u8 else 0, cfg.rope_theta, cfg.rms_eps, 0)
