@@ -22,6 +22,7 @@
 //
 // Tensor memory (512 columns): S0 0..127, S1 128..255, O 256..256+DV-1, P0 and P1 (64 columns each) behind it.
 // Every wait is bounded (mbar_wait) and reports through the status word.
+#include <float.h>
 #include <math_constants.h>
 
 #include <atomic>
@@ -261,7 +262,12 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (biased) {
             using E = typename std::conditional<F16, __half, __nv_bfloat16>::type;
             const E* kb = reinterpret_cast<const E*>(p.key_bias) + (size_t)b * p.bias_stride;
-            for (int i = r; i < ntiles * kBK; i += kBM) sBias[i] = i < kv_total ? float(kb[i]) * 1.4426950408889634f : 0.f;
+            // A finite value stays finite: bf16's lowest, times log2(e), would be -inf, and a sequence all of whose keys have it gets the mean of its
+            // values, as any equal scores do.
+            for (int i = r; i < ntiles * kBK; i += kBM) {
+                const float v = i < kv_total ? float(kb[i]) : 0.f, w = v * 1.4426950408889634f;
+                sBias[i] = isinf(w) && !isinf(v) ? copysignf(FLT_MAX, v) : w;
+            }
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
         for (int j = 0; j < ntiles && ok; ++j) {

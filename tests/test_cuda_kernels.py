@@ -1307,3 +1307,27 @@ def test_sdpa_with_a_value_per_key(ops, dtype, D, S):
         ops.sdpa_masked(torch.zeros(9000, 64, device="cuda", dtype=dtype), *(torch.zeros(9000, 64, device="cuda", dtype=dtype),) * 2,
                         torch.zeros(1, 9000, device="cuda", dtype=dtype), 1, 9000, 1, 64, 64)
     ops.check_status("sdpa_masked")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D,S", [(64, 1), (64, 100), (64, 129), (64, 384), (128, 257)])
+def test_sdpa_of_a_sequence_that_is_all_padding(ops, dtype, D, S):
+    """Every key of a sequence at the type's lowest (or largest) finite value: softmax sees equal biases. The 16-bit value times log2(e) does not fit 32
+    bits in bf16. NaN in a mask stays NaN."""
+    B, H = 4, 2
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q, k, v = (torch.randn(B * S, H * D, device="cuda", generator=g).to(dtype) for _ in range(3))
+    bias = torch.zeros(B, S, device="cuda", dtype=dtype)
+    bias[1], bias[2] = torch.finfo(dtype).min, torch.finfo(dtype).max
+    bias[3, : S // 2] = float("-inf")                     # some keys not there, the others at the lowest value
+    bias[3, S // 2:] = torch.finfo(dtype).min
+    qd, kd, vd = (t.reshape(B, S, H, D).transpose(1, 2).double() for t in (q, k, v))
+    want = (torch.softmax(qd @ kd.transpose(-1, -2) / D ** 0.5 + bias.double()[:, None, None], -1) @ vd).transpose(1, 2).reshape(B, S, H * D)
+    out = ops.sdpa_masked(q, k, v, bias, B, S, H, D, H * D).reshape(B, S, H * D)
+    # probabilities and the result in 16 bits; a score beside 65504 log2(e) is rounded to 2^-7, so a probability of fp16 is off by 2^-8 ln 2 at most
+    rel = 2.0 ** -9 + 2.0 ** -8 if dtype == torch.float16 else 2.0 ** -7
+    for b in range(B):
+        assert _rel_err(out[b], want[b]) < rel, b
+    bias[0, S - 1] = float("nan")
+    assert ops.sdpa_masked(q, k, v, bias, B, S, H, D, H * D).reshape(B, -1)[0].isnan().all()
+    ops.check_status("sdpa_masked")
