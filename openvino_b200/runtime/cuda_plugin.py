@@ -1583,8 +1583,8 @@ class CudaCompiledModel(CompiledModel):
                 raise RuntimeError("string tensors are not supported on this device")
             return torch.from_numpy(np.ascontiguousarray(arr))
 
-        def to_device(t: Tensor) -> torch.Tensor:
-            x = t.torch() if t.is_remote else host_view(t).to(dev, non_blocking=True)
+        def to_device(t: Tensor, host: Optional[torch.Tensor]) -> torch.Tensor:
+            x = t.torch() if t.is_remote else (host_view(t) if host is None else host).to(dev, non_blocking=True)
             if x.dtype == torch.float32 and self.precision is not None:
                 x = x.to(self.precision)
             return x
@@ -1599,7 +1599,7 @@ class CudaCompiledModel(CompiledModel):
         graph_cache: Dict[tuple, object] = {}
         request._cuda_graphs = graph_cache
 
-        def run_graphed(xs: List[torch.Tensor]):
+        def run_graphed(xs: List[torch.Tensor], hosts: List[Optional[torch.Tensor]]):
             key = tuple((tuple(x.shape), x.dtype) for x in xs)
             entry = graph_cache.get(key)
             if entry is None:                       # first call: eager (warms up workspaces and one-time kernel set-up)
@@ -1629,6 +1629,9 @@ class CudaCompiledModel(CompiledModel):
                     graph_cache[key] = "eager"
                     return program.run(xs, None)
                 graph_cache[key] = entry
+                for i, (h, s_) in enumerate(zip(hosts, static_in)):
+                    if h is not None and h.dtype == s_.dtype:
+                        reserve(i, s_)
                 g.replay()
                 return list(entry[2])
             g, static_in, static_out = entry
@@ -1639,28 +1642,39 @@ class CudaCompiledModel(CompiledModel):
 
         # Host inputs of a captured shape go through pinned memory of this request straight into the graph's buffers: a copy from pageable memory
         # waits for the device (encoder with three inputs: 16 x 384 1677 -> 1654 us, 1 x 40 467 -> 437 us). A request's inference ends with
-        # a synchronisation, so its pinned memory is free again when the next one starts.
-        staging: Dict[tuple, list] = {}
+        # a synchronisation, so its pinned memory is free again when the next one starts. There is one piece per input, as large as the largest
+        # captured shape needs, and it is allocated when that shape is captured: the allocation takes far longer than the replays that follow save.
+        staging: Dict[int, torch.Tensor] = {}
+        staged_views: Dict[tuple, List[Optional[torch.Tensor]]] = {}     # the pieces in the type and shape of a captured shape's inputs
+        request._cuda_staging = staging
 
-        def run_staged(ins: List[Tensor]):
-            """The outputs, or None where the shape has not been captured yet or an input lies on the device."""
-            if not graph_cache or any(t.is_remote for t in ins):
-                return None
-            hosts = [host_view(t) for t in ins]
+        def reserve(i: int, like: torch.Tensor) -> None:
+            size = like.numel() * like.element_size()
+            if i not in staging or staging[i].numel() < size:
+                staged_views.clear()
+                staging[i] = torch.empty(size, dtype=torch.uint8, pin_memory=True)
+
+        def run_staged(hosts: List[torch.Tensor], ins: List[Tensor]):
+            """The outputs, or None where the shape has not been captured yet."""
             key = tuple((tuple(h.shape), self.precision if h.dtype == torch.float32 and self.precision is not None else h.dtype) for h in hosts)
             entry = graph_cache.get(key)
             if not isinstance(entry, tuple):
                 return None
             g, static_in, static_out = entry
-            pins = staging.setdefault(key, [None] * len(hosts))
-            for i, (h, s_) in enumerate(zip(hosts, static_in)):
-                if h.dtype != s_.dtype:             # converted on the device
-                    s_.copy_(to_device(ins[i]), non_blocking=True)
-                    continue
-                if pins[i] is None:
-                    pins[i] = torch.empty(h.shape, dtype=h.dtype, pin_memory=True)
-                pins[i].copy_(h)
-                s_.copy_(pins[i], non_blocking=True)
+            straight = [h.dtype == s_.dtype for h, s_ in zip(hosts, static_in)]      # the others are converted on the device
+            for i, s_ in enumerate(static_in):
+                if straight[i]:
+                    reserve(i, s_)                       # (captured from inputs on the device, or in another type)
+            views = staged_views.get(key)
+            if views is None or any(v is None and st for v, st in zip(views, straight)):
+                views = staged_views[key] = [staging[i][:s_.numel() * s_.element_size()].view(s_.dtype).view(s_.shape) if straight[i] else None
+                                             for i, s_ in enumerate(static_in)]
+            for t, h, s_, v, st in zip(ins, hosts, static_in, views, straight):
+                if st:
+                    v.copy_(h)
+                    s_.copy_(v, non_blocking=True)
+                else:
+                    s_.copy_(to_device(t, h), non_blocking=True)
             g.replay()
             return list(static_out)
 
@@ -1670,16 +1684,19 @@ class CudaCompiledModel(CompiledModel):
                 with (self._state_lock if self._has_state else contextlib.nullcontext()), stream_lock:
                     program.ctx.variables = ctx_vars
                     with torch.cuda.stream(stream):
-                        outs = run_staged(ins) if graphs_on else None
+                        outs = None
+                        hosts = [None if t.is_remote else host_view(t) for t in ins]
+                        if graphs_on and graph_cache and not any(t.is_remote for t in ins):
+                            outs = run_staged(hosts, ins)
                         if outs is None:
-                            xs = [to_device(t) for t in ins]
-                            outs = run_graphed(xs) if graphs_on else program.run(xs, prof)
+                            xs = [to_device(t, h) for t, h in zip(ins, hosts)]
+                            outs = run_graphed(xs, hosts) if graphs_on else program.run(xs, prof)
                         res = self._finish(outs, req)
                     stream.synchronize()
             else:
                 with self._state_lock:
                     program.ctx.variables = ctx_vars
-                    outs = program.run([to_device(t) for t in ins], prof)
+                    outs = program.run([to_device(t, None) for t in ins], prof)
                     res = self._finish(outs, req)
                     torch.cuda.current_stream(self.device).synchronize()
             if prof is not None:

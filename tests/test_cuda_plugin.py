@@ -224,3 +224,28 @@ def test_host_inputs_of_a_captured_shape(core, precision):
     req.set_input_tensor(0, Tensor(x))
     req.infer()
     assert np.array_equal(req.get_output_tensor(0).data, x * 2 + 7)
+
+
+def test_pinned_inputs_are_allocated_with_the_capture(core, monkeypatch):
+    """No pinned memory is allocated by a replay, and a request keeps one piece per input, of the largest captured shape."""
+    a, b = ops.parameter([-1, 8], Type.f32, name="a"), ops.parameter([-1, 8], Type.i32, name="b")
+    m = Model([ops.add(a, ops.convert(b, "f32"))], [a, b], "two_inputs")
+    req = core.compile_model(m, "CUDA", {props.hint.inference_precision: "f32"}).create_infer_request()
+    sizes, plain = [], torch.empty
+
+    def counted(*args, **kw):
+        t = plain(*args, **kw)
+        if kw.get("pin_memory"):
+            sizes.append(t.numel() * t.element_size())
+        return t
+    monkeypatch.setattr(torch, "empty", counted)
+    for rows in (4, 64, 16):
+        for call in range(4):
+            x, y = np.full((rows, 8), float(rows + call), np.float32), np.full((rows, 8), call, np.int32)
+            del sizes[:]
+            assert np.array_equal(req.infer([x, y])[0], x + y.astype(np.float32))
+            assert call < 2 or not sizes, (rows, call, sizes)      # eager, captured, replayed
+    for rows in (64, 4, 16):
+        x, y = np.random.RandomState(rows).rand(rows, 8).astype(np.float32), np.full((rows, 8), rows, np.int32)
+        assert np.array_equal(req.infer([x, y])[0], x + y.astype(np.float32))
+    assert sum(s.numel() for s in req._cuda_staging.values()) == 2 * 64 * 8 * 4
