@@ -187,7 +187,7 @@ def build_native_test(test_source: Path, sanitize: str = "", force: bool = False
     capi = sorted((CSRC / "capi").glob("*.cpp"))
     if core_subset is not None:           # a driver that needs only some translation units (and no C API)
         core, capi = [s for s in core if s.stem in set(core_subset)], []
-    hdrs = sorted((CSRC / "core").glob("*.hpp")) + sorted((PKG / "include").rglob("*.h")) + sorted((CSRC / "cuda").glob("comm_layout.h"))
+    hdrs = sorted((CSRC / "core").glob("*.hpp")) + sorted((PKG / "include").rglob("*.h")) + sorted((CSRC / "cuda").glob("comm_layout.h")) + sorted((CSRC / "cuda").glob("cluster_table.h"))
     if not force and not _stale(exe, core + capi + hdrs + [test_source]):
         return exe
     # the distribution's compiler knows where its sanitizer runtimes are; a compiler wrapper named by CXX may not

@@ -217,7 +217,7 @@ int gemm_pair(const ovb_gemm_args* a, cudaStream_t stream);
 // gemm_few.cu: products of up to 64 tokens with quantised weights.
 bool gemm_few_takes(const ovb_gemm_args* a);
 int gemm_few(const ovb_gemm_args* a, cudaStream_t stream);
-// Clusters of this many CTAs that the device holds, one CTA of gemm_few.cu's size per SM, asked of the driver once.
+// Clusters of this many CTAs that the current device holds, one CTA of gemm_few.cu's size per SM, asked of the driver once per device.
 int cluster_capacity(int size);
 // The RMS norm of a product's few rows, by the whole CTA: every thread holds HOLD pieces of eight columns of each of T rows of x (it reads the rows in
 // whole, whatever part of K its CTA has) and calls put(token, piece of eight columns, normalised values). `part`: [warps][TMAX] floats of shared

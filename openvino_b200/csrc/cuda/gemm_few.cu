@@ -17,6 +17,7 @@
 // A decode step of 24 tokens (8B, four layers, u8): 684 -> 609 us, products 414 -> 345; of 32 tokens (70B, two layers, fp8): 868 -> 777 us.
 #include <mutex>
 
+#include "cluster_table.h"
 #include "gemm_common.cuh"
 
 namespace ovb {
@@ -449,34 +450,37 @@ static bool few_layout(int wmode, int nt, FewPlan* f) {
     return f->smem <= kFewSmem;
 }
 
-int cluster_capacity(int splits) {
-    static std::mutex mu;
-    static int table[9] = {0, 148, 74, 45, 35, 27, 22, 18, 16};       // (without a device)
-    std::lock_guard<std::mutex> lk(mu);
-    if (table[0] == 0) {
-        table[0] = 1;
-        auto kern = gemm_few_kernel<OVB_W_U4>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem) == cudaSuccess) {
-            for (int s = 2; s <= 8; ++s) {
-                cudaLaunchConfig_t cfg;
-                memset(&cfg, 0, sizeof(cfg));
-                cfg.gridDim = dim3(s * 64);
-                cfg.blockDim = dim3(kFewThreads);
-                cfg.dynamicSmemBytes = kFewSmem;
-                cudaLaunchAttribute attr[1];
-                attr[0].id = cudaLaunchAttributeClusterDimension;
-                attr[0].val.clusterDim.x = s;
-                attr[0].val.clusterDim.y = 1;
-                attr[0].val.clusterDim.z = 1;
-                cfg.attrs = attr;
-                cfg.numAttrs = 1;
-                int n = 0;
-                if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0) table[s] = n;
-            }
-        }
+static int ask_cluster_capacity(int size) {
+    auto kern = gemm_few_kernel<OVB_W_U4>;
+    int n = 0;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(size * 64);
+    cfg.blockDim = dim3(kFewThreads);
+    cfg.dynamicSmemBytes = kFewSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
+        return 0;
     }
-    return table[splits];
+    return n;
+}
+
+int cluster_capacity(int size) {
+    static ClusterTable table;
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        dev = -1;
+    }
+    return table.get(dev, size, [size] { return ask_cluster_capacity(size); });
 }
 
 // Splits of K. Time of a candidate (us): rounds of tiles, each as long as its stages take an SM or their bytes take HBM at 6.3 TB/s, whichever is

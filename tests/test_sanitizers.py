@@ -11,6 +11,7 @@ executable of its own (no Python in the process, so no preloaded sanitizer runti
                                 one-shot packets, fence + flags, in-switch barrier) with the kernels' index arithmetic,
                                 including a rank that skips a step (the others time out with a status, the next step
                                 works); under TSan.
+* ``cluster_table.cpp``       - cluster capacities of several devices, asked by several threads; under TSan.
 """
 import os
 import subprocess
@@ -55,6 +56,13 @@ def test_runtime_threads_under_thread_sanitizer():
     exe = build.build_native_test(NATIVE / "runtime_threads.cpp", "thread", core_subset=("runtime", "sched", "types"))
     r = _run(exe, [], {"TSAN_OPTIONS": "halt_on_error=1"})
     assert r.returncode == 0 and "RUNTIME_THREADS_OK" in r.stdout, (r.stdout[-2000:], r.stderr[-6000:])
+    assert "WARNING: ThreadSanitizer" not in r.stderr, r.stderr[-6000:]
+
+
+def test_cluster_capacities_belong_to_their_device():
+    exe = build.build_native_test(NATIVE / "cluster_table.cpp", "thread", core_subset=())
+    r = _run(exe, [], {"TSAN_OPTIONS": "halt_on_error=1"})
+    assert r.returncode == 0 and "CLUSTER_TABLE_OK" in r.stdout, (r.stdout[-2000:], r.stderr[-6000:])
     assert "WARNING: ThreadSanitizer" not in r.stderr, r.stderr[-6000:]
 
 
