@@ -864,14 +864,19 @@ def _sdpa(n, ins, ctx):
         return [out.reshape(B, S, H, D).transpose(1, 2)]
     if (K is not None and not causal and mask is not None and mask.dim() == 4 and mask.dtype == q.dtype and q.dim() == 4 and q.dtype in (torch.float16, torch.bfloat16)
             and q.shape[-1] in (64, 128) and q.shape == k.shape == v.shape and k.dtype == v.dtype == q.dtype and len(ins) <= 5
-            and mask.shape[1] == mask.shape[2] == 1 and mask.shape[3] == q.shape[2] <= 8192 and mask.shape[0] in (1, q.shape[0])):
-        # a value per key (a padding mask), added to the scores inside the kernel
+            and mask.shape[1] == mask.shape[2] == 1 and mask.shape[3] == q.shape[2] <= 8192 and mask.shape[0] in (1, q.shape[0])
+            and (q.shape[3] == 64 or q.shape[2] >= 128)):
+        # A value per key (a padding mask), added to the scores inside the kernel, which wants the heads side by side in the rows of their tokens. In another
+        # order three copies come first, which only long sequences pay for (us, fp16, 16 heads, in place / with copies / torch's attention: heads of 64,
+        # 16 x 384 tokens 36 / 85 / 71, 1 x 1024 17 / 28 / 62, 2 x 2048 98 / 129 / 235; of 128, 1 x 1024 20 / 37 / 62, 2 x 2048 135 / 217 / 239, 1 x 8192 with 8
+        # heads 500 / 614 / 606). Heads of 128 with a few keys gain nothing: 1 x 128 7.1 / - / 6.7, 1 x 40 with 12 heads 7.1 / - / 5.0.
         B, H, S, D = q.shape
-        q, k, v = (_dense(t.transpose(1, 2)).reshape(B * S, H * D) for t in (q, k, v))
-        if all(t.data_ptr() % 16 == 0 for t in (q, k, v)):
-            out = K.sdpa_masked(q, k, v, mask.reshape(mask.shape[0], S).contiguous(), B, S, H, D, H * D, scale=scale)
-            return [out.reshape(B, S, H, D).transpose(1, 2)]
-        q, k, v = (t.reshape(B, S, H, D).transpose(1, 2) for t in (q, k, v))
+        rows = [t.transpose(1, 2) for t in (q, k, v)]
+        if 1024 <= S <= (8192 if D == 64 else 2048) or all(t.is_contiguous() for t in rows):
+            rows = [_dense(t).reshape(B * S, H * D) for t in rows]
+            if all(t.data_ptr() % 16 == 0 for t in rows):
+                out = K.sdpa_masked(*rows, mask.reshape(mask.shape[0], S).contiguous(), B, S, H, D, H * D, scale=scale)
+                return [out.reshape(B, S, H, D).transpose(1, 2)]
     return [F.scaled_dot_product_attention(q, k.to(q.dtype), v.to(q.dtype), attn_mask=None if causal else mask, is_causal=bool(causal) and mask is None, scale=scale)]
 
 

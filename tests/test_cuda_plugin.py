@@ -249,3 +249,24 @@ def test_pinned_inputs_are_allocated_with_the_capture(core, monkeypatch):
         x, y = np.random.RandomState(rows).rand(rows, 8).astype(np.float32), np.full((rows, 8), rows, np.int32)
         assert np.array_equal(req.infer([x, y])[0], x + y.astype(np.float32))
     assert sum(s.numel() for s in req._cuda_staging.values()) == 2 * 64 * 8 * 4
+
+
+@pytest.mark.parametrize("order,S,D,inside", [("tokens first", 40, 64, True), ("heads first", 40, 64, False), ("heads first", 1024, 64, True), ("tokens first", 40, 128, False),
+                                              ("tokens first", 200, 128, True)])
+def test_padding_masks_stay_inside_the_kernel_where_that_is_faster(core, monkeypatch, order, S, D, inside):
+    """Queries, keys and values whose heads lie side by side go to the kernel as they are; in another order only where the copies pay."""
+    from openvino_b200.ops import cuda as K
+    B, H = 2, 3
+    shape = [B, S, H, D] if order == "tokens first" else [B, H, S, D]
+    params = [ops.parameter(shape, Type.f16, name=n) for n in "qkv"] + [ops.parameter([B, 1, 1, S], Type.f16, name="mask")]
+    heads = [ops.transpose(p, np.array([0, 2, 1, 3])) if order == "tokens first" else p for p in params[:3]]
+    m = Model([ops.scaled_dot_product_attention(*heads, params[3])], params, "masked_attention")
+    calls, plain = [], K.sdpa_masked
+    monkeypatch.setattr(K, "sdpa_masked", lambda *a, **kw: calls.append(1) or plain(*a, **kw))
+    rng = np.random.RandomState(S)
+    x = [rng.randn(*shape).astype(np.float16) for _ in range(3)] + [np.where(np.arange(S) < [[S], [S // 2]], 0.0, -10000.0).astype(np.float16).reshape(B, 1, 1, S)]
+    got = core.compile_model(m, "CUDA", {props.hint.inference_precision: "f16"}).create_infer_request().infer(x)[0]
+    assert bool(calls) == inside
+    q, k, v = (torch.from_numpy(t).double() if order != "tokens first" else torch.from_numpy(t).double().transpose(1, 2) for t in x[:3])
+    want = torch.softmax(q @ k.transpose(-1, -2) / D ** 0.5 + torch.from_numpy(x[3]).double(), -1) @ v
+    assert float((torch.from_numpy(got.astype(np.float64)) - want).norm() / want.norm()) < 2.0 ** -9        # probabilities and the result in fp16
