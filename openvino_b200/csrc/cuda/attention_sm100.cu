@@ -79,20 +79,20 @@ __host__ __device__ constexpr int tile_tokens(int g) { return kBM / g / 8 * 8; }
 // KH / RH / VH: 64-column (128-byte) parts of a key row, of its shared second part, and of a value row. A part that reaches past
 // the end of a cache row is filled with zeros by the copy, so any size that is a multiple of 8 is served; what the query tile
 // holds behind a head's columns meets those zeros. GT: query heads per KV head, 0 = at run time (p.group).
-// Dense heads of 64 keep S and P once (256 columns of tensor memory), so that two CTAs share an SM and one's exponentials run beside the other's
-// products; the scores are read twice, 32 at a time, instead of being held. 16 x 384 tokens, 16 heads, with a mask: 49 us with one CTA per SM, 36 here.
-constexpr bool two_dense_ctas(int kh, int rh, int vh, int src) { return src == SRC_DENSE && kh == 1 && rh == 0 && vh == 1; }
-
-template <int KH, int RH, int VH, int GT, int SRC, bool F16>
-__global__ void __launch_bounds__(192, two_dense_ctas(KH, RH, VH, SRC) ? 2 : 1)
+// BIAS (dense): a value per key is added to its scaled scores.
+// TWO (dense heads of 64): S and P are kept once (256 columns of tensor memory), so that two CTAs share an SM and one's exponentials run beside the
+// other's products; the scores are read twice, 32 at a time, instead of being held.
+template <int KH, int RH, int VH, int GT, int SRC, bool F16, bool BIAS = false, bool TWO = false>
+__global__ void __launch_bounds__(192, TWO ? 2 : 1)
 pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                      const __grid_constant__ CUtensorMap tmR, PaKParams p, int* status) {
+    static_assert(SRC == SRC_DENSE || (!BIAS && !TWO), "dense attention");
     constexpr bool PAGED = SRC != SRC_DENSE;                   // ragged batch with a descriptor
     constexpr int DK = (KH + RH) * 64, DV = VH * 64;
     const int G = GT > 0 ? GT : p.group;
     const int TOK = tile_tokens(G);            // tokens per tile
     constexpr int Q_BYTES = kBM * DK * 2, K_BYTES = kBK * DK * 2, V_BYTES = kBK * DV * 2;
-    constexpr int SB = two_dense_ctas(KH, RH, VH, SRC) ? 1 : 2;   // copies of S and P
+    constexpr int SB = TWO ? 1 : 2;            // copies of S and P
     constexpr uint32_t TM_S = 0, TM_O = SB * 128, TM_P = SB * 128 + DV, TM_COLS = SB == 1 ? 256 : 512;   // tensor-memory columns
     constexpr uint32_t IDESC_QK = umma_idesc_f16(kBM, kBK, !F16);
     constexpr uint32_t IDESC_PV = umma_idesc_f16(kBM, DV, !F16) | (1u << 16);   // B operand MN-major
@@ -114,7 +114,7 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* s_work = const_cast<int*>(abort_flag) + 1;   // [2]
-    float* sBias = reinterpret_cast<float*>(bars + 32);   // SRC_DENSE with a bias: of all keys, times log2(e)
+    float* sBias = reinterpret_cast<float*>(bars + 32);   // BIAS: of all keys, times log2(e)
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = blockIdx.y;
@@ -257,9 +257,8 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const uint32_t lane_base = tmem + (uint32_t(warp * 32) << 16);
         float m_used = -CUDART_INF_F, l_sum = 0.f;
         bool ok = true;
-        const bool biased = SRC == SRC_DENSE && p.key_bias != nullptr;
-        const float scale = biased ? 1.f : p.scale_log2;      // (biased scores are scaled when the bias is added)
-        if (biased) {
+        const float scale = BIAS ? 1.f : p.scale_log2;        // (biased scores are scaled when the bias is added)
+        if (BIAS) {
             using E = typename std::conditional<F16, __half, __nv_bfloat16>::type;
             const E* kb = reinterpret_cast<const E*>(p.key_bias) + (size_t)b * p.bias_stride;
             // A finite value stays finite: bf16's lowest, times log2(e), would be -inf, and a sequence all of whose keys have it gets the mean of its
@@ -291,7 +290,7 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 tmem_ld_x16(lane_base + TM_S + c, w);
                 tmem_ld_x16(lane_base + TM_S + c + 16, w + 16);
                 tmem_ld_wait();
-                if (biased) {
+                if (BIAS) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 4) {
                         const float4 kb = *reinterpret_cast<const float4*>(sBias + j0 + c + i);
@@ -324,7 +323,7 @@ pa_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 tmem_ld_wait();
                 tc_fence_before_sync();
                 mbar_arrive(&s_free[st]);
-                if (biased) {
+                if (BIAS) {
 #pragma unroll
                     for (int i = 0; i < kBK; i += 4) {
                         const float4 kb = *reinterpret_cast<const float4*>(sBias + j0 + i);
@@ -814,18 +813,18 @@ int launch_duo(PaKParams p, int num_q_tiles, cudaStream_t stream) {
 
 constexpr int kMaxBiasedKeys = 8192;
 
-template <int KH, int RH, int VH, int G, int SRC, bool F16>
+template <int KH, int RH, int VH, int G, int SRC, bool F16, bool BIAS = false, bool TWO = false>
 int launch_tc_parts(const PaKParams& p, int num_q_tiles, cudaStream_t stream) {
     const int TOK = tile_tokens(G > 0 ? G : p.group);
     constexpr int plain = kBM * (KH + RH) * 128 + 2 * kBK * (KH + RH + VH) * 128 + 256 + 1024;
-    const int smem = plain + (SRC == SRC_DENSE && p.key_bias != nullptr ? ceil_div(p.dense_S, kBK) * kBK * 4 : 0);
-    auto kern = pa_prefill_tc_kernel<KH, RH, VH, G, SRC, F16>;
+    const int smem = plain + (BIAS ? ceil_div(p.dense_S, kBK) * kBK * 4 : 0);
+    auto kern = pa_prefill_tc_kernel<KH, RH, VH, G, SRC, F16, BIAS, TWO>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     OVB_CHECK_CUDA(cudaGetDevice(&dev));
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
-        OVB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, plain + (SRC == SRC_DENSE ? kMaxBiasedKeys * 4 : 0)));
+        OVB_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, plain + (BIAS ? kMaxBiasedKeys * 4 : 0)));
         configured.fetch_or(bit, std::memory_order_release);
     }
     const CUtensorMapDataType dt = F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -854,11 +853,30 @@ int launch_tc_parts(const PaKParams& p, int num_q_tiles, cudaStream_t stream) {
 }
 
 // Heads of one size D packed without gaps.
-template <int D, int G, bool PAGED, bool F16>
+void pack_heads(PaKParams* p, int D) {
+    p->q_head = p->o_head = p->dv_store = p->k_row = p->v_row = p->k_head = p->v_head = D;
+    p->ldo = p->Hq * D;
+}
+
+template <int D, int G>
 int launch_tc(PaKParams p, int num_q_tiles, cudaStream_t stream) {
-    p.q_head = p.o_head = p.dv_store = p.k_row = p.v_row = p.k_head = p.v_head = D;
-    p.ldo = p.Hq * D;
-    return launch_tc_parts<D / 64, 0, D / 64, G, PAGED ? SRC_PAGED : SRC_DENSE, F16>(p, num_q_tiles, stream);
+    pack_heads(&p, D);
+    return launch_tc_parts<D / 64, 0, D / 64, G, SRC_PAGED, false>(p, num_q_tiles, stream);
+}
+
+// Two CTAs to an SM where there are more CTAs than SMs (heads of 64, fp16, us with one / with two: 16 x 384 tokens, 16 heads, with a mask 49 / 36); a
+// CTA that has its SM to itself is faster with S and P twice (1 x 1024, 16 heads 14.6 / 18.0; 4 x 200, 12 heads 7.7 / 8.8; 1 x 40 5.4 / 6.0).
+template <int D, bool F16>
+int launch_dense(PaKParams p, int num_q_tiles, cudaStream_t stream) {
+    pack_heads(&p, D);
+    constexpr int P = D / 64;
+    if constexpr (D == 64) {
+        if (num_q_tiles * p.Hkv > 148)
+            return p.key_bias != nullptr ? launch_tc_parts<P, 0, P, 1, SRC_DENSE, F16, true, true>(p, num_q_tiles, stream)
+                                         : launch_tc_parts<P, 0, P, 1, SRC_DENSE, F16, false, true>(p, num_q_tiles, stream);
+    }
+    return p.key_bias != nullptr ? launch_tc_parts<P, 0, P, 1, SRC_DENSE, F16, true>(p, num_q_tiles, stream)
+                                 : launch_tc_parts<P, 0, P, 1, SRC_DENSE, F16>(p, num_q_tiles, stream);
 }
 
 }  // namespace
@@ -890,20 +908,20 @@ int launch_prefill_tc(const PaKParams& p, int D, int G, bool paged, bool f16, in
         }
         if (D == 128) {
             switch (G) {
-                case 1: return launch_tc<128, 1, true, false>(p, num_q_tiles, stream);
-                case 2: return launch_tc<128, 2, true, false>(p, num_q_tiles, stream);
-                case 4: return launch_tc<128, 4, true, false>(p, num_q_tiles, stream);
-                case 8: return launch_tc<128, 8, true, false>(p, num_q_tiles, stream);
+                case 1: return launch_tc<128, 1>(p, num_q_tiles, stream);
+                case 2: return launch_tc<128, 2>(p, num_q_tiles, stream);
+                case 4: return launch_tc<128, 4>(p, num_q_tiles, stream);
+                case 8: return launch_tc<128, 8>(p, num_q_tiles, stream);
             }
         } else if (D == 64) {
             switch (G) {
-                case 1: return launch_tc<64, 1, true, false>(p, num_q_tiles, stream);
-                case 4: return launch_tc<64, 4, true, false>(p, num_q_tiles, stream);
+                case 1: return launch_tc<64, 1>(p, num_q_tiles, stream);
+                case 4: return launch_tc<64, 4>(p, num_q_tiles, stream);
             }
         }
     } else if (!paged && G == 1) {
-        if (D == 64) return f16 ? launch_tc<64, 1, false, true>(p, num_q_tiles, stream) : launch_tc<64, 1, false, false>(p, num_q_tiles, stream);
-        if (D == 128) return f16 ? launch_tc<128, 1, false, true>(p, num_q_tiles, stream) : launch_tc<128, 1, false, false>(p, num_q_tiles, stream);
+        if (D == 64) return f16 ? launch_dense<64, true>(p, num_q_tiles, stream) : launch_dense<64, false>(p, num_q_tiles, stream);
+        if (D == 128) return f16 ? launch_dense<128, true>(p, num_q_tiles, stream) : launch_dense<128, false>(p, num_q_tiles, stream);
     }
     return ERR_UNSUPPORTED;
 }

@@ -1314,7 +1314,7 @@ def test_sdpa_with_a_value_per_key(ops, dtype, D, S):
 def test_sdpa_of_a_sequence_that_is_all_padding(ops, dtype, D, S):
     """Every key of a sequence at the type's lowest (or largest) finite value: softmax sees equal biases. The 16-bit value times log2(e) does not fit 32
     bits in bf16. NaN in a mask stays NaN."""
-    B, H = 4, 2
+    B, H = 4, 16 if S == 384 else 2                       # (more CTAs than SMs: the form with two CTAs on an SM)
     g = torch.Generator(device="cuda").manual_seed(S)
     q, k, v = (torch.randn(B * S, H * D, device="cuda", generator=g).to(dtype) for _ in range(3))
     bias = torch.zeros(B, S, device="cuda", dtype=dtype)
@@ -1331,3 +1331,23 @@ def test_sdpa_of_a_sequence_that_is_all_padding(ops, dtype, D, S):
     bias[0, S - 1] = float("nan")
     assert ops.sdpa_masked(q, k, v, bias, B, S, H, D, H * D).reshape(B, -1)[0].isnan().all()
     ops.check_status("sdpa_masked")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D,S", [(64, 1), (64, 100), (64, 128), (64, 129), (64, 640), (128, 1), (128, 127), (128, 257), (128, 384)])
+def test_sdpa_dense_causal_and_not(ops, dtype, causal, D, S):
+    """Dense attention without a mask, one CTA per query tile, both head sizes, edges of the tiles of 128 keys, more CTAs than SMs (two to an SM for heads of
+    64) and fewer, against softmax in 64 bits."""
+    B, H = 3, 2 if S < 600 and (D, S) != (64, 129) else 30
+    qkv = torch.randn(B * S, 3 * H * D, device="cuda", generator=torch.Generator(device="cuda").manual_seed(S)).to(dtype)
+    q, k, v = (qkv[:, i * H * D:] for i in range(3))
+    out = ops.sdpa_dense(q, k, v, B, S, H, D, 3 * H * D, causal=causal)
+    qd, kd, vd = (t[:, :H * D].reshape(B, S, H, D).transpose(1, 2).double() for t in (q, k, v))
+    s = qd @ kd.transpose(-1, -2) / D ** 0.5
+    if causal:
+        s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = (torch.softmax(s, -1) @ vd).transpose(1, 2).reshape(B * S, H * D)
+    # probabilities rounded to 16 bits, and the result once more
+    assert _rel_err(out, want) < (2.0 ** -9 if dtype == torch.float16 else 2.0 ** -7)
+    ops.check_status("sdpa_dense")
