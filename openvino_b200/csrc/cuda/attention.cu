@@ -19,6 +19,7 @@
 #include <atomic>
 
 #include "attention.cuh"
+#include "cluster_table.h"
 #include "common.cuh"
 #include "debug_bounds.cuh"
 #include "gemm_common.cuh"
@@ -824,36 +825,75 @@ int launch_decode_combine(const PaKParams& p, int dv, cudaStream_t stream) {
     return 0;
 }
 
-template <int DK, int DV, int G, bool KVU8, int NST, bool ROPE = false>
-static int launch_decode_sizes(const PaKParams& p, cudaStream_t stream) {
-    constexpr int PAGE = 16;
-    const int warp_bytes = KVU8 ? NST * 2 * (PAGE * DK + PAGE * 4) + PAGE * DK * 2 : NST * PAGE * (DK + DV) * 2;
-    const int smem = 16 * DK * 2 + 4 * warp_bytes + 128 + (ROPE ? 2 * DK * 2 + DK / 2 * 8 : 0) + (G > 0 && p.cluster ? p.nsplit * G * (DV + 4) * 4 : 0);
-    constexpr int most = 16 * DK * 2 + 4 * (KVU8 ? NST * 2 * (PAGE * DK + PAGE * 4) + PAGE * DK * 2 : NST * PAGE * (DK + DV) * 2) + 128 + 2 * DK * 2 + DK / 2 * 8 + 8 * (G > 0 ? G : 1) * (DV + 4) * 4;
-    auto kern = pa_decode_kernel<DK, DV, G, PAGE, KVU8, NST, ROPE>;
-    static std::atomic<uint64_t> configured{0};
-    if (int rc = set_smem_once(configured, reinterpret_cast<const void*>(kern), most)) return rc;
-    dim3 grid(p.B, p.Hkv * (G > 0 ? 1 : (p.group + 7) / 8), p.nsplit);
-    if (G > 0 && p.cluster) {
-        cudaLaunchConfig_t cfg;
-        memset(&cfg, 0, sizeof(cfg));
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3(128);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[2];
+// A decode kernel's shared memory, and whether the splits of a step are clusters that sum themselves.
+template <int DK, int DV, int G, bool KVU8, int NST, bool ROPE>
+struct DecodeForm {
+    static constexpr int kPage = 16;
+    static constexpr int kWarp = KVU8 ? NST * 2 * (kPage * DK + kPage * 4) + kPage * DK * 2 : NST * kPage * (DK + DV) * 2;
+    static constexpr int kAlone = 16 * DK * 2 + 4 * kWarp + 128 + (ROPE ? 2 * DK * 2 + DK / 2 * 8 : 0), kShare = G * (DV + 4) * 4;      // kShare: a split's sums
+    static constexpr int kMost = kAlone + 8 * kShare;
+
+    static void config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int B, int Hkv, int nsplit, cudaStream_t stream) {
+        memset(cfg, 0, sizeof(*cfg));
+        cfg->gridDim = dim3(B, Hkv, nsplit);
+        cfg->blockDim = dim3(128);
+        cfg->dynamicSmemBytes = kAlone + nsplit * kShare;
+        cfg->stream = stream;
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 1;
         attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = p.nsplit;
+        attr[0].val.clusterDim.z = nsplit;
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = pdl_enabled() ? 2 : 1;
-        OVB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<PaKParams>(p)));
+        cfg->attrs = attr;
+        cfg->numAttrs = pdl_enabled() ? 2 : 1;
+    }
+
+    static int setup() {
+        static std::atomic<uint64_t> configured{0};
+        return set_smem_once(configured, reinterpret_cast<const void*>(pa_decode_kernel<DK, DV, G, kPage, KVU8, NST, ROPE>), kMost);
+    }
+
+    // A split's sums take 528 bytes of shared memory per query head beside the 103 KB (byte cache: 70) of a CTA, and a cluster needs its SMs together. Where
+    // all clusters of a step are resident, they cost less than a launch for the sum: us without / with them, each with the rotation, 32 / 8 heads
+    // of 16-bit keys: 1 sequence of 1000 keys 10.9 / 9.6, 8 of 1000 13.7 / 12.6, 16 of 500 14.7 / 14.0. A second wave of clusters costs more than it
+    // saves, the more so the larger they are: 10 of 1000 (80 clusters of 4, 71 fit) 15.4 / 19.8, 4 of 2000 (32 of 8, 15 fit) 16.0 / 29.0, 20 of 500
+    // (160 of 2, 148 fit) 20.1 / 22.2. The byte cache leaves two places free: 32 clusters of 8, where 33 fit, took 24.2 us with two query heads per KV head
+    // and 17.4 without. Eight query heads double what is sent: 16-bit keys gain nothing anywhere (0.97 to 1.06), bytes from 200 CTAs on (0.85 to 0.95;
+    // below 0.91 to 1.09).
+    static bool clusters(int B, int Hkv, int nsplit) {
+        if (G == 0 || nsplit < 2 || nsplit > 8 || (G == 8 && (!KVU8 || B * Hkv * nsplit < 200)) || setup() != 0) return false;
+        static ClusterTable table;
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess) return false;
+        const int resident = table.get(dev, nsplit, [&] {
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute attr[2];
+            config(&cfg, attr, B, Hkv, nsplit, nullptr);
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, pa_decode_kernel<DK, DV, G, kPage, KVU8, NST, ROPE>, &cfg) != cudaSuccess) (void)cudaGetLastError();
+            return n;
+        });
+        return B * Hkv <= resident - (KVU8 ? 2 : 0);
+    }
+};
+
+template <int DK, int DV, int G, bool KVU8, int NST, bool ROPE = false>
+static int launch_decode_sizes(PaKParams p, cudaStream_t stream) {
+    using Form = DecodeForm<DK, DV, G, KVU8, NST, ROPE>;
+    auto kern = pa_decode_kernel<DK, DV, G, Form::kPage, KVU8, NST, ROPE>;
+    if (int rc = Form::setup()) return rc;
+    p.cluster = p.cluster && Form::clusters(p.B, p.Hkv, p.nsplit);
+    if (p.cluster) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[2];
+        Form::config(&cfg, attr, p.B, p.Hkv, p.nsplit, stream);
+        OVB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
         return 0;
     }
-    OVB_CHECK_CUDA(launch_pdl(kern, dim3(grid), dim3(128), smem, stream, p));
+    dim3 grid(p.B, p.Hkv * (G > 0 ? 1 : (p.group + 7) / 8), p.nsplit);
+    OVB_CHECK_CUDA(launch_pdl(kern, dim3(grid), dim3(128), Form::kAlone, stream, p));
     OVB_CHECK_CUDA(cudaGetLastError());
     return p.nsplit > 1 ? launch_decode_combine(p, DV, stream) : 0;
 }
@@ -933,12 +973,31 @@ int64_t ovb_pa_scratch_bytes(int B, int Hq, int D, int max_context_len) {
     return (int64_t)B * Hq * 32 * (D + 2) * (int64_t)sizeof(float);
 }
 
-// A step whose CTAs are all resident at once: launches count, and what they would do costs little inside the attention (one sequence of 650
-// keys, 32 / 8 heads: rotation 2.3, attention 6.0 and sum 3.4 us as three launches). With more CTAs every wave of them pays for it (64 sequences of
-// 1150: 60 us as three launches, 71 as one).
-static bool decode_is_small(const ovb_pa_args* a) { return a->B * a->Hkv * decode_nsplit(a->B, a->Hkv, a->max_context_len) <= 444; }
+// Up to this many CTAs the rotation inside the attention is the faster way: its launch is saved, and every CTA hides its part behind its first pages. us as a
+// launch of its own / inside (32 / 8 heads, 16-bit keys): 1 sequence of 250 keys 8.9 / 7.9, 16 of 250 12.0 / 9.6, 55 of 250 (440 CTAs) 22.2 / 19.8, 64 of 250
+// (512) 23.6 / 20.5. In 870 steps of 8 to 1600 CTAs it took 0.71 to 1.01 of the time, 0.97 in the mean from 1200 on, behind that up to 1.03.
+constexpr int kRotateCtas = 1536;
 
-int ovb_decode_attention_rotates(const ovb_pa_args* a) { return ovb_decode_attention_takes(a) && !a->kv_u8 && decode_is_small(a); }
+int ovb_decode_attention_rotates(const ovb_pa_args* a) {
+    return ovb_decode_attention_takes(a) && !a->kv_u8 && a->B * a->Hkv * decode_nsplit(a->B, a->Hkv, a->max_context_len) <= kRotateCtas;
+}
+
+int ovb_decode_attention_clusters(const ovb_pa_args* a, int rotates) {
+    if (!ovb_decode_attention_takes(a) || a->scratch == nullptr) return 0;
+    const int ns = decode_nsplit(a->B, a->Hkv, a->max_context_len);
+    switch (a->Hq / a->Hkv) {
+#define OVB_FORM(g)                                                                                                                  \
+    case g:                                                                                                                          \
+        return a->kv_u8 ? DecodeForm<128, 128, g, true, 3, false>::clusters(a->B, a->Hkv, ns)                                        \
+                        : rotates ? DecodeForm<128, 128, g, false, 3, true>::clusters(a->B, a->Hkv, ns) : DecodeForm<128, 128, g, false, 3, false>::clusters(a->B, a->Hkv, ns);
+        OVB_FORM(1)
+        OVB_FORM(2)
+        OVB_FORM(4)
+        OVB_FORM(8)
+#undef OVB_FORM
+    }
+    return 0;
+}
 
 int ovb_decode_attention_takes(const ovb_pa_args* a) {
     const int G = a->Hkv > 0 ? a->Hq / a->Hkv : 0;
@@ -996,7 +1055,7 @@ static int paged_attention(const ovb_pa_args* a, const int* positions, const int
         p.nsplit = ns;
         int kps = (a->max_context_len + ns - 1) / ns;
         p.keys_per_split = ((kps + 63) / 64) * 64;   // whole pages, and page index % 4 == warp stays aligned
-        p.cluster = alone && ns >= 2 && ns <= 8 && decode_is_small(a);
+        p.cluster = alone;                            // where clusters() says so
         if (a->kv_u8) {
             switch (G) {
                 case 1: return launch_decode<128, 1, true>(p, stream);

@@ -281,11 +281,12 @@ typedef struct {
 } ovb_pa_args;
 int ovb_paged_attention(const ovb_pa_args* a, ovb_stream_t stream);
 // A decode step's attention with what surrounds it. `positions` (and slot_map, theta as in ovb_rope_kv_write; NULL: not): q points at the fused qkv
-// rows before the rotation; queries and the new key are rotated and the new rows written to the cache. The splits of a small step are summed
-// in the same launch.
+// rows before the rotation; queries and the new key are rotated and the new rows written to the cache. The splits are summed in the same launch
+// where they are clusters.
 int ovb_decode_attention(const ovb_pa_args* a, const int* positions, const int* slot_map, float theta, ovb_stream_t stream);
 int ovb_decode_attention_takes(const ovb_pa_args* a);
 int ovb_decode_attention_rotates(const ovb_pa_args* a);      // 1: the rotation inside the attention is the faster way
+int ovb_decode_attention_clusters(const ovb_pa_args* a, int rotates);      // 1: the splits are clusters, which sum themselves (scratch given)
 int64_t ovb_pa_scratch_bytes(int B, int Hq, int D, int max_context_len);
 // 1: a prefill or mixed step of T tokens in B sequences (16-bit cache, head size 128) runs two query tiles per CTA, 0: one.
 int ovb_pa_two_query_tiles(int T, int B, int Hq, int Hkv);

@@ -1351,3 +1351,33 @@ def test_sdpa_dense_causal_and_not(ops, dtype, causal, D, S):
     # probabilities rounded to 16 bits, and the result once more
     assert _rel_err(out, want) < (2.0 ** -9 if dtype == torch.float16 else 2.0 ** -7)
     ops.check_status("sdpa_dense")
+
+
+@pytest.mark.parametrize("Hq,Hkv,B,ctx,u8,clusters", [
+    (32, 8, 1, 1000, False, 1), (32, 8, 8, 1000, False, 1), (32, 8, 10, 1000, False, 0), (32, 8, 1, 2000, False, 1), (32, 8, 2, 2000, False, 0), (32, 8, 4, 2000, False, 0),
+    (32, 8, 18, 500, False, 1), (32, 8, 20, 500, False, 0), (32, 8, 1, 250, False, 0), (32, 8, 1, 4000, False, 0), (64, 8, 1, 1000, False, 0), (16, 8, 4, 2000, False, 1),
+    (16, 8, 4, 2000, True, 0), (32, 8, 24, 500, True, 1), (32, 8, 28, 500, True, 0), (64, 8, 4, 500, True, 0), (64, 8, 8, 1000, True, 1)])
+def test_splits_are_clusters_where_all_are_resident(ops, Hq, Hkv, B, ctx, u8, clusters):
+    """Both sides of the rule at sizes that were measured (one more wave of clusters costs up to twice the attention), and the result of either form."""
+    import ctypes as C
+    D, dev = 128, "cuda"
+    a = ops.PaArgs()
+    a.scratch = a.q = a.out = a.k_cache = a.v_cache = 16
+    a.B = a.T = B
+    a.Hq, a.Hkv, a.D, a.block_size, a.max_q_len, a.max_context_len, a.kv_u8 = Hq, Hkv, D, 16, 1, 1 << (ctx - 1).bit_length(), 1 if u8 else 0
+    assert ops.lib().ovb_decode_attention_clusters(C.byref(a), 0 if u8 else 1) == clusters
+    g = torch.Generator(device=dev).manual_seed(B)
+    blocks = (ctx + 15) // 16
+    tables, begins = torch.randperm(B * blocks, device=dev, generator=g).int(), torch.arange(B + 1, dtype=torch.int32, device=dev) * blocks
+    past, sub = torch.full((B,), ctx - 1, dtype=torch.int32, device=dev), torch.arange(B + 1, dtype=torch.int32, device=dev)
+    q = torch.randn(B, (Hq + 2 * Hkv) * D, device=dev, generator=g).bfloat16()
+    if u8:
+        kv = [torch.randint(0, 256, (B * blocks, Hkv, 16, D), device=dev, dtype=torch.uint8, generator=g) for _ in range(2)]
+        meta = dict(k_meta=torch.full((B * blocks, Hkv, 16, 2), 0.01, device=dev).half(), v_meta=torch.full((B * blocks, Hkv, 16, 2), 0.01, device=dev).half())
+    else:
+        kv, meta = [torch.randn(B * blocks, Hkv, 16, D, device=dev, generator=g).bfloat16() for _ in range(2)], {}
+    args = (q, *kv, past, sub, tables, begins, Hq, Hkv, D)
+    got = ops.decode_attention(*args, max_context_len=a.max_context_len, **meta)
+    want = ops.paged_attention(*args, max_context_len=a.max_context_len, max_q_len=1, **meta)
+    assert _rel_err(got, want.double()) < 1e-3         # the same products, the splits' sums in another order
+    ops.check_status("decode attention")
