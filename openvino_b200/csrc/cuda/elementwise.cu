@@ -1221,10 +1221,11 @@ int ovb_embed_tokens(int* ids, const int* tok_src, const int* last_token, const 
     return 0;
 }
 
-// Rows that several CTAs share: few of them, long, and readable in 16-byte pieces. (64 rows of 128256: 8.4 us, shared 5.9; from 148 rows on every SM
-// has a row of its own.)
+// Rows that several CTAs share: few of them, long, and readable in 16-byte pieces. us with one CTA per row / with eight, logits in L2: 1 row of 32000 3.9 / 2.6,
+// 16 of 32000 3.0 / 3.0, 32 of 65536 3.8 / 3.6, 40 of 65536 4.0 / 4.3, 64 of 128256 5.8 / 5.3, 8 of 16384 2.7 / 2.7. Eight CTAs of 512 threads for each of
+// 74 rows are resident at a time; a second wave doubles the time (80 of 128256 6.6 / 7.6, 128: 8.9 / 11.4).
 static bool argmax_in_pieces(const void* logits, int ld, int rows, int vocab) {
-    return rows < 148 && vocab >= 16384 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+    return rows <= 74 && vocab >= 32000 && vocab >= 2000 * rows && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
 }
 
 static int launch_argmax_pieces(const void* logits, int ld, int rows, int vocab, void* out_ids, int ids_i32, float* out_max, const int* tok_dst, int* last_token,

@@ -1381,3 +1381,15 @@ def test_splits_are_clusters_where_all_are_resident(ops, Hq, Hkv, B, ctx, u8, cl
     want = ops.paged_attention(*args, max_context_len=a.max_context_len, max_q_len=1, **meta)
     assert _rel_err(got, want.double()) < 1e-3         # the same products, the splits' sums in another order
     ops.check_status("decode attention")
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 32000), (5, 32003), (16, 32000), (17, 32000), (74, 148000), (75, 152000)])
+def test_argmax_on_both_sides_of_its_rule(ops, rows, vocab):
+    """Rows shared by eight CTAs and rows of one CTA, an odd tail, the largest entry in the first and in the last piece, ties to the lowest index."""
+    l = torch.randn(rows, (vocab + 7) // 8 * 8, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows)).bfloat16()[:, :vocab]
+    l[0, vocab - 1] = 60.0
+    l[rows - 1, 2] = l[rows - 1, vocab - 2] = 61.0
+    out = torch.empty(rows, dtype=torch.int32, device="cuda")
+    ops.argmax(l, out=out)
+    assert torch.equal(out.long(), l.float().argmax(-1)) and int(out[rows - 1]) == 2
+    ops.check_status("argmax")
