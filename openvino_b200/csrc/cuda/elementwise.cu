@@ -48,7 +48,9 @@ union Pack8 {
 
 // ------------------------------------------------------------------------------------ RMSNorm
 // One CTA per row; cols % 8 == 0. Row is kept in registers (up to 8 vectors per thread).
-template <int THREADS, int MAXV>
+// AHEAD: the weights come with the row, not behind its sum, and the warps meet at one barrier: a step of few tokens waits for these loads. With many rows the
+// registers cost resident CTAs. Rows by index: AHEAD only.
+template <int THREADS, int MAXV, bool AHEAD>
 __global__ void __launch_bounds__(THREADS)
 rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                const __nv_bfloat16* __restrict__ gamma, __nv_bfloat16* __restrict__ y,
@@ -58,7 +60,7 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
     const size_t row = blockIdx.x;
     const int nvec = cols >> 3;
     size_t from = row;
-    if (row_idx != nullptr) {
+    if (AHEAD && row_idx != nullptr) {
         int id = row_idx[row];
         if (id < 0 || id >= x_rows) {            // as an embedding does
             (void)OVB_DBG_ROW(-1, 1);
@@ -67,12 +69,13 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
         from = (size_t)id;
     }
     const uint4* xr = reinterpret_cast<const uint4*>(x + from * cols);
-    // the weights come with the row, not behind the sum: a step of few tokens waits for these loads
-    uint4 gv[MAXV];
+    uint4 gv[AHEAD ? MAXV : 1];
+    if (AHEAD) {
 #pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-        const int v = threadIdx.x + i * THREADS;
-        if (v < nvec) gv[i] = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+        for (int i = 0; i < MAXV; ++i) {
+            const int v = threadIdx.x + i * THREADS;
+            if (v < nvec) gv[AHEAD ? i : 0] = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+        }
     }
     const uint4* rr = residual ? reinterpret_cast<const uint4*>(residual + row * cols) : nullptr;
     float vals[MAXV][8];
@@ -103,18 +106,22 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restr
             for (int j = 0; j < 8; ++j) ss += vals[i][j] * vals[i][j];
         }
     }
-    // every warp sums all warps' parts: one barrier
-    ss = warp_sum(ss);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    const float tot = warp_sum((threadIdx.x & 31) < THREADS / 32 ? red[threadIdx.x & 31] : 0.f);
+    float tot;
+    if (AHEAD) {                                 // every warp sums all warps' parts: one barrier
+        ss = warp_sum(ss);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+        __syncthreads();
+        tot = warp_sum((threadIdx.x & 31) < THREADS / 32 ? red[threadIdx.x & 31] : 0.f);
+    } else {
+        tot = block_sum<THREADS>(ss, red);
+    }
     const float inv = rsqrtf(tot / float(cols) + eps);
 #pragma unroll
     for (int i = 0; i < MAXV; ++i) {
         const int v = threadIdx.x + i * THREADS;
         if (v < nvec) {
             Pack8 g, o;
-            g.u = gv[i];
+            g.u = AHEAD ? gv[AHEAD ? i : 0] : reinterpret_cast<const uint4*>(gamma)[v];
 #pragma unroll
             for (int j = 0; j < 8; ++j) o.b[j] = __float2bfloat16_rn(vals[i][j] * inv * __bfloat162float(g.b[j]));
             reinterpret_cast<uint4*>(y + row * cols)[v] = o.u;
@@ -1055,7 +1062,13 @@ static int rmsnorm(const void* x, const void* residual, const void* gamma, void*
     auto Y = (__nv_bfloat16*)y;
     auto RO = (__nv_bfloat16*)residual_out;
     const int nvec = cols / 8;
-    auto kern = nvec <= 256 ? rmsnorm_kernel<256, 1> : nvec <= 512 ? rmsnorm_kernel<256, 2> : nvec <= 1024 ? rmsnorm_kernel<256, 4> : rmsnorm_kernel<256, 8>;
+    // us without / with the weights ahead: 1 row of 4096 2.1 / 1.7, 300 of 4096 2.4 / 2.2, 300 of 8192 3.1 / 3.1, 1024 of 4096 3.4 / 3.7, 8192 of 4096 24.9 / 27.0, 8192 of 16384
+    // 97 / 123.
+    const bool ahead = row_idx != nullptr || rows <= (cols <= 8192 ? 300 : 148);
+    auto kern = nvec <= 256    ? (ahead ? rmsnorm_kernel<256, 1, true> : rmsnorm_kernel<256, 1, false>)
+                : nvec <= 512  ? (ahead ? rmsnorm_kernel<256, 2, true> : rmsnorm_kernel<256, 2, false>)
+                : nvec <= 1024 ? (ahead ? rmsnorm_kernel<256, 4, true> : rmsnorm_kernel<256, 4, false>)
+                               : (ahead ? rmsnorm_kernel<256, 8, true> : rmsnorm_kernel<256, 8, false>);
     OVB_CHECK_CUDA(launch_pdl(kern, dim3(rows), dim3(256), 0, stream, X, R, G, Y, RO, cols, eps, row_idx, x_rows));
     OVB_CHECK_CUDA(cudaGetLastError());
     return 0;

@@ -1393,3 +1393,17 @@ def test_argmax_on_both_sides_of_its_rule(ops, rows, vocab):
     ops.argmax(l, out=out)
     assert torch.equal(out.long(), l.float().argmax(-1)) and int(out[rows - 1]) == 2
     ops.check_status("argmax")
+
+
+@pytest.mark.parametrize("rows", [1, 148, 149, 300, 301])
+@pytest.mark.parametrize("cols", [256, 2048, 2056, 4096, 8192, 8200, 16384])
+def test_rmsnorm_forms(ops, rows, cols):
+    """Both forms of the norm (weights ahead of the sum or behind it) at the limits of the rule, with a residual and without, against 64 bits."""
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    x, r, gamma = (torch.randn(n, cols, device="cuda", generator=g).bfloat16() for n in (rows, rows, 1))
+    for res in (None, r):
+        y = ops.rmsnorm(x, gamma[0], 1e-5, residual=res)
+        y = y[0] if isinstance(y, tuple) else y
+        h = x.double() if res is None else (x.float() + res.float()).bfloat16().double()
+        want = h * torch.rsqrt(h.square().mean(-1, keepdim=True) + 1e-5) * gamma.double()
+        assert ((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()        # one rounding to 16 bits
