@@ -511,17 +511,31 @@ static bool few_plan(int wmode, int T, int N, int K, int forced, FewPlan* best) 
     return best_t < 1e30;
 }
 
-// Where it is the faster one, against gemm_sm100.cu (us with the norm before it; cold weights). u4: 128256 x 4096 16 tokens 67 / 89, 37 tokens 84 / 96, 64
-// tokens 98 / 98; 4096 x 14336 24 tokens 16 / 24; 4096 x 4096 24 tokens 11 / 11. u8: 128256 x 4096 24 tokens 94 / 110, 64 tokens 117 / 127; 6144 x 4096 37
-// tokens 15 / 19. fp8: 57344 x 8192 32 tokens 89 / 113; 8192 x 28672 64 tokens 57 / 80. With more than 48 tokens the MMAs bind a stage: u4 weights, half
-// the bytes, gain nothing (a step of 64 tokens 690 / 697), and 8-bit tiles that fill one CTA per SM a little more than once suit the two smaller CTAs
-// of gemm_sm100.cu better (28672 x 4096, 64 tokens: 40.5 / 36.6).
+// Where it is the faster one, against gemm_sm100.cu: the smallest K, by token columns (16, 32, 48, 64) and tiles of 128 rows (up to 8, 16, 32, 64, 148, 296,
+// more). A tile costs the exchange of its sums and its epilogue, which grow with the tokens and which short sums do not hide, and 149 to 296 tiles
+// are one wave of the other kernel's two CTAs per SM and two rounds here. us here / there, launches one after the other with cold weights: u4, 16
+// tokens 128256 x 4096 65.5 / 89, 4096 x 14336 14.9 / 18.2, 28672 x 1024 11.5 / 10.8; 37 tokens 28672 x 4096 26.6 / 28.2, 4096 x 4096 11.0 / 10.2, 20480 x
+// 1024 14.6 / 11.5; u8, 24 tokens 6144 x 4096 11.8 / 14.6, 1024 x 1024 7.4 / 5.4; 48 tokens 24576 x 2048 20.0 / 19.2; 64 tokens 8192 x 28672 58 / 74, 1024 x
+// 1024 10.8 / 6.9, 28672 x 4096 40.5 / 36.6. With 64 token columns the MMAs bind a stage, so that half the bytes gain u4 weights nothing.
+static bool few_is_faster(int wmode, int T, int tiles, int K) {
+    constexpr int never = 1 << 30;
+    static constexpr int u4[4][7] = {{256, 256, 256, 256, 1024, 1536, 256}, {2048, 2048, 6144, 3072, 3072, 3072, 1536}, {6144, 2048, 6144, 2048, 3072, 4096, 3072},
+                                     {never, never, never, never, never, never, never}};
+    static constexpr int bytes[4][7] = {{256, 256, 256, 256, 1024, 1024, 256}, {2048, 2048, 4096, 1024, 2048, 2048, 1024}, {6144, 2048, 3072, 1024, 2048, 4096, 1536},
+                                        {6144, 2048, 4096, 2048, 3072, 8192, 3072}};
+    const int col = tiles <= 8 ? 0 : tiles <= 16 ? 1 : tiles <= 32 ? 2 : tiles <= 64 ? 3 : tiles <= 148 ? 4 : tiles <= 296 ? 5 : 6, row = (T - 1) / 16;
+    // the other kernel shares such a K better: u4, 16 tokens 4096 x 2048 7.2 / 6.1, 8192 x 1024 7.7 / 6.9
+    if (wmode == OVB_W_U4 && row == 0 && ((col == 2 && K > 1024 && K < 4096) || (col == 3 && K >= 1024 && K < 2048))) return false;
+    // a few tiles more than clusters of two: one CTA per tile leaves half of the SMs idle (10240 x 6144 u8, 64 tokens 27.6 / 23.6, 10240 x 8192, 37 tokens 28.3 / 27.3)
+    if (wmode != OVB_W_U4 && tiles > 74 && tiles <= 90 && K >= 6144 && K <= 8192) return false;
+    return K >= (wmode == OVB_W_U4 ? u4 : bytes)[row][col];
+}
+
 bool gemm_few_takes(const ovb_gemm_args* a) {
     if (!is_quant(a->wmode) || a->T > kFewTokens || a->comm != nullptr || a->group_offsets != nullptr || a->group_mode == 3 || a->block_t != 0) return false;
     if (a->N % TILE_N != 0 || a->K % kFewStageK != 0 || a->group_size % 128 != 0 || a->w_kb_stride != 0) return false;
     if (a->splits > 8 || a->splits > a->K / kFewStageK) return false;
-    const int tiles = a->N / TILE_N;
-    if (a->splits == 0 && a->T > 48 && (a->wmode == OVB_W_U4 || (tiles > 148 && tiles <= 296 && a->K <= 4096))) return false;
+    if (a->splits == 0 && !few_is_faster(a->wmode, a->T, a->N / TILE_N, a->K)) return false;
     FewPlan f;
     return few_plan(a->wmode, a->T, a->N, a->K, a->splits, &f);
 }

@@ -1458,7 +1458,15 @@ static int comm_packets(int world, int mode) {
     return world <= 2;
 }
 
-int ovb_gemm_route(const ovb_gemm_args* a) { return ovb::gemm_ring_takes(a) || ovb::gemm_stream_takes(a) ? 2 : ovb::gemm_pair_takes(a) ? 1 : 0; }
+int ovb_gemm_kernel(const ovb_gemm_args* a) {
+    using namespace ovb;
+    return gemm_ring_takes(a) ? OVB_GEMM_RING : gemm_stream_takes(a) ? OVB_GEMM_STREAM : gemm_few_takes(a) ? OVB_GEMM_FEW : gemm_pair_takes(a) ? OVB_GEMM_PAIR : OVB_GEMM_SINGLE;
+}
+
+int ovb_gemm_route(const ovb_gemm_args* a) {
+    const int k = ovb_gemm_kernel(a);
+    return k == OVB_GEMM_RING || k == OVB_GEMM_STREAM ? 2 : k == OVB_GEMM_PAIR ? 1 : 0;
+}
 
 int ovb_gemm_norms(const ovb_gemm_args* a) {
     using namespace ovb;
@@ -1511,11 +1519,11 @@ int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream_) {
                     "ovb_gemm: grouped GEMM needs tile-packed weights (u4 or 16-bit), N %% 128 == 0, K %% 64 == 0 and no communicator");
     }
     const int bt = a->block_t ? a->block_t : pick_block_t(a->T);
-    const bool ring = gemm_ring_takes(a), streamed = !ring && gemm_stream_takes(a), few = !ring && !streamed && gemm_few_takes(a);
-    if (ring || streamed || few || gemm_pair_takes(a)) {
+    const int kernel = ovb_gemm_kernel(a);
+    if (kernel != OVB_GEMM_SINGLE) {
         // a selective build keeps this kernel's variant for the token counts of the recorded ones, which other sizes of the same range need
         g_cc_gemm_used[((f16 ? OVB_W_BF16 : a->wmode) * 2 + (f16 ? 1 : 0)) & 15].fetch_or(1u << bt_bit(bt), std::memory_order_relaxed);
-        return ring ? gemm_ring(a, stream) : streamed ? gemm_stream(a, stream) : few ? gemm_few(a, stream) : gemm_pair(a, stream);
+        return kernel == OVB_GEMM_RING ? gemm_ring(a, stream) : kernel == OVB_GEMM_STREAM ? gemm_stream(a, stream) : kernel == OVB_GEMM_FEW ? gemm_few(a, stream) : gemm_pair(a, stream);
     }
     const int splits = (swiglu || grouped) ? 1 : a->splits;   // 0: chosen at launch, where the kernel variant and its cluster occupancy are known
     const int64_t tiles = (int64_t)ceil_div(a->N, TILE_N) * ceil_div(a->T, bt);

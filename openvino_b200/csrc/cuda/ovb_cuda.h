@@ -108,6 +108,9 @@ typedef struct {
 int ovb_gemm(const ovb_gemm_args* a, ovb_stream_t stream);
 // The kernel that ovb_gemm runs this problem on: 0 single CTAs (gemm_sm100.cu, gemm_few.cu), 1 pairs of CTAs (gemm_pair.cu), 2 few tokens (gemm_ring.cu, gemm_stream.cu).
 int ovb_gemm_route(const ovb_gemm_args* a);
+// The same, by its file: gemm_sm100.cu, gemm_pair.cu, gemm_stream.cu, gemm_ring.cu, gemm_few.cu.
+enum { OVB_GEMM_SINGLE = 0, OVB_GEMM_PAIR = 1, OVB_GEMM_STREAM = 2, OVB_GEMM_RING = 3, OVB_GEMM_FEW = 4 };
+int ovb_gemm_kernel(const ovb_gemm_args* a);
 // 1: ovb_gemm takes x_norm in (products of up to four tokens); the fields x_norm and x_rows themselves are not looked at.
 int ovb_gemm_norms(const ovb_gemm_args* a);
 // Bytes of split-K workspace / number of counters that ovb_gemm may need for the given problem.

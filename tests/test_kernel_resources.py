@@ -86,3 +86,31 @@ def test_few_tokens_leave_clusters_that_would_share_many_tiles(gemm, N, K, T, ro
     a.x = a.w = a.out = 16
     a.T, a.N, a.K, a.ldx, a.group_size, a.wmode = T, N, K, K, 128, ops.W_U4
     assert ops.lib().ovb_gemm_route(C.byref(a)) == route
+
+
+SINGLE, PAIR, STREAM, RING, FEW = range(5)
+
+
+@pytest.mark.parametrize("fmt,N,K,splits,T,kernel", [
+    # what the test of the few-token kernel runs with a number of splits: one stage of K, odd shares of K, several rounds of tiles
+    *[(f, N, K, s, T, FEW) for f, T in (("u4", 5), ("u8", 33), ("f8", 64))
+      for N, K, splits in ((128, 256, (1,)), (256, 1280, (2, 3, 5)), (512, 2048, (4, 6, 7, 8)), (128 * 150, 256, (1,)), (128 * 76, 512, (2,)), (128 * 19, 2048, (8,))) for s in splits],
+    # both sides of the rule, at sizes that were measured on both kernels
+    ("u4", 128256, 4096, 0, 16, FEW), ("u4", 4096, 14336, 0, 16, FEW), ("u4", 28672, 1024, 0, 16, SINGLE), ("u4", 4096, 2048, 0, 16, SINGLE), ("u4", 8192, 1024, 0, 8, SINGLE), ("u4", 8192, 2048, 0, 8, FEW), ("u4", 4096, 1024, 0, 16, FEW),
+    ("u4", 28672, 4096, 0, 37, FEW), ("u4", 4096, 4096, 0, 37, SINGLE), ("u4", 20480, 1024, 0, 37, SINGLE), ("u4", 128256, 4096, 0, 64, SINGLE),
+    ("u8", 6144, 4096, 0, 24, FEW), ("u8", 1024, 1024, 0, 24, SINGLE), ("u8", 24576, 2048, 0, 48, SINGLE), ("f8", 8192, 28672, 0, 64, FEW), ("f8", 1024, 1024, 0, 64, SINGLE),
+    ("u8", 28672, 4096, 0, 64, SINGLE), ("u8", 128256, 4096, 0, 64, FEW), ("f8", 10240, 8192, 0, 37, SINGLE), ("f8", 10240, 14336, 0, 37, FEW),
+    ("u4", 512, 2048, 0, 65, SINGLE), ("u4", 512, 2048 + 128, 0, 16, SINGLE), ("u4", 512 + 32, 2048, 0, 16, SINGLE),
+    ("u4", 2048, 4096, 0, 1, RING), ("u4", 2048, 4096, 0, 4, RING), ("u4", 2048, 4096, 0, 5, FEW), ("u4", 2048, 4096 - 256, 0, 1, STREAM), ("u4", 1280, 8192, 0, 3, RING),
+    ("u8", 512, 2048, 0, 4, STREAM), ("f8", 512, 2048, 0, 4, STREAM), ("u8", 128256, 4096, 0, 4, FEW), ("dense", 512, 2048, 0, 8, STREAM), ("dense", 512, 2048, 0, 9, SINGLE),
+    ("dense", 28672, 4096, 0, 512, PAIR)])
+def test_products_run_on_the_kernel_for_their_size(gemm, fmt, N, K, splits, T, kernel):
+    """Which kernel the products run on that the kernels' own tests compute."""
+    import ctypes as C
+    from openvino_b200.ops import cuda as ops
+    a = ops.GemmArgs()
+    a.x = a.w = a.out = a.scales = 16
+    a.T, a.N, a.K, a.ldx, a.group_size, a.splits = T, N, K, K, 128, splits
+    a.wmode = {"u4": ops.W_U4, "u8": ops.W_U8, "f8": ops.W_F8, "dense": ops.W_BF16}[fmt]
+    a.w_tiled = 1 if fmt == "dense" else 0
+    assert ops.lib().ovb_gemm_kernel(C.byref(a)) == kernel
