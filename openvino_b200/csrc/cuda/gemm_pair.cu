@@ -458,10 +458,11 @@ static int pick_cut(int bt, int rest, int pairs) {
 // Token tile: the smallest estimate of waves x (tile + 32); the constant stands for what a wave costs beside its MMAs (the pair that
 // finishes last, the epilogue of the last tile). With 999 tokens a 256-token tile of the 4096 x 4096 product fills 64 of 74 pairs
 // once, 6144 rows fill them 1.3 times and take 192-token tiles (two full waves) instead.
-// A cut last wave has to be cheaper by 4 %: its parts read the weights once each. us without / with it, gate and up of 28672 x 4096:
-// 512 tokens 101 / 87, 999: 168 / 159, 2048: 315 / 309; 4096 x 14336, 4096 tokens: 346 / 324. Where nearly every pair has a tile it costs as
-// much as it gives (4096 x 4096, 1024 tokens, one cut wave of 64 tiles: 31 / 34 us), and so it does where the sum is short (4096 x 1024,
-// 4096 tokens: 36.3 / 37.0).
+// A cut last wave has to be cheaper by 3 %. Its parts read their 256 weight rows once each and take 166 of these units with 32 tokens, 182 with 64, 214 with
+// 128 (100 products of 192 to 3000 tokens, K 2048 to 14336). us without / with it, gate and up of 28672 x 4096: 512 tokens 98.8 / 89.6, 999: 166.7 /
+// 160.3; 4096 x 14336, 4096 tokens: 331 / 315; 19200 x 2048, 512 tokens: 48.6 / 37.4. Where 72 parts stand for 12 tiles it costs as much as it gives or more
+// (10240 x 8192, 768 tokens: 101 / 109, 8192 x 4096, 900: 66 / 75), and so it does where nearly every pair has a tile (4096 x 4096, 1024 tokens,
+// one cut wave of 64 tiles: 31 / 34) and where the sum is short (4096 x 1024, 4096 tokens: 36.3 / 37.0).
 constexpr int kCutMinK = 2048;
 static int pick_pair_tile(int T, int N, int K, int pairs, int* cut) {
     const int tiles_n = ceil_div(N, 256);
@@ -472,10 +473,10 @@ static int pick_pair_tile(int T, int N, int K, int pairs, int* cut) {
         if (t < best_t * 0.999) { best_t = t; best = bt; }
     }
     if (cut == nullptr || K < kCutMinK || (int64_t)tiles_n * ceil_div(T, 64) > (1 << 24)) return best;
-    best_t *= 0.96;
+    best_t *= 0.97;
     for (int bt = 256; bt >= 64; bt -= 32) {
         const int tiles = tiles_n * ceil_div(T, bt), parts = tiles < pairs ? 1 : pick_cut(bt, tiles % pairs, pairs);
-        const double t = (double)(tiles / pairs) * (bt + 32) + bt / parts + 64;
+        const double t = (double)(tiles / pairs) * (bt + 32) + 0.5 * bt / parts + 150;
         if (parts > 1 && t < best_t) { best_t = t; best = bt; best_cut = parts; }
     }
     *cut = best_cut;
