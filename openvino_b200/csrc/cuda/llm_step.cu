@@ -79,6 +79,8 @@ static int check_layer(const ovb_llm_step* s, const ovb_llm_layer* l, int i) {
 
 extern "C" {
 
+int ovb_llm_struct_bytes(int which) { return which == 0 ? (int)sizeof(ovb_llm_weight) : which == 1 ? (int)sizeof(ovb_llm_layer) : (int)sizeof(ovb_llm_step); }
+
 int64_t ovb_llm_scratch_bytes(const ovb_llm_step* s) {
     using namespace ovb;
     int64_t most = 0;

@@ -347,6 +347,7 @@ typedef struct {
     int launches;             // out: operations launched by ovb_llm_step_run
 } ovb_llm_step;
 int64_t ovb_llm_scratch_bytes(const ovb_llm_step* s);
+int ovb_llm_struct_bytes(int which);        // sizes of 0: ovb_llm_weight, 1: ovb_llm_layer, 2: ovb_llm_step, for callers that lay them out themselves
 int ovb_llm_step_run(ovb_llm_step* s, ovb_stream_t stream);
 
 // The same with a value per key that is added to its scaled scores (a padding mask): key_bias[b * bias_stride + j], in the type of q; bias_stride 0:

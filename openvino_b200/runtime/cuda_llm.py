@@ -429,10 +429,13 @@ class CudaLlmExecutor(LlmExecutor):
         self.full_logits = comm.alloc((max(max_seqs, 1), cfg.vocab_size)) if self.tp_size > 1 else None
         self._expert_windows = {}
 
+    def _is_native(self) -> bool:
+        return self.tp_size == 1 and not self.cfg.num_experts and all(p.mode != K.W_F32 for lw in self.w.layers for p in (lw.qkv, lw.o, lw.gate_up, lw.down))
+
     # -- one forward pass over the buffers of `sb`
     def _forward(self, sb: StepBuffers, shp: StepShape) -> None:
         cfg, w, ws = self.cfg, self.w, self.ws
-        if self.tp_size == 1 and not cfg.num_experts and all(p.mode != K.W_F32 for lw in w.layers for p in (lw.qkv, lw.o, lw.gate_up, lw.down)):
+        if self._is_native():
             return self._forward_native(sb, shp)
         T, B = shp.T, shp.B
         D = cfg.head_dim
@@ -495,8 +498,9 @@ class CudaLlmExecutor(LlmExecutor):
         self.kernel_launches += n + 5
 
     def _forward_native(self, sb: StepBuffers, shp: StepShape) -> None:
-        """The pass of a dense model on one GPU: one call into the kernel library, which launches what `_forward` launches one by one. The addresses
-        are collected anew for every pass."""
+        """The pass of a dense model on one GPU as one call into the kernel library, with the results of `_forward` up to the order of 32-bit sums. It takes
+        fewer launches: ids with their embedding, norms inside products of up to four tokens, the rotation inside the attention of small decode steps,
+        the last norm with its gather. The addresses are collected anew for every pass."""
         cfg, w, ws, T, B = self.cfg, self.w, self.ws, shp.T, shp.B
         if T > sb.Tcap or B > sb.Bcap:
             raise ValueError("a step of %d tokens in %d sequences does not fit buffers of %d and %d" % (T, B, sb.Tcap, sb.Bcap))

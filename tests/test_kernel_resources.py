@@ -88,6 +88,15 @@ def test_few_tokens_leave_clusters_that_would_share_many_tiles(gemm, N, K, T, ro
     assert ops.lib().ovb_gemm_route(C.byref(a)) == route
 
 
+def test_step_descriptors_have_the_size_of_the_c_structs(gemm):
+    import ctypes as C
+    import struct
+    from openvino_b200.ops import cuda as ops
+    sizes = [struct.calcsize("<" + ops.LLM_WEIGHT), struct.calcsize(ops.LLM_LAYER), C.sizeof(ops.LlmStep)]
+    assert [ops.lib().ovb_llm_struct_bytes(i) for i in range(3)] == sizes
+    assert C.sizeof(dict(ops.LlmStep._fields_)["head"]) == sizes[0]
+
+
 SINGLE, PAIR, STREAM, RING, FEW = range(5)
 
 

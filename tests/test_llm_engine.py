@@ -123,3 +123,119 @@ def test_prefix_caching_reuses_kv_blocks_and_keeps_the_tokens():
     assert results[True][0] == results[False][0]
     assert results[True][2] == 2 * 64                                  # two later requests x four cached blocks of 16 tokens
     assert results[True][1] == results[False][1] - 2 * 64
+
+
+def _fill_step(ex, spans, blocks, vocab, seed):
+    """A step of ``spans`` (earlier tokens, new tokens) whose blocks are handed out in turn."""
+    import numpy as np
+    from openvino_b200.genai.pipeline import step_shape
+    from openvino_b200.genai.scheduler import Scheduler, SchedulerConfig, Sequence
+    rng = np.random.RandomState(seed)
+    T = sum(n for _, n in spans)
+    sched = Scheduler(SchedulerConfig(max_num_batched_tokens=max(T, 64), max_num_seqs=len(spans), num_kv_blocks=blocks, block_size=16))
+    free, seqs = list(rng.permutation(blocks)), []
+    for i, (past, n) in enumerate(spans):
+        s = Sequence(i, rng.randint(0, vocab, past + n).astype(np.int32), 0)
+        s.num_computed, s.blocks = past, [int(free.pop()) for _ in range((past + n + 15) // 16)]
+        sched.admit(s)
+        seqs.append(s)
+    step = sched.place(seqs, [n for _, n in spans])
+    sb = ex.decode if step.max_q_len == 1 and len(seqs) <= ex.decode.Bcap else ex.prefill
+    sched.fill(step, {name: sb.view(name, host=0).numpy() for name in sb.offsets})
+    return sb, step_shape(step)
+
+
+STEPS = [
+    [(33, 1)],                                              # norms inside the products, the rotation inside the attention
+    [(700, 1), (3, 1), (15, 1), (16, 1)],
+    [(5 * i, 1) for i in range(5)],                         # the gathered norm as a launch of its own
+    [(1100 + i, 1) for i in range(65)],                     # rotation, attention and sum as launches of their own
+    [(40, 1), (0, 37), (100, 20), (7, 1)],                  # decoding beside portions of prompts
+    [(0, 1023)], [(0, 1025)],
+]
+
+
+@pytest.mark.parametrize("fmt,kv,gate,bias,window", [("int4", "bf16", True, False, 0), ("bf16", "bf16", True, False, 100), ("int8", "u8", True, False, 0),
+                                                     ("fp8", "bf16", False, False, 0), ("bf16", "u8", False, True, 0), ("int4", "bf16", False, True, 0)])
+def test_native_step_against_the_launches_one_by_one(fmt, kv, gate, bias, window, monkeypatch):
+    """One call into the kernel library against `_forward`'s own launches: logits, tokens and all cache rows. Where they differ, 32-bit sums were added in
+    another order, so that a 16-bit value between two kernels is a neighbour now and then: far less than the 2^-8 of rounding all of them once. A
+    wrong pointer, size, flag or stride shows as a difference of the order of one."""
+    from openvino_b200.models.llm_config import TINY_LLAMA
+    from openvino_b200.ops import cuda as K
+    from openvino_b200.runtime.cuda_llm import CudaLlmExecutor, LlmWeights
+
+    cfg = TINY_LLAMA.with_(weight_format=fmt, sliding_window=window)
+    w = LlmWeights.random(cfg, "cuda", seed=4)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    for lw in w.layers:
+        lw.gate_up.swiglu = gate
+        lw.norm1.normal_(1.0, 0.1, generator=g)
+        lw.norm2.normal_(1.0, 0.1, generator=g)
+        for p in (lw.qkv, lw.o, lw.gate_up, lw.down) if bias else ():
+            p.bias = torch.randn(p.N, device="cuda", generator=g).bfloat16()
+    w.final_norm.normal_(1.0, 0.1, generator=g)
+    blocks = 65 * 73
+    ex = CudaLlmExecutor(cfg, w, blocks, max_batch_tokens=1100, max_seqs=65, max_blocks_per_seq=80, use_cuda_graphs=False, kv_cache_precision=kv)
+    caches = [t for t in ex.k_cache + ex.v_cache + ex.k_meta + ex.v_meta if t is not None]
+    for t in caches:
+        t.copy_(torch.randint(100, 156, t.shape, device="cuda", generator=g).to(t.dtype) if t.dtype == torch.uint8 else
+                torch.rand(t.shape, device="cuda", generator=g) * 0.01 + 0.01 if t.dtype == torch.float16 else torch.randn(t.shape, device="cuda", generator=g))
+    before = [t.clone() for t in caches]
+
+    def rel(a, b):
+        a, b = a.double(), b.double()
+        return float((a - b).norm() / b.norm())
+    for n, spans in enumerate(STEPS):
+        sb, shape = _fill_step(ex, spans, blocks, cfg.vocab_size, n)
+        got = []
+        for native in (True, False):
+            for t, v in zip(caches, before):
+                t.copy_(v)
+            sb.logits.zero_()
+            ex.last_token.fill_(-7)
+            monkeypatch.setattr(CudaLlmExecutor, "_is_native", lambda self, native=native: native)
+            ex.upload(sb)
+            tokens = ex.run(sb, shape)
+            got.append((sb.logits[:shape.B].clone(), tokens.clone(), ex.last_token.clone(), [t.clone() for t in caches]))
+        K.check_status("native step")
+        (la, ta, fa, ca), (lb, tb, fb, cb) = got
+        assert rel(la, lb) < 2.0 ** -8, (n, rel(la, lb))
+        best = lb.float().gather(1, ta.long()[:, None])[:, 0]
+        assert (best >= lb.float().max(1).values - 0.02 * lb.float().abs().max()).all(), n        # the same token, or one as good
+        assert torch.equal(fa == -7, fb == -7)
+        slots = sb.view("slot_map")[:shape.T].long()
+        new = torch.zeros(blocks * 16, dtype=torch.bool, device="cuda")
+        new[slots] = True
+        new = new.reshape(blocks, 1, 16, 1)
+        for a, b, v in zip(ca, cb, before):
+            assert torch.equal(a.masked_fill(new, 0), v.masked_fill(new, 0)), n                   # nothing but the step's rows was written
+            a, b = (t.permute(0, 2, 1, 3).reshape(blocks * 16, -1)[slots] for t in (a, b))
+            if a.dtype == torch.uint8:
+                assert (a.int() - b.int()).abs().max() <= 2, n
+            else:
+                assert rel(a, b) < 2.0 ** -8, n
+
+
+def test_native_step_shares_the_memory_for_expanded_weights(monkeypatch):
+    """Quantised products of many tokens expand their weights: one piece of memory for the four products of a layer, sized for the largest."""
+    from openvino_b200.models.llm_config import LLAMA3_8B
+    from openvino_b200.ops import cuda as K
+    from openvino_b200.runtime.cuda_llm import CudaLlmExecutor, LlmWeights
+
+    cfg = LLAMA3_8B.with_(num_layers=1, vocab_size=512)
+    ex = CudaLlmExecutor(cfg, LlmWeights.random(cfg, "cuda", seed=2), 80, max_batch_tokens=1100, max_seqs=1, max_blocks_per_seq=80, use_cuda_graphs=False)
+    asked, plain = [], K._gemm_scratch
+    monkeypatch.setattr(K, "_gemm_scratch", lambda n, d: asked.append(n) or plain(n, d))
+    for T in (1023, 1024, 1100):
+        sb, shape = _fill_step(ex, [(0, T)], 80, cfg.vocab_size, T)
+        out = []
+        for native in (True, False):
+            monkeypatch.setattr(CudaLlmExecutor, "_is_native", lambda self, native=native: native)
+            del asked[:]
+            ex.upload(sb)
+            ex.run(sb, shape)
+            out.append((sb.logits[:1].clone(), ex.k_cache[0].clone(), ex.v_cache[0].clone(), max(asked, default=0)))
+        K.check_status("native step")
+        assert (out[0][3] > 0) == (T >= 1024) and out[0][3] == out[1][3]
+        assert all(torch.equal(a, b) for a, b in zip(out[0][:3], out[1][:3])), T                  # the same kernels in the same order
