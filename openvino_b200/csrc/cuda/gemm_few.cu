@@ -26,10 +26,12 @@ constexpr int kFewGroups = 3;                                  // groups of four
 constexpr int kFewIssuers = 2;                                 // warps that issue MMAs
 constexpr int kFewStageK = 256;                                // columns of K of a stage: 128 for either issuer
 constexpr int kFewThreads = (12 + 4 * kFewGroups) * 32;
+constexpr int kFewBound = 896;                                 // (see kFewSmem)
 constexpr int kFewMaxRing = 12, kFewMaxX = 8, kFewA = 3;        // slots of packed weights, of tokens, of expanded weights
 constexpr int kFewBarBytes = 1024;
-// 8 KB of registers (72 a thread) and 11 KB of shared memory stay free: the blocks of a norm or a rotation fit beside a CTA, so that it starts, and
-// requests its weights, while they still run.
+// 40 KB of registers (u4: 768 threads of 72; 8-bit weights start 640) and 11 KB of shared memory stay free: a block of a norm or a rotation (256
+// threads of up to 40) fits beside a CTA, so that it starts, and requests its weights, while they still run. The kernel's launch bound names 896
+// threads, more than any plan starts, for these 72 registers: bound to 768 it takes 80, and 16 KB would be left.
 constexpr int kFewSmem = 216 * 1024;
 constexpr int kFewTokens = 64;                                 // largest T
 
@@ -79,7 +81,7 @@ __device__ __forceinline__ void few_mma_stage(uint32_t d, uint32_t ta, uint64_t 
 }
 
 template <int WMODE>
-__global__ void __launch_bounds__(896, 1)
+__global__ void __launch_bounds__(kFewBound, 1)
 gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const FewParams p) {
     using E = __nv_bfloat16;
     constexpr int SLOT = few_slot(WMODE), PAIRS = few_pairs(WMODE);

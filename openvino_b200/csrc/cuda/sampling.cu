@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const E* __restr
 // order: CTA, warp, piece of 256, lane). What bounds it then is the way between the CTAs, about 1.3 us for a step of the bisection: every CTA pushes its count and
 // mass to all (st.async) and adds up the eight itself, in the same order. Once no CTA keeps more than kShareList entries, the kept ones go to all
 // CTAs, each of which takes the remaining steps by itself.
-// 24 rows of 128256 entries, top-k 50 and top-p 0.95: 73 us a step with one CTA per row, 38 here.
+// (A thread holds 16 words of its row and the steps of two forms in 64 registers, two CTAs to an SM: some 30 words are parked in local memory.)
 constexpr int kShareThreads = 512, kShareCtas = 8, kShareList = 512;
 
 struct ShareBox {                         // what the CTAs of a row send one another
@@ -687,9 +687,11 @@ static int sample_rows(const E* logits, int ld, int rows, int vocab, float tempe
                        cudaStream_t stream) {
     OVB_REQUIRE(logits && out_ids && rows > 0 && vocab > 0 && temperature > 0.f, "ovb_sample: bad arguments (temperature must be > 0)");
     if constexpr (sizeof(E) == 2) {
-        // A cluster holds up to 8 x 512 x 32 entries. It takes 27 us with up to 16 rows and 0.95 us for each more, a CTA per row 12 us and 0.57 us per 1000
-        // entries, whatever the rows (128256 entries: 24 rows 42 / 85, 64 rows 83 / 85; 32000: 8 rows 28 / 38, 64 rows 80 / 38). Without top-k the kept set
-        // is large, its steps are all between the CTAs, and the token of a flat distribution would depend on the order of its sums.
+        // A cluster holds up to 8 x 512 x 32 entries. It takes 26 us with up to 12 rows, 38 with up to 36 (their 296 CTAs are resident at a time), 71 with 48, 76 with
+        // 64; a CTA per row takes the same for any of these numbers of rows: 33 us with 16384 entries, 39 with 32000, 51 with 65536, 85 with 128256 (top-k 50,
+        // top-p 0.95, logits in L2). At the line: 6 rows of 16384 entries 26 / 33, 11 of 32000 26 / 39, 24 of 65536 37 / 52, 37 of 100352 62 / 76, 47 of 128256
+        // 71 / 86; behind it 24 of 16384 36 / 34, 37 of 65536 59 / 52, 74 of 128256 94 / 87. Without top-k the kept set is large, its steps are all between the
+        // CTAs, and the token of a flat distribution would depend on the order of its sums.
         if (top_k > 0 && top_k < vocab && vocab >= 16384 && (int64_t)rows * 2700 <= vocab && vocab <= kShareCtas * kShareThreads * 32 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
             cudaLaunchConfig_t cfg;
             memset(&cfg, 0, sizeof(cfg));
