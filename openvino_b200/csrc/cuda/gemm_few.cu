@@ -1,6 +1,6 @@
 // Products of up to 64 tokens with quantised weights: out[T, N] = epilogue(X[T, K] * dequant(W[N, K])^T), a decode step's or a short prompt's.
 //
-// What has to bound it: the read of the weights. The kernel of gemm_sm100.cu, which ran all of these sizes before, takes up to three times as long
+// What has to bound it: the read of the weights. The kernel of gemm_sm100.cu, which keeps short sums (few_is_faster), takes up to three times as long
 // as that read: the one warp that issues its MMAs competes with the expanding warps for issue slots, and a launch costs 8 to 10 us beyond its
 // bytes, most of it in the reduction over the splits of K.
 //  * One CTA per SM, persistent: warp 0 streams the weights into a ring (requested before the kernel that writes the tokens is done), warp 1 the
@@ -8,8 +8,8 @@
 //    warps (one per quarter of the tensor memory's lanes) expand, each a stage of its own.
 //  * A stage is 256 columns of K: one copy for the weights, one for the tokens. With 128 columns the copying lanes, between busy warps, were what
 //    the kernel waited for (128256 x 4096 u4, 16 tokens: 82 us, now 69; u8 107, now 90: 5.9 TB/s).
-//  * Two issuing warps, each with an accumulator of its own: an MMA of 128 x 16 x 16 takes the issuing warp 37 cycles alone and up to 116 between
-//    warps that expand, the tensor pipe 19.
+//  * Two issuing warps, each with an accumulator of its own: between warps that expand, one of them was what the kernel waited for (128256 x 4096 u8,
+//    24 tokens now: 5.8 TB/s, issue slots 58 % busy, tensor pipe 19 %).
 //  * The S CTAs of a cluster share the columns of K. Partial sums are pushed: every CTA owns a share of the tile's outputs, the others store their
 //    sums straight into its shared memory (st.async, counted on an mbarrier), it adds them in the order of the ranks (the same bits on every run)
 //    and writes the outputs. One way through the cluster instead of a barrier, a read and a barrier.
@@ -200,7 +200,7 @@ gemm_few_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     } else if (warp >= 8 - kFewIssuers && warp < 8) {
         // ------------------------------------------------------------ MMA issuers (warp-uniform, see gemm_sm100.cu)
         // Two warps, one for the first 128 columns of every stage and one for the others, each with an accumulator of its own: the waits,
-        // eight MMAs and commits take a warp 600 to 900 cycles between the expanding warps, longer than the read of their weights.
+        // eight MMAs and commits of a stage take one warp, between the expanding ones, longer than the read of its weights.
         const uint32_t idesc = umma_idesc_f16(TILE_N, NT, true);
         const int me = warp - (8 - kFewIssuers);
         const uint64_t desc0 = umma_desc_k_sw128(smem_u32(xbuf) + me * (xbytes >> 1), 1024);
@@ -515,19 +515,19 @@ static bool few_plan(int wmode, int T, int N, int K, int forced, FewPlan* best) 
 
 // Where it is the faster one, against gemm_sm100.cu: the smallest K, by token columns (16, 32, 48, 64) and tiles of 128 rows (up to 8, 16, 32, 64, 148, 296,
 // more). A tile costs the exchange of its sums and its epilogue, which grow with the tokens and which short sums do not hide, and 149 to 296 tiles
-// are one wave of the other kernel's two CTAs per SM and two rounds here. us here / there, launches one after the other with cold weights: u4, 16
-// tokens 128256 x 4096 65.5 / 89, 4096 x 14336 14.9 / 18.2, 28672 x 1024 11.5 / 10.8; 37 tokens 28672 x 4096 26.6 / 28.2, 4096 x 4096 11.0 / 10.2, 20480 x
-// 1024 14.6 / 11.5; u8, 24 tokens 6144 x 4096 11.8 / 14.6, 1024 x 1024 7.4 / 5.4; 48 tokens 24576 x 2048 20.0 / 19.2; 64 tokens 8192 x 28672 58 / 74, 1024 x
-// 1024 10.8 / 6.9, 28672 x 4096 40.5 / 36.6. With 64 token columns the MMAs bind a stage, so that half the bytes gain u4 weights nothing.
+// are one wave of the other kernel's two CTAs per SM and two rounds here. Measured with cold weights behind a norm, which is included, and back to back; a
+// product stays here where either way it is not the slower one, since behind a longer kernel that leaves SMs idle (a short prompt's attention) its weights are
+// fetched meanwhile (37 tokens, 4096 x 4096 u4 after the attention: 5 us less than the other kernel; behind a norm 0.96 of it, back to back 1.05).
+// us here / there, back to back: u4, 16 tokens 128256 x 4096 65.5 / 89, 4096 x 14336 14.9 / 18.2, 28672 x 1024 11.5 / 10.8; 37 tokens 28672 x 4096 26.6 /
+// 28.2, 20480 x 1024 14.6 / 11.5; u8, 24 tokens 6144 x 4096 11.8 / 14.6, 1024 x 1024 7.4 / 5.4; 48 tokens 24576 x 2048 20.0 / 19.2; 64 tokens 8192 x 28672
+// 58 / 74, 1024 x 1024 10.8 / 6.9, 28672 x 4096 40.5 / 36.6. With 64 token columns the MMAs bind a stage, so that half the bytes gain u4 weights little.
 static bool few_is_faster(int wmode, int T, int tiles, int K) {
     constexpr int never = 1 << 30;
-    static constexpr int u4[4][7] = {{256, 256, 256, 256, 1024, 1536, 256}, {2048, 2048, 6144, 3072, 3072, 3072, 1536}, {6144, 2048, 6144, 2048, 3072, 4096, 3072},
+    static constexpr int u4[4][7] = {{256, 256, 256, 256, 1024, 1536, 256}, {2048, 2048, 3072, 2048, 2048, 3072, 1536}, {6144, 2048, 3072, 2048, 3072, 4096, 3072},
                                      {never, never, never, never, never, never, never}};
-    static constexpr int bytes[4][7] = {{256, 256, 256, 256, 1024, 1024, 256}, {2048, 2048, 4096, 1024, 2048, 2048, 1024}, {6144, 2048, 3072, 1024, 2048, 4096, 1536},
-                                        {6144, 2048, 4096, 2048, 3072, 8192, 3072}};
+    static constexpr int bytes[4][7] = {{256, 256, 256, 256, 512, 1024, 256}, {2048, 2048, 3072, 1536, 2048, 2048, 1024}, {6144, 2048, 2048, 1024, 1536, 4096, 1536},
+                                        {8192, 2048, 4096, 2048, 3072, 8192, 3072}};
     const int col = tiles <= 8 ? 0 : tiles <= 16 ? 1 : tiles <= 32 ? 2 : tiles <= 64 ? 3 : tiles <= 148 ? 4 : tiles <= 296 ? 5 : 6, row = (T - 1) / 16;
-    // the other kernel shares such a K better: u4, 16 tokens 4096 x 2048 7.2 / 6.1, 8192 x 1024 7.7 / 6.9
-    if (wmode == OVB_W_U4 && row == 0 && ((col == 2 && K > 1024 && K < 4096) || (col == 3 && K >= 1024 && K < 2048))) return false;
     // a few tiles more than clusters of two: one CTA per tile leaves half of the SMs idle (10240 x 6144 u8, 64 tokens 27.6 / 23.6, 10240 x 8192, 37 tokens 28.3 / 27.3)
     if (wmode != OVB_W_U4 && tiles > 74 && tiles <= 90 && K >= 6144 && K <= 8192) return false;
     return K >= (wmode == OVB_W_U4 ? u4 : bytes)[row][col];

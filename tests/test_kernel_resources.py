@@ -105,8 +105,8 @@ SINGLE, PAIR, STREAM, RING, FEW = range(5)
     *[(f, N, K, s, T, FEW) for f, T in (("u4", 5), ("u8", 33), ("f8", 64))
       for N, K, splits in ((128, 256, (1,)), (256, 1280, (2, 3, 5)), (512, 2048, (4, 6, 7, 8)), (128 * 150, 256, (1,)), (128 * 76, 512, (2,)), (128 * 19, 2048, (8,))) for s in splits],
     # both sides of the rule, at sizes that were measured on both kernels
-    ("u4", 128256, 4096, 0, 16, FEW), ("u4", 4096, 14336, 0, 16, FEW), ("u4", 28672, 1024, 0, 16, SINGLE), ("u4", 4096, 2048, 0, 16, SINGLE), ("u4", 8192, 1024, 0, 8, SINGLE), ("u4", 8192, 2048, 0, 8, FEW), ("u4", 4096, 1024, 0, 16, FEW),
-    ("u4", 28672, 4096, 0, 37, FEW), ("u4", 4096, 4096, 0, 37, SINGLE), ("u4", 20480, 1024, 0, 37, SINGLE), ("u4", 128256, 4096, 0, 64, SINGLE),
+    ("u4", 128256, 4096, 0, 16, FEW), ("u4", 4096, 14336, 0, 16, FEW), ("u4", 28672, 1024, 0, 16, SINGLE), ("u4", 4096, 1024, 0, 16, FEW), ("u4", 4096, 2048, 0, 37, SINGLE),
+    ("u4", 28672, 4096, 0, 37, FEW), ("u4", 4096, 4096, 0, 37, FEW), ("u4", 20480, 1024, 0, 37, SINGLE), ("u4", 128256, 4096, 0, 64, SINGLE),
     ("u8", 6144, 4096, 0, 24, FEW), ("u8", 1024, 1024, 0, 24, SINGLE), ("u8", 24576, 2048, 0, 48, SINGLE), ("f8", 8192, 28672, 0, 64, FEW), ("f8", 1024, 1024, 0, 64, SINGLE),
     ("u8", 28672, 4096, 0, 64, SINGLE), ("u8", 128256, 4096, 0, 64, FEW), ("f8", 10240, 8192, 0, 37, SINGLE), ("f8", 10240, 14336, 0, 37, FEW),
     ("u4", 512, 2048, 0, 65, SINGLE), ("u4", 512, 2048 + 128, 0, 16, SINGLE), ("u4", 512 + 32, 2048, 0, 16, SINGLE),
